@@ -472,10 +472,16 @@ def work(case):
 
 
 def tolerance(case):
-    kind = case["kind"]
-    return {"step": {"rel": 5e-3, "max": 0.5}, "dry": {"rel": 1e-3, "max": 0.1}, "acoustic": {"rel": 1e-3, "max": 0.5},
-            "scalar": {"rel": 1e-4, "max": 0.05}, "momentum": {"rel": 1e-4, "max": 0.05},
-            "tke": {"rel": 1e-5, "max": 1e-3}, "gradient": {"rel": 1e-4, "max": 0.05}}[kind]
+    """About four times what a correct implementation in binary32 differs by:
+    the operators measured against `exact`, the whole steps between two runs
+    whose starting words differ in their last bit.  The radiation histories
+    (a ratio of two small differences of winds, averaged) set the acoustic
+    stage's bound; a limiter's branch taken the other way in a cell sets the
+    gradient's."""
+    return {"step": {"rel": 1e-4, "max": 5e-3}, "dry": {"rel": 2e-5, "max": 1e-4},
+            "acoustic": {"rel": 2e-2, "max": 0.5}, "scalar": {"rel": 4e-4, "max": 1e-2},
+            "momentum": {"rel": 5e-5, "max": 5e-3}, "tke": {"rel": 2e-7, "max": 1e-4},
+            "gradient": {"rel": 2e-2, "max": 0.9}}[case["kind"]]
 
 
 # ------------------------------------------------- the same in 64 bits (torch)
