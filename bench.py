@@ -98,10 +98,13 @@ KERNEL_WORDS_PER_CELL = {
     # moist step: terrain/open acoustic stage
     # in: u v w pp3d qk pk1 pk2 mm ppten ppterm piadv rr0 rrf0 wten rru rrv rrw; out: w pp3d ppd rru rrv rrw
     "tos_column_kernel": 23,
-    # in: ppd thv uten vten gxu gyv u v; out: u v
-    "tos_pgrad_kernel": 10,
-    # flat column: in ppd thv uten vten u v; out u v
-    "tos_flat_pgrad_kernel": 8,
+    # in: u v piadv ppterm ppten qk pk1 pk2 mm wten; in+out: w pp3d rrw; out: ppd (the uniform column reads rr0
+    # and rrf0 besides)
+    "tos_column_march_kernel": 17,
+    # in: ppd thv uten vten gxu gyv; in+out: u v rru rrv
+    "tos_pgrad_kernel": 14,
+    # flat column: in ppd thv uten vten; in+out: u v rru rrv
+    "tos_flat_pgrad_kernel": 12,
     # in: ppx ppi ua va wa ppterm piadv c1 c2 rf0 rr0 thv; out: ppd pp3d rru rrv rrw u v w qk pk1 pk2 mm
     "tos_prepare_kernel": 24,
     # in: scalar rru rrv rrw divx rr0 c1 c2; out: tendency

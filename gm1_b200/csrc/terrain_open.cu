@@ -39,6 +39,7 @@ namespace {
 constexpr int kTosWarps = 8;     // k-parallel warps of the column pass
 constexpr int kTosMaxNk = 160;   // column pass keeps 10 words per level per column in shared memory
 constexpr int kTosArrays = 7;
+constexpr int kFlatLevels = 2;   // the same of the flat pressure gradient, which has no vertical coupling
 constexpr int kPgLevels = 4;     // levels whose loads the pressure-gradient march issues together
 constexpr int kA2Levels = 2;     // levels per warp whose column-pass loads are issued together (phase A2)
 constexpr int kColLevels = 2;    // the same for phases A3 and C
@@ -49,6 +50,7 @@ struct TosArgs {
     gm1b_terrain_metrics m;
     int ni, nj, nk, nrk, n, nloop;
     unsigned abl, diag;
+    int acc;  // this small step's pressure gradient sums rru and rrv (the march pass follows)
     float dts, rdx, rdy, dz, alph, beta, asq, kdiv, temx, temy, tavg, zt, rzt, halfcp;
     float cgs[3], cgt[3];
     // the stretched terrain column (vmode 1): CM1-indexed sigma (nk+2),
@@ -326,8 +328,17 @@ __global__ void __launch_bounds__(256) tos_flat_edge_kernel(TosArgs p) {
 // flat column pressure gradient (sound.F:318-342): every face i = 1..ni+1,
 // j = 1..nj+1 takes u + (dts*dtu0)*(uten - pgrad), dtu0 = 1 on the faces
 // param.F:9182-9219 admits (a periodic side's boundary face included), 0
-// elsewhere; one thread per (j, i), marching k
+// elsewhere; one thread per (j, i) and kFlatLevels levels.  With the running
+// sums it moves 12 words a cell: 640x768x80 0.322 ms, 5.9 TB/s (marching the
+// column level by level without them, 8 words: 0.351 ms)
 // ---------------------------------------------------------------------------
+// this small step's word of the running rru / rrv average: the sum so far (0
+// before the first step), the step's velocity, the mean after the last
+__device__ __forceinline__ float running(const TosArgs &p, float sum, float vel) {
+    const float s = sum + vel;
+    return p.n == p.nloop ? s * p.tavg : s;
+}
+
 __global__ void __launch_bounds__(128) tos_flat_pgrad_kernel(TosArgs p) {
     const Ix X{p.ni, p.nj};
     const int ni = p.ni, nj = p.nj, nk = p.nk;
@@ -341,17 +352,40 @@ __global__ void __launch_bounds__(128) tos_flat_pgrad_kernel(TosArgs p) {
     const float wv = (i <= ni && (j > 1 || ps) && (j < nj + 1 || pn)) ? 1.0f : 0.0f;
     const float tem1 = (p.rdx * 1005.7f) * 0.5f, tem2 = (p.rdy * 1005.7f) * 0.5f;
     const float du = p.dts * wu, dv = p.dts * wv;
-    for (int k = 1; k <= nk; ++k) {
-        const unsigned c = X.p(k, j, i);
-        const float pc = __ldg(a.ppd + c), tc = __ldg(a.thv + c);
-        float pu = tem1 * (pc - __ldg(a.ppd + X.p(k, j, i - 1)));
-        pu = pu * (tc + __ldg(a.thv + X.p(k, j, i - 1)));
-        const unsigned xu = X.u(k, j + 2, i + 2);
-        a.u3d[xu] = a.u3d[xu] + du * (__ldg(a.uten + xu) - pu);
-        float pv = tem2 * (pc - __ldg(a.ppd + X.p(k, j - 1, i)));
-        pv = pv * (tc + __ldg(a.thv + X.p(k, j - 1, i)));
-        const unsigned xv = X.v(k, j + 2, i + 2);
-        a.v3d[xv] = a.v3d[xv] + dv * (__ldg(a.vten + xv) - pv);
+    const bool sums = p.acc && p.n > 1;
+    const unsigned row = (unsigned)(ni + 2);
+    // kFlatLevels levels per thread, every load issued before the first store
+    const int k0 = 1 + blockIdx.z * kFlatLevels;
+    float pc[kFlatLevels], pi[kFlatLevels], pj[kFlatLevels], tc[kFlatLevels], ti[kFlatLevels], tj[kFlatLevels];
+    float ut[kFlatLevels], uu[kFlatLevels], vt[kFlatLevels], vv[kFlatLevels], ru[kFlatLevels], rv[kFlatLevels];
+#pragma unroll
+    for (int q = 0; q < kFlatLevels; ++q) {
+        const int k = min(k0 + q, nk);
+        const unsigned c = X.p(k, j, i), xu = X.u(k, j + 2, i + 2), xv = X.v(k, j + 2, i + 2);
+        pc[q] = __ldg(a.ppd + c), pi[q] = __ldg(a.ppd + c - 1), pj[q] = __ldg(a.ppd + c - row);
+        tc[q] = __ldg(a.thv + c), ti[q] = __ldg(a.thv + c - 1), tj[q] = __ldg(a.thv + c - row);
+        ut[q] = __ldg(a.uten + xu), uu[q] = a.u3d[xu];
+        vt[q] = __ldg(a.vten + xv), vv[q] = a.v3d[xv];
+        ru[q] = sums ? a.rru[xu] : 0.0f;
+        rv[q] = sums ? a.rrv[xv] : 0.0f;
+    }
+#pragma unroll
+    for (int q = 0; q < kFlatLevels; ++q) {
+        const int k = k0 + q;
+        if (k > nk) break;
+        const unsigned xu = X.u(k, j + 2, i + 2), xv = X.v(k, j + 2, i + 2);
+        float pu = tem1 * (pc[q] - pi[q]);
+        pu = pu * (tc[q] + ti[q]);
+        const float un = uu[q] + du * (ut[q] - pu);
+        a.u3d[xu] = un;
+        float pv = tem2 * (pc[q] - pj[q]);
+        pv = pv * (tc[q] + tj[q]);
+        const float vn = vv[q] + dv * (vt[q] - pv);
+        a.v3d[xv] = vn;
+        if (p.acc) {
+            a.rru[xu] = running(p, ru[q], un);
+            a.rrv[xv] = running(p, rv[q], vn);
+        }
     }
 }
 
@@ -374,7 +408,9 @@ __global__ void __launch_bounds__(128) tos_pgrad_kernel(TosArgs p) {
     const bool du = j >= 1 && j <= nj && i >= 2 && i <= ni;
     const bool dv = j >= 2 && j <= nj && i >= 1 && i <= ni;
     const bool dh = p.diag && p.n == p.nloop && !(p.abl & GM1B_TOS_PRESSURE_ADVECTION);
-    if (!du && !dv && !dh) return;
+    const bool acc = p.acc && j >= 1 && i >= 1;  // rru and rrv take every face, the boundary ones as they are
+    if (!du && !dv && !dh && !acc) return;
+    const bool sums = acc && p.n > 1;
     const int iw = du ? i - 1 : i, js = dv ? j - 1 : j;   // neighbour points (own point when unused)
     float pc = __ldg(a.ppd + X.p(1, j, i)), pw = __ldg(a.ppd + X.p(1, j, iw)), ps = __ldg(a.ppd + X.p(1, js, i));
     float vc = 0.0f, vw = 0.0f, vs = 0.0f;  // vertical difference at level k (zero at k = 1)
@@ -387,11 +423,12 @@ __global__ void __launch_bounds__(128) tos_pgrad_kernel(TosArgs p) {
     for (int k0 = 1; k0 <= nk; k0 += kPgLevels) {
         float lp[kPgLevels], lw[kPgLevels], ls[kPgLevels], lth[kPgLevels], lthw[kPgLevels], lths[kPgLevels];
         float lgx[kPgLevels], lgy[kPgLevels], lut[kPgLevels], luu[kPgLevels], lvt[kPgLevels], lvv[kPgLevels];
+        float lru[kPgLevels], lrv[kPgLevels];
 #pragma unroll
         for (int q = 0; q < kPgLevels; ++q) {
             const int k = k0 + q;
             lp[q] = lw[q] = ls[q] = lth[q] = lthw[q] = lths[q] = 0.0f;
-            lgx[q] = lgy[q] = lut[q] = luu[q] = lvt[q] = lvv[q] = 0.0f;
+            lgx[q] = lgy[q] = lut[q] = luu[q] = lvt[q] = lvv[q] = lru[q] = lrv[q] = 0.0f;
             if (k > nk) continue;
             if (k < nk) {
                 lp[q] = __ldg(a.ppd + X.p(k + 1, j, i));
@@ -399,19 +436,19 @@ __global__ void __launch_bounds__(128) tos_pgrad_kernel(TosArgs p) {
                 ls[q] = __ldg(a.ppd + X.p(k + 1, js, i));
             }
             lth[q] = __ldg(a.thv + X.p(k, j, i));
+            const unsigned ou = X.u(k, j + 2, i + 2), ov = X.v(k, j + 2, i + 2);
+            if (du || acc) luu[q] = a.u3d[ou];
+            if (dv || acc) lvv[q] = a.v3d[ov];
+            if (sums) lru[q] = a.rru[ou], lrv[q] = a.rrv[ov];
             if (du) {
-                const unsigned o = X.u(k, j + 2, i + 2);
                 lthw[q] = __ldg(a.thv + X.p(k, j, iw));
                 lgx[q] = __ldg(m.gxu + ((unsigned)k * (unsigned)nj + (unsigned)(j - 1)) * (unsigned)(ni + 1) + (unsigned)(i - 1));
-                lut[q] = __ldg(a.uten + o);
-                luu[q] = a.u3d[o];
+                lut[q] = __ldg(a.uten + ou);
             }
             if (dv) {
-                const unsigned o = X.v(k, j + 2, i + 2);
                 lths[q] = __ldg(a.thv + X.p(k, js, i));
                 lgy[q] = __ldg(m.gyv + ((unsigned)k * (unsigned)(nj + 1) + (unsigned)(j - 1)) * (unsigned)ni + (unsigned)(i - 1));
-                lvt[q] = __ldg(a.vten + o);
-                lvv[q] = a.v3d[o];
+                lvt[q] = __ldg(a.vten + ov);
             }
         }
 #pragma unroll
@@ -435,7 +472,8 @@ __global__ void __launch_bounds__(128) tos_pgrad_kernel(TosArgs p) {
                 const float vsum = (vc1 + vw1) + (vc + vw);
                 const float tr = (0.125f * vsum) * (gxu_lo + gxu_hi);
                 const float pg = (p.halfcp * th) * (hz + tr);
-                a.u3d[X.u(k, j + 2, i + 2)] = luu[q] + p.dts * (lut[q] - pg);
+                luu[q] = luu[q] + p.dts * (lut[q] - pg);
+                a.u3d[X.u(k, j + 2, i + 2)] = luu[q];
                 gxu_lo = gxu_hi;
             }
             if (dv) {
@@ -445,8 +483,13 @@ __global__ void __launch_bounds__(128) tos_pgrad_kernel(TosArgs p) {
                 const float vsum = (vc1 + vs1) + (vc + vs);
                 const float tr = (0.125f * vsum) * (gyv_lo + gyv_hi);
                 const float pg = (p.halfcp * th) * (hz + tr);
-                a.v3d[X.v(k, j + 2, i + 2)] = lvv[q] + p.dts * (lvt[q] - pg);
+                lvv[q] = lvv[q] + p.dts * (lvt[q] - pg);
+                a.v3d[X.v(k, j + 2, i + 2)] = lvv[q];
                 gyv_lo = gyv_hi;
+            }
+            if (acc) {
+                a.rru[X.u(k, j + 2, i + 2)] = running(p, lru[q], luu[q]);
+                a.rrv[X.v(k, j + 2, i + 2)] = running(p, lrv[q], lvv[q]);
             }
             pc = pc1, pw = pw1, ps = ps1;
             vc = vc1, vw = vw1, vs = vs1;
@@ -925,6 +968,344 @@ __global__ void __launch_bounds__(32 * kTosWarps, 3) tos_column_kernel(TosArgs p
 }
 
 // ---------------------------------------------------------------------------
+// column pass of one small step with every phase on and no diagnostics (the
+// composed steps and the compact stage; tos_column_kernel below keeps the
+// diagnostic words and the ablations).  CTA = 32 consecutive columns of row
+// j, kMarchWarps warps each marching up its own run of consecutive levels.
+// One pass forms fpk and the tridiagonal row of each level: what levels k-1
+// and k share (the transformed velocities, w, pk1 + qk, pk2 - qk, pp3d and
+// pp3d + fpk) stays in registers, so each word is loaded once and each
+// level's terrain terms are formed once; the next level's loads are in
+// flight while a level computes.  Only a run's first level needs the run
+// below (its pp3d + fpk, one shared word after a barrier).  Shared memory
+// holds five words per level and column: pp3d + fpk, aa, bb, cc (then the
+// eliminated cc) and dd (then ed, then w).  rru and rrv are summed by the
+// pressure-gradient pass, which holds u and v.
+// Bound by load latency and the barriers around the sweep (24 warps an SM:
+// the five shared words and 80 registers allow three CTAs).  Measured on one
+// B200, per launch: flat column 640x768x80 1.583 -> 0.898 ms, uniform column
+// 256x256x80 271 -> 169 us against the phase-by-phase pass; 16 warps 1.007 ms,
+// 10 warps 1.048, 4 warps 1.228, two CTAs an SM 1.175, four (64 registers)
+// 1.144.
+// ---------------------------------------------------------------------------
+constexpr int kMarchWarps = 8;
+constexpr int kMarchArrays = 5;
+
+// the transformed face velocities of one level, and (terrain column) their
+// density-weighted twins
+template <int VM> struct Faces {
+    float xw, xe, ys, yn;      // VM 2: the face velocities as they are
+    float rw, re, rs, rn;      // VM 1: times the face's own base density
+    float ws;                  // VM 0/1: (uw + ue)*dzdx + (vs + vn)*dzdy
+};
+
+template <int VM>
+__device__ __forceinline__ Faces<VM> march_faces(const TosArgs &p, const Ix &X, int k, int y, int x, float rgw,
+                                                 float rge, float rgs, float rgn, float dzdx, float dzdy) {
+    const gm1b_terrain_open_arrays &a = p.a;
+    Faces<VM> f{};
+    const unsigned qu = X.u(k, y, x), qv = X.v(k, y, x);
+    const float uw = __ldg(a.u3d + qu), ue = __ldg(a.u3d + qu + 1);
+    const float vs = __ldg(a.v3d + qv), vn = __ldg(a.v3d + qv + (unsigned)(p.ni + 6));
+    if (VM == 2) {
+        f.xw = uw, f.xe = ue, f.ys = vs, f.yn = vn;
+        return f;
+    }
+    f.xw = uw * rgw, f.xe = ue * rge, f.ys = vs * rgs, f.yn = vn * rgn;
+    if (k == 1) f.ws = (uw + ue) * dzdx + (vs + vn) * dzdy;
+    if (VM == 1) {
+        const unsigned q = X.w(k, y, x), row = (unsigned)(p.ni + 6);
+        const float rc = __ldg(p.rho0p + q);
+        f.rw = (0.5f * (__ldg(p.rho0p + q - 1) + rc)) * f.xw;
+        f.re = (0.5f * (rc + __ldg(p.rho0p + q + 1))) * f.xe;
+        f.rs = (0.5f * (__ldg(p.rho0p + q - row) + rc)) * f.ys;
+        f.rn = (0.5f * (rc + __ldg(p.rho0p + q + row))) * f.yn;
+    }
+    return f;
+}
+
+// dum3 and hadvp at w level kf from the faces of levels kf (h) and kf-1 (l)
+template <int VM>
+__device__ __forceinline__ void march_terms(const TosArgs &p, int kf, const Faces<VM> &h, const Faces<VM> &l,
+                                            float dzdx, float dzdy, float gz, float rk, float rl, float rrf0,
+                                            float &d3, float &ha) {
+    const float r2 = col_r2<VM>(p, kf);
+    const float r1 = 1.0f - r2;
+    const float height = (col_sigf<VM>(p, kf) - p.zt) * p.rzt;
+    float uh = h.xw + h.xe, ul = l.xw + l.xe, vh = h.ys + h.yn, vl = l.ys + l.yn;
+    float xt = (r2 * uh + r1 * ul) * dzdx, yt = (r2 * vh + r1 * vl) * dzdy;
+    d3 = ((0.5f * (xt + yt)) * height) * gz;
+    if (VM == 1) {
+        uh = h.rw + h.re, ul = l.rw + l.re;
+        vh = h.rs + h.rn, vl = l.rs + l.rn;
+    } else {
+        uh = rk * h.xw + rk * h.xe, ul = rl * l.xw + rl * l.xe;
+        vh = rk * h.ys + rk * h.yn, vl = rl * l.ys + rl * l.yn;
+    }
+    xt = (r2 * uh + r1 * ul) * dzdx, yt = (r2 * vh + r1 * vl) * dzdy;
+    ha = (((0.5f * (xt + yt)) * height) * gz) * rrf0;
+}
+
+// the words of one level that no other level of the run reads
+struct MarchLoad {
+    float pc, pe, pw, pn, ps, qk, pk1, pk2, ppten, ppterm, pp, mm, wt, w1, rr0, rrf;
+    template <int VM>
+    __device__ __forceinline__ void load(const TosArgs &p, const Ix &X, int k, int j, int i) {
+        const gm1b_terrain_open_arrays &a = p.a;
+        const unsigned c = X.p(k, j, i), row = (unsigned)(p.ni + 2), qw = X.w(k, j + 2, i + 2);
+        pc = __ldg(a.piadv + c);
+        pe = __ldg(a.piadv + c + 1);
+        pw = __ldg(a.piadv + c - 1);
+        pn = __ldg(a.piadv + c + row);
+        ps = __ldg(a.piadv + c - row);
+        qk = __ldg(a.qk + c);
+        pk1 = __ldg(a.pk1 + c);
+        pk2 = __ldg(a.pk2 + c);
+        ppten = __ldg(a.ppten + c);
+        ppterm = __ldg(a.ppterm + c);
+        pp = a.pp3d[c];
+        mm = __ldg(a.mm + c);
+        wt = __ldg(a.wten + qw);
+        w1 = a.w3d[qw + (unsigned)(p.nj + 6) * (unsigned)(p.ni + 6)];
+        rr0 = rrf = 0.0f;
+        if (VM != 2) {
+            rr0 = __ldg(p.m.rr0 + X.m(k - 1, j - 1, i - 1));
+            rrf = k < p.nk ? __ldg(p.m.rrf0 + X.m(k, j - 1, i - 1)) : 0.0f;
+        }
+    }
+};
+
+template <int VM>
+__global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(TosArgs p) {
+    extern __shared__ float sh[];
+    const Ix X{p.ni, p.nj};
+    const int ni = p.ni, nk = p.nk, L = nk + 2;
+    const int lane = threadIdx.x, wy = threadIdx.y;
+    const bool live = blockIdx.x * 32 + lane + 1 <= ni;
+    // lanes past the row's end repeat its last column and store nothing
+    const int i = live ? (int)(blockIdx.x * 32) + lane + 1 : ni;
+    const int j = blockIdx.y + 1, y = j + 2, x = i + 2;
+    const gm1b_terrain_open_arrays &a = p.a;
+    const gm1b_terrain_metrics &m = p.m;
+    const bool last = p.n == p.nloop;
+    float *s_sum = sh + lane, *s_aa = s_sum + L * 32, *s_bb = s_aa + L * 32, *s_cc = s_bb + L * 32,
+          *s_dd = s_cc + L * 32;
+    const int run = (nk + kMarchWarps - 1) / kMarchWarps;
+    const int k_lo = 1 + wy * run, k_hi = min(nk, k_lo + run - 1);
+    const bool busy = k_lo <= nk;
+    float f_base = 0.0f, f_mm = 0.0f, f_sum = 0.0f;  // the run's first row, completed after the barrier
+    if (busy) {
+        float gz = 0.0f, dzdx = 0.0f, dzdy = 0.0f, rgw = 0.0f, rge = 0.0f, rgs = 0.0f, rgn = 0.0f;
+        if (VM != 2) {
+            const int i0 = i - 1, j0 = j - 1;
+            gz = __ldg(m.gz + X.h(j0, i0));
+            dzdx = __ldg(m.dzdx + X.h(j0, i0));
+            dzdy = __ldg(m.dzdy + X.h(j0, i0));
+            rgw = __ldg(m.rgzu + (size_t)j0 * (ni + 1) + i0), rge = __ldg(m.rgzu + (size_t)j0 * (ni + 1) + i0 + 1);
+            rgs = __ldg(m.rgzv + (size_t)j0 * ni + i0), rgn = __ldg(m.rgzv + (size_t)(j0 + 1) * ni + i0);
+        }
+        Faces<VM> fc = march_faces<VM>(p, X, k_lo, y, x, rgw, rge, rgs, rgn, dzdx, dzdy);
+        MarchLoad ld;
+        ld.load<VM>(p, X, k_lo, j, i);
+        float wk = a.w3d[X.w(k_lo, y, x)];
+        float a1m = 0.0f, a2m = 0.0f, ppm = 0.0f, summ = 0.0f, d3k = 0.0f, hak = 0.0f, rk = 0.0f;
+        if (VM == 0) rk = __ldg(m.rho0_3d + X.m(k_lo - 1, 0, 0));
+        if (k_lo >= 2) {
+            const unsigned cm = X.p(k_lo - 1, j, i);
+            const float qm = __ldg(a.qk + cm);
+            a1m = __ldg(a.pk1 + cm) + qm;
+            a2m = __ldg(a.pk2 + cm) - qm;
+            ppm = a.pp3d[cm];
+            if (VM != 2) {
+                const Faces<VM> fl = march_faces<VM>(p, X, k_lo - 1, y, x, rgw, rge, rgs, rgn, dzdx, dzdy);
+                const float rl = VM == 0 ? __ldg(m.rho0_3d + X.m(k_lo - 2, 0, 0)) : 0.0f;
+                march_terms<VM>(p, k_lo, fc, fl, dzdx, dzdy, gz, rk, rl,
+                                __ldg(m.rrf0 + X.m(k_lo - 1, j - 1, i - 1)), d3k, hak);
+            }
+        } else if (VM != 2) {
+            wk = (0.5f * fc.ws) * gz;  // bc.F:1151-1178: the surface w of this small step
+        }
+        if (k_lo == 1) s_dd[32] = wk;
+#pragma unroll 1
+        for (int k = k_lo; k <= k_hi; ++k) {
+            // the next level's words, in flight while this one computes (the
+            // last level loads its own again)
+            const int kn = k < k_hi ? k + 1 : k_hi;
+            MarchLoad nx;
+            nx.load<VM>(p, X, kn, j, i);
+            const int kf = VM == 2 ? kn : (k < nk ? k + 1 : nk);
+            const Faces<VM> fn = march_faces<VM>(p, X, kf, y, x, rgw, rge, rgs, rgn, dzdx, dzdy);
+            const float a1k = ld.pk1 + ld.qk, a2k = ld.pk2 - ld.qk, wk1 = ld.w1;
+            float fpk;
+            if (VM == 2) {
+                // sound.F:491-509 on the flat column (as in tos_column_kernel)
+                float div = (fc.xe - fc.xw) * p.rdx + (fc.yn - fc.ys) * p.rdy;
+                if (fabsf(div) < 1.0e-30f) div = 0.0f;
+                float hx = fc.xw * (ld.pc - ld.pw) + fc.xe * (ld.pe - ld.pc);
+                hx = (-hx) * p.temx;
+                float hy = fc.ys * (ld.pc - ld.ps) + fc.yn * (ld.pn - ld.pc);
+                hy = (-hy) * p.temy;
+                const float vert = wk * a1k + wk1 * a2k;
+                fpk = ((p.dts * (ld.ppten - ld.ppterm * div)) + (hx + hy)) + p.beta * vert;
+            } else {
+                float d3k1 = 0.0f, hak1 = 0.0f, rk1 = 0.0f;
+                if (k < nk) {
+                    if (VM == 0) rk1 = __ldg(m.rho0_3d + X.m(k, 0, 0));
+                    march_terms<VM>(p, k + 1, fn, fc, dzdx, dzdy, gz, rk1, rk, ld.rrf, d3k1, hak1);
+                }
+                const float hzd = (fc.xe - fc.xw) * p.rdx + (fc.yn - fc.ys) * p.rdy;
+                const float vtd = (d3k1 - d3k) * col_rdsf<VM>(p, k);
+                float div = gz * (hzd + vtd);
+                if (fabsf(div) < 1.0e-20f) div = 0.0f;
+                const float w1 = k == 1 ? 0.0f : wk, w2 = k == nk ? 0.0f : wk1;
+                fpk = p.dts * (ld.ppten - ld.ppterm * div) + p.beta * ((-ld.qk) * (w2 - w1));
+                const float rxe = VM ? fc.re : rk * fc.xe, rxw = VM ? fc.rw : rk * fc.xw;
+                const float ryn = VM ? fc.rn : rk * fc.yn, rys = VM ? fc.rs : rk * fc.ys;
+                const float ww2 = hak1 + p.beta * wk1, ww1 = hak + p.beta * wk;
+                const float xa = (p.temx * rxe) * (ld.pe - ld.pc) + (p.temx * rxw) * (ld.pc - ld.pw);
+                const float ya = (p.temy * ryn) * (ld.pn - ld.pc) + (p.temy * rys) * (ld.pc - ld.ps);
+                float hz = (-(xa + ya)) * ld.rr0;
+                hz = hz * gz;
+                fpk = fpk + (hz + (ww1 * ld.pk1 + ww2 * ld.pk2));
+                d3k = d3k1, hak = hak1, rk = rk1;
+            }
+            const float sum = ld.pp + fpk;
+            s_sum[k * 32] = sum;
+            if (k >= 2) {
+                const float mmk = ld.mm;
+                s_aa[k * 32] = k >= 3 ? (-p.asq) * (mmk * a1m) : 0.0f;
+                s_cc[k * 32] = k < nk ? (-p.asq) * ((-mmk) * a2k) : 0.0f;
+                const float dg = (-a1k) + a2m;
+                s_bb[k * 32] = 1.0f - p.asq * (mmk * dg);
+                const float pd = ld.pp - ppm;
+                const float fwk = p.dts * ld.wt + p.beta * ((-mmk) * pd);
+                const float base = wk + fwk;
+                if (k == k_lo)
+                    f_base = base, f_mm = mmk, f_sum = sum;
+                else
+                    s_dd[k * 32] = base + p.alph * ((-mmk) * (sum - summ));
+            }
+            if (k == nk) s_dd[(nk + 1) * 32] = wk1;
+            a1m = a1k, a2m = a2k, ppm = ld.pp, summ = sum, wk = wk1;
+            ld = nx, fc = fn;
+        }
+    }
+    // phase C's words (pp3d of level k is read here before this thread writes
+    // it there): the first levels' in flight over the barriers and the sweep
+    float lrw[kColLevels], cpp[kColLevels], ca1[kColLevels], ca2[kColLevels];
+    auto c_loads = [&](int kb) {
+#pragma unroll
+        for (int q = 0; q < kColLevels; ++q) {
+            const int k = min(kb + q, k_hi);
+            const unsigned c = X.p(k, j, i);
+            lrw[q] = a.rrw[X.w(k, y, x)];
+            cpp[q] = a.pp3d[c];
+            const float qk = __ldg(a.qk + c);
+            ca1[q] = __ldg(a.pk1 + c) + qk;
+            ca2[q] = __ldg(a.pk2 + c) - qk;
+        }
+    };
+    if (busy) c_loads(k_lo);
+    __syncthreads();
+    if (busy && k_lo >= 2) s_dd[k_lo * 32] = f_base + p.alph * ((-f_mm) * (f_sum - s_sum[(k_lo - 1) * 32]));
+    __syncthreads();
+    // Thomas sweep, one lane per column, as in tos_column_kernel
+    if (wy == 0) {
+        float ec = 0.0f, ed = 0.0f, wn = 0.0f;
+        float aa = s_aa[2 * 32], bb = s_bb[2 * 32], cc = s_cc[2 * 32], dd = s_dd[2 * 32];
+        for (int k = 2; k <= nk; ++k) {
+            float naa = 0.0f, nbb = 0.0f, ncc = 0.0f, ndd = 0.0f;
+            if (k < nk) {
+                naa = s_aa[(k + 1) * 32];
+                nbb = s_bb[(k + 1) * 32];
+                ncc = s_cc[(k + 1) * 32];
+                ndd = s_dd[(k + 1) * 32];
+            }
+            const float piv = k == 2 ? bb : aa * ec + bb;
+            const float inv = rcp_rn(piv);
+            if (k < nk) {
+                ec = (-cc) * inv;
+                ed = (k == 2 ? dd : dd - aa * ed) * inv;
+                s_cc[k * 32] = ec;
+                s_dd[k * 32] = ed;
+            } else {
+                wn = (dd - aa * ed) * inv;
+                s_dd[k * 32] = wn;
+            }
+            aa = naa, bb = nbb, cc = ncc, dd = ndd;
+        }
+        for (int kb = nk - 1; kb >= 2; kb -= kThomasChunk) {
+            float ce[kThomasChunk], ee[kThomasChunk];
+#pragma unroll
+            for (int q = 0; q < kThomasChunk; ++q) {
+                const int k = kb - q;
+                ce[q] = k >= 2 ? s_cc[k * 32] : 0.0f;
+                ee[q] = k >= 2 ? s_dd[k * 32] : 0.0f;
+            }
+#pragma unroll
+            for (int q = 0; q < kThomasChunk; ++q) {
+                const int k = kb - q;
+                if (k < 2) break;
+                wn = ce[q] * wn + ee[q];
+                s_dd[k * 32] = wn;
+            }
+        }
+    }
+    __syncthreads();
+    // pressure update, filter, halo copy, rrw average
+    if (!busy || !live) return;
+    const bool fill = !last;
+    const bool east = i == ni, north = j == p.nj;
+    for (int kb = k_lo; kb <= k_hi; kb += kColLevels) {
+        if (kb != k_lo) c_loads(kb);
+#pragma unroll
+        for (int q = 0; q < kColLevels; ++q) {
+            const int k = kb + q;
+            if (k > k_hi) break;
+            const unsigned c = X.p(k, j, i), qw = X.w(k, y, x);
+            const float wk = s_dd[k * 32], wk1 = s_dd[(k + 1) * 32];
+            a.w3d[qw] = wk;
+            const float w1 = (k == 1 && VM != 2) ? 0.0f : wk, w2 = (k == nk && VM != 2) ? 0.0f : wk1;
+            const float old = cpp[q];
+            const float vt = w1 * ca1[q] + w2 * ca2[q];
+            float up = s_sum[k * 32] + p.alph * vt;
+            if (fabsf(up) < (VM == 2 ? 1.0e-30f : 1.0e-20f)) up = 0.0f;
+            const float tend = p.kdiv * (up - old);
+            const float pd = up + tend;
+            a.pp3d[c] = up;
+            a.ppd[c] = pd;
+            if (p.nrk == 3 && last) a.ppx[c] = tend;
+            if (fill && (i == 1 || east || j == 1 || north)) {  // bcp: the halo takes its clamped interior neighbour
+                const int rows[3] = {j, j == 1 ? 0 : -1, north ? p.nj + 1 : -1};
+                const int cols[3] = {i, i == 1 ? 0 : -1, east ? ni + 1 : -1};
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    if (rows[r] < 0) continue;
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) {
+                        if (cols[e] < 0 || (r == 0 && e == 0)) continue;
+                        a.ppd[X.p(k, rows[r], cols[e])] = pd;
+                    }
+                }
+            }
+            const float sw = lrw[q] + (last ? wk * p.alph : wk);
+            a.rrw[qw] = last ? sw * p.tavg : sw;
+            if (east || north) {  // rrw on faces ni+1 and rows nj+1
+#pragma unroll
+                for (int e = 1; e < 4; ++e) {
+                    const int dx = e & 1, dy = e >> 1;
+                    if ((dx && !east) || (dy && !north)) continue;
+                    const unsigned ew = X.w(k, y + dy, x + dx);
+                    const float wv = a.w3d[ew];
+                    const float se = a.rrw[ew] + (last ? wv * p.alph : wv);
+                    a.rrw[ew] = last ? se * p.tavg : se;
+                }
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // radiation histories (radbcew4/radbcns4): one warp per boundary line, the
 // clamped phase speeds of all levels in parallel, their column mean summed
 // in level order by lane 0
@@ -1328,6 +1709,13 @@ int32_t terrain_open_stage(int32_t ni, int32_t nj, int32_t nk, int32_t nrk, floa
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(tos_column_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)((size_t)kTosArrays * (kTosMaxNk + 2) * 32 * sizeof(float)));
+        const int march_most = (int)((size_t)kMarchArrays * (kTosMaxNk + 2) * 32 * sizeof(float));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(tos_column_march_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, march_most);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(tos_column_march_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, march_most);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(tos_column_march_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, march_most);
         if (e != cudaSuccess) {
             gm1b_set_error("cudaFuncSetAttribute(tos_column_kernel): %s", cudaGetErrorString(e));
             return GM1B_ERR_CUDA;
@@ -1341,8 +1729,17 @@ int32_t terrain_open_stage(int32_t ni, int32_t nj, int32_t nk, int32_t nrk, floa
     }
     if (!launch_ok("tos_prepare_kernel")) return GM1B_ERR_CUDA;
     const dim3 pg_grid((ni + 2 + 31) / 32, (nj + 2 + 3) / 4), col_grid((ni + 31) / 32, nj);
+    constexpr uint32_t column_phases = GM1B_TOS_PRESSURE_GRADIENT | GM1B_TOS_TRANSFORMED_DIVERGENCE |
+                                       GM1B_TOS_PRESSURE_ADVECTION | GM1B_TOS_IMPLICIT_SOLVE |
+                                       GM1B_TOS_BETWEEN_STEP_FILL;
+    const dim3 march_grid((ni + 31) / 32, nj), march_block(32, kMarchWarps);
+    const size_t march_smem = (size_t)kMarchArrays * (size_t)(nk + 2) * 32 * sizeof(float);
     for (int n = 1; n <= nloop; ++n) {
         p.n = n;
+        // the march pass runs whole small steps; an ablated step and the step
+        // that leaves the diagnostic words take the general column pass
+        const bool march = (ablations & column_phases) == column_phases && !(p.diag && n == nloop);
+        p.acc = march ? 1 : 0;
         if ((ablations & GM1B_TOS_OPEN_CONSUMPTION) && p.vmode == 2) {
             ProfScope ps("tos_flat_edge_kernel", st);
             tos_flat_edge_kernel<<<grid_for((size_t)nk * (nj + ni), 256), 256, 0, st>>>(p);
@@ -1356,7 +1753,8 @@ int32_t terrain_open_stage(int32_t ni, int32_t nj, int32_t nk, int32_t nrk, floa
         }
         if ((ablations & GM1B_TOS_PRESSURE_GRADIENT) && p.vmode == 2) {
             ProfScope ps("tos_flat_pgrad_kernel", st);
-            tos_flat_pgrad_kernel<<<dim3((ni + 1 + 31) / 32, (nj + 1 + 3) / 4), dim3(32, 4), 0, st>>>(p);
+            tos_flat_pgrad_kernel<<<dim3((ni + 1 + 31) / 32, (nj + 1 + 3) / 4, (nk + kFlatLevels - 1) / kFlatLevels),
+                                    dim3(32, 4), 0, st>>>(p);
             ps.stop();
             if (!launch_ok("tos_flat_pgrad_kernel")) return GM1B_ERR_CUDA;
         } else if (ablations & GM1B_TOS_PRESSURE_GRADIENT) {
@@ -1365,7 +1763,17 @@ int32_t terrain_open_stage(int32_t ni, int32_t nj, int32_t nk, int32_t nrk, floa
             ps.stop();
             if (!launch_ok("tos_pgrad_kernel")) return GM1B_ERR_CUDA;
         }
-        {
+        if (march) {
+            ProfScope ps("tos_column_march_kernel", st);
+            if (p.vmode == 2)
+                tos_column_march_kernel<2><<<march_grid, march_block, march_smem, st>>>(p);
+            else if (p.vmode == 1)
+                tos_column_march_kernel<1><<<march_grid, march_block, march_smem, st>>>(p);
+            else
+                tos_column_march_kernel<0><<<march_grid, march_block, march_smem, st>>>(p);
+            ps.stop();
+            if (!launch_ok("tos_column_march_kernel")) return GM1B_ERR_CUDA;
+        } else {
             ProfScope ps("tos_column_kernel", st);
             if (p.vmode == 2)
                 tos_column_kernel<2><<<col_grid, dim3(32, kTosWarps), col_smem, st>>>(p);

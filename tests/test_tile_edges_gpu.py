@@ -1,0 +1,70 @@
+"""The marching kernels at the sizes where their tiles can go wrong: the
+edges of the 31- and 32-wide tiles and of the 4-, 7- and 8-row blocks, runs
+of levels that do not divide the column, the shortest columns.  Against the
+oracle, every float32 word identical."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(d):
+    return {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in d.items()}
+
+
+def _differ(got, want, names):
+    torch.cuda.synchronize()
+    return [n for n in names if not np.array_equal(got[n].cpu().numpy().view(np.uint32), want[n].view(np.uint32))]
+
+
+def _t(x):
+    return torch.from_numpy(np.array(x, dtype=np.float32)).cuda()
+
+
+def _profiles(nk):
+    rng = np.random.default_rng(nk)
+    return dict(mh=rng.uniform(0.3, 3.0, nk + 2).astype(np.float32), mf=rng.uniform(0.3, 3.0, nk + 3).astype(np.float32),
+                rdz=float(np.float32(1.0) / np.float32(100.0)))
+
+
+@pytest.mark.parametrize("column", ["uniform", "terrain", "flat"])
+@pytest.mark.parametrize("ni,nj,nk", [(31, 4, 4), (32, 3, 7), (33, 5, 8), (64, 3, 9), (65, 4, 17), (3, 3, 160)])
+def test_compact_acoustic_stage(column, ni, nj, nk):
+    """The column pass that marches runs of levels, without diagnostics."""
+    from gm1_b200 import terrain_open as tos
+    from gm1_b200.momentum import StretchedMomentumColumn
+    from gm1_b200.vertical import uniform_vertical_levels
+    from oracle import terrain_open as orc
+    from tests.golden.make_golden import terrain_open_fixture
+    from tests.test_oracle_momentum import _padded_rho0
+
+    a, m = terrain_open_fixture(ni, nj, nk, 40 + ni + nk)
+    ref = {k: v.copy() for k, v in a.items()}
+    dev, mdev = _dev(a), _dev(m)
+    kw = dict(ni=ni, nj=nj, nk=nk, dt=2.0, nsound=6, dx=450.0, dy=520.0)
+    compiled = tos.compile_cuda_psolver3_terrain_open(retain_column_diagnostics=False)
+    for n in tos.COLUMN_DIAGNOSTIC_NAMES:
+        dev[n] = torch.zeros(1, device="cuda")
+    rho0p = _padded_rho0(m["rho0_3d"], ni, nj, nk)
+    mdev["rho0_padded"] = _t(rho0p)
+    if column == "flat":
+        p = _profiles(nk)
+        vertical = StretchedMomentumColumn(True, None, mh=_t(p["mh"]), mf=_t(p["mf"]), rdz=p["rdz"])
+    elif column == "terrain":
+        lv = uniform_vertical_levels(nk, 210.0)
+        p = {"sigma": lv.sigma, "sigmaf": lv.sigmaf, "rds": lv.rds, "rdsf": lv.rdsf, "ztop": lv.ztop_m, "rho0p": rho0p}
+        vertical = StretchedMomentumColumn(False, None, **{n: _t(p[n]) for n in ("sigma", "sigmaf", "rds", "rdsf")},
+                                           ztop=lv.ztop_m)
+    for nrk in (1, 2, 3):
+        if column == "uniform":
+            orc.terrain_open_stage(ref, m, nrk=nrk, dz=210.0, **kw)
+            tos.launch_cuda_psolver3_terrain_open_stage(dev, mdev, nrk=nrk, dz=210.0, compiled=compiled, **kw)
+        else:
+            (orc.terrain_open_stage_flat if column == "flat" else orc.terrain_open_stage_column)(ref, m, p, nrk=nrk, **kw)
+            tos.launch_cuda_gm1_child_psolver3_open_stage(dev, mdev, nrk=nrk, vertical=vertical, compiled=compiled, **kw)
+        names = [n for n in tos.COMPARE_OUTPUT_NAMES if not n.startswith("tri_")] + ["scalar"]
+        assert _differ(dev, ref, names) == [], nrk
