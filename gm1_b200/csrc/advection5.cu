@@ -7,14 +7,14 @@
 //   lateral-side tendency of the reference kernel
 //   cm1_adv5_scalar_tendency_v1      src/cm1core/cuda_advection5.py:669
 //
-// Design (B200): the scalar advection is ONE fused pass.  A CTA owns a 32x4
-// column tile and marches up a chunk of levels: at each level the x and y
-// face fluxes of the tile (33 x 4 and 32 x 5 faces) are formed once into
-// shared memory, the vertical flux of the upper face is formed in a register
-// and carried to the next level as the lower face, and the tendency is
-// written.  The face-flux scratch arrays of the reference (three passes
-// through HBM) are optional outputs here.  WENO smoothness weights are
-// binary64 as in the reference.
+// Design (B200): the scalar advection is ONE fused pass in which a warp owns
+// a row of 32 x faces and marches up a chunk of levels: the lanes exchange
+// their x face fluxes by shuffle (31 cells per 32 lanes), the upper vertical
+// flux is carried to the next level as the lower one.  The face-flux scratch
+// arrays of the reference (three passes through HBM) are optional outputs
+// here.  WENO smoothness weights are binary64 as in the reference.
+#include <algorithm>
+
 #include "gm1b_common.cuh"
 #include "weno.cuh"
 
@@ -128,94 +128,15 @@ __global__ void __launch_bounds__(kAX *kAY)
     }
 }
 
-// ---------------------------------------------------------------------------
-// fused scalar advection: grid (ceil(ni/32), ceil(nj/4), chunks of levels)
-// ---------------------------------------------------------------------------
+// the upwind reconstruction at a face from the six points around it (both
+// upwind stencils): one reconstruction of selected points, so that a warp
+// whose lanes differ in the sign of m does not form both
 template <bool WENO>
-__device__ __forceinline__ float vertical_flux(const float *__restrict__ s, const PaddedDims &d,
-                                               const gm1b_scalar_advection5_arrays &a, int k, int j, int i, int y,
-                                               int x, double eps, float wepsf) {
-    const int nk = d.nk;
-    if (k <= 1 || k >= nk + 1) return 0.0f;
-    const float m = a.rrw[d.s(k, y, x)];
-#define SK(kk) __ldg(s + d.s((kk), y, x))
-    float r;
-    if (k == 2) {
-        if (m >= 0.0f)
-            r = a.c1[d.c(k - 1, j, i)] * SK(k - 1) + a.c2[d.c(k - 1, j, i)] * SK(k);
-        else if (WENO)
-            r = upstrpd(SK(k + 1), SK(k), SK(k - 1), wepsf);
-        else
-            r = flx3(SK(k + 1), SK(k), SK(k - 1));
-    } else if (k == nk) {
-        const bool up = WENO ? (m > 0.0f) : (m >= 0.0f);
-        if (up)
-            r = WENO ? upstrpd(SK(k - 2), SK(k - 1), SK(k), wepsf) : flx3(SK(k - 2), SK(k - 1), SK(k));
-        else
-            r = a.c1[d.c(k - 1, j, i)] * SK(k - 1) + a.c2[d.c(k - 1, j, i)] * SK(k);
-    } else if (k == 3) {
-        if (m >= 0.0f)
-            r = WENO ? upstrpd(SK(k - 2), SK(k - 1), SK(k), wepsf) : flx3(SK(k - 2), SK(k - 1), SK(k));
-        else
-            r = recon<WENO>(SK(k + 2), SK(k + 1), SK(k), SK(k - 1), SK(k - 2), eps);
-    } else if (k == nk - 1) {
-        if (m >= 0.0f)
-            r = recon<WENO>(SK(k - 3), SK(k - 2), SK(k - 1), SK(k), SK(k + 1), eps);
-        else if (WENO)
-            r = upstrpd(SK(k + 1), SK(k), SK(k - 1), wepsf);
-        else
-            r = flx3(SK(k + 1), SK(k), SK(k - 1));
-    } else if (m >= 0.0f) {
-        r = recon<WENO>(SK(k - 3), SK(k - 2), SK(k - 1), SK(k), SK(k + 1), eps);
-    } else {
-        r = recon<WENO>(SK(k + 2), SK(k + 1), SK(k), SK(k - 1), SK(k - 2), eps);
-    }
-#undef SK
-    return m * r;
+__device__ __forceinline__ float upwind(float m, float s0, float s1, float s2, float s3, float s4, float s5,
+                                        double eps) {
+    const bool pos = m >= 0.0f;
+    return m * recon<WENO>(pos ? s0 : s5, pos ? s1 : s4, pos ? s2 : s3, pos ? s3 : s2, pos ? s4 : s1, eps);
 }
-
-template <bool WENO>
-__device__ __forceinline__ float x_face_flux(const float *__restrict__ s, const PaddedDims &d, const float *rru,
-                                             int k, int y, int x, double eps) {
-    const float m = __ldg(rru + d.u(k, y, x));
-    const float *row = s + d.s(k, y, 0);
-    float r;
-    if (m >= 0.0f)
-        r = recon<WENO>(__ldg(row + x - 3), __ldg(row + x - 2), __ldg(row + x - 1), __ldg(row + x), __ldg(row + x + 1),
-                        eps);
-    else
-        r = recon<WENO>(__ldg(row + x + 2), __ldg(row + x + 1), __ldg(row + x), __ldg(row + x - 1), __ldg(row + x - 2),
-                        eps);
-    return m * r;
-}
-
-template <bool WENO>
-__device__ __forceinline__ float y_face_flux(const float *__restrict__ s, const PaddedDims &d, const float *rrv,
-                                             int k, int y, int x, double eps) {
-    const float m = __ldg(rrv + d.v(k, y, x));
-    const size_t sy = (size_t)(d.ni + 2 * NG);
-    const float *col = s + d.s(k, 0, x);
-    float r;
-    if (m >= 0.0f)
-        r = recon<WENO>(__ldg(col + (y - 3) * sy), __ldg(col + (y - 2) * sy), __ldg(col + (y - 1) * sy),
-                        __ldg(col + y * sy), __ldg(col + (y + 1) * sy), eps);
-    else
-        r = recon<WENO>(__ldg(col + (y + 2) * sy), __ldg(col + (y + 1) * sy), __ldg(col + y * sy),
-                        __ldg(col + (y - 1) * sy), __ldg(col + (y - 2) * sy), eps);
-    return m * r;
-}
-
-// ---------------------------------------------------------------------------
-// tiled fused scalar advection: grid (ceil(ni/32), ceil(nj/8), level chunks)
-//
-// Per level the CTA stages the scalar plane of its 32x8 tile plus a 3-cell
-// halo (38 x 14 words) in shared memory and forms every x and y face flux of
-// the tile once from it; each thread keeps the six levels k-2..k+3 of its own
-// column in registers for the vertical flux of face k+1, whose value is
-// carried to the next level as the lower face.  Offsets are 32-bit.
-// ---------------------------------------------------------------------------
-constexpr int kTX5 = 32, kTY5 = 8;
-constexpr int kPX = kTX5 + 6, kPY = kTY5 + 6;
 
 template <bool WENO>
 __device__ __forceinline__ float z_face(const float win[6], float m, float c1, float c2, int face, int nk,
@@ -248,10 +169,8 @@ __device__ __forceinline__ float z_face(const float win[6], float m, float c1, f
             r = upstrpd(L(face + 1), L(face), L(face - 1), wepsf);
         else
             r = flx3(L(face + 1), L(face), L(face - 1));
-    } else if (m >= 0.0f) {
-        r = recon<WENO>(L(face - 3), L(face - 2), L(face - 1), L(face), L(face + 1), eps);
     } else {
-        r = recon<WENO>(L(face + 2), L(face + 1), L(face), L(face - 1), L(face - 2), eps);
+        return upwind<WENO>(m, L(face - 3), L(face - 2), L(face - 1), L(face), L(face + 1), L(face + 2), eps);
     }
 #undef L
     return m * r;
@@ -268,146 +187,151 @@ struct VertCol {
     float rdz;
 };
 
+constexpr int kFaceOut = 31;    // cells a warp of 32 x faces completes
+constexpr int kFifthRows = 8;   // rows (warps) per CTA of the fifth-order pass, each independent
+constexpr int kWenoRows = 8;    // rows per CTA of the WENO pass: 8 rows of y faces complete 7 rows of cells
+
+// levels per chunk when the caller leaves it open: long chunks re-read and
+// re-form less (each chunk starts with six window loads and its lower face
+// flux), short ones give a small plane warps enough for 148 SMs
+inline int default_chunk(int row_warps, int nk, bool weno) {
+    const int want = 148 * (weno ? 32 : 48);  // warps in flight worth of work
+    int chunk = nk;
+    while (chunk > 4 && (long long)row_warps * ((nk + chunk - 1) / chunk) < 2LL * want) chunk = (chunk + 1) / 2;
+    return chunk;
+}
+
+// One warp = the faces x = x0 .. x0+31 of one row and a chunk of levels.  A
+// lane forms the x flux of its face and takes the next face's from the lane
+// above, so 31 cells per warp need no second flux and no divergent edge.  The
+// fifth-order pass forms both y fluxes of a cell (cheaper than handing one
+// down through shared memory behind a barrier); the WENO pass, whose flux
+// costs four binary64 divisions, hands each y flux to the row below through
+// shared memory, one barrier a level, the eighth row forming a flux only.
+// Words come through L1, which holds a row's neighbours: the passes are bound
+// by instruction issue (fifth order) and the binary64 weights (WENO).
+// Measured on one B200, per launch at 640x768x80: fifth order 1.105 -> 0.446
+// ms, WENO 2.572 -> 1.355 against CTAs that stage each level's plane in shared
+// memory (WENO with 24 warps an SM 1.437, with 16 rows 1.836).
 template <bool WENO>
-__global__ void __launch_bounds__(kTX5 *kTY5)
-    scalar_advection5_tiled_kernel(gm1b_scalar_advection5_arrays a, PaddedDims d, int levels_per_chunk, float rdx,
+__global__ void __launch_bounds__(32 * (WENO ? kWenoRows : kFifthRows), WENO ? 4 : 5)
+    scalar_advection5_march_kernel(gm1b_scalar_advection5_arrays a, PaddedDims d, int levels_per_chunk, float rdx,
                                    float rdy, float rdsf, double eps, float wepsf, unsigned obc, VertCol vc) {
-    __shared__ float s_plane[kPY][kPX];
-    __shared__ float s_fx[kTY5][kTX5 + 1];
-    __shared__ float s_fy[kTY5 + 1][kTX5];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int tid = ty * kTX5 + tx;
-    const int i0 = blockIdx.x * kTX5, j0 = blockIdx.y * kTY5;
-    const int i = i0 + tx, j = j0 + ty;
+    constexpr int ROWS = WENO ? kWenoRows : kFifthRows;
+    __shared__ float s_fy[WENO ? 2 : 1][WENO ? ROWS : 1][32], s_vm[WENO ? 2 : 1][WENO ? ROWS : 1][32];
+    const int lane = threadIdx.x, ty = threadIdx.y;
     const int ni = d.ni, nj = d.nj, nk = d.nk;
-    const int sx = ni + 2 * NG, sy = nj + 2 * NG;        // scalar / w plane
-    const int ux = ni + 1 + 2 * NG;                      // u row length
-    const int vy = nj + 1 + 2 * NG;                      // v rows
+    const int sx = ni + 2 * NG, sy = nj + 2 * NG, ux = ni + 1 + 2 * NG, vy = nj + 1 + 2 * NG;
     const int splane = sx * sy, uplane = ux * sy, vplane = sx * vy, cplane = ni * nj;
-    const bool cell = i < ni && j < nj;
-    const int x = i + NG, y = j + NG;
-    const int k_begin = 1 + blockIdx.z * levels_per_chunk;
+    const int xtiles = ni / kFaceOut + 1;  // tiles in one grid dimension, which takes any plane
+    const int i = blockIdx.x % xtiles * kFaceOut + lane;
+    const int row = blockIdx.x / xtiles * (WENO ? ROWS - 1 : ROWS) + ty;
+    if (!WENO && row >= nj) return;  // whole warps: the fifth-order pass has no barrier
+    // rows and faces past the domain repeat its last ones and store nothing
+    const int j = min(row, WENO ? nj : nj - 1), f = min(i, ni);
+    const int x = f + NG, y = j + NG;
+    const bool cell = i < ni && row < nj && lane < kFaceOut && (!WENO || ty < ROWS - 1);
+    const int k_begin = 1 + blockIdx.y * levels_per_chunk;
     const int k_end = min(nk, k_begin + levels_per_chunk - 1);
     const float *s = a.scalar;
     const bool owned = cell && (obc != 0u || (i >= 3 && i + 3 < ni && j >= 3 && j + 3 < nj));
-    const bool east_face = cell && (tx == kTX5 - 1 || i == ni - 1);
-    const bool north_face = cell && (ty == kTY5 - 1 || j == nj - 1);
-    const float gz = cell ? __ldg(a.gz + j * ni + i) : 0.0f;
-    const int col = y * sx + x;  // offset of this column inside a scalar/w plane
-    // register window of this column: win[q] = level (k+1) - 3 + q, k = k_begin - 1 initially
-    float win[6];
+    const int col = y * sx + x;          // this point in a scalar / w plane
+    const int uc = y * ux + x, cc = min(j, nj - 1) * ni + min(f, ni - 1);
+    const bool north = WENO && j == nj;  // the row of faces nj only
+    const bool wo = i == 0 && (obc & 15u) == 2u, eo = i + 1 == ni && ((obc >> 4) & 15u) == 2u;
+    const bool so = j == 0 && ((obc >> 8) & 15u) == 2u, no = j + 1 == nj && ((obc >> 12) & 15u) == 2u;
+    const float gz = __ldg(a.gz + cc);
+    float win[6];  // levels k-3 .. k+2 of this point; shifted to k-2 .. k+3 for face k+1
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-        const int lev = k_begin - 3 + q;  // face k_begin needs levels k_begin-3 .. k_begin+2
-        win[q] = (cell && lev >= 0 && lev <= nk + 1) ? __ldg(s + lev * splane + col) : 0.0f;
+        const int lev = k_begin - 3 + q;
+        win[q] = (!north && lev >= 0 && lev <= nk + 1) ? __ldg(s + lev * splane + col) : 0.0f;
     }
     float fz_lo = 0.0f;
     if (cell) {
-        const int f = k_begin;
-        if (f >= 2 && f <= nk) {
-            const float m = __ldg(a.rrw + f * splane + col);
-            const float c1 = (f == 2 || f == nk) ? __ldg(a.c1 + (f - 1) * cplane + j * ni + i) : 0.0f;
-            const float c2 = (f == 2 || f == nk) ? __ldg(a.c2 + (f - 1) * cplane + j * ni + i) : 0.0f;
-            fz_lo = z_face<WENO>(win, m, c1, c2, f, nk, eps, wepsf);
+        if (k_begin >= 2) {
+            const bool end = k_begin == 2 || k_begin == nk;
+            const float m = __ldg(a.rrw + k_begin * splane + col);
+            const float c1 = end ? __ldg(a.c1 + (k_begin - 1) * cplane + cc) : 0.0f;
+            const float c2 = end ? __ldg(a.c2 + (k_begin - 1) * cplane + cc) : 0.0f;
+            fz_lo = z_face<WENO>(win, m, c1, c2, k_begin, nk, eps, wepsf);
+        } else if (a.flux_z != nullptr) {
+            a.flux_z[splane + col] = 0.0f;
         }
-        if (a.flux_z != nullptr && k_begin == 1) a.flux_z[1 * splane + col] = 0.0f;
     }
+#pragma unroll 1
     for (int k = k_begin; k <= k_end; ++k) {
-        // stage the scalar plane of level k: tile columns x0-3 .. x0+34, rows y0-3 .. y0+10
-        const float *plane = s + k * splane;
-        for (int q = tid; q < kPX * kPY; q += kTX5 * kTY5) {
-            const int py = q / kPX, px = q - py * kPX;
-            const int gx = i0 + px, gy = j0 + py;  // padded coords (tile origin x0 - 3 = i0)
-            s_plane[py][px] = (gx < sx && gy < sy) ? __ldg(plane + gy * sx + gx) : 0.0f;
+        const float *pt = s + k * splane + col;
+        // the level's words, all in flight together
+        const float mw = __ldg(a.rru + k * uplane + uc);
+        const float ms = __ldg(a.rrv + k * vplane + col);
+        float mn = 0.0f;
+        if (!WENO) mn = __ldg(a.rrv + k * vplane + col + sx);
+        float px[6], py[7];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) px[q] = q == 3 ? 0.0f : __ldg(pt + (q - 3));
+#pragma unroll
+        for (int q = 0; q < 7; ++q) py[q] = (q == 3 || (WENO && q == 6)) ? 0.0f : __ldg(pt + (q - 3) * sx);
+        const float zn = (!north && k + 3 <= nk + 1) ? __ldg(pt + 3 * splane) : 0.0f;
+        const int fz = k + 1;
+        float mz = 0.0f, c1 = 0.0f, c2 = 0.0f;
+        if (fz <= nk && !north) {
+            mz = __ldg(a.rrw + fz * splane + col);
+            if (fz == 2 || fz == nk) {
+                c1 = __ldg(a.c1 + (fz - 1) * cplane + cc);
+                c2 = __ldg(a.c2 + (fz - 1) * cplane + cc);
+            }
         }
-        // shift the column window to levels k-2 .. k+3 (face k+1)
+        const int c = (k - 1) * cplane + cc;
+        const float div = __ldg(a.divx + c);
+        const float rr0 = __ldg(a.rr0 + (vc.mode == 2 ? (k - 1) * cplane : c));
+        float sv = win[3];
+        if (north) sv = __ldg(pt);
+        px[3] = py[3] = sv;
+        const float fx = upwind<WENO>(mw, px[0], px[1], px[2], px[3], px[4], px[5], eps);
+        const float fy = upwind<WENO>(ms, py[0], py[1], py[2], py[3], py[4], py[5], eps);
+        float fw = fx, fe = __shfl_down_sync(0xffffffffu, fx, 1);
+        const float ue = __shfl_down_sync(0xffffffffu, mw, 1);
+        float fs = fy, fn;
+        if (WENO) {
+            const int buf = k & 1;
+            s_fy[buf][ty][lane] = fy;
+            s_vm[buf][ty][lane] = ms;
+            __syncthreads();
+            const int up = min(ty + 1, ROWS - 1);
+            fn = s_fy[buf][up][lane];
+            mn = s_vm[buf][up][lane];
+        } else {
+            fn = upwind<WENO>(mn, py[1], py[2], py[3], py[4], py[5], py[6], eps);
+        }
 #pragma unroll
         for (int q = 0; q < 5; ++q) win[q] = win[q + 1];
-        {
-            const int lev = k + 3;
-            win[5] = (cell && lev <= nk + 1) ? __ldg(s + lev * splane + col) : 0.0f;
-        }
-        __syncthreads();
+        win[5] = zn;
         if (cell) {
-            const float *urow = a.rru + k * uplane + y * ux;
-            const float mw = __ldg(urow + x);
-            const float fw = mw * (mw >= 0.0f ? recon<WENO>(s_plane[ty + 3][tx], s_plane[ty + 3][tx + 1],
-                                                            s_plane[ty + 3][tx + 2], s_plane[ty + 3][tx + 3],
-                                                            s_plane[ty + 3][tx + 4], eps)
-                                              : recon<WENO>(s_plane[ty + 3][tx + 5], s_plane[ty + 3][tx + 4],
-                                                            s_plane[ty + 3][tx + 3], s_plane[ty + 3][tx + 2],
-                                                            s_plane[ty + 3][tx + 1], eps));
-            s_fx[ty][tx] = fw;
-            if (a.flux_x != nullptr) a.flux_x[k * uplane + y * ux + x] = fw;
-            if (east_face) {
-                const float me = __ldg(urow + x + 1);
-                const float fe = me * (me >= 0.0f ? recon<WENO>(s_plane[ty + 3][tx + 1], s_plane[ty + 3][tx + 2],
-                                                                s_plane[ty + 3][tx + 3], s_plane[ty + 3][tx + 4],
-                                                                s_plane[ty + 3][tx + 5], eps)
-                                                  : recon<WENO>(s_plane[ty + 3][tx + 6], s_plane[ty + 3][tx + 5],
-                                                                s_plane[ty + 3][tx + 4], s_plane[ty + 3][tx + 3],
-                                                                s_plane[ty + 3][tx + 2], eps));
-                s_fx[ty][tx + 1] = fe;
-                if (a.flux_x != nullptr && i == ni - 1) a.flux_x[k * uplane + y * ux + x + 1] = fe;
+            if (a.flux_x != nullptr) {
+                a.flux_x[k * uplane + uc] = fw;
+                if (i == ni - 1) a.flux_x[k * uplane + uc + 1] = fe;
             }
-            const float *vplane_k = a.rrv + k * vplane;
-            const float ms = __ldg(vplane_k + y * sx + x);
-            const float fs = ms * (ms >= 0.0f ? recon<WENO>(s_plane[ty][tx + 3], s_plane[ty + 1][tx + 3],
-                                                            s_plane[ty + 2][tx + 3], s_plane[ty + 3][tx + 3],
-                                                            s_plane[ty + 4][tx + 3], eps)
-                                              : recon<WENO>(s_plane[ty + 5][tx + 3], s_plane[ty + 4][tx + 3],
-                                                            s_plane[ty + 3][tx + 3], s_plane[ty + 2][tx + 3],
-                                                            s_plane[ty + 1][tx + 3], eps));
-            s_fy[ty][tx] = fs;
-            if (a.flux_y != nullptr) a.flux_y[k * vplane + y * sx + x] = fs;
-            if (north_face) {
-                const float mn = __ldg(vplane_k + (y + 1) * sx + x);
-                const float fn = mn * (mn >= 0.0f ? recon<WENO>(s_plane[ty + 1][tx + 3], s_plane[ty + 2][tx + 3],
-                                                                s_plane[ty + 3][tx + 3], s_plane[ty + 4][tx + 3],
-                                                                s_plane[ty + 5][tx + 3], eps)
-                                                  : recon<WENO>(s_plane[ty + 6][tx + 3], s_plane[ty + 5][tx + 3],
-                                                                s_plane[ty + 4][tx + 3], s_plane[ty + 3][tx + 3],
-                                                                s_plane[ty + 2][tx + 3], eps));
-                s_fy[ty + 1][tx] = fn;
-                if (a.flux_y != nullptr && j == nj - 1) a.flux_y[k * vplane + (y + 1) * sx + x] = fn;
+            if (a.flux_y != nullptr) {
+                a.flux_y[k * vplane + col] = fs;
+                if (j == nj - 1) a.flux_y[k * vplane + col + sx] = fn;
             }
-        }
-        __syncthreads();
-        if (cell) {
             float fz_hi = 0.0f;
-            const int f = k + 1;
-            if (f <= nk) {
-                const float m = __ldg(a.rrw + f * splane + col);
-                const float c1 = (f == 2 || f == nk) ? __ldg(a.c1 + (f - 1) * cplane + j * ni + i) : 0.0f;
-                const float c2 = (f == 2 || f == nk) ? __ldg(a.c2 + (f - 1) * cplane + j * ni + i) : 0.0f;
-                fz_hi = z_face<WENO>(win, m, c1, c2, f, nk, eps, wepsf);
-            }
-            if (a.flux_z != nullptr) a.flux_z[f * splane + col] = fz_hi;
+            if (fz <= nk) fz_hi = z_face<WENO>(win, mz, c1, c2, fz, nk, eps, wepsf);
+            if (a.flux_z != nullptr) a.flux_z[fz * splane + col] = fz_hi;
             if (owned) {
-                float fw = s_fx[ty][tx], fe = s_fx[ty][tx + 1];
-                float fs = s_fy[ty][tx], fn = s_fy[ty + 1][tx];
-                // this cell's value from the register window (levels k-2..k+3):
-                // the shared plane may already hold level k+1 for threads
-                // that moved on
-                const float sv = win[2];
-                const float *urow = a.rru + k * uplane + y * ux;
-                const float *vcol = a.rrv + k * vplane + x;
-                const float uw = __ldg(urow + x), ue = __ldg(urow + x + 1);
-                const float vs = __ldg(vcol + y * sx), vn = __ldg(vcol + (y + 1) * sx);
-                const bool iw = (i == 0) && ((obc & 15u) == 2u) && uw >= 0.0f;
-                const bool ie = (i + 1 == ni) && (((obc >> 4) & 15u) == 2u) && ue <= 0.0f;
-                const bool js = (j == 0) && (((obc >> 8) & 15u) == 2u) && vs >= 0.0f;
-                const bool jn = (j + 1 == nj) && (((obc >> 12) & 15u) == 2u) && vn <= 0.0f;
+                const bool iw = wo && mw >= 0.0f, ie = eo && ue <= 0.0f;
+                const bool js = so && ms >= 0.0f, jn = no && mn <= 0.0f;
                 if (iw) fw = fe;
                 if (ie) fe = fw;
                 if (js) fs = fn;
                 if (jn) fn = fs;
                 float ax = (fw - fe) * rdx;
                 float ay = (fs - fn) * rdy;
-                if (iw) ax = ax - (sv * (ue - uw)) * rdx;
-                if (ie) ax = ax - (sv * (ue - uw)) * rdx;
-                if (js) ay = ay - (sv * (vn - vs)) * rdy;
-                if (jn) ay = ay - (sv * (vn - vs)) * rdy;
+                if (iw) ax = ax - (sv * (ue - mw)) * rdx;
+                if (ie) ax = ax - (sv * (ue - mw)) * rdx;
+                if (js) ay = ay - (sv * (mn - ms)) * rdy;
+                if (jn) ay = ay - (sv * (mn - ms)) * rdy;
                 float az;
                 if (vc.mode == 2) {
                     const float mhk = __ldg(vc.mh + k);
@@ -426,100 +350,12 @@ __global__ void __launch_bounds__(kTX5 *kTY5)
                     else
                         az = (fz_lo - fz_hi) * r;
                 }
-                const int c = (k - 1) * cplane + j * ni + i;
                 float total = (ax + ay) + az;
-                total = total + sv * __ldg(a.divx + c);
-                if (vc.mode == 2)
-                    a.tendency[c] = total * __ldg(a.rr0 + (k - 1) * cplane);
-                else
-                    a.tendency[c] = (total * __ldg(a.rr0 + c)) * gz;
+                total = total + sv * div;
+                a.tendency[c] = vc.mode == 2 ? total * rr0 : (total * rr0) * gz;
             }
             fz_lo = fz_hi;
         }
-    }
-}
-
-template <bool WENO>
-__global__ void __launch_bounds__(kAX *kAY)
-    scalar_advection5_kernel(gm1b_scalar_advection5_arrays a, PaddedDims d, int levels_per_chunk, float rdx,
-                             float rdy, float rdsf, double eps, float wepsf, unsigned obc) {
-    __shared__ float s_fx[kAY][kAX + 1];
-    __shared__ float s_fy[kAY + 1][kAX];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i = blockIdx.x * kAX + tx;
-    const int j = blockIdx.y * kAY + ty;
-    const int ni = d.ni, nj = d.nj, nk = d.nk;
-    const bool cell = i < ni && j < nj;
-    const int x = i + NG, y = j + NG;
-    const int k_begin = 1 + blockIdx.z * levels_per_chunk;
-    const int k_end = min(nk, k_begin + levels_per_chunk - 1);
-    const float *s = a.scalar;
-    const bool owned = cell && (obc != 0u || (i >= 3 && i + 3 < ni && j >= 3 && j + 3 < nj));
-    const bool east_face = cell && (tx == kAX - 1 || i == ni - 1);
-    const bool north_face = cell && (ty == kAY - 1 || j == nj - 1);
-    float fz_lo = 0.0f;
-    if (cell) {
-        fz_lo = vertical_flux<WENO>(s, d, a, k_begin, j, i, y, x, eps, wepsf);
-        if (a.flux_z != nullptr && k_begin == 1) a.flux_z[d.s(1, y, x)] = 0.0f;
-    }
-    for (int k = k_begin; k <= k_end; ++k) {
-        if (cell) {
-            const float fw = x_face_flux<WENO>(s, d, a.rru, k, y, x, eps);
-            s_fx[ty][tx] = fw;
-            if (a.flux_x != nullptr) a.flux_x[d.u(k, y, x)] = fw;
-            if (east_face) {
-                const float fe = x_face_flux<WENO>(s, d, a.rru, k, y, x + 1, eps);
-                s_fx[ty][tx + 1] = fe;
-                if (a.flux_x != nullptr && i == ni - 1) a.flux_x[d.u(k, y, x + 1)] = fe;
-            }
-            const float fs = y_face_flux<WENO>(s, d, a.rrv, k, y, x, eps);
-            s_fy[ty][tx] = fs;
-            if (a.flux_y != nullptr) a.flux_y[d.v(k, y, x)] = fs;
-            if (north_face) {
-                const float fn = y_face_flux<WENO>(s, d, a.rrv, k, y + 1, x, eps);
-                s_fy[ty + 1][tx] = fn;
-                if (a.flux_y != nullptr && j == nj - 1) a.flux_y[d.v(k, y + 1, x)] = fn;
-            }
-        }
-        __syncthreads();
-        if (cell) {
-            const float fz_hi = vertical_flux<WENO>(s, d, a, k + 1, j, i, y, x, eps, wepsf);
-            if (a.flux_z != nullptr) a.flux_z[d.s(k + 1, y, x)] = fz_hi;
-            if (owned) {
-                float fw = s_fx[ty][tx], fe = s_fx[ty][tx + 1];
-                float fs = s_fy[ty][tx], fn = s_fy[ty + 1][tx];
-                const float sv = __ldg(s + d.s(k, y, x));
-                const float uw = __ldg(a.rru + d.u(k, y, x)), ue = __ldg(a.rru + d.u(k, y, x + 1));
-                const float vs = __ldg(a.rrv + d.v(k, y, x)), vn = __ldg(a.rrv + d.v(k, y + 1, x));
-                const bool iw = (i == 0) && ((obc & 15u) == 2u) && uw >= 0.0f;
-                const bool ie = (i + 1 == ni) && (((obc >> 4) & 15u) == 2u) && ue <= 0.0f;
-                const bool js = (j == 0) && (((obc >> 8) & 15u) == 2u) && vs >= 0.0f;
-                const bool jn = (j + 1 == nj) && (((obc >> 12) & 15u) == 2u) && vn <= 0.0f;
-                if (iw) fw = fe;
-                if (ie) fe = fw;
-                if (js) fs = fn;
-                if (jn) fn = fs;
-                float ax = (fw - fe) * rdx;
-                float ay = (fs - fn) * rdy;
-                if (iw) ax = ax - (sv * (ue - uw)) * rdx;
-                if (ie) ax = ax - (sv * (ue - uw)) * rdx;
-                if (js) ay = ay - (sv * (vn - vs)) * rdy;
-                if (jn) ay = ay - (sv * (vn - vs)) * rdy;
-                float az;
-                if (k == 1)
-                    az = (-fz_hi) * rdsf;
-                else if (k == nk)
-                    az = fz_lo * rdsf;
-                else
-                    az = (fz_lo - fz_hi) * rdsf;
-                float total = (ax + ay) + az;
-                total = total + sv * __ldg(a.divx + d.c(k - 1, j, i));
-                a.tendency[d.c(k - 1, j, i)] =
-                    (total * __ldg(a.rr0 + d.c(k - 1, j, i))) * __ldg(a.gz + (size_t)j * ni + i);
-            }
-            fz_lo = fz_hi;
-        }
-        __syncthreads();
     }
 }
 
@@ -609,23 +445,20 @@ int32_t scalar_advection5_launch(int32_t ni, int32_t nj, int32_t nk, const gm1b_
         }
     }
     const bool weno = wflag != 0 && nrk == 3;
-    // default level chunk per CTA (measured at 256x256x80 on B200): short
-    // chunks give the fifth-order pass more CTAs to overlap its per-level
-    // staging (4 levels: 0.154 ms, 16: 0.191 ms); the WENO pass is bound by its
-    // binary64 weights and is flat between 4 and 16
-    int chunk = levels_per_chunk > 0 ? levels_per_chunk : (weno ? 16 : 4);
-    if (chunk > nk) chunk = nk;
     const PaddedDims d{ni, nj, nk};
-    const dim3 grid((ni + kTX5 - 1) / kTX5, (nj + kTY5 - 1) / kTY5, (nk + chunk - 1) / chunk);
+    const int xtiles = ni / kFaceOut + 1;  // faces 0..ni
+    const int rows = weno ? kWenoRows - 1 : kFifthRows, ytiles = (nj + rows - 1) / rows;
+    const int chunk = levels_per_chunk > 0 ? std::min(levels_per_chunk, nk) : default_chunk(xtiles * nj, nk, weno);
+    const dim3 grid(xtiles * ytiles, (nk + chunk - 1) / chunk);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float rdx = 1.0f / dx, rdy = 1.0f / dy, rdsf = 1.0f / dz;
     ProfScope ps(weno ? "scalar_advection5_weno_kernel" : "scalar_advection5_kernel", st);
     if (weno)
-        scalar_advection5_tiled_kernel<true>
-            <<<grid, dim3(kTX5, kTY5), 0, st>>>(a, d, chunk, rdx, rdy, rdsf, weps, (float)weps, lateral_obc, vc);
+        scalar_advection5_march_kernel<true>
+            <<<grid, dim3(32, kWenoRows), 0, st>>>(a, d, chunk, rdx, rdy, rdsf, weps, (float)weps, lateral_obc, vc);
     else
-        scalar_advection5_tiled_kernel<false>
-            <<<grid, dim3(kTX5, kTY5), 0, st>>>(a, d, chunk, rdx, rdy, rdsf, weps, (float)weps, lateral_obc, vc);
+        scalar_advection5_march_kernel<false>
+            <<<grid, dim3(32, kFifthRows), 0, st>>>(a, d, chunk, rdx, rdy, rdsf, weps, (float)weps, lateral_obc, vc);
     ps.stop();
     if (cudaPeekAtLastError() != cudaSuccess) {
         gm1b_set_error("scalar_advection5_kernel: %s", cudaGetErrorString(cudaGetLastError()));

@@ -68,3 +68,30 @@ def test_compact_acoustic_stage(column, ni, nj, nk):
             tos.launch_cuda_gm1_child_psolver3_open_stage(dev, mdev, nrk=nrk, vertical=vertical, compiled=compiled, **kw)
         names = [n for n in tos.COMPARE_OUTPUT_NAMES if not n.startswith("tri_")] + ["scalar"]
         assert _differ(dev, ref, names) == [], nrk
+
+
+@pytest.mark.parametrize("nrk", [1, 3])
+@pytest.mark.parametrize("ni,nj,nk,chunk", [(30, 8, 8, None), (31, 13, 9, 4), (32, 14, 11, 5), (61, 15, 8, 1),
+                                            (62, 9, 21, None), (8, 8, 40, 7)])
+def test_scalar_advection(ni, nj, nk, chunk, nrk):
+    """Open sides with the face fluxes written, each word of the tendency and
+    the fluxes (the warps' shared faces among them)."""
+    from gm1_b200.advection import launch_cuda_scalar_advection5, padded_shapes
+    from oracle import advection as adv
+
+    rng = np.random.default_rng(ni + nk)
+    sh = padded_shapes(ni, nj, nk)
+    f = lambda s, lo, hi: rng.uniform(lo, hi, s).astype(np.float32)  # noqa: E731
+    h = {"scalar": f(sh["scalar"], -1, 1), "rru": f(sh["u"], -9, 9), "rrv": f(sh["v"], -9, 9), "rrw": f(sh["w"], -2, 2),
+         "c1": f(sh["face"], 0.3, 0.7), "c2": f(sh["face"], 0.3, 0.7), "rr0": f(sh["cell"], 0.8, 3.0),
+         "gz": f((nj, ni), 0.8, 1.2), "divx": f(sh["cell"], -1e-3, 1e-3), "tendency": np.zeros(sh["cell"], np.float32),
+         "flux_x": np.zeros(sh["u"], np.float32), "flux_y": np.zeros(sh["v"], np.float32),
+         "flux_z": np.zeros(sh["w"], np.float32)}
+    h["scalar"][:, :, : ni // 2] = 0.0  # whole stencils of zeros, and edges of them
+    d = _dev(h)
+    kw = dict(ni=ni, nj=nj, nk=nk, nrk=nrk, dx=400.0, dy=350.0, dz=150.0, weps=1.0e-20)
+    adv.scalar_advection5(h, lateral_obc=0x2222, **kw)
+    launch_cuda_scalar_advection5(
+        d["scalar"], {k: d[k] for k in ("rru", "rrv", "rrw")}, {k: d[k] for k in ("c1", "c2", "rr0", "gz")}, d["divx"],
+        d["tendency"], {q: d["flux_" + q] for q in "xyz"}, lateral_sides=(2, 2, 2, 2), levels_per_chunk=chunk, **kw)
+    assert _differ(d, h, ("tendency", "flux_x", "flux_y", "flux_z")) == []
