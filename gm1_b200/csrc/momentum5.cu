@@ -12,9 +12,9 @@
 // Design (B200): three launches instead of the reference's six.  (1) every
 // u and v face's mass flux; (2) rrw and divx together (each cell forms the
 // two rrw words its divergence needs, writing its own); (3) one momentum
-// pass where a thread owns the u face, the v face and the w face at its
-// (k, y, x).  Upwind face fluxes read the six points that hold both upwind
-// stencils before the mass-flux sign is known, so no load waits on it.
+// pass whose warps march rows of u, v or w faces up the column (below).
+// Upwind face fluxes read the six points that hold both upwind stencils
+// before the mass-flux sign is known, so no load waits on it.
 // Binary32 one operation at a time in the reference's order: word-identical.
 #include "gm1b_common.cuh"
 
@@ -67,11 +67,6 @@ __device__ __forceinline__ int cyw(const MomArgs &a, int j) {
 __device__ __forceinline__ int fyw(const MomArgs &a, int j) {
     return (a.per[2] && j < 0) ? j + a.nj : ((a.per[3] && j > a.nj) ? j - a.nj : j);
 }
-// face-level c2 at Fortran face kface, clamped column
-__device__ __forceinline__ float c2m(const MomArgs &a, int kface, int j, int i) {
-    return __ldg(a.c2 + ic(a, kface - 1, clampn(j, a.nj), clampn(i, a.ni)));
-}
-
 // x * the column's vertical reciprocal at mass level k (uniform rdz, the
 // terrain branch's rdsf(k), or the flat column's (x*rdz)*mh(k))
 __device__ __forceinline__ float zmass(const MomArgs &a, float x, int k) {
@@ -101,130 +96,6 @@ __device__ __forceinline__ float up5(float m, float s0, float s1, float s2, floa
 #define RU(k, y, x) a.rru[iu(a, (k), (y), (x))]
 #define RV(k, y, x) a.rrv[iv(a, (k), (y), (x))]
 #define RW(k, y, x) a.rrw[iw(a, (k), (y), (x))]
-
-__device__ float u_fx(const MomArgs &a, int k, int j, int face) {
-    const int y = j + G, x = face + G;
-    const float m = 0.5f * (RU(k, y, fxw(a, face) + G) + RU(k, y, fxw(a, face + 1) + G));
-    return up5(m, LU(k, y, x - 2), LU(k, y, x - 1), LU(k, y, x), LU(k, y, x + 1), LU(k, y, x + 2), LU(k, y, x + 3));
-}
-
-__device__ float u_fy_base(const MomArgs &a, int k, int face, int i_face) {
-    const int y = face + G, x = i_face + G;
-    const float m = 0.5f * (RV(k, y, cxw(a, i_face) + G) + RV(k, y, cxw(a, i_face - 1) + G));
-    return up5(m, LU(k, y - 3, x), LU(k, y - 2, x), LU(k, y - 1, x), LU(k, y, x), LU(k, y + 1, x), LU(k, y + 2, x));
-}
-
-__device__ float u_fy(const MomArgs &a, int k, int face, int i_face) {
-    const int y = face + G;
-    const float mt = RV(k, y, cxw(a, i_face) + G) + RV(k, y, cxw(a, i_face - 1) + G);
-    if (face == 0 && a.opn[2] && mt >= 0.0f) return u_fy_base(a, k, 1, i_face);
-    if (face == a.nj && a.opn[3] && mt <= 0.0f) return u_fy_base(a, k, a.nj - 1, i_face);
-    return u_fy_base(a, k, face, i_face);
-}
-
-__device__ float v_fx_base(const MomArgs &a, int k, int j_face, int face) {
-    const int y = j_face + G, x = face + G;
-    const float m = 0.5f * (RU(k, cyw(a, j_face) + G, x) + RU(k, cyw(a, j_face - 1) + G, x));
-    return up5(m, LV(k, y, x - 3), LV(k, y, x - 2), LV(k, y, x - 1), LV(k, y, x), LV(k, y, x + 1), LV(k, y, x + 2));
-}
-
-__device__ float v_fx(const MomArgs &a, int k, int j_face, int face) {
-    const int x = face + G;
-    const float mt = RU(k, cyw(a, j_face) + G, x) + RU(k, cyw(a, j_face - 1) + G, x);
-    if (face == 0 && a.opn[0] && mt >= 0.0f) return v_fx_base(a, k, j_face, 1);
-    if (face == a.ni && a.opn[1] && mt <= 0.0f) return v_fx_base(a, k, j_face, a.ni - 1);
-    return v_fx_base(a, k, j_face, face);
-}
-
-__device__ float v_fy(const MomArgs &a, int k, int face, int i) {
-    const int y = face + G, x = i + G;
-    const float m = 0.5f * (RV(k, fyw(a, face) + G, x) + RV(k, fyw(a, face + 1) + G, x));
-    return up5(m, LV(k, y - 2, x), LV(k, y - 1, x), LV(k, y, x), LV(k, y + 1, x), LV(k, y + 2, x), LV(k, y + 3, x));
-}
-
-__device__ float w_fx_base(const MomArgs &a, int kf, int j, int face) {
-    const int y = j + G, x = face + G;
-    const float c2 = 0.5f * (c2m(a, kf, j, face - 1) + c2m(a, kf, j, face)), c1 = 1.0f - c2;
-    const float m = c2 * RU(kf, y, x) + c1 * RU(kf - 1, y, x);
-    return up5(m, LW(kf, y, x - 3), LW(kf, y, x - 2), LW(kf, y, x - 1), LW(kf, y, x), LW(kf, y, x + 1),
-               LW(kf, y, x + 2));
-}
-
-__device__ float w_fx(const MomArgs &a, int kf, int j, int face) {
-    const int y = j + G, x = face + G;
-    const float c2 = 0.5f * (c2m(a, kf, j, face - 1) + c2m(a, kf, j, face)), c1 = 1.0f - c2;
-    const float m = c2 * RU(kf, y, x) + c1 * RU(kf - 1, y, x);
-    if (face == 0 && a.opn[0] && m >= 0.0f) return w_fx_base(a, kf, j, 1);
-    if (face == a.ni && a.opn[1] && m <= 0.0f) return w_fx_base(a, kf, j, a.ni - 1);
-    return w_fx_base(a, kf, j, face);
-}
-
-__device__ float w_fy_base(const MomArgs &a, int kf, int face, int i) {
-    const int y = face + G, x = i + G;
-    const float c2 = 0.5f * (c2m(a, kf, face - 1, i) + c2m(a, kf, face, i)), c1 = 1.0f - c2;
-    const float m = c2 * RV(kf, y, x) + c1 * RV(kf - 1, y, x);
-    return up5(m, LW(kf, y - 3, x), LW(kf, y - 2, x), LW(kf, y - 1, x), LW(kf, y, x), LW(kf, y + 1, x),
-               LW(kf, y + 2, x));
-}
-
-__device__ float w_fy(const MomArgs &a, int kf, int face, int i) {
-    const int y = face + G, x = i + G;
-    const float c2 = 0.5f * (c2m(a, kf, face - 1, i) + c2m(a, kf, face, i)), c1 = 1.0f - c2;
-    const float m = c2 * RV(kf, y, x) + c1 * RV(kf - 1, y, x);
-    if (face == 0 && a.opn[2] && m >= 0.0f) return w_fy_base(a, kf, 1, i);
-    if (face == a.nj && a.opn[3] && m <= 0.0f) return w_fy_base(a, kf, a.nj - 1, i);
-    return w_fy_base(a, kf, face, i);
-}
-
-// vertical flux of u (is_u) or v at Fortran face kface of column (j, i)
-__device__ float uv_z(const MomArgs &a, bool is_u, int kface, int j, int i) {
-    const int y = j + G, x = i + G, nk = a.nk;
-    float m, c2;
-    if (is_u) {
-        m = 0.5f * (RW(kface, y, cxw(a, i) + G) + RW(kface, y, cxw(a, i - 1) + G));
-        c2 = 0.5f * (c2m(a, kface, j, i - 1) + c2m(a, kface, j, i));
-    } else {
-        m = 0.5f * (RW(kface, cyw(a, j) + G, x) + RW(kface, cyw(a, j - 1) + G, x));
-        c2 = 0.5f * (c2m(a, kface, j - 1, i) + c2m(a, kface, j, i));
-    }
-    const float c1 = 1.0f - c2;
-#define Q(l) (is_u ? LU((l), y, x) : LV((l), y, x))
-    float r;
-    if (kface == 2) {
-        r = m >= 0.0f ? c1 * Q(1) + c2 * Q(2) : flx3(Q(3), Q(2), Q(1));
-    } else if (kface == nk) {
-        r = m >= 0.0f ? flx3(Q(nk - 2), Q(nk - 1), Q(nk)) : c1 * Q(nk - 1) + c2 * Q(nk);
-    } else if (kface == 3) {
-        r = m >= 0.0f ? flx3(Q(1), Q(2), Q(3)) : flx5(Q(5), Q(4), Q(3), Q(2), Q(1));
-    } else if (kface == nk - 1) {
-        r = m >= 0.0f ? flx5(Q(kface - 3), Q(kface - 2), Q(kface - 1), Q(kface), Q(kface + 1))
-                      : flx3(Q(kface + 1), Q(kface), Q(kface - 1));
-    } else {
-        return up5(m, Q(kface - 3), Q(kface - 2), Q(kface - 1), Q(kface), Q(kface + 1), Q(kface + 2));
-    }
-#undef Q
-    return m * r;
-}
-
-__device__ float w_z(const MomArgs &a, int k, int j, int i) {
-    const int y = j + G, x = i + G, nk = a.nk;
-    const float m = 0.5f * (RW(k, y, x) + RW(k + 1, y, x));
-#define Q(l) LW((l), y, x)
-    float r;
-    if (k == 1) {
-        r = m >= 0.0f ? 0.5f * (Q(1) + Q(2)) : flx3(Q(3), Q(2), Q(1));
-    } else if (k == 2) {
-        r = m >= 0.0f ? flx3(Q(1), Q(2), Q(3)) : flx5(Q(5), Q(4), Q(3), Q(2), Q(1));
-    } else if (k == nk - 1) {
-        r = m >= 0.0f ? flx5(Q(k - 2), Q(k - 1), Q(k), Q(k + 1), Q(k + 2)) : flx3(Q(k + 2), Q(k + 1), Q(k));
-    } else if (k == nk) {
-        r = m >= 0.0f ? flx3(Q(k - 1), Q(k), Q(k + 1)) : 0.5f * (Q(k) + Q(k + 1));
-    } else {
-        return up5(m, Q(k - 2), Q(k - 1), Q(k), Q(k + 1), Q(k + 2), Q(k + 3));
-    }
-#undef Q
-    return m * r;
-}
 
 // (1) horizontal mass fluxes; grid: x over 0..ni, y over 0..nj, z over k = 1..nk
 __global__ void __launch_bounds__(128) mom5_mass_kernel(MomArgs a) {
@@ -291,117 +162,312 @@ __global__ void __launch_bounds__(128) mom5_rrw_divx_kernel(MomArgs a) {
     a.divx[ic(a, k0, j, i)] = fabsf(value) < 1.0e-20f ? 0.0f : value;
 }
 
-// (3) advu / advv / advw; grid: x over 0..ni, y over 0..nj, z over k = 1..nk
-__global__ void __launch_bounds__(128) mom5_adv_kernel(MomArgs a) {
-    const int xx = blockIdx.x * 32 + threadIdx.x, yy = blockIdx.y * 4 + threadIdx.y, k = blockIdx.z + 1;
-    const int ni = a.ni, nj = a.nj, nk = a.nk, k0 = k - 1;
-    if (xx > ni || yy > nj) return;
-    // advu at face f = xx of row j = yy
+// ---------------------------------------------------------------------------
+// (3) advu / advv / advw.  A warp owns 32 x faces of one row of one component
+// and marches up a chunk of levels: each lane forms the x flux of one face
+// and takes the next face's from the lane above (31 points per 32 lanes, no
+// divergent edge), the upper vertical flux is carried down as the next
+// level's lower one and the column's six levels stay in registers; only the
+// two y fluxes of a point are formed apart.  The three components of a tile
+// are neighbouring CTAs (blockIdx.x % 3), so their shared mass fluxes meet in
+// L2.  Bound by instruction issue (the upwind selects on the half-rate ALU).
+// Measured on one B200, per launch at 640x768x80: 3.085 ms with a thread per
+// point forming all its fluxes, 1.596 here (32 warps an SM; 24 warps 1.775, 16
+// warps 1.889).
+// ---------------------------------------------------------------------------
+constexpr int kMomOut = 31;   // points a warp of 32 faces completes
+constexpr int kMomRows = 4;   // rows (independent warps) per CTA
+
+// vertical flux of u or v at Fortran face kf from levels kf-3 .. kf+2 (win)
+__device__ __forceinline__ float uv_z(const float win[6], float m, float c2, int kf, int nk) {
+#define Q(l) win[(l) - kf + 3]
+    float r;
+    if (kf == 2)
+        r = m >= 0.0f ? (1.0f - c2) * Q(1) + c2 * Q(2) : flx3(Q(3), Q(2), Q(1));
+    else if (kf == nk)
+        r = m >= 0.0f ? flx3(Q(kf - 2), Q(kf - 1), Q(kf)) : (1.0f - c2) * Q(kf - 1) + c2 * Q(kf);
+    else if (kf == 3)
+        r = m >= 0.0f ? flx3(Q(1), Q(2), Q(3)) : flx5(Q(5), Q(4), Q(3), Q(2), Q(1));
+    else if (kf == nk - 1)
+        r = m >= 0.0f ? flx5(Q(kf - 3), Q(kf - 2), Q(kf - 1), Q(kf), Q(kf + 1)) : flx3(Q(kf + 1), Q(kf), Q(kf - 1));
+    else
+        return up5(m, Q(kf - 3), Q(kf - 2), Q(kf - 1), Q(kf), Q(kf + 1), Q(kf + 2));
+#undef Q
+    return m * r;
+}
+
+// vertical flux of w at mass level k from levels k-2 .. k+3 (win)
+__device__ __forceinline__ float w_z(const float win[6], float m, int k, int nk) {
+#define Q(l) win[(l) - k + 2]
+    float r;
+    if (k == 1)
+        r = m >= 0.0f ? 0.5f * (Q(1) + Q(2)) : flx3(Q(3), Q(2), Q(1));
+    else if (k == 2)
+        r = m >= 0.0f ? flx3(Q(1), Q(2), Q(3)) : flx5(Q(5), Q(4), Q(3), Q(2), Q(1));
+    else if (k == nk - 1)
+        r = m >= 0.0f ? flx5(Q(k - 2), Q(k - 1), Q(k), Q(k + 1), Q(k + 2)) : flx3(Q(k + 2), Q(k + 1), Q(k));
+    else if (k == nk)
+        r = m >= 0.0f ? flx3(Q(k - 1), Q(k), Q(k + 1)) : 0.5f * (Q(k) + Q(k + 1));
+    else
+        return up5(m, Q(k - 2), Q(k - 1), Q(k), Q(k + 1), Q(k + 2), Q(k + 3));
+#undef Q
+    return m * r;
+}
+
+// six points of a row (the two upwind stencils of a face) around p[0], and
+// the seven of a column of row stride sy (both faces of a point); the centre
+// is the column window's
+__device__ __forceinline__ void row6(const float *p, float c, float q[6]) {
+#pragma unroll
+    for (int e = 0; e < 6; ++e) q[e] = e == 3 ? c : __ldg(p + (e - 3));
+}
+__device__ __forceinline__ void col7(const float *p, int sy, float c, float q[7]) {
+#pragma unroll
+    for (int e = 0; e < 7; ++e) q[e] = e == 3 ? c : __ldg(p + (e - 3) * sy);
+}
+__device__ __forceinline__ float below(float v) { return __shfl_down_sync(0xffffffffu, v, 1); }  // the next face's
+__device__ __forceinline__ void shift(float win[6], float next) {
+#pragma unroll
+    for (int q = 0; q < 5; ++q) win[q] = win[q + 1];
+    win[5] = next;
+}
+
+// advu at the faces f of row j
+__device__ __forceinline__ void march_u(const MomArgs &a, int tile, int j, int k_lo, int k_hi) {
+    const int ni = a.ni, nj = a.nj, nk = a.nk, lane = threadIdx.x;
+    if (j >= nj) return;
     const int ff = a.per[0] ? 0 : 1, lf = a.per[1] ? ni : ni - 1;
-    if (yy < nj && xx >= ff && xx <= lf) {
-        const int j = yy, f = xx, y = j + G, x = f + G, west = cxw(a, f - 1), east = cxw(a, f);
-        const float advx = -(u_fx(a, k, j, f) - u_fx(a, k, j, f - 1)) * a.rdx;
-        float advy = -(u_fy(a, k, j + 1, f) - u_fy(a, k, j, f)) * a.rdy;
-        const float uc = LU(k, y, x);
-        if (j == 0 && a.opn[2]) {
-            const float m = RV(k, G, east + G) + RV(k, G, west + G);
-            if (m >= 0.0f) {
-                const float corr = (RV(k, G + 1, west + G) - RV(k, G, west + G)) + (RV(k, G + 1, east + G) - RV(k, G, east + G));
-                advy = advy - bcorr(a, uc * 0.5f, corr, a.rdy, __ldg(a.vh + y));
-            }
-        } else if (j == nj - 1 && a.opn[3]) {
-            const float m = RV(k, G + nj, east + G) + RV(k, G + nj, west + G);
-            if (m <= 0.0f) {
-                const float corr = (RV(k, y + 1, west + G) - RV(k, y, west + G)) + (RV(k, y + 1, east + G) - RV(k, y, east + G));
-                advy = advy - bcorr(a, uc * 0.5f, corr, a.rdy, __ldg(a.vh + y));
-            }
-        }
-        float advz;
-        if (k == 1) advz = zmass(a, -uv_z(a, true, 2, j, f), k);
-        else if (k == nk) advz = zmass(a, uv_z(a, true, nk, j, f), k);
-        else advz = zmass(a, -(uv_z(a, true, k + 1, j, f) - uv_z(a, true, k, j, f)), k);
-        float total = (advx + advy) + advz;
-        total = total + uc * (0.5f * (a.divx[ic(a, k0, j, east)] + a.divx[ic(a, k0, j, west)]));
-        const float scale = a.vmode == 2 ? __ldg(a.rr0 + ic(a, k0, 0, 0))
-                                         : __ldg(a.gzu + (size_t)j * (ni + 1) + f) /
-                                               (0.5f * (__ldg(a.rho0 + ic(a, k0, j, west)) + __ldg(a.rho0 + ic(a, k0, j, east))));
-        const unsigned p = iu(a, k, y, x);
-        a.uten[p] = a.uten[p] + total * scale;
+    if (ff + tile * kMomOut > lf) return;
+    const int f = min(ff + tile * kMomOut + lane, lf + 1);  // the flux u_fx(f - 1)
+    const bool own = lane < kMomOut && ff + tile * kMomOut + lane <= lf;
+    const int ux = ni + 1 + 2 * G, sx = ni + 2 * G, uz = (nj + 2 * G) * ux, vz = (nj + 1 + 2 * G) * sx,
+              wz = (nj + 2 * G) * sx, cz = ni * nj;
+    const int y = j + G, o = y * ux + f + G;
+    const int ra = y * ux + fxw(a, f - 1) + G, rb = y * ux + fxw(a, f) + G;
+    const int e = cxw(a, f), w = cxw(a, f - 1);
+    const int se = y * sx + e + G, sw = y * sx + w + G;          // rrv / rrw columns east and west of the face
+    const int ce = j * ni + clampn(e, ni), cw = j * ni + clampn(w, ni);  // divx and rho0
+    const int c2e = j * ni + clampn(f, ni), c2w = j * ni + clampn(f - 1, ni);
+    const bool so = j == 0 && a.opn[2], no = j == nj - 1 && a.opn[3];
+    const float gzu = a.vmode == 2 ? 0.0f : __ldg(a.gzu + j * (ni + 1) + min(f, ni)), vh = __ldg(a.vh + y);
+    float win[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const int l = k_lo - 3 + q;
+        win[q] = l >= 0 && l <= nk + 1 ? __ldg(a.u3d + l * uz + o) : 0.0f;
     }
-    // advv at face g = yy of column i = xx
+    auto c2f = [&](int kf) {
+        return kf == 2 || kf == nk ? 0.5f * (__ldg(a.c2 + (kf - 1) * cz + c2w) + __ldg(a.c2 + (kf - 1) * cz + c2e)) : 0.0f;
+    };
+    float zlo = 0.0f;
+    if (k_lo >= 2)
+        zlo = uv_z(win, 0.5f * (__ldg(a.rrw + k_lo * wz + se) + __ldg(a.rrw + k_lo * wz + sw)), c2f(k_lo), k_lo, nk);
+#pragma unroll 1
+    for (int k = k_lo; k <= k_hi; ++k) {
+        const float *pt = a.u3d + k * uz + o;
+        const float uc = win[3];
+        float px[6], py[7];
+        row6(pt, uc, px);
+        col7(pt, ux, uc, py);
+        const float next = k + 3 <= nk + 1 ? __ldg(pt + 3 * uz) : 0.0f;
+        const float ma = __ldg(a.rru + k * uz + ra), mb = __ldg(a.rru + k * uz + rb);
+        const float *rv = a.rrv + k * vz;
+        const float vse = __ldg(rv + se), vsw = __ldg(rv + sw), vne = __ldg(rv + se + sx), vnw = __ldg(rv + sw + sx);
+        float mz = 0.0f, c2 = 0.0f;
+        if (k < nk) {
+            mz = 0.5f * (__ldg(a.rrw + (k + 1) * wz + se) + __ldg(a.rrw + (k + 1) * wz + sw));
+            c2 = c2f(k + 1);
+        }
+        const float de = __ldg(a.divx + (k - 1) * cz + ce), dw = __ldg(a.divx + (k - 1) * cz + cw);
+        float *out = a.uten + k * uz + o;
+        const float ten = own ? *out : 0.0f;
+        const float scale = a.vmode == 2 ? __ldg(a.rr0 + (k - 1) * cz)
+                                         : gzu / (0.5f * (__ldg(a.rho0 + (k - 1) * cz + cw) + __ldg(a.rho0 + (k - 1) * cz + ce)));
+        const float fw = up5(0.5f * (ma + mb), px[0], px[1], px[2], px[3], px[4], px[5]);
+        const float fe = below(fw);
+        const float ms = vse + vsw, mn = vne + vnw;
+        const float fs0 = up5(0.5f * ms, py[0], py[1], py[2], py[3], py[4], py[5]);
+        const float fn0 = up5(0.5f * mn, py[1], py[2], py[3], py[4], py[5], py[6]);
+        // inflow through an open side's face takes the inner neighbour's flux
+        const bool sub_s = so && ms >= 0.0f, sub_n = no && mn <= 0.0f;
+        const float fs = sub_s ? fn0 : fs0, fn = sub_n ? fs0 : fn0;
+        shift(win, next);
+        const float zhi = k < nk ? uv_z(win, mz, c2, k + 1, nk) : 0.0f;
+        const float advx = -(fe - fw) * a.rdx;
+        float advy = -(fn - fs) * a.rdy;
+        if (sub_s || sub_n) {
+            const float corr = (vnw - vsw) + (vne - vse);
+            advy = advy - bcorr(a, uc * 0.5f, corr, a.rdy, vh);
+        }
+        const float advz = zmass(a, k == 1 ? -zhi : k == nk ? zlo : -(zhi - zlo), k);
+        float total = (advx + advy) + advz;
+        total = total + uc * (0.5f * (de + dw));
+        if (own) *out = ten + total * scale;
+        zlo = zhi;
+    }
+}
+
+// advv at the faces g of rows, columns i
+__device__ __forceinline__ void march_v(const MomArgs &a, int tile, int g, int k_lo, int k_hi) {
+    const int ni = a.ni, nj = a.nj, nk = a.nk, lane = threadIdx.x;
     const int fr = a.per[2] ? 0 : 1, lr = a.per[3] ? nj : nj - 1;
-    if (xx < ni && yy >= fr && yy <= lr) {
-        const int g = yy, i = xx, y = g + G, x = i + G, south = cyw(a, g - 1), north = cyw(a, g);
-        float advx = -(v_fx(a, k, g, i + 1) - v_fx(a, k, g, i)) * a.rdx;
-        const float advy = -(v_fy(a, k, g, i) - v_fy(a, k, g - 1, i)) * a.rdy;
-        const float vc = LV(k, y, x);
-        if (i == 0 && a.opn[0]) {
-            const float m = RU(k, north + G, G) + RU(k, south + G, G);
-            if (m >= 0.0f) {
-                const float corr = (RU(k, south + G, G + 1) - RU(k, south + G, G)) + (RU(k, north + G, G + 1) - RU(k, north + G, G));
-                advx = advx - bcorr(a, vc * 0.5f, corr, a.rdx, __ldg(a.uh + G));
-            }
-        } else if (i == ni - 1 && a.opn[1]) {
-            const float m = RU(k, north + G, G + ni) + RU(k, south + G, G + ni);
-            if (m <= 0.0f) {
-                const float corr = (RU(k, south + G, x + 1) - RU(k, south + G, x)) + (RU(k, north + G, x + 1) - RU(k, north + G, x));
-                advx = advx - bcorr(a, vc * 0.5f, corr, a.rdx, __ldg(a.uh + x));
-            }
-        }
-        float advz;
-        if (k == 1) advz = zmass(a, -uv_z(a, false, 2, g, i), k);
-        else if (k == nk) advz = zmass(a, uv_z(a, false, nk, g, i), k);
-        else advz = zmass(a, -(uv_z(a, false, k + 1, g, i) - uv_z(a, false, k, g, i)), k);
-        float total = (advx + advy) + advz;
-        total = total + vc * (0.5f * (a.divx[ic(a, k0, north, i)] + a.divx[ic(a, k0, south, i)]));
-        const float scale = a.vmode == 2 ? __ldg(a.rr0 + ic(a, k0, 0, 0))
-                                         : __ldg(a.gzv + (size_t)g * ni + i) /
-                                               (0.5f * (__ldg(a.rho0 + ic(a, k0, south, i)) + __ldg(a.rho0 + ic(a, k0, north, i))));
-        const unsigned p = iv(a, k, y, x);
-        a.vten[p] = a.vten[p] + total * scale;
+    if (g < fr || g > lr || tile * kMomOut >= ni) return;
+    const int i0 = tile * kMomOut + lane, i = min(i0, ni);  // the flux v_fx(i)
+    const bool own = lane < kMomOut && i0 < ni;
+    const int ux = ni + 1 + 2 * G, sx = ni + 2 * G, uz = (nj + 2 * G) * ux, vz = (nj + 1 + 2 * G) * sx,
+              wz = (nj + 2 * G) * sx, cz = ni * nj;
+    const int y = g + G, x = i + G, o = y * sx + x;
+    const int north = cyw(a, g), south = cyw(a, g - 1);
+    const int un = (north + G) * ux + x, us = (south + G) * ux + x;
+    const int rs = (fyw(a, g - 1) + G) * sx + x, rc = (fyw(a, g) + G) * sx + x, rn = (fyw(a, g + 1) + G) * sx + x;
+    const int sn = (north + G) * sx + x, ss = (south + G) * sx + x;  // rrw
+    const int ic0 = min(i, ni - 1);
+    const int cn = clampn(north, nj) * ni + ic0, cs = clampn(south, nj) * ni + ic0;
+    const int c2n = clampn(g, nj) * ni + ic0, c2s = clampn(g - 1, nj) * ni + ic0;
+    const bool wo = i == 0 && a.opn[0], eo = i == ni - 1 && a.opn[1];
+    const float gzv = a.vmode == 2 ? 0.0f : __ldg(a.gzv + g * ni + ic0), uh = __ldg(a.uh + x);
+    float win[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const int l = k_lo - 3 + q;
+        win[q] = l >= 0 && l <= nk + 1 ? __ldg(a.v3d + l * vz + o) : 0.0f;
     }
-    // advw at Fortran face kf = k + 1 (2..nk) of column (yy, xx)
-    if (xx < ni && yy < nj && k < nk) {
-        const int kf = k + 1, j = yy, i = xx, y = j + G, x = i + G;
-        const float dfx = -(w_fx(a, kf, j, i + 1) - w_fx(a, kf, j, i)), dfy = -(w_fy(a, kf, j + 1, i) - w_fy(a, kf, j, i));
-        float advx = a.vmode == 2 ? (dfx * a.rdx) * __ldg(a.uh + x) : dfx * (a.rdx * __ldg(a.uh + x));
-        float advy = a.vmode == 2 ? (dfy * a.rdy) * __ldg(a.vh + y) : dfy * (a.rdy * __ldg(a.vh + y));
-        const float c2 = __ldg(a.c2 + ic(a, kf - 1, j, i)), c1 = 1.0f - c2;
-        const float wc = LW(kf, y, x);
-        if (i == 0 && a.opn[0]) {
-            const float m = c2 * RU(kf, y, G) + c1 * RU(kf - 1, y, G);
-            if (m >= 0.0f) {
-                const float corr = c1 * (RU(kf - 1, y, G + 1) - RU(kf - 1, y, G)) + c2 * (RU(kf, y, G + 1) - RU(kf, y, G));
-                advx = advx - bcorr(a, wc, corr, a.rdx, __ldg(a.uh + x));
-            }
-        } else if (i == ni - 1 && a.opn[1]) {
-            const float m = c2 * RU(kf, y, G + ni) + c1 * RU(kf - 1, y, G + ni);
-            if (m <= 0.0f) {
-                const float corr = c1 * (RU(kf - 1, y, x + 1) - RU(kf - 1, y, x)) + c2 * (RU(kf, y, x + 1) - RU(kf, y, x));
-                advx = advx - bcorr(a, wc, corr, a.rdx, __ldg(a.uh + x));
-            }
+    auto c2f = [&](int kf) {
+        return kf == 2 || kf == nk ? 0.5f * (__ldg(a.c2 + (kf - 1) * cz + c2s) + __ldg(a.c2 + (kf - 1) * cz + c2n)) : 0.0f;
+    };
+    float zlo = 0.0f;
+    if (k_lo >= 2)
+        zlo = uv_z(win, 0.5f * (__ldg(a.rrw + k_lo * wz + sn) + __ldg(a.rrw + k_lo * wz + ss)), c2f(k_lo), k_lo, nk);
+#pragma unroll 1
+    for (int k = k_lo; k <= k_hi; ++k) {
+        const float *pt = a.v3d + k * vz + o;
+        const float vc = win[3];
+        float px[6], py[7];
+        row6(pt, vc, px);
+        col7(pt, sx, vc, py);
+        const float next = k + 3 <= nk + 1 ? __ldg(pt + 3 * vz) : 0.0f;
+        const float uN = __ldg(a.rru + k * uz + un), uS = __ldg(a.rru + k * uz + us);
+        const float *rv = a.rrv + k * vz;
+        const float ma = __ldg(rv + rs), mb = __ldg(rv + rc), mc = __ldg(rv + rn);
+        float mz = 0.0f, c2 = 0.0f;
+        if (k < nk) {
+            mz = 0.5f * (__ldg(a.rrw + (k + 1) * wz + sn) + __ldg(a.rrw + (k + 1) * wz + ss));
+            c2 = c2f(k + 1);
         }
-        if (j == 0 && a.opn[2]) {
-            const float m = c2 * RV(kf, G, x) + c1 * RV(kf - 1, G, x);
-            if (m >= 0.0f) {
-                const float corr = c1 * (RV(kf - 1, G + 1, x) - RV(kf - 1, G, x)) + c2 * (RV(kf, G + 1, x) - RV(kf, G, x));
-                advy = advy - bcorr(a, wc, corr, a.rdy, __ldg(a.vh + y));
-            }
-        } else if (j == nj - 1 && a.opn[3]) {
-            const float m = c2 * RV(kf, G + nj, x) + c1 * RV(kf - 1, G + nj, x);
-            if (m <= 0.0f) {
-                const float corr = c1 * (RV(kf - 1, y + 1, x) - RV(kf - 1, y, x)) + c2 * (RV(kf, y + 1, x) - RV(kf, y, x));
-                advy = advy - bcorr(a, wc, corr, a.rdy, __ldg(a.vh + y));
-            }
+        const float dn = __ldg(a.divx + (k - 1) * cz + cn), ds = __ldg(a.divx + (k - 1) * cz + cs);
+        float *out = a.vten + k * vz + o;
+        const float ten = own ? *out : 0.0f;
+        const float scale = a.vmode == 2 ? __ldg(a.rr0 + (k - 1) * cz)
+                                         : gzv / (0.5f * (__ldg(a.rho0 + (k - 1) * cz + cs) + __ldg(a.rho0 + (k - 1) * cz + cn)));
+        const float mw = uN + uS;
+        const float fw0 = up5(0.5f * mw, px[0], px[1], px[2], px[3], px[4], px[5]);
+        const float fe0 = below(fw0), me = below(mw), uNe = below(uN), uSe = below(uS);
+        const bool sub_w = wo && mw >= 0.0f, sub_e = eo && me <= 0.0f;
+        const float fw = sub_w ? fe0 : fw0, fe = sub_e ? fw0 : fe0;
+        const float fs = up5(0.5f * (ma + mb), py[0], py[1], py[2], py[3], py[4], py[5]);
+        const float fn = up5(0.5f * (mb + mc), py[1], py[2], py[3], py[4], py[5], py[6]);
+        shift(win, next);
+        const float zhi = k < nk ? uv_z(win, mz, c2, k + 1, nk) : 0.0f;
+        float advx = -(fe - fw) * a.rdx;
+        const float advy = -(fn - fs) * a.rdy;
+        if (sub_w || sub_e) {
+            const float corr = (uSe - uS) + (uNe - uN);
+            advx = advx - bcorr(a, vc * 0.5f, corr, a.rdx, uh);
         }
-        const float advz = zface(a, -(w_z(a, kf, j, i) - w_z(a, kf - 1, j, i)), kf);
+        const float advz = zmass(a, k == 1 ? -zhi : k == nk ? zlo : -(zhi - zlo), k);
         float total = (advx + advy) + advz;
-        total = total + wc * (c2 * a.divx[ic(a, kf - 1, j, i)] + c1 * a.divx[ic(a, kf - 2, j, i)]);
-        const float scale = a.vmode == 2 ? __ldg(a.rrf0 + ic(a, kf - 1, 0, 0))
-                                         : __ldg(a.rrf0 + ic(a, kf - 1, j, i)) * __ldg(a.gz + (size_t)j * ni + i);
-        const unsigned p = iw(a, kf, y, x);
-        a.wten[p] = a.wten[p] + total * scale;
+        total = total + vc * (0.5f * (dn + ds));
+        if (own) *out = ten + total * scale;
+        zlo = zhi;
     }
+}
+
+// advw at the w levels kf = k + 1 (2..nk) of row j, columns i
+__device__ __forceinline__ void march_w(const MomArgs &a, int tile, int j, int k_lo, int k_hi) {
+    const int ni = a.ni, nj = a.nj, nk = a.nk, lane = threadIdx.x;
+    if (j >= nj || tile * kMomOut >= ni || k_lo >= nk) return;
+    const int i0 = tile * kMomOut + lane, i = min(i0, ni);  // the flux w_fx(i)
+    const bool own = lane < kMomOut && i0 < ni;
+    const int ux = ni + 1 + 2 * G, sx = ni + 2 * G, uz = (nj + 2 * G) * ux, vz = (nj + 1 + 2 * G) * sx,
+              wz = (nj + 2 * G) * sx, cz = ni * nj;
+    const int y = j + G, x = i + G, o = y * sx + x, ou = y * ux + x;
+    const int ic0 = min(i, ni - 1), cc = j * ni + ic0;
+    const int cw = j * ni + clampn(i - 1, ni), ce = j * ni + clampn(i, ni);
+    const int cs = clampn(j - 1, nj) * ni + ic0, cn = clampn(j + 1, nj) * ni + ic0;
+    const bool wo = i == 0 && a.opn[0], eo = i == ni - 1 && a.opn[1];
+    const bool so = j == 0 && a.opn[2], no = j == nj - 1 && a.opn[3];
+    const float uh = __ldg(a.uh + min(x, ni + 2 * G - 1)), vh = __ldg(a.vh + y);
+    const float gz = a.vmode == 2 ? 0.0f : __ldg(a.gz + cc);
+    float win[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const int l = k_lo - 2 + q;
+        win[q] = l >= 0 && l <= nk + 2 ? __ldg(a.w3d + l * wz + o) : 0.0f;
+    }
+    float rw = __ldg(a.rrw + (k_lo + 1) * wz + o);  // rrw(kf)
+    float zlo = w_z(win, 0.5f * (__ldg(a.rrw + k_lo * wz + o) + rw), k_lo, nk);
+    float rul = __ldg(a.rru + k_lo * uz + ou), rsl = __ldg(a.rrv + k_lo * vz + o), rnl = __ldg(a.rrv + k_lo * vz + o + sx);
+    float dl = __ldg(a.divx + (k_lo - 1) * cz + cc);
+#pragma unroll 1
+    for (int k = k_lo; k <= k_hi && k < nk; ++k) {
+        const int kf = k + 1;
+        const float *pt = a.w3d + kf * wz + o;
+        const float wc = win[3];  // the window still ends at kf + 2
+        float px[6], py[7];
+        row6(pt, wc, px);
+        col7(pt, sx, wc, py);
+        const float next = kf + 3 <= nk + 2 ? __ldg(pt + 3 * wz) : 0.0f;
+        const float *c2p = a.c2 + (kf - 1) * cz;
+        const float kw = __ldg(c2p + cw), ke = __ldg(c2p + ce), ks = __ldg(c2p + cs), kn = __ldg(c2p + cn), c2 = __ldg(c2p + cc);
+        const float ru = __ldg(a.rru + kf * uz + ou), rs = __ldg(a.rrv + kf * vz + o), rn = __ldg(a.rrv + kf * vz + o + sx);
+        const float rwn = __ldg(a.rrw + (kf + 1) * wz + o), dh = __ldg(a.divx + (kf - 1) * cz + cc);
+        float *out = a.wten + kf * wz + o;
+        const float ten = own ? *out : 0.0f;
+        const float scale = a.vmode == 2 ? __ldg(a.rrf0 + (kf - 1) * cz) : __ldg(a.rrf0 + (kf - 1) * cz + cc) * gz;
+        const float c1 = 1.0f - c2;
+        const float c2x = 0.5f * (kw + ke), c2s = 0.5f * (ks + c2), c2n = 0.5f * (c2 + kn);
+        const float mw = c2x * ru + (1.0f - c2x) * rul;
+        const float ms = c2s * rs + (1.0f - c2s) * rsl, mn = c2n * rn + (1.0f - c2n) * rnl;
+        const float fw0 = up5(mw, px[0], px[1], px[2], px[3], px[4], px[5]);
+        const float fe0 = below(fw0), me = below(mw), rue = below(ru), rule = below(rul);
+        const float fs0 = up5(ms, py[0], py[1], py[2], py[3], py[4], py[5]);
+        const float fn0 = up5(mn, py[1], py[2], py[3], py[4], py[5], py[6]);
+        const float fw = wo && mw >= 0.0f ? fe0 : fw0, fe = eo && me <= 0.0f ? fw0 : fe0;
+        const float fs = so && ms >= 0.0f ? fn0 : fs0, fn = no && mn <= 0.0f ? fs0 : fn0;
+        shift(win, next);
+        const float zhi = w_z(win, 0.5f * (rw + rwn), kf, nk);
+        const float dfx = -(fe - fw), dfy = -(fn - fs);
+        float advx = a.vmode == 2 ? (dfx * a.rdx) * uh : dfx * (a.rdx * uh);
+        float advy = a.vmode == 2 ? (dfy * a.rdy) * vh : dfy * (a.rdy * vh);
+        // the open sides' corrections weigh with the cell's own c2
+        if ((wo && c2 * ru + c1 * rul >= 0.0f) || (eo && c2 * rue + c1 * rule <= 0.0f)) {
+            const float corr = c1 * (rule - rul) + c2 * (rue - ru);
+            advx = advx - bcorr(a, wc, corr, a.rdx, uh);
+        }
+        if ((so && c2 * rs + c1 * rsl >= 0.0f) || (no && c2 * rn + c1 * rnl <= 0.0f)) {
+            const float corr = c1 * (rnl - rsl) + c2 * (rn - rs);
+            advy = advy - bcorr(a, wc, corr, a.rdy, vh);
+        }
+        const float advz = zface(a, -(zhi - zlo), kf);
+        float total = (advx + advy) + advz;
+        total = total + wc * (c2 * dh + c1 * dl);
+        if (own) *out = ten + total * scale;
+        zlo = zhi, rw = rwn, rul = ru, rsl = rs, rnl = rn, dl = dh;
+    }
+}
+
+__global__ void __launch_bounds__(32 * kMomRows, 8) mom5_adv_kernel(MomArgs a, int levels_per_chunk) {
+    // all tiles in one grid dimension, which takes any plane
+    const int tiles = a.ni / kMomOut + 1, bt = blockIdx.x / 3;
+    const int tile = bt % tiles, row = bt / tiles * kMomRows + threadIdx.y;
+    const int k_lo = 1 + blockIdx.y * levels_per_chunk, k_hi = min(a.nk, k_lo + levels_per_chunk - 1);
+    const int component = blockIdx.x % 3;
+    if (component == 0)
+        march_u(a, tile, row, k_lo, k_hi);
+    else if (component == 1)
+        march_v(a, tile, row, k_lo, k_hi);
+    else
+        march_w(a, tile, row, k_lo, k_hi);
 }
 
 bool launch_ok(const char *what) {
@@ -514,9 +580,14 @@ int enqueue_mass(const MomArgs &a, cudaStream_t st) {
 }
 
 int enqueue_transport(const MomArgs &a, cudaStream_t st) {
-    const dim3 g_face((a.ni + 1 + 31) / 32, (a.nj + 1 + 3) / 4, a.nk);
+    const int tiles = a.ni / kMomOut + 1, ytiles = (a.nj + 1 + kMomRows - 1) / kMomRows;
+    // long chunks re-load and re-form less (each starts with six window loads
+    // and its lower flux), short ones give a small plane warps enough: halve
+    // until two rounds of 24 warps on each of 148 SMs, or four levels, are left
+    int chunk = a.nk;
+    while (chunk > 4 && 3LL * tiles * (a.nj + 1) * ((a.nk + chunk - 1) / chunk) < 2LL * 148 * 24) chunk = (chunk + 1) / 2;
     ProfScope ps("mom5_adv_kernel", st);
-    mom5_adv_kernel<<<g_face, dim3(32, 4), 0, st>>>(a);
+    mom5_adv_kernel<<<dim3(3 * tiles * ytiles, (a.nk + chunk - 1) / chunk), dim3(32, kMomRows), 0, st>>>(a, chunk);
     ps.stop();
     return launch_ok("mom5_adv_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }

@@ -95,3 +95,20 @@ def test_scalar_advection(ni, nj, nk, chunk, nrk):
         d["scalar"], {k: d[k] for k in ("rru", "rrv", "rrw")}, {k: d[k] for k in ("c1", "c2", "rr0", "gz")}, d["divx"],
         d["tendency"], {q: d["flux_" + q] for q in "xyz"}, lateral_sides=(2, 2, 2, 2), levels_per_chunk=chunk, **kw)
     assert _differ(d, h, ("tendency", "flux_x", "flux_y", "flux_z")) == []
+
+
+@pytest.mark.parametrize("sides", [(2, 2, 2, 2), (1, 1, 1, 1)])
+@pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (32, 9, 10), (62, 11, 13), (63, 12, 33)])
+def test_momentum_advection(ni, nj, nk, sides):
+    from gm1_b200 import momentum as mom
+    from oracle import momentum as orc
+    from tests.golden.make_golden import momentum_fixture
+    from tests.test_oracle_momentum import OUTS
+
+    a, m, _ = momentum_fixture(ni, nj, nk, 7 * ni + nk)
+    kw = dict(ni=ni, nj=nj, nk=nk, dx=500.0, dy=450.0, dz=150.0, lateral_sides=sides)
+    dev = _dev({**a, **m})
+    out = mom.launch_cuda_terrain_open_momentum_advection5(dev, dev, nrk=1, **kw)
+    ref = {**a, **m, "divx": np.zeros((nk, nj, ni), np.float32)}
+    orc.momentum_advection5(ref, **kw)
+    assert _differ({**dev, "divx": out.divx}, ref, OUTS) == []
