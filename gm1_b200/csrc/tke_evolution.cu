@@ -18,8 +18,9 @@
 //    and 32 x 5 per level) in shared memory, so every face flux is formed
 //    once, and each cell adds its horizontal divergence and vertical
 //    diffusion to tketen.  No device scratch.
-//  * an RK stage is elementwise over the face levels: each cell forms its six
-//    face fluxes (fifth order, WENO5 at nrk = 3) from the stage-start field.
+//  * an RK stage marches warps of 32 x faces up the face levels: each x and
+//    vertical face flux (fifth order, WENO5 at nrk = 3) is formed once, from
+//    the stage-start field.
 //  * binary32 one operation at a time in the reference's order, binary64
 //    WENO weights: word-identical to the reference twin.
 #include "gm1b_common.cuh"
@@ -362,78 +363,26 @@ __global__ void __launch_bounds__(kTT) tke_turbt_flat_kernel(TkeArgs a, float dt
 }
 
 // ------------------------------------------------------------- RK stage
-__device__ __forceinline__ float rru_at(const TkeArgs &a, int k, int j, int f) {
-    return a.rru[((unsigned)k * (unsigned)(a.nj + 2 * kG) + (unsigned)(j + kG)) * (unsigned)(a.ni + 1 + 2 * kG) +
-                 (unsigned)(f + kG)];
-}
-__device__ __forceinline__ float rrv_at(const TkeArgs &a, int k, int f, int i) {
-    return a.rrv[((unsigned)k * (unsigned)(a.nj + 1 + 2 * kG) + (unsigned)(f + kG)) * (unsigned)(a.ni + 2 * kG) +
-                 (unsigned)(i + kG)];
-}
-__device__ __forceinline__ float rrw_at(const TkeArgs &a, int k, int j, int i) {
-    return a.rrw[((unsigned)k * (unsigned)(a.nj + 2 * kG) + (unsigned)(j + kG)) * (unsigned)(a.ni + 2 * kG) +
-                 (unsigned)(i + kG)];
-}
-
-// mass flux through x face `face` of row j (axis 0) or y face `face` of
-// column `row` (axis 1) at face level f
-__device__ __forceinline__ float face_mass(const TkeArgs &a, int axis, int f, int row, int face) {
-    if (axis == 0) {
-        const float c2 = 0.5f * (cellc(a, a.c2, f, row, face - 1) + cellc(a, a.c2, f, row, face));
-        return c2 * rru_at(a, f + 1, row, face) + (1.0f - c2) * rru_at(a, f, row, face);
-    }
-    const float c2 = 0.5f * (cellc(a, a.c2, f, face - 1, row) + cellc(a, a.c2, f, face, row));
-    return c2 * rrv_at(a, f + 1, face, row) + (1.0f - c2) * rrv_at(a, f, face, row);
-}
-
 template <bool W>
 __device__ __forceinline__ float rec5(float s1, float s2, float s3, float s4, float s5, double eps) {
     if (W) return weno5(s1, s2, s3, s4, s5, eps);
     return flx5(s1, s2, s3, s4, s5);
 }
 
-// face flux with its own mass (no open-side substitution)
+// the upwind flux at a face from the six points around it: one reconstruction
+// of selected points, so a warp of mixed signs does not form both
 template <bool W>
-__device__ float face_flux_plain(const TkeArgs &a, const float *q, int axis, int f, int row, int face, double eps) {
-    const float m = face_mass(a, axis, f, row, face);
-    float v[5];
-    const int sgn = m >= 0.0f ? 1 : -1;
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {
-        const int off = sgn > 0 ? s - 3 : 2 - s;
-        v[s] = axis == 0 ? cellc(a, q, f, row, face + off) : cellc(a, q, f, face + off, row);
-    }
-    return m * rec5<W>(v[0], v[1], v[2], v[3], v[4], eps);
+__device__ __forceinline__ float up6(float m, float s0, float s1, float s2, float s3, float s4, float s5, double eps) {
+    const bool pos = m >= 0.0f;
+    return m * rec5<W>(pos ? s0 : s5, pos ? s1 : s4, pos ? s2 : s3, pos ? s3 : s2, pos ? s4 : s1, eps);
 }
 
-// face flux with the open-side substitution: inflow through the first face
-// (or the last face) takes the flux of its inner neighbour face; the mass
-// returned is the face's own
+// vertical flux at staggered index ks (cuda_tke_evolution.py:194-203) from
+// levels ks-3 .. ks+2 of the column (win)
 template <bool W>
-__device__ float face_flux(const TkeArgs &a, const float *q, int axis, int f, int row, int face, double eps,
-                           float *mass) {
-    const int n = axis == 0 ? a.ni : a.nj;
-    const float m = face_mass(a, axis, f, row, face);
-    *mass = m;
-    if (face == 0 && m >= 0.0f) return face_flux_plain<W>(a, q, axis, f, row, 1, eps);
-    if (face == n && m <= 0.0f) return face_flux_plain<W>(a, q, axis, f, row, n - 1, eps);
-    float v[5];
-    const int sgn = m >= 0.0f ? 1 : -1;
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {
-        const int off = sgn > 0 ? s - 3 : 2 - s;
-        v[s] = axis == 0 ? cellc(a, q, f, row, face + off) : cellc(a, q, f, face + off, row);
-    }
-    return m * rec5<W>(v[0], v[1], v[2], v[3], v[4], eps);
-}
-
-// vertical flux at staggered index ks (cuda_tke_evolution.py:194-203)
-template <bool W>
-__device__ float vert_flux(const TkeArgs &a, const float *q, int ks, int j, int i, double eps) {
-    const int nk = a.nk;
-    const float m = 0.5f * (rrw_at(a, ks, j, i) + rrw_at(a, ks + 1, j, i));
+__device__ __forceinline__ float vert_flux(const float win[6], float m, int ks, int nk, double eps) {
     const float wf = (float)eps;
-#define Q(k) q[f3(a, (k), j, i)]
+#define Q(k) win[(k) - ks + 3]
     float r;
     if (ks == 1) {
         r = m >= 0.0f ? 0.5f * (Q(0) + Q(1)) : (W ? upstrpd(Q(2), Q(1), Q(0), wf) : flx3(Q(2), Q(1), Q(0)));
@@ -444,86 +393,160 @@ __device__ float vert_flux(const TkeArgs &a, const float *q, int ks, int j, int 
         r = (W ? m > 0.0f : m >= 0.0f) ? rec5<W>(Q(ks - 3), Q(ks - 2), Q(ks - 1), Q(ks), Q(ks + 1), eps)
                                        : (W ? upstrpd(Q(ks + 1), Q(ks), Q(ks - 1), wf) : flx3(Q(ks + 1), Q(ks), Q(ks - 1)));
     } else if (ks == nk) {
-        r = (W ? m > 0.0f : m >= 0.0f) ? (W ? upstrpd(Q(nk - 2), Q(nk - 1), Q(nk), wf) : flx3(Q(nk - 2), Q(nk - 1), Q(nk)))
-                                       : 0.5f * (Q(nk - 1) + Q(nk));
-    } else if (m >= 0.0f) {
-        r = rec5<W>(Q(ks - 3), Q(ks - 2), Q(ks - 1), Q(ks), Q(ks + 1), eps);
+        r = (W ? m > 0.0f : m >= 0.0f) ? (W ? upstrpd(Q(ks - 2), Q(ks - 1), Q(ks), wf) : flx3(Q(ks - 2), Q(ks - 1), Q(ks)))
+                                       : 0.5f * (Q(ks - 1) + Q(ks));
     } else {
-        r = rec5<W>(Q(ks + 2), Q(ks + 1), Q(ks), Q(ks - 1), Q(ks - 2), eps);
+        return up6<W>(m, Q(ks - 3), Q(ks - 2), Q(ks - 1), Q(ks), Q(ks + 1), Q(ks + 2), eps);
     }
 #undef Q
     return m * r;
 }
 
-// grid: x over i, y over j, z over face level f = 0..nk; nxt2 optional.
+constexpr int kStageOut = 31;   // cells a warp of 32 x faces completes
+constexpr int kStageRows = 4;   // rows per CTA of the fifth-order stage, each independent
+constexpr int kStageWRows = 8;  // rows per CTA of the WENO stage: 8 rows of y faces complete 7 rows of cells
+
+// A warp owns the x faces i0 .. i0+31 of one row and marches up a chunk of
+// face levels: each lane forms the x flux of one face and takes the next
+// face's from the lane above, the upper vertical flux and the mass fluxes of
+// the level above are carried down, the column's six levels stay in
+// registers.  The fifth-order stage forms both y fluxes of a cell; the WENO
+// stage hands each to the row below through shared memory (one barrier a
+// level), the last row forming a flux only.  Columns beyond the open sides
+// repeat the edge ones.  Bound by instruction issue (fifth order) and the
+// binary64 weights (WENO); a step's three flat stages at 640x768x80 took 5.04 ms
+// with six fluxes per cell and take 2.87 here (24 warps an SM for WENO: 16
+// warps 1.787 ms a stage, 24 1.624).
 // FLAT: the flat column's advw (gm1_flat_tke_advw_rk_v1,
 // src/cm1core/cuda_gm1_flat_stretched_closure.py:401-449; adv.F:3252-3355
 // with terrain_flag=.false.): vertical divergence -(dumz(k)-dumz(k-1))*rdz
 // *mf(k), the column's c1/c2 in the divergence correction and its rrf0, the
 // open-side divergence piece (q*d)*rdx evaluated left to right, no gz.
 template <bool W, bool FLAT>
-__global__ void __launch_bounds__(128) tke_rk_stage_kernel(TkeArgs a, const float *__restrict__ cur,
-                                                           float *__restrict__ nxt, float *__restrict__ nxt2,
-                                                           float dttmp, double eps) {
-    // The x face fluxes pass to the next lane by warp shuffle and the y face
-    // fluxes to the next warp row through shared memory (the last lane or row
-    // forms its outer one itself): each face flux is formed once, by the same
-    // function of the same arguments.
-    __shared__ float s_fy[4][32], s_my[4][32];
-    const int lane = threadIdx.x, row = threadIdx.y;
-    const int i = blockIdx.x * 32 + lane, j = blockIdx.y * 4 + row, f = blockIdx.z;
+__global__ void __launch_bounds__(32 * (W ? kStageWRows : kStageRows), W ? 3 : 8)
+    tke_rk_stage_kernel(TkeArgs a, const float *__restrict__ cur, float *__restrict__ nxt, float *__restrict__ nxt2,
+                        int levels_per_chunk, float dttmp, double eps) {
+    constexpr int ROWS = W ? kStageWRows : kStageRows;
+    __shared__ float s_fy[W ? 2 : 1][W ? ROWS : 1][32], s_my[W ? 2 : 1][W ? ROWS : 1][32];
+    const int lane = threadIdx.x, ty = threadIdx.y;
     const int ni = a.ni, nj = a.nj, nk = a.nk;
-    const bool inner = f > 0 && f < nk;  // uniform over the block
-    float mw = 0.0f, me = 0.0f, ms = 0.0f, mn = 0.0f, fx0 = 0.0f, fx1 = 0.0f, fy0 = 0.0f, fy1 = 0.0f;
-    if (inner) {
-        if (j < nj && i <= ni) fx0 = face_flux<W>(a, cur, 0, f, j, i, eps, &mw);
-        fx1 = __shfl_down_sync(0xffffffffu, fx0, 1);
-        me = __shfl_down_sync(0xffffffffu, mw, 1);
-        if (lane == 31 && j < nj && i < ni) fx1 = face_flux<W>(a, cur, 0, f, j, i + 1, eps, &me);
-        if (i < ni && j <= nj) fy0 = face_flux<W>(a, cur, 1, f, i, j, eps, &ms);
-        s_fy[row][lane] = fy0;
-        s_my[row][lane] = ms;
+    const int ux = ni + 1 + 2 * kG, sx = ni + 2 * kG, uz = (nj + 2 * kG) * ux, vz = (nj + 1 + 2 * kG) * sx,
+              wz = (nj + 2 * kG) * sx, cz = ni * nj;
+    const int tiles = ni / kStageOut + 1;  // all tiles in one grid dimension, which takes any plane
+    const int i0 = blockIdx.x % tiles * kStageOut + lane, row = blockIdx.x / tiles * (W ? ROWS - 1 : ROWS) + ty;
+    if (!W && row >= nj) return;  // whole warps: the fifth-order stage has no barrier
+    // faces and rows past the domain repeat its last ones and store nothing
+    const int i = min(i0, ni), j = min(row, W ? nj : nj - 1);
+    const bool own = i0 < ni && row < nj && lane < kStageOut && (!W || ty < ROWS - 1);
+    const int jc = min(j, nj - 1), ic = min(i, ni - 1), cc = jc * ni + ic;
+    const int ou = (jc + kG) * ux + i + kG, ov = (j + kG) * sx + ic + kG, ow = (jc + kG) * sx + ic + kG;
+    int xo[6], yo[7];  // clamped columns and rows of the two stencils, as offsets in a level
+#pragma unroll
+    for (int q = 0; q < 6; ++q) xo[q] = jc * ni + clampi(i + q - 3, ni);
+#pragma unroll
+    for (int q = 0; q < 7; ++q) yo[q] = clampi(j + q - 3, nj) * ni + ic;
+    // window of the own column: levels f_lo-4 .. f_lo+1, shifted to f-3 .. f+2
+    const int f_lo = blockIdx.y * levels_per_chunk, f_hi = min(nk, f_lo + levels_per_chunk - 1);
+    if (f_lo == 0 && own) {
+        nxt[cc] = 0.0f;
+        if (nxt2) nxt2[cc] = 0.0f;
     }
-    __syncthreads();
-    if (inner && row < 3) {
-        fy1 = s_fy[row + 1][lane];
-        mn = s_my[row + 1][lane];
-    }
-    if (i >= ni || j >= nj) return;
-    const unsigned z = f3(a, f, j, i);
-    if (!inner) {
+    if (f_hi == nk && own) {
+        const unsigned z = (unsigned)nk * (unsigned)cz + (unsigned)cc;
         nxt[z] = 0.0f;
         if (nxt2) nxt2[z] = 0.0f;
-        return;
     }
-    if (row == 3) fy1 = face_flux<W>(a, cur, 1, f, i, j + 1, eps, &mn);
-    float ax = -1.0f * ((fx1 - fx0) * a.rdx);
-    float ay = -1.0f * ((fy1 - fy0) * a.rdy);
-    const float c2 = a.c2[z], c1 = 1.0f - c2;
-    const float q = cur[z];
-    if ((i == 0 && mw >= 0.0f) || (i == ni - 1 && me <= 0.0f)) {
-        const float du = c1 * (rru_at(a, f, j, i + 1) - rru_at(a, f, j, i)) +
-                         c2 * (rru_at(a, f + 1, j, i + 1) - rru_at(a, f + 1, j, i));
-        ax = FLAT ? ax - ((q * du) * a.rdx) : ax - q * (du * a.rdx);
+    const int k_lo = max(f_lo, 1), k_hi = min(f_hi, nk - 1);
+    if (k_lo > k_hi) return;  // the whole CTA
+    float win[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const int l = k_lo - 3 + q;
+        win[q] = l >= 0 && l <= nk ? cur[l * cz + cc] : 0.0f;
     }
-    if ((j == 0 && ms >= 0.0f) || (j == nj - 1 && mn <= 0.0f)) {
-        const float dv = c1 * (rrv_at(a, f, j + 1, i) - rrv_at(a, f, j, i)) +
-                         c2 * (rrv_at(a, f + 1, j + 1, i) - rrv_at(a, f + 1, j, i));
-        ay = FLAT ? ay - ((q * dv) * a.rdy) : ay - q * (dv * a.rdy);
+    float rw = __ldg(a.rrw + (k_lo + 1) * wz + ow);
+    float zlo = vert_flux<W>(win, 0.5f * (__ldg(a.rrw + k_lo * wz + ow) + rw), k_lo, nk, eps);
+    float rul = __ldg(a.rru + k_lo * uz + ou), rsl = __ldg(a.rrv + k_lo * vz + ov), rnl = 0.0f;
+    if (!W) rnl = __ldg(a.rrv + k_lo * vz + ov + sx);
+    float dl = __ldg(a.divx + (k_lo - 1) * cz + cc);
+    const float gz = FLAT ? 0.0f : __ldg(a.gz + cc);
+#pragma unroll 1
+    for (int f = k_lo; f <= k_hi; ++f) {
+        const float *lev = cur + f * cz;
+        const float q = win[3];
+        float px[6], py[7];
+#pragma unroll
+        for (int e = 0; e < 6; ++e) px[e] = __ldg(lev + xo[e]);
+#pragma unroll
+        for (int e = 0; e < 7; ++e) py[e] = W && e == 6 ? 0.0f : __ldg(lev + yo[e]);
+        const float next = f + 3 <= nk ? __ldg(lev + 3 * cz + cc) : 0.0f;
+        const float *c2p = a.c2 + f * cz;
+        const float kw = __ldg(c2p + xo[2]), ke = __ldg(c2p + xo[3]), ks = __ldg(c2p + yo[2]), kn = __ldg(c2p + yo[3]);
+        const float c2 = __ldg(c2p + cc);
+        const float ru = __ldg(a.rru + (f + 1) * uz + ou), rs = __ldg(a.rrv + (f + 1) * vz + ov);
+        const float rwn = __ldg(a.rrw + (f + 2) * wz + ow), dh = __ldg(a.divx + f * cz + cc);
+        const unsigned z = (unsigned)f * (unsigned)cz + (unsigned)cc;
+        const float base = a.tkea[z], ten = __ldg(a.tketen + z);
+        const float rrf = FLAT ? __ldg(a.rrf0 + f * cz) : __ldg(a.rrf0 + z);
+        const float c2x = 0.5f * (kw + ke), c2y = 0.5f * (ks + kn);
+        const float mw = c2x * ru + (1.0f - c2x) * rul, ms = c2y * rs + (1.0f - c2y) * rsl;
+        const float fx0 = up6<W>(mw, px[0], px[1], px[2], px[3], px[4], px[5], eps);
+        const float fy0 = up6<W>(ms, py[0], py[1], py[2], py[3], py[4], py[5], eps);
+        const float fx1 = __shfl_down_sync(0xffffffffu, fx0, 1), me = __shfl_down_sync(0xffffffffu, mw, 1);
+        const float rue = __shfl_down_sync(0xffffffffu, ru, 1), rule = __shfl_down_sync(0xffffffffu, rul, 1);
+        float fy1, mn, rn = 0.0f;
+        if (W) {
+            s_fy[f & 1][ty][lane] = fy0;
+            s_my[f & 1][ty][lane] = ms;
+            __syncthreads();
+            const int up = min(ty + 1, ROWS - 1);
+            fy1 = s_fy[f & 1][up][lane];
+            mn = s_my[f & 1][up][lane];
+        } else {
+            rn = __ldg(a.rrv + (f + 1) * vz + ov + sx);
+            const float c2n = 0.5f * (kn + __ldg(c2p + yo[4]));
+            mn = c2n * rn + (1.0f - c2n) * rnl;
+            fy1 = up6<W>(mn, py[1], py[2], py[3], py[4], py[5], py[6], eps);
+        }
+        // inflow through an open side's face takes the inner neighbour's flux
+        const bool sw = i == 0 && mw >= 0.0f, se = i == ni - 1 && me <= 0.0f;
+        const bool ss = j == 0 && ms >= 0.0f, sn = j == nj - 1 && mn <= 0.0f;
+        float ax = -1.0f * (((se ? fx0 : fx1) - (sw ? fx1 : fx0)) * a.rdx);
+        float ay = -1.0f * (((sn ? fy0 : fy1) - (ss ? fy1 : fy0)) * a.rdy);
+        const float c1 = 1.0f - c2;
+        if (sw || se) {
+            const float du = c1 * (rule - rul) + c2 * (rue - ru);
+            ax = FLAT ? ax - ((q * du) * a.rdx) : ax - q * (du * a.rdx);
+        }
+        if (ss || sn) {
+            if (W) {
+                rn = __ldg(a.rrv + (f + 1) * vz + ov + sx);
+                rnl = __ldg(a.rrv + f * vz + ov + sx);
+            }
+            const float dv = c1 * (rnl - rsl) + c2 * (rn - rs);
+            ay = FLAT ? ay - ((q * dv) * a.rdy) : ay - q * (dv * a.rdy);
+        }
+#pragma unroll
+        for (int e = 0; e < 5; ++e) win[e] = win[e + 1];
+        win[5] = next;
+        const float zhi = vert_flux<W>(win, 0.5f * (rw + rwn), f + 1, nk, eps);
+        const float dvf = zhi - zlo;
+        const float az = FLAT ? ((-dvf) * a.rdz) * __ldg(a.mfp + f + 1) : -1.0f * (dvf * a.rdz);
+        float total = (ax + ay) + az;
+        // the divergence correction: the flat text reads the column's c2 here
+        // (the open-side pieces above read the cell's)
+        const float c2d = FLAT ? __ldg(c2p) : c2, c1d = FLAT ? 1.0f - c2d : c1;
+        total = total + q * (c2d * dh + c1d * dl);
+        const float wten = FLAT ? ten + total * rrf : ten + total * (rrf * gz);
+        const float value = base + dttmp * wten;
+        if (own) {
+            const float out = value < 1e-10f ? 0.0f : value;
+            nxt[z] = out;
+            if (nxt2) nxt2[z] = out;
+        }
+        zlo = zhi, rw = rwn, rul = ru, rsl = rs, dl = dh;
+        if (!W) rnl = rn;
     }
-    const float dvf = vert_flux<W>(a, cur, f + 1, j, i, eps) - vert_flux<W>(a, cur, f, j, i, eps);
-    const float az = FLAT ? ((-dvf) * a.rdz) * a.mfp[f + 1] : -1.0f * (dvf * a.rdz);
-    float total = (ax + ay) + az;
-    // the divergence correction: the flat text reads the column's c2 here
-    // (the open-side pieces above read the cell's)
-    const float c2d = FLAT ? a.c2[f3(a, f, 0, 0)] : c2, c1d = FLAT ? 1.0f - c2d : c1;
-    total = total + q * (c2d * a.divx[f3(a, f, j, i)] + c1d * a.divx[f3(a, f - 1, j, i)]);
-    const float wten = FLAT ? a.tketen[z] + total * a.rrf0[f3(a, f, 0, 0)]
-                            : a.tketen[z] + total * (a.rrf0[z] * a.gz[(size_t)j * ni + i]);
-    const float value = a.tkea[z] + dttmp * wten;
-    const float out = value < 1e-10f ? 0.0f : value;
-    nxt[z] = out;
-    if (nxt2) nxt2[z] = out;
 }
 
 bool launch_ok(const char *what) {
@@ -623,30 +646,32 @@ int enqueue_diffusion(const TkeArgs &a, float dt, cudaStream_t st) {
     return launch_ok("tke_turbt_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }
 
+// Levels per chunk: long chunks re-load and re-form less (each starts with
+// six window loads and its lower flux), short ones give a small plane warps
+// enough: halve until two rounds of `warps` on each of 148 SMs, or four
+// levels, are left.
+int stage_chunk(const TkeArgs &a, int warps) {
+    const long long rows = (long long)(a.ni / kStageOut + 1) * a.nj;
+    int chunk = a.nk + 1;
+    while (chunk > 4 && rows * ((a.nk + chunk) / chunk) < 2LL * 148 * warps) chunk = (chunk + 1) / 2;
+    return chunk;
+}
+
+template <bool FLAT>
 int enqueue_stage(const TkeArgs &a, const float *cur, float *nxt, float *nxt2, int nrk, float dt, cudaStream_t st) {
     const float dttmp = dt / (float)(4 - nrk);
     const double eps = (double)(100.0f * 1e-18f);
-    const dim3 grid((a.ni + 31) / 32, (a.nj + 3) / 4, a.nk + 1), block(32, 4);
-    ProfScope ps("tke_rk_stage_kernel", st);
-    if (nrk == 3)
-        tke_rk_stage_kernel<true, false><<<grid, block, 0, st>>>(a, cur, nxt, nxt2, dttmp, eps);
+    const bool weno = nrk == 3;
+    const int rows = weno ? kStageWRows - 1 : kStageRows, chunk = stage_chunk(a, weno ? 16 : 24);
+    const dim3 grid((a.ni / kStageOut + 1) * ((a.nj + rows - 1) / rows), (a.nk + chunk) / chunk);
+    const char *name = FLAT ? "tke_rk_stage_flat_kernel" : "tke_rk_stage_kernel";
+    ProfScope ps(name, st);
+    if (weno)
+        tke_rk_stage_kernel<true, FLAT><<<grid, dim3(32, kStageWRows), 0, st>>>(a, cur, nxt, nxt2, chunk, dttmp, eps);
     else
-        tke_rk_stage_kernel<false, false><<<grid, block, 0, st>>>(a, cur, nxt, nxt2, dttmp, eps);
+        tke_rk_stage_kernel<false, FLAT><<<grid, dim3(32, kStageRows), 0, st>>>(a, cur, nxt, nxt2, chunk, dttmp, eps);
     ps.stop();
-    return launch_ok("tke_rk_stage_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
-}
-
-int enqueue_stage_flat(const TkeArgs &a, const float *cur, float *nxt, int nrk, float dt, cudaStream_t st) {
-    const float dttmp = dt / (float)(4 - nrk);
-    const double eps = (double)(100.0f * 1e-18f);
-    const dim3 grid((a.ni + 31) / 32, (a.nj + 3) / 4, a.nk + 1), block(32, 4);
-    ProfScope ps("tke_rk_stage_flat_kernel", st);
-    if (nrk == 3)
-        tke_rk_stage_kernel<true, true><<<grid, block, 0, st>>>(a, cur, nxt, nullptr, dttmp, eps);
-    else
-        tke_rk_stage_kernel<false, true><<<grid, block, 0, st>>>(a, cur, nxt, nullptr, dttmp, eps);
-    ps.stop();
-    return launch_ok("tke_rk_stage_flat_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
+    return launch_ok(name) ? GM1B_OK : GM1B_ERR_CUDA;
 }
 
 // Flat column arguments: the arrays the flat turbt and RK stage read.
@@ -759,7 +784,7 @@ extern "C" int32_t gm1b_tke_rk_stage_flat(int32_t ni, int32_t nj, int32_t nk,
         gm1b_set_error("gm1b_tke_rk_stage_flat: need distinct cur and nxt and nrk in 1..3");
         return GM1B_ERR_ARGUMENT;
     }
-    return enqueue_stage_flat(a, cur, nxt, nrk, dt, static_cast<cudaStream_t>(stream));
+    return enqueue_stage<true>(a, cur, nxt, nullptr, nrk, dt, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int32_t gm1b_tke_rk_stage(int32_t ni, int32_t nj, int32_t nk, const gm1b_tke_evolution_arrays *arrays,
@@ -772,7 +797,7 @@ extern "C" int32_t gm1b_tke_rk_stage(int32_t ni, int32_t nj, int32_t nk, const g
         gm1b_set_error("gm1b_tke_rk_stage: need distinct cur and nxt and nrk in 1..3");
         return GM1B_ERR_ARGUMENT;
     }
-    return enqueue_stage(a, cur, nxt, nullptr, nrk, dt, static_cast<cudaStream_t>(stream));
+    return enqueue_stage<false>(a, cur, nxt, nullptr, nrk, dt, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int32_t gm1b_tke_evolution(int32_t ni, int32_t nj, int32_t nk, const gm1b_tke_evolution_arrays *arrays,
@@ -789,9 +814,9 @@ extern "C" int32_t gm1b_tke_evolution(int32_t ni, int32_t nj, int32_t nk, const 
     int s = enqueue_diffusion(a, dt, st);
     // stage 1: tke3d -> workspace; stage 2: workspace -> tke3d; stage 3:
     // tke3d -> tkea (each cell reads only its own tkea word) and workspace
-    if (s == GM1B_OK) s = enqueue_stage(a, tke3d, workspace, nullptr, 1, dt, st);
-    if (s == GM1B_OK) s = enqueue_stage(a, workspace, tke3d, nullptr, 2, dt, st);
-    if (s == GM1B_OK) s = enqueue_stage(a, tke3d, workspace, tkea, 3, dt, st);
+    if (s == GM1B_OK) s = enqueue_stage<false>(a, tke3d, workspace, nullptr, 1, dt, st);
+    if (s == GM1B_OK) s = enqueue_stage<false>(a, workspace, tke3d, nullptr, 2, dt, st);
+    if (s == GM1B_OK) s = enqueue_stage<false>(a, tke3d, workspace, tkea, 3, dt, st);
     if (s != GM1B_OK) return s;
     const size_t bytes = (size_t)(nk + 1) * nj * ni * sizeof(float);
     const cudaError_t e = cudaMemcpyAsync(tke3d, workspace, bytes, cudaMemcpyDeviceToDevice, st);

@@ -112,3 +112,26 @@ def test_momentum_advection(ni, nj, nk, sides):
     ref = {**a, **m, "divx": np.zeros((nk, nj, ni), np.float32)}
     orc.momentum_advection5(ref, **kw)
     assert _differ({**dev, "divx": out.divx}, ref, OUTS) == []
+
+
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (32, 14, 11), (62, 15, 12), (7, 9, 40)])
+def test_tke_stages(ni, nj, nk, flat):
+    from gm1_b200 import tke_evolution as te
+    from oracle import tke_evolution as orc
+    from tests.golden.make_golden import tke_evolution_fixture
+
+    a = tke_evolution_fixture(ni, nj, nk, seed=ni + nk)
+    dev = _dev(a)
+    ws, p = torch.empty_like(dev["tke3d"]), _profiles(nk)
+    kw = dict(ni=ni, nj=nj, nk=nk, dx=500.0, dy=450.0, dt=2.0)
+    for nrk in (1, 2, 3):
+        nxt = np.zeros_like(a["tke3d"])
+        if flat:
+            orc.tke_rk_stage_flat(a, p["mf"], a["tke3d"], nxt, nrk=nrk, rdz=p["rdz"], **kw)
+            te.launch_cuda_flat_tke_rk_stage(dev, mf_profile=_t(p["mf"]), workspace=ws, nrk=nrk, rdz=p["rdz"], **kw)
+        else:
+            orc.tke_rk_stage(a, a["tke3d"], nxt, nrk=nrk, dz=150.0, **kw)
+            te.launch_cuda_tke_rk_stage(dev, workspace=ws, nrk=nrk, dz=150.0, **kw)
+        a["tke3d"] = nxt
+        assert _differ(dev, a, ("tke3d",)) == [], nrk
