@@ -135,3 +135,17 @@ def test_tke_stages(ni, nj, nk, flat):
             te.launch_cuda_tke_rk_stage(dev, workspace=ws, nrk=nrk, dz=150.0, **kw)
         a["tke3d"] = nxt
         assert _differ(dev, a, ("tke3d",)) == [], nrk
+
+
+@pytest.mark.parametrize("ni,nj,nk", [(31, 7, 8), (32, 8, 9), (33, 7, 10), (7, 7, 17), (8, 9, 201)])
+def test_flat_tke_diffusion(ni, nj, nk):
+    from gm1_b200 import tke_evolution as te
+    from oracle import tke_evolution as orc
+    from tests.golden.make_golden import tke_evolution_fixture
+
+    a = tke_evolution_fixture(ni, nj, nk, seed=3 * ni + nk)
+    dev = _dev(a)
+    kw = dict(ni=ni, nj=nj, nk=nk, dx=500.0, dy=450.0, rdz=_profiles(nk)["rdz"], dt=2.0)
+    orc.tke_diffusion_flat(a, **kw)
+    te.launch_cuda_flat_tke_diffusion(dev, **kw)
+    assert _differ(dev, a, ("tketen",)) == []
