@@ -50,7 +50,8 @@ struct TosArgs {
     gm1b_terrain_metrics m;
     int ni, nj, nk, nrk, n, nloop;
     unsigned abl, diag;
-    int acc;  // this small step's pressure gradient sums rru and rrv (the march pass follows)
+    int acc;   // this small step's pressure gradient sums rru and rrv (the march pass follows)
+    int edge;  // the march pass leaves the next small step's open-side velocities
     float dts, rdx, rdy, dz, alph, beta, asq, kdiv, temx, temy, tavg, zt, rzt, halfcp;
     float cgs[3], cgt[3];
     // the stretched terrain column (vmode 1): CM1-indexed sigma (nk+2),
@@ -983,13 +984,16 @@ __global__ void __launch_bounds__(32 * kTosWarps, 3) tos_column_kernel(TosArgs p
 // pressure-gradient pass, which holds u and v.
 // Bound by load latency and the barriers around the sweep (24 warps an SM:
 // the five shared words and 80 registers allow three CTAs).  Measured on one
-// B200, per launch: flat column 640x768x80 1.583 -> 0.898 ms, uniform column
-// 256x256x80 271 -> 169 us against the phase-by-phase pass; 16 warps 1.007 ms,
-// 10 warps 1.048, 4 warps 1.228, two CTAs an SM 1.175, four (64 registers)
-// 1.144.
+// B200, per launch: flat column 640x768x80 1.583 -> 0.878 ms, uniform column
+// 256x256x80 271 -> 177 us against the phase-by-phase pass and its separate
+// open-edge launch of 11 us; 16 warps 1.007 ms, 10 warps 1.048, 4 warps 1.228,
+// two CTAs an SM 1.175, four (64 registers) 1.144, four without the next
+// level's prefetch 1.179; the last phase's loads two levels at a time 0.900,
+// one 0.962.
 // ---------------------------------------------------------------------------
 constexpr int kMarchWarps = 8;
 constexpr int kMarchArrays = 5;
+constexpr int kMarchLevels = 4;  // levels of the last phase whose loads are issued together
 
 // the transformed face velocities of one level, and (terrain column) their
 // density-weighted twins
@@ -1005,8 +1009,8 @@ __device__ __forceinline__ Faces<VM> march_faces(const TosArgs &p, const Ix &X, 
     const gm1b_terrain_open_arrays &a = p.a;
     Faces<VM> f{};
     const unsigned qu = X.u(k, y, x), qv = X.v(k, y, x);
-    const float uw = __ldg(a.u3d + qu), ue = __ldg(a.u3d + qu + 1);
-    const float vs = __ldg(a.v3d + qv), vn = __ldg(a.v3d + qv + (unsigned)(p.ni + 6));
+    const float uw = a.u3d[qu], ue = a.u3d[qu + 1];
+    const float vs = a.v3d[qv], vn = a.v3d[qv + (unsigned)(p.ni + 6)];
     if (VM == 2) {
         f.xw = uw, f.xe = ue, f.ys = vs, f.yn = vn;
         return f;
@@ -1075,8 +1079,54 @@ struct MarchLoad {
     }
 };
 
+// the open-side normal velocity of one small step at level k of boundary line
+// `line` (row j of the west 0 / east 1 side, column i of the south 2 / north 3
+// side), from the words before it: tos_edge_kernel's and tos_flat_edge_kernel's
+// expressions
 template <int VM>
-__global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(TosArgs p) {
+__device__ __forceinline__ float edge_velocity(const TosArgs &p, const Ix &X, int side, int line, int k) {
+    const gm1b_terrain_open_arrays &a = p.a;
+    const gm1b_terrain_metrics &m = p.m;
+    const int ni = p.ni, nj = p.nj, nk = p.nk, t = line + 2;
+    const bool ew = side < 2, lo = side == 0 || side == 2;
+    // q0, q1: the two faces of the edge cell; the open one is q0 on the west
+    // and south sides, q1 on the others
+    const int f0 = side == 0 || side == 2 ? 3 : ew ? ni + 2 : nj + 2;
+    const float *q = ew ? a.u3d : a.v3d;
+    auto at = [&](int kk, int f) { return q[ew ? X.u(kk, t, f) : X.v(kk, f, t)]; };
+    const float q0 = at(k, f0), q1 = at(k, f0 + 1), old = lo ? q0 : q1;
+    const unsigned o = ew ? X.u(k, t, lo ? f0 : f0 + 1) : X.v(k, lo ? f0 : f0 + 1, t);
+    const float ten = __ldg((ew ? a.uten : a.vten) + o);
+    const float rd = ew ? p.rdx : p.rdy;
+    const float hmet = __ldg((ew ? a.uh : a.vh) + (lo ? 3 : ew ? ni + 2 : nj + 2));
+    const float *rad = side == 0 ? a.radbcw : side == 1 ? a.radbce : side == 2 ? a.radbcs : a.radbcn;
+    const float r = -rad[(size_t)k * (size_t)(ew ? nj + 6 : ni + 6) + t];
+    if (VM == 2) {
+        const float tnd = ((r * (q1 - q0)) * rd) * hmet + ten;
+        return old + p.dts * tnd;
+    }
+    const int j0 = ew ? line - 1 : (side == 2 ? 0 : nj - 1), i0 = ew ? (side == 0 ? 0 : ni - 1) : line - 1;
+    // the face's velocity at w level kf
+    auto atw = [&](int kf, int f) {
+        if (kf == 1) return (p.cgs[0] * at(1, f) + p.cgs[1] * at(2, f)) + p.cgs[2] * at(3, f);
+        if (kf == nk + 1) return (p.cgt[0] * at(nk, f) + p.cgt[1] * at(nk - 1, f)) + p.cgt[2] * at(nk - 2, f);
+        const float r2 = col_r2<VM>(p, kf), r1 = 1.0f - r2;
+        return r1 * at(kf - 1, f) + r2 * at(kf, f);
+    };
+    const float *rg = ew ? m.rgzu + (size_t)j0 * (ni + 1) + i0 : m.rgzv + (size_t)j0 * ni + i0;
+    const float rg0 = rg[0], rg1 = rg[ew ? 1 : ni];
+    const float *gmet = ew ? m.gx : m.gy;
+    float hz = m.gz[X.h(j0, i0)] * (q1 * rg1 - q0 * rg0);
+    hz = (hz * rd) * hmet;
+    float vt = gmet[X.m(k, j0, i0)] * (atw(k + 1, f0 + 1) + atw(k + 1, f0)) -
+               gmet[X.m(k - 1, j0, i0)] * (atw(k, f0 + 1) + atw(k, f0));
+    vt = (0.5f * vt) * col_rdsf<VM>(p, k);
+    const float tnd = r * (hz + vt) + ten;
+    return old + p.dts * tnd;
+}
+
+template <int VM>
+__global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(const __grid_constant__ TosArgs p) {
     extern __shared__ float sh[];
     const Ix X{p.ni, p.nj};
     const int ni = p.ni, nk = p.nk, L = nk + 2;
@@ -1131,7 +1181,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(T
             // the next level's words, in flight while this one computes (the
             // last level loads its own again)
             const int kn = k < k_hi ? k + 1 : k_hi;
-            MarchLoad nx;
+            MarchLoad nx = {};
             nx.load<VM>(p, X, kn, j, i);
             const int kf = VM == 2 ? kn : (k < nk ? k + 1 : nk);
             const Faces<VM> fn = march_faces<VM>(p, X, kf, y, x, rgw, rge, rgs, rgn, dzdx, dzdy);
@@ -1192,10 +1242,10 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(T
     }
     // phase C's words (pp3d of level k is read here before this thread writes
     // it there): the first levels' in flight over the barriers and the sweep
-    float lrw[kColLevels], cpp[kColLevels], ca1[kColLevels], ca2[kColLevels];
+    float lrw[kMarchLevels], cpp[kMarchLevels], ca1[kMarchLevels], ca2[kMarchLevels];
     auto c_loads = [&](int kb) {
 #pragma unroll
-        for (int q = 0; q < kColLevels; ++q) {
+        for (int q = 0; q < kMarchLevels; ++q) {
             const int k = min(kb + q, k_hi);
             const unsigned c = X.p(k, j, i);
             lrw[q] = a.rrw[X.w(k, y, x)];
@@ -1253,13 +1303,12 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(T
     }
     __syncthreads();
     // pressure update, filter, halo copy, rrw average
-    if (!busy || !live) return;
     const bool fill = !last;
     const bool east = i == ni, north = j == p.nj;
-    for (int kb = k_lo; kb <= k_hi; kb += kColLevels) {
+    for (int kb = k_lo; busy && live && kb <= k_hi; kb += kMarchLevels) {
         if (kb != k_lo) c_loads(kb);
 #pragma unroll
-        for (int q = 0; q < kColLevels; ++q) {
+        for (int q = 0; q < kMarchLevels; ++q) {
             const int k = kb + q;
             if (k > k_hi) break;
             const unsigned c = X.p(k, j, i), qw = X.w(k, y, x);
@@ -1302,6 +1351,37 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(T
                 }
             }
         }
+    }
+    // the next small step's normal velocities on the open sides (ssopenbc*):
+    // this CTA alone reads and writes its own boundary faces, so the step
+    // needs no launch for them.  New words wait in shared memory until every
+    // level has read the old ones.
+    if (!p.edge) return;
+    // the sides this CTA touches, one bit each
+    const unsigned sides = (blockIdx.x == 0 ? 1u : 0u) | (blockIdx.x == gridDim.x - 1 ? 2u : 0u) | (j == 1 ? 4u : 0u) |
+                           (j == p.nj ? 8u : 0u);
+    if (sides == 0u) return;
+    const int tid = wy * 32 + lane;
+    float *s_we = sh + L * 32, *s_s = s_we + L * 32, *s_n = s_s + L * 32;  // the swept aa, bb and cc
+    auto open = [&](int side) {
+        return ((sides >> side) & 1u) != 0u && (VM != 2 || ((p.obc >> (4 * side)) & 15u) == 2u);
+    };
+    for (int e = tid; e < 2 * nk; e += 32 * kMarchWarps) {
+        const int side = e / nk, k = e % nk + 1;
+        if (open(side)) s_we[k * 32 + side] = edge_velocity<VM>(p, X, side, j, k);
+    }
+    for (int k = 1 + wy; k <= nk; k += kMarchWarps) {
+        if (open(2) && live) s_s[k * 32 + lane] = edge_velocity<VM>(p, X, 2, i, k);
+        if (open(3) && live) s_n[k * 32 + lane] = edge_velocity<VM>(p, X, 3, i, k);
+    }
+    __syncthreads();
+    for (int e = tid; e < 2 * nk; e += 32 * kMarchWarps) {
+        const int side = e / nk, k = e % nk + 1;
+        if (open(side)) a.u3d[X.u(k, y, side == 0 ? 3 : ni + 3)] = s_we[k * 32 + side];
+    }
+    for (int k = 1 + wy; k <= nk; k += kMarchWarps) {
+        if (open(2) && live) a.v3d[X.v(k, 3, x)] = s_s[k * 32 + lane];
+        if (open(3) && live) a.v3d[X.v(k, p.nj + 3, x)] = s_n[k * 32 + lane];
     }
 }
 
@@ -1734,18 +1814,23 @@ int32_t terrain_open_stage(int32_t ni, int32_t nj, int32_t nk, int32_t nrk, floa
                                        GM1B_TOS_BETWEEN_STEP_FILL;
     const dim3 march_grid((ni + 31) / 32, nj), march_block(32, kMarchWarps);
     const size_t march_smem = (size_t)kMarchArrays * (size_t)(nk + 2) * 32 * sizeof(float);
+    bool edges_left = false;
     for (int n = 1; n <= nloop; ++n) {
         p.n = n;
         // the march pass runs whole small steps; an ablated step and the step
         // that leaves the diagnostic words take the general column pass
         const bool march = (ablations & column_phases) == column_phases && !(p.diag && n == nloop);
         p.acc = march ? 1 : 0;
-        if ((ablations & GM1B_TOS_OPEN_CONSUMPTION) && p.vmode == 2) {
+        p.edge = march && n < nloop && (ablations & GM1B_TOS_OPEN_CONSUMPTION) ? 1 : 0;
+        // (a march pass has left the open sides of the step that follows it)
+        const bool open_sides = (ablations & GM1B_TOS_OPEN_CONSUMPTION) && !edges_left;
+        edges_left = p.edge != 0;
+        if (open_sides && p.vmode == 2) {
             ProfScope ps("tos_flat_edge_kernel", st);
             tos_flat_edge_kernel<<<grid_for((size_t)nk * (nj + ni), 256), 256, 0, st>>>(p);
             ps.stop();
             if (!launch_ok("tos_flat_edge_kernel")) return GM1B_ERR_CUDA;
-        } else if (ablations & GM1B_TOS_OPEN_CONSUMPTION) {
+        } else if (open_sides) {
             ProfScope ps("tos_edge_kernel", st);
             tos_edge_kernel<<<2 * nj + 2 * ni, 128, 4 * (size_t)(nk + 2) * sizeof(float), st>>>(p);
             ps.stop();
