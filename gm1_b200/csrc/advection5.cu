@@ -210,13 +210,18 @@ inline int default_chunk(int row_warps, int nk, bool weno) {
 // shared memory, one barrier a level, the eighth row forming a flux only.
 // Words come through L1, which holds a row's neighbours: the passes are bound
 // by instruction issue (fifth order) and the binary64 weights (WENO).
-// Measured on one B200, per launch at 640x768x80: fifth order 1.105 -> 0.446
-// ms, WENO 2.572 -> 1.355 against CTAs that stage each level's plane in shared
-// memory (WENO with 24 warps an SM 1.437, with 16 rows 1.836).
-template <bool WENO>
-__global__ void __launch_bounds__(32 * (WENO ? kWenoRows : kFifthRows), WENO ? 4 : 5)
-    scalar_advection5_march_kernel(gm1b_scalar_advection5_arrays a, PaddedDims d, int levels_per_chunk, float rdx,
-                                   float rdy, float rdsf, double eps, float wepsf, unsigned obc, VertCol vc) {
+// Measured on one B200, per launch at 640x768x80: fifth order 1.105 -> 0.430
+// ms, WENO 2.572 -> 1.290 against CTAs that stage each level's plane in shared
+// memory (WENO with 24 warps an SM 1.336, with 16 rows 1.836; fifth order with
+// 24 warps 0.402 but 72 us for 68 at 256x256x80, with 40 warps 0.602).
+// Warps away from open sides, at levels away from the column's ends and with
+// no flux outputs take a finish without those branches.
+template <bool WENO, bool FLAT>
+__global__ void __launch_bounds__(32 * (WENO ? kWenoRows : kFifthRows), WENO ? 4 : 4)
+    scalar_advection5_march_kernel(const __grid_constant__ gm1b_scalar_advection5_arrays a,
+                                   const __grid_constant__ PaddedDims d, int levels_per_chunk, float rdx, float rdy,
+                                   float rdsf, double eps, float wepsf, unsigned obc,
+                                   const __grid_constant__ VertCol vc) {
     constexpr int ROWS = WENO ? kWenoRows : kFifthRows;
     __shared__ float s_fy[WENO ? 2 : 1][WENO ? ROWS : 1][32], s_vm[WENO ? 2 : 1][WENO ? ROWS : 1][32];
     const int lane = threadIdx.x, ty = threadIdx.y;
@@ -237,15 +242,16 @@ __global__ void __launch_bounds__(32 * (WENO ? kWenoRows : kFifthRows), WENO ? 4
     const bool owned = cell && (obc != 0u || (i >= 3 && i + 3 < ni && j >= 3 && j + 3 < nj));
     const int col = y * sx + x;          // this point in a scalar / w plane
     const int uc = y * ux + x, cc = min(j, nj - 1) * ni + min(f, ni - 1);
-    const bool north = WENO && j == nj;  // the row of faces nj only
     const bool wo = i == 0 && (obc & 15u) == 2u, eo = i + 1 == ni && ((obc >> 4) & 15u) == 2u;
     const bool so = j == 0 && ((obc >> 8) & 15u) == 2u, no = j + 1 == nj && ((obc >> 12) & 15u) == 2u;
-    const float gz = __ldg(a.gz + cc);
+    const bool edge = __any_sync(0xffffffffu, wo || eo) || so || no || a.flux_x != nullptr || a.flux_y != nullptr ||
+                      a.flux_z != nullptr;
+    const float gz = FLAT ? 0.0f : __ldg(a.gz + cc);
     float win[6];  // levels k-3 .. k+2 of this point; shifted to k-2 .. k+3 for face k+1
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
         const int lev = k_begin - 3 + q;
-        win[q] = (!north && lev >= 0 && lev <= nk + 1) ? __ldg(s + lev * splane + col) : 0.0f;
+        win[q] = (lev >= 0 && lev <= nk + 1) ? __ldg(s + lev * splane + col) : 0.0f;
     }
     float fz_lo = 0.0f;
     if (cell) {
@@ -272,26 +278,18 @@ __global__ void __launch_bounds__(32 * (WENO ? kWenoRows : kFifthRows), WENO ? 4
         for (int q = 0; q < 6; ++q) px[q] = q == 3 ? 0.0f : __ldg(pt + (q - 3));
 #pragma unroll
         for (int q = 0; q < 7; ++q) py[q] = (q == 3 || (WENO && q == 6)) ? 0.0f : __ldg(pt + (q - 3) * sx);
-        const float zn = (!north && k + 3 <= nk + 1) ? __ldg(pt + 3 * splane) : 0.0f;
+        const float zn = k + 3 <= nk + 1 ? __ldg(pt + 3 * splane) : 0.0f;
         const int fz = k + 1;
-        float mz = 0.0f, c1 = 0.0f, c2 = 0.0f;
-        if (fz <= nk && !north) {
-            mz = __ldg(a.rrw + fz * splane + col);
-            if (fz == 2 || fz == nk) {
-                c1 = __ldg(a.c1 + (fz - 1) * cplane + cc);
-                c2 = __ldg(a.c2 + (fz - 1) * cplane + cc);
-            }
-        }
+        const float mz = __ldg(a.rrw + fz * splane + col);  // level nk+1 exists and is not used
         const int c = (k - 1) * cplane + cc;
         const float div = __ldg(a.divx + c);
-        const float rr0 = __ldg(a.rr0 + (vc.mode == 2 ? (k - 1) * cplane : c));
-        float sv = win[3];
-        if (north) sv = __ldg(pt);
+        const float rr0 = __ldg(a.rr0 + (FLAT ? (k - 1) * cplane : c));
+        const float r = FLAT ? __ldg(vc.mh + k) : vc.mode == 1 ? __ldg(vc.rdsf + k) : rdsf;
+        const float sv = win[3];
         px[3] = py[3] = sv;
         const float fx = upwind<WENO>(mw, px[0], px[1], px[2], px[3], px[4], px[5], eps);
         const float fy = upwind<WENO>(ms, py[0], py[1], py[2], py[3], py[4], py[5], eps);
         float fw = fx, fe = __shfl_down_sync(0xffffffffu, fx, 1);
-        const float ue = __shfl_down_sync(0xffffffffu, mw, 1);
         float fs = fy, fn;
         if (WENO) {
             const int buf = k & 1;
@@ -307,55 +305,68 @@ __global__ void __launch_bounds__(32 * (WENO ? kWenoRows : kFifthRows), WENO ? 4
 #pragma unroll
         for (int q = 0; q < 5; ++q) win[q] = win[q + 1];
         win[5] = zn;
-        if (cell) {
-            if (a.flux_x != nullptr) {
-                a.flux_x[k * uplane + uc] = fw;
-                if (i == ni - 1) a.flux_x[k * uplane + uc + 1] = fe;
-            }
-            if (a.flux_y != nullptr) {
-                a.flux_y[k * vplane + col] = fs;
-                if (j == nj - 1) a.flux_y[k * vplane + col + sx] = fn;
-            }
-            float fz_hi = 0.0f;
-            if (fz <= nk) fz_hi = z_face<WENO>(win, mz, c1, c2, fz, nk, eps, wepsf);
-            if (a.flux_z != nullptr) a.flux_z[fz * splane + col] = fz_hi;
-            if (owned) {
-                const bool iw = wo && mw >= 0.0f, ie = eo && ue <= 0.0f;
-                const bool js = so && ms >= 0.0f, jn = no && mn <= 0.0f;
-                if (iw) fw = fe;
-                if (ie) fe = fw;
-                if (js) fs = fn;
-                if (jn) fn = fs;
-                float ax = (fw - fe) * rdx;
-                float ay = (fs - fn) * rdy;
-                if (iw) ax = ax - (sv * (ue - mw)) * rdx;
-                if (ie) ax = ax - (sv * (ue - mw)) * rdx;
-                if (js) ay = ay - (sv * (mn - ms)) * rdy;
-                if (jn) ay = ay - (sv * (mn - ms)) * rdy;
-                float az;
-                if (vc.mode == 2) {
-                    const float mhk = __ldg(vc.mh + k);
-                    if (k == 1)
-                        az = ((-fz_hi) * vc.rdz) * mhk;
-                    else if (k == nk)
-                        az = (fz_lo * vc.rdz) * mhk;
-                    else
-                        az = ((-(fz_hi - fz_lo)) * vc.rdz) * mhk;
-                } else {
-                    const float r = vc.mode == 1 ? __ldg(vc.rdsf + k) : rdsf;
-                    if (k == 1)
-                        az = (-fz_hi) * r;
-                    else if (k == nk)
-                        az = fz_lo * r;
-                    else
-                        az = (fz_lo - fz_hi) * r;
+        float fz_hi = 0.0f;
+        if (!edge && fz > 3 && fz < nk - 1) {
+            fz_hi = upwind<WENO>(mz, win[0], win[1], win[2], win[3], win[4], win[5], eps);
+            const float ax = (fw - fe) * rdx, ay = (fs - fn) * rdy;
+            const float az = FLAT ? ((-(fz_hi - fz_lo)) * vc.rdz) * r : (fz_lo - fz_hi) * r;
+            float total = (ax + ay) + az;
+            total = total + sv * div;
+            if (owned) a.tendency[c] = FLAT ? total * rr0 : (total * rr0) * gz;
+        } else {
+            const float ue = __shfl_down_sync(0xffffffffu, mw, 1);
+            if (cell) {
+                if (a.flux_x != nullptr) {
+                    a.flux_x[k * uplane + uc] = fw;
+                    if (i == ni - 1) a.flux_x[k * uplane + uc + 1] = fe;
                 }
-                float total = (ax + ay) + az;
-                total = total + sv * div;
-                a.tendency[c] = vc.mode == 2 ? total * rr0 : (total * rr0) * gz;
+                if (a.flux_y != nullptr) {
+                    a.flux_y[k * vplane + col] = fs;
+                    if (j == nj - 1) a.flux_y[k * vplane + col + sx] = fn;
+                }
+                if (fz <= nk) {
+                    const bool end = fz == 2 || fz == nk;
+                    const float c1 = end ? __ldg(a.c1 + (fz - 1) * cplane + cc) : 0.0f;
+                    const float c2 = end ? __ldg(a.c2 + (fz - 1) * cplane + cc) : 0.0f;
+                    fz_hi = z_face<WENO>(win, mz, c1, c2, fz, nk, eps, wepsf);
+                }
+                if (a.flux_z != nullptr) a.flux_z[fz * splane + col] = fz_hi;
+                if (owned) {
+                    const bool iw = wo && mw >= 0.0f, ie = eo && ue <= 0.0f;
+                    const bool js = so && ms >= 0.0f, jn = no && mn <= 0.0f;
+                    if (iw) fw = fe;
+                    if (ie) fe = fw;
+                    if (js) fs = fn;
+                    if (jn) fn = fs;
+                    float ax = (fw - fe) * rdx;
+                    float ay = (fs - fn) * rdy;
+                    if (iw) ax = ax - (sv * (ue - mw)) * rdx;
+                    if (ie) ax = ax - (sv * (ue - mw)) * rdx;
+                    if (js) ay = ay - (sv * (mn - ms)) * rdy;
+                    if (jn) ay = ay - (sv * (mn - ms)) * rdy;
+                    float az;
+                    if (FLAT) {
+                        if (k == 1)
+                            az = ((-fz_hi) * vc.rdz) * r;
+                        else if (k == nk)
+                            az = (fz_lo * vc.rdz) * r;
+                        else
+                            az = ((-(fz_hi - fz_lo)) * vc.rdz) * r;
+                    } else {
+                        if (k == 1)
+                            az = (-fz_hi) * r;
+                        else if (k == nk)
+                            az = fz_lo * r;
+                        else
+                            az = (fz_lo - fz_hi) * r;
+                    }
+                    float total = (ax + ay) + az;
+                    total = total + sv * div;
+                    a.tendency[c] = FLAT ? total * rr0 : (total * rr0) * gz;
+                }
             }
-            fz_lo = fz_hi;
         }
+        fz_lo = fz_hi;
     }
 }
 
@@ -453,12 +464,15 @@ int32_t scalar_advection5_launch(int32_t ni, int32_t nj, int32_t nk, const gm1b_
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float rdx = 1.0f / dx, rdy = 1.0f / dy, rdsf = 1.0f / dz;
     ProfScope ps(weno ? "scalar_advection5_weno_kernel" : "scalar_advection5_kernel", st);
+    auto launch = [&](auto kernel, int rows_per_cta) {
+        kernel<<<grid, dim3(32, rows_per_cta), 0, st>>>(a, d, chunk, rdx, rdy, rdsf, weps, (float)weps, lateral_obc, vc);
+    };
     if (weno)
-        scalar_advection5_march_kernel<true>
-            <<<grid, dim3(32, kWenoRows), 0, st>>>(a, d, chunk, rdx, rdy, rdsf, weps, (float)weps, lateral_obc, vc);
+        vc.mode == 2 ? launch(scalar_advection5_march_kernel<true, true>, kWenoRows)
+                     : launch(scalar_advection5_march_kernel<true, false>, kWenoRows);
     else
-        scalar_advection5_march_kernel<false>
-            <<<grid, dim3(32, kFifthRows), 0, st>>>(a, d, chunk, rdx, rdy, rdsf, weps, (float)weps, lateral_obc, vc);
+        vc.mode == 2 ? launch(scalar_advection5_march_kernel<false, true>, kFifthRows)
+                     : launch(scalar_advection5_march_kernel<false, false>, kFifthRows);
     ps.stop();
     if (cudaPeekAtLastError() != cudaSuccess) {
         gm1b_set_error("scalar_advection5_kernel: %s", cudaGetErrorString(cudaGetLastError()));

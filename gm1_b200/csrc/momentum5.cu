@@ -69,19 +69,19 @@ __device__ __forceinline__ int fyw(const MomArgs &a, int j) {
 }
 // x * the column's vertical reciprocal at mass level k (uniform rdz, the
 // terrain branch's rdsf(k), or the flat column's (x*rdz)*mh(k))
-__device__ __forceinline__ float zmass(const MomArgs &a, float x, int k) {
-    if (a.vmode == 2) return (x * a.rdzm) * __ldg(a.mh + k);
+template <bool FLAT> __device__ __forceinline__ float zmass(const MomArgs &a, float x, int k) {
+    if (FLAT) return (x * a.rdzm) * __ldg(a.mh + k);
     return x * (a.vmode == 1 ? __ldg(a.rdsf + k) : a.rdz);
 }
 // the same at w level kf (rds(kf) / (x*rdz)*mf(kf))
-__device__ __forceinline__ float zface(const MomArgs &a, float x, int kf) {
-    if (a.vmode == 2) return (x * a.rdzm) * __ldg(a.mf + kf);
+template <bool FLAT> __device__ __forceinline__ float zface(const MomArgs &a, float x, int kf) {
+    if (FLAT) return (x * a.rdzm) * __ldg(a.mf + kf);
     return x * (a.vmode == 1 ? __ldg(a.rds + kf) : a.rdz);
 }
 // a boundary correction: uniform and terrain ((q*c)*(r*h)) as adv.F is
 // grouped in the uniform text; the flat text groups it ((q*c)*r)*h
-__device__ __forceinline__ float bcorr(const MomArgs &a, float q, float c, float r, float h) {
-    return a.vmode == 2 ? ((q * c) * r) * h : q * (c * (r * h));
+template <bool FLAT> __device__ __forceinline__ float bcorr(float q, float c, float r, float h) {
+    return FLAT ? ((q * c) * r) * h : q * (c * (r * h));
 }
 
 __device__ __forceinline__ float up5(float m, float s0, float s1, float s2, float s3, float s4, float s5) {
@@ -172,8 +172,9 @@ __global__ void __launch_bounds__(128) mom5_rrw_divx_kernel(MomArgs a) {
 // are neighbouring CTAs (blockIdx.x % 3), so their shared mass fluxes meet in
 // L2.  Bound by instruction issue (the upwind selects on the half-rate ALU).
 // Measured on one B200, per launch at 640x768x80: 3.085 ms with a thread per
-// point forming all its fluxes, 1.596 here (32 warps an SM; 24 warps 1.775, 16
-// warps 1.889).
+// point forming all its fluxes, 1.596 with one finish for every line, 1.127
+// here (32 warps an SM; 24 warps 1.169, 40 warps 1.267, two levels a trip
+// 1.353).
 // ---------------------------------------------------------------------------
 constexpr int kMomOut = 31;   // points a warp of 32 faces completes
 constexpr int kMomRows = 4;   // rows (independent warps) per CTA
@@ -233,6 +234,7 @@ __device__ __forceinline__ void shift(float win[6], float next) {
 }
 
 // advu at the faces f of row j
+template <bool FLAT>
 __device__ __forceinline__ void march_u(const MomArgs &a, int tile, int j, int k_lo, int k_hi) {
     const int ni = a.ni, nj = a.nj, nk = a.nk, lane = threadIdx.x;
     if (j >= nj) return;
@@ -248,8 +250,8 @@ __device__ __forceinline__ void march_u(const MomArgs &a, int tile, int j, int k
     const int se = y * sx + e + G, sw = y * sx + w + G;          // rrv / rrw columns east and west of the face
     const int ce = j * ni + clampn(e, ni), cw = j * ni + clampn(w, ni);  // divx and rho0
     const int c2e = j * ni + clampn(f, ni), c2w = j * ni + clampn(f - 1, ni);
-    const bool so = j == 0 && a.opn[2], no = j == nj - 1 && a.opn[3];
-    const float gzu = a.vmode == 2 ? 0.0f : __ldg(a.gzu + j * (ni + 1) + min(f, ni)), vh = __ldg(a.vh + y);
+    const bool so = j == 0 && a.opn[2], no = j == nj - 1 && a.opn[3], edge = so || no;
+    const float gzu = FLAT ? 0.0f : __ldg(a.gzu + j * (ni + 1) + min(f, ni)), vh = __ldg(a.vh + y);
     float win[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
@@ -273,33 +275,36 @@ __device__ __forceinline__ void march_u(const MomArgs &a, int tile, int j, int k
         const float ma = __ldg(a.rru + k * uz + ra), mb = __ldg(a.rru + k * uz + rb);
         const float *rv = a.rrv + k * vz;
         const float vse = __ldg(rv + se), vsw = __ldg(rv + sw), vne = __ldg(rv + se + sx), vnw = __ldg(rv + sw + sx);
-        float mz = 0.0f, c2 = 0.0f;
-        if (k < nk) {
-            mz = 0.5f * (__ldg(a.rrw + (k + 1) * wz + se) + __ldg(a.rrw + (k + 1) * wz + sw));
-            c2 = c2f(k + 1);
-        }
+        // (level nk+1's is not used)
+        const float mz = 0.5f * (__ldg(a.rrw + (k + 1) * wz + se) + __ldg(a.rrw + (k + 1) * wz + sw));
         const float de = __ldg(a.divx + (k - 1) * cz + ce), dw = __ldg(a.divx + (k - 1) * cz + cw);
         float *out = a.uten + k * uz + o;
         const float ten = own ? *out : 0.0f;
-        const float scale = a.vmode == 2 ? __ldg(a.rr0 + (k - 1) * cz)
+        const float scale = FLAT ? __ldg(a.rr0 + (k - 1) * cz)
                                          : gzu / (0.5f * (__ldg(a.rho0 + (k - 1) * cz + cw) + __ldg(a.rho0 + (k - 1) * cz + ce)));
         const float fw = up5(0.5f * (ma + mb), px[0], px[1], px[2], px[3], px[4], px[5]);
         const float fe = below(fw);
         const float ms = vse + vsw, mn = vne + vnw;
         const float fs0 = up5(0.5f * ms, py[0], py[1], py[2], py[3], py[4], py[5]);
         const float fn0 = up5(0.5f * mn, py[1], py[2], py[3], py[4], py[5], py[6]);
-        // inflow through an open side's face takes the inner neighbour's flux
-        const bool sub_s = so && ms >= 0.0f, sub_n = no && mn <= 0.0f;
-        const float fs = sub_s ? fn0 : fs0, fn = sub_n ? fs0 : fn0;
         shift(win, next);
-        const float zhi = k < nk ? uv_z(win, mz, c2, k + 1, nk) : 0.0f;
         const float advx = -(fe - fw) * a.rdx;
-        float advy = -(fn - fs) * a.rdy;
-        if (sub_s || sub_n) {
-            const float corr = (vnw - vsw) + (vne - vse);
-            advy = advy - bcorr(a, uc * 0.5f, corr, a.rdy, vh);
+        float advy, advz, zhi;
+        if (!edge && k >= 3 && k < nk - 2) {
+            zhi = up5(mz, win[0], win[1], win[2], win[3], win[4], win[5]);
+            advy = -(fn0 - fs0) * a.rdy;
+            advz = zmass<FLAT>(a, -(zhi - zlo), k);
+        } else {
+            // inflow through an open side's face takes the inner neighbour's flux
+            const bool sub_s = so && ms >= 0.0f, sub_n = no && mn <= 0.0f;
+            zhi = k < nk ? uv_z(win, mz, c2f(k + 1), k + 1, nk) : 0.0f;
+            advy = -((sub_n ? fs0 : fn0) - (sub_s ? fn0 : fs0)) * a.rdy;
+            if (sub_s || sub_n) {
+                const float corr = (vnw - vsw) + (vne - vse);
+                advy = advy - bcorr<FLAT>(uc * 0.5f, corr, a.rdy, vh);
+            }
+            advz = zmass<FLAT>(a, k == 1 ? -zhi : k == nk ? zlo : -(zhi - zlo), k);
         }
-        const float advz = zmass(a, k == 1 ? -zhi : k == nk ? zlo : -(zhi - zlo), k);
         float total = (advx + advy) + advz;
         total = total + uc * (0.5f * (de + dw));
         if (own) *out = ten + total * scale;
@@ -308,6 +313,7 @@ __device__ __forceinline__ void march_u(const MomArgs &a, int tile, int j, int k
 }
 
 // advv at the faces g of rows, columns i
+template <bool FLAT>
 __device__ __forceinline__ void march_v(const MomArgs &a, int tile, int g, int k_lo, int k_hi) {
     const int ni = a.ni, nj = a.nj, nk = a.nk, lane = threadIdx.x;
     const int fr = a.per[2] ? 0 : 1, lr = a.per[3] ? nj : nj - 1;
@@ -324,8 +330,8 @@ __device__ __forceinline__ void march_v(const MomArgs &a, int tile, int g, int k
     const int ic0 = min(i, ni - 1);
     const int cn = clampn(north, nj) * ni + ic0, cs = clampn(south, nj) * ni + ic0;
     const int c2n = clampn(g, nj) * ni + ic0, c2s = clampn(g - 1, nj) * ni + ic0;
-    const bool wo = i == 0 && a.opn[0], eo = i == ni - 1 && a.opn[1];
-    const float gzv = a.vmode == 2 ? 0.0f : __ldg(a.gzv + g * ni + ic0), uh = __ldg(a.uh + x);
+    const bool wo = i == 0 && a.opn[0], eo = i == ni - 1 && a.opn[1], edge = __any_sync(0xffffffffu, wo || eo);
+    const float gzv = FLAT ? 0.0f : __ldg(a.gzv + g * ni + ic0), uh = __ldg(a.uh + x);
     float win[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
@@ -349,32 +355,35 @@ __device__ __forceinline__ void march_v(const MomArgs &a, int tile, int g, int k
         const float uN = __ldg(a.rru + k * uz + un), uS = __ldg(a.rru + k * uz + us);
         const float *rv = a.rrv + k * vz;
         const float ma = __ldg(rv + rs), mb = __ldg(rv + rc), mc = __ldg(rv + rn);
-        float mz = 0.0f, c2 = 0.0f;
-        if (k < nk) {
-            mz = 0.5f * (__ldg(a.rrw + (k + 1) * wz + sn) + __ldg(a.rrw + (k + 1) * wz + ss));
-            c2 = c2f(k + 1);
-        }
+        const float mz = 0.5f * (__ldg(a.rrw + (k + 1) * wz + sn) + __ldg(a.rrw + (k + 1) * wz + ss));
         const float dn = __ldg(a.divx + (k - 1) * cz + cn), ds = __ldg(a.divx + (k - 1) * cz + cs);
         float *out = a.vten + k * vz + o;
         const float ten = own ? *out : 0.0f;
-        const float scale = a.vmode == 2 ? __ldg(a.rr0 + (k - 1) * cz)
+        const float scale = FLAT ? __ldg(a.rr0 + (k - 1) * cz)
                                          : gzv / (0.5f * (__ldg(a.rho0 + (k - 1) * cz + cs) + __ldg(a.rho0 + (k - 1) * cz + cn)));
         const float mw = uN + uS;
         const float fw0 = up5(0.5f * mw, px[0], px[1], px[2], px[3], px[4], px[5]);
-        const float fe0 = below(fw0), me = below(mw), uNe = below(uN), uSe = below(uS);
-        const bool sub_w = wo && mw >= 0.0f, sub_e = eo && me <= 0.0f;
-        const float fw = sub_w ? fe0 : fw0, fe = sub_e ? fw0 : fe0;
+        const float fe0 = below(fw0);
         const float fs = up5(0.5f * (ma + mb), py[0], py[1], py[2], py[3], py[4], py[5]);
         const float fn = up5(0.5f * (mb + mc), py[1], py[2], py[3], py[4], py[5], py[6]);
         shift(win, next);
-        const float zhi = k < nk ? uv_z(win, mz, c2, k + 1, nk) : 0.0f;
-        float advx = -(fe - fw) * a.rdx;
         const float advy = -(fn - fs) * a.rdy;
-        if (sub_w || sub_e) {
-            const float corr = (uSe - uS) + (uNe - uN);
-            advx = advx - bcorr(a, vc * 0.5f, corr, a.rdx, uh);
+        float advx, advz, zhi;
+        if (!edge && k >= 3 && k < nk - 2) {
+            zhi = up5(mz, win[0], win[1], win[2], win[3], win[4], win[5]);
+            advx = -(fe0 - fw0) * a.rdx;
+            advz = zmass<FLAT>(a, -(zhi - zlo), k);
+        } else {
+            const float me = below(mw), uNe = below(uN), uSe = below(uS);
+            const bool sub_w = wo && mw >= 0.0f, sub_e = eo && me <= 0.0f;
+            zhi = k < nk ? uv_z(win, mz, c2f(k + 1), k + 1, nk) : 0.0f;
+            advx = -((sub_e ? fw0 : fe0) - (sub_w ? fe0 : fw0)) * a.rdx;
+            if (sub_w || sub_e) {
+                const float corr = (uSe - uS) + (uNe - uN);
+                advx = advx - bcorr<FLAT>(vc * 0.5f, corr, a.rdx, uh);
+            }
+            advz = zmass<FLAT>(a, k == 1 ? -zhi : k == nk ? zlo : -(zhi - zlo), k);
         }
-        const float advz = zmass(a, k == 1 ? -zhi : k == nk ? zlo : -(zhi - zlo), k);
         float total = (advx + advy) + advz;
         total = total + vc * (0.5f * (dn + ds));
         if (own) *out = ten + total * scale;
@@ -383,6 +392,7 @@ __device__ __forceinline__ void march_v(const MomArgs &a, int tile, int g, int k
 }
 
 // advw at the w levels kf = k + 1 (2..nk) of row j, columns i
+template <bool FLAT>
 __device__ __forceinline__ void march_w(const MomArgs &a, int tile, int j, int k_lo, int k_hi) {
     const int ni = a.ni, nj = a.nj, nk = a.nk, lane = threadIdx.x;
     if (j >= nj || tile * kMomOut >= ni || k_lo >= nk) return;
@@ -396,8 +406,9 @@ __device__ __forceinline__ void march_w(const MomArgs &a, int tile, int j, int k
     const int cs = clampn(j - 1, nj) * ni + ic0, cn = clampn(j + 1, nj) * ni + ic0;
     const bool wo = i == 0 && a.opn[0], eo = i == ni - 1 && a.opn[1];
     const bool so = j == 0 && a.opn[2], no = j == nj - 1 && a.opn[3];
+    const bool edge = __any_sync(0xffffffffu, wo || eo) || so || no;
     const float uh = __ldg(a.uh + min(x, ni + 2 * G - 1)), vh = __ldg(a.vh + y);
-    const float gz = a.vmode == 2 ? 0.0f : __ldg(a.gz + cc);
+    const float gz = FLAT ? 0.0f : __ldg(a.gz + cc);
     float win[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
@@ -423,32 +434,42 @@ __device__ __forceinline__ void march_w(const MomArgs &a, int tile, int j, int k
         const float rwn = __ldg(a.rrw + (kf + 1) * wz + o), dh = __ldg(a.divx + (kf - 1) * cz + cc);
         float *out = a.wten + kf * wz + o;
         const float ten = own ? *out : 0.0f;
-        const float scale = a.vmode == 2 ? __ldg(a.rrf0 + (kf - 1) * cz) : __ldg(a.rrf0 + (kf - 1) * cz + cc) * gz;
+        const float scale = FLAT ? __ldg(a.rrf0 + (kf - 1) * cz) : __ldg(a.rrf0 + (kf - 1) * cz + cc) * gz;
         const float c1 = 1.0f - c2;
         const float c2x = 0.5f * (kw + ke), c2s = 0.5f * (ks + c2), c2n = 0.5f * (c2 + kn);
         const float mw = c2x * ru + (1.0f - c2x) * rul;
         const float ms = c2s * rs + (1.0f - c2s) * rsl, mn = c2n * rn + (1.0f - c2n) * rnl;
         const float fw0 = up5(mw, px[0], px[1], px[2], px[3], px[4], px[5]);
-        const float fe0 = below(fw0), me = below(mw), rue = below(ru), rule = below(rul);
+        const float fe0 = below(fw0);
         const float fs0 = up5(ms, py[0], py[1], py[2], py[3], py[4], py[5]);
         const float fn0 = up5(mn, py[1], py[2], py[3], py[4], py[5], py[6]);
-        const float fw = wo && mw >= 0.0f ? fe0 : fw0, fe = eo && me <= 0.0f ? fw0 : fe0;
-        const float fs = so && ms >= 0.0f ? fn0 : fs0, fn = no && mn <= 0.0f ? fs0 : fn0;
         shift(win, next);
-        const float zhi = w_z(win, 0.5f * (rw + rwn), kf, nk);
-        const float dfx = -(fe - fw), dfy = -(fn - fs);
-        float advx = a.vmode == 2 ? (dfx * a.rdx) * uh : dfx * (a.rdx * uh);
-        float advy = a.vmode == 2 ? (dfy * a.rdy) * vh : dfy * (a.rdy * vh);
-        // the open sides' corrections weigh with the cell's own c2
-        if ((wo && c2 * ru + c1 * rul >= 0.0f) || (eo && c2 * rue + c1 * rule <= 0.0f)) {
-            const float corr = c1 * (rule - rul) + c2 * (rue - ru);
-            advx = advx - bcorr(a, wc, corr, a.rdx, uh);
+        const float mz = 0.5f * (rw + rwn);
+        float advx, advy, zhi;
+        if (!edge && kf > 2 && kf < nk - 1) {
+            zhi = up5(mz, win[0], win[1], win[2], win[3], win[4], win[5]);
+            const float dfx = -(fe0 - fw0), dfy = -(fn0 - fs0);
+            advx = FLAT ? (dfx * a.rdx) * uh : dfx * (a.rdx * uh);
+            advy = FLAT ? (dfy * a.rdy) * vh : dfy * (a.rdy * vh);
+        } else {
+            const float me = below(mw), rue = below(ru), rule = below(rul);
+            const float fw = wo && mw >= 0.0f ? fe0 : fw0, fe = eo && me <= 0.0f ? fw0 : fe0;
+            const float fs = so && ms >= 0.0f ? fn0 : fs0, fn = no && mn <= 0.0f ? fs0 : fn0;
+            zhi = w_z(win, mz, kf, nk);
+            const float dfx = -(fe - fw), dfy = -(fn - fs);
+            advx = FLAT ? (dfx * a.rdx) * uh : dfx * (a.rdx * uh);
+            advy = FLAT ? (dfy * a.rdy) * vh : dfy * (a.rdy * vh);
+            // the open sides' corrections weigh with the cell's own c2
+            if ((wo && c2 * ru + c1 * rul >= 0.0f) || (eo && c2 * rue + c1 * rule <= 0.0f)) {
+                const float corr = c1 * (rule - rul) + c2 * (rue - ru);
+                advx = advx - bcorr<FLAT>(wc, corr, a.rdx, uh);
+            }
+            if ((so && c2 * rs + c1 * rsl >= 0.0f) || (no && c2 * rn + c1 * rnl <= 0.0f)) {
+                const float corr = c1 * (rnl - rsl) + c2 * (rn - rs);
+                advy = advy - bcorr<FLAT>(wc, corr, a.rdy, vh);
+            }
         }
-        if ((so && c2 * rs + c1 * rsl >= 0.0f) || (no && c2 * rn + c1 * rnl <= 0.0f)) {
-            const float corr = c1 * (rnl - rsl) + c2 * (rn - rs);
-            advy = advy - bcorr(a, wc, corr, a.rdy, vh);
-        }
-        const float advz = zface(a, -(zhi - zlo), kf);
+        const float advz = zface<FLAT>(a, -(zhi - zlo), kf);
         float total = (advx + advy) + advz;
         total = total + wc * (c2 * dh + c1 * dl);
         if (own) *out = ten + total * scale;
@@ -456,18 +477,22 @@ __device__ __forceinline__ void march_w(const MomArgs &a, int tile, int j, int k
     }
 }
 
-__global__ void __launch_bounds__(32 * kMomRows, 8) mom5_adv_kernel(MomArgs a, int levels_per_chunk) {
+// (lines of points away from open sides, at levels away from the column's
+// ends, take a finish without those branches)
+template <bool FLAT>
+__global__ void __launch_bounds__(32 * kMomRows, 8) mom5_adv_kernel(const __grid_constant__ MomArgs a,
+                                                                     int levels_per_chunk) {
     // all tiles in one grid dimension, which takes any plane
     const int tiles = a.ni / kMomOut + 1, bt = blockIdx.x / 3;
     const int tile = bt % tiles, row = bt / tiles * kMomRows + threadIdx.y;
     const int k_lo = 1 + blockIdx.y * levels_per_chunk, k_hi = min(a.nk, k_lo + levels_per_chunk - 1);
     const int component = blockIdx.x % 3;
     if (component == 0)
-        march_u(a, tile, row, k_lo, k_hi);
+        march_u<FLAT>(a, tile, row, k_lo, k_hi);
     else if (component == 1)
-        march_v(a, tile, row, k_lo, k_hi);
+        march_v<FLAT>(a, tile, row, k_lo, k_hi);
     else
-        march_w(a, tile, row, k_lo, k_hi);
+        march_w<FLAT>(a, tile, row, k_lo, k_hi);
 }
 
 bool launch_ok(const char *what) {
@@ -587,7 +612,11 @@ int enqueue_transport(const MomArgs &a, cudaStream_t st) {
     int chunk = a.nk;
     while (chunk > 4 && 3LL * tiles * (a.nj + 1) * ((a.nk + chunk - 1) / chunk) < 2LL * 148 * 24) chunk = (chunk + 1) / 2;
     ProfScope ps("mom5_adv_kernel", st);
-    mom5_adv_kernel<<<dim3(3 * tiles * ytiles, (a.nk + chunk - 1) / chunk), dim3(32, kMomRows), 0, st>>>(a, chunk);
+    const dim3 grid(3 * tiles * ytiles, (a.nk + chunk - 1) / chunk), block(32, kMomRows);
+    if (a.vmode == 2)
+        mom5_adv_kernel<true><<<grid, block, 0, st>>>(a, chunk);
+    else
+        mom5_adv_kernel<false><<<grid, block, 0, st>>>(a, chunk);
     ps.stop();
     return launch_ok("mom5_adv_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }
