@@ -107,6 +107,16 @@ class ProfScope {
     cudaEvent_t start_;
 };
 
+// the composed step's own launches: several open fills (GM1B_FILL_*) at once,
+// and theta with the three moisture rows packed into their filled carriers
+struct OpenFill {
+    int kind;
+    float *q;
+};
+int32_t open_fills(int32_t ni, int32_t nj, int32_t nk, const OpenFill *fills, int n, cudaStream_t st);
+int32_t pack_scalars_open(int32_t ni, int32_t nj, int32_t nk, const float *th0, const float *const scalar[4],
+                          float *const padded[4], cudaStream_t st);
+
 }  // namespace gm1b
 
 // thread-local error message of the last failed entry point

@@ -7,8 +7,9 @@
 // :1635-1685; the Kessler transition, src/cm1core/cuda_gm1_kessler_large_step.py:183;
 // solve3, src/cm1core/cuda_cartesian_finish.py:739).
 //
-// The same launches in the same order as the package's Python composition
-// (gm1_b200.moist_step.MoistLargeStep), so the two give the same words; the
+// The same operators in the same order as the package's Python composition
+// (gm1_b200.moist_step.MoistLargeStep), so the two give the same words (here
+// the fills and packs of a phase share launches); the
 // uniform column runs the terrain operator family on flat metrics, a
 // stretched column the flat (terrain_flag=.false.) family.  Each RK stage's
 // theta and moisture advection, momentum/pressure boundaries and TKE stage
@@ -344,8 +345,8 @@ int pre_acoustic(Step &h, int nrk, cudaStream_t st) {
     gm1b_eqtset2_arrays e{s.th0, s.qv0, s.pi0, nullptr, nullptr, s.th3d, s.q3d, s.pp3d,
                           s.thv, s.ppterm, s.dum8, s.thterm, s.piadv};
     TRY(gm1b_eqtset2_stage_terms(c.ni, c.nj, c.nk, &e, 0, st));
-    TRY(gm1b_open_fill(c.ni, c.nj, c.nk, 0, s.thv, st));   // pressure
-    TRY(gm1b_open_fill(c.ni, c.nj, c.nk, 1, s.dum8, st));  // scalar
+    const OpenFill fills[2] = {{GM1B_FILL_PRESSURE, s.thv}, {GM1B_FILL_SCALAR, s.dum8}};
+    TRY(open_fills(c.ni, c.nj, c.nk, fills, 2, st));
     TRY(zero(s.uten, z.u * sizeof(float), st, "zero uten"));
     TRY(zero(s.vten, z.v * sizeof(float), st, "zero vten"));
     TRY(zero(s.wten, z.w * sizeof(float), st, "zero wten"));
@@ -421,11 +422,7 @@ int advect(Step &h, float *padded, float *tendency, double weps, int nrk, cudaSt
 }
 
 int theta_advection(Step &h, int nrk, cudaStream_t st) {
-    const gm1b_moist_step_config &c = h.c;
     const gm1b_moist_state &s = h.s;
-    TRY(gm1b_theta_transport_pack(c.ni, c.nj, c.nk, s.th0, s.th3d, s.theta_padded, st));
-    TRY(gm1b_open_fill(c.ni, c.nj, c.nk, 1, s.theta_padded, st));
-    TRY(zero(s.theta_adv, Sizes(c).mass * sizeof(float), st, "zero theta_adv"));
     return advect(h, s.theta_padded, s.theta_adv, weps_of(10.0f), nrk, st);
 }
 
@@ -448,11 +445,7 @@ int species_advection(Step &h, int r, int nrk, cudaStream_t st) {
     const gm1b_moist_metrics &m = h.m;
     const Sizes z(c);
     const Species sp = species(h, r);
-    float *q = s.q3d + (size_t)r * z.mass;
     float *adv = s.moist_adv + (size_t)r * z.mass;
-    TRY(gm1b_pack_scalar(c.ni, c.nj, c.nk, q, sp.padded, st));
-    TRY(gm1b_open_fill(c.ni, c.nj, c.nk, 1, sp.padded, st));
-    TRY(zero(adv, z.mass * sizeof(float), st, "zero moist_adv"));
     const double weps = weps_of(1.0e-2f);
     if (nrk < 3) return advect(h, sp.padded, adv, weps, nrk, st);
     gm1b_pdef_chain_arrays a{s.qa + (size_t)r * z.mass, sp.padded, m.rho0_3d, m.gz, m.rgz, m.rr0, m.c1, m.c2,
@@ -475,6 +468,14 @@ int record_wait(cudaEvent_t ev, cudaStream_t from, cudaStream_t to) {
 int scalar_moist(Step &h, int nrk, cudaStream_t st) {
     const gm1b_moist_step_config &c = h.c;
     const gm1b_moist_state &s = h.s;
+    {
+        // every scalar's carrier in one launch; the advections write whole
+        // tendencies on these whole-domain sides, so nothing is zeroed
+        const size_t mass = Sizes(c).mass;
+        const float *scalar[4] = {s.th3d, s.q3d, s.q3d + mass, s.q3d + 2 * mass};
+        float *padded[4] = {s.theta_padded, species(h, 0).padded, species(h, 1).padded, species(h, 2).padded};
+        TRY(pack_scalars_open(c.ni, c.nj, c.nk, s.th0, scalar, padded, st));
+    }
     if (c.concurrent) {
         // fork the theta and species lanes from st, join them back
         TRY(ok(cudaEventRecord(h.ev[0], st), "cudaEventRecord") ? GM1B_OK : GM1B_ERR_CUDA);
@@ -493,18 +494,17 @@ int scalar_moist(Step &h, int nrk, cudaStream_t st) {
     return gm1b_scalar_moist_rk_compose(z.mass, kNumq, &a, nrk, c.dt, st);
 }
 
-int momentum_boundaries(Step &h, cudaStream_t st) {
+// the momentum boundaries, and between the stages pi's
+int boundaries(Step &h, int nrk, cudaStream_t st) {
     const gm1b_moist_step_config &c = h.c;
     const gm1b_moist_state &s = h.s;
     const gm1b_moist_metrics &m = h.m;
-    TRY(gm1b_open_fill(c.ni, c.nj, c.nk, 2, s.u3d, st));
-    TRY(gm1b_open_fill(c.ni, c.nj, c.nk, 3, s.v3d, st));
-    TRY(gm1b_open_fill(c.ni, c.nj, c.nk, 4, s.w3d, st));
+    const OpenFill fills[4] = {
+        {GM1B_FILL_U, s.u3d}, {GM1B_FILL_V, s.v3d}, {GM1B_FILL_W, s.w3d}, {GM1B_FILL_PRESSURE, s.pp3d}};
+    TRY(open_fills(c.ni, c.nj, c.nk, fills, nrk < 3 ? 4 : 3, st));
     if (c.stretched) return GM1B_OK;  // solve2.F:1676: bcwsfc is a terrain_flag statement
     return gm1b_bcwsfc(c.ni, c.nj, c.nk, s.u3d, s.v3d, s.w3d, m.gz, m.dzdx, m.dzdy, st);
 }
-
-int scalar_boundaries(Step &h, cudaStream_t st) { return gm1b_open_fill(h.c.ni, h.c.nj, h.c.nk, 0, h.s.pp3d, st); }
 
 int tke_rk(Step &h, int nrk, cudaStream_t st) {
     const gm1b_moist_step_config &c = h.c;
@@ -523,8 +523,7 @@ int tke_rk(Step &h, int nrk, cudaStream_t st) {
 int stage_tail(Step &h, int nrk, cudaStream_t st) {
     if (!h.c.concurrent) {
         TRY(scalar_moist(h, nrk, st));
-        TRY(momentum_boundaries(h, st));
-        if (nrk < 3) TRY(scalar_boundaries(h, st));
+        TRY(boundaries(h, nrk, st));
         return tke_rk(h, nrk, st);
     }
     cudaStream_t bnd = h.side[1 + kNumq], tke = h.side[2 + kNumq];
@@ -532,8 +531,7 @@ int stage_tail(Step &h, int nrk, cudaStream_t st) {
     TRY(ok(cudaStreamWaitEvent(bnd, h.ev[8], 0), "cudaStreamWaitEvent") ? GM1B_OK : GM1B_ERR_CUDA);
     TRY(ok(cudaStreamWaitEvent(tke, h.ev[8], 0), "cudaStreamWaitEvent") ? GM1B_OK : GM1B_ERR_CUDA);
     TRY(scalar_moist(h, nrk, st));
-    TRY(momentum_boundaries(h, bnd));
-    if (nrk < 3) TRY(scalar_boundaries(h, bnd));
+    TRY(boundaries(h, nrk, bnd));
     TRY(tke_rk(h, nrk, tke));
     TRY(record_wait(h.ev[9], bnd, st));
     return record_wait(h.ev[10], tke, st);

@@ -12,9 +12,12 @@
 //   solve3 density                                  src/cm1core/cuda_gm1_forecast.py:548 (gm1_solve3_density_v1)
 //
 // Design (B200): each piece is an elementwise or per-line pass with the
-// reference's operation order; the open fills run as the reference's two
-// ordered passes (first direction of the family, then the second), so a
-// halo corner takes the words CM1's sequential loops leave there.
+// reference's operation order; an open fill leaves in one launch the words of
+// the reference's two ordered passes (first direction of the family, then
+// the second), the halo corners among them.
+#include <algorithm>
+#include <cmath>
+
 #include "gm1b_common.cuh"
 #include "weno.cuh"
 
@@ -49,41 +52,101 @@ struct FillGeom {
     int nk;
 };
 
-// one pass: ew = 1 fills the west/east halo columns of rows y0-1..yl+1,
-// ew = 0 the south/north halo rows of columns x0-1..xl+1
-__global__ void __launch_bounds__(256) open_fill_pass_kernel(FillGeom f, int ew, int zero) {
-    const int nlev = f.k1 - f.k0 + 1;
-    const unsigned lines = ew ? (unsigned)(f.yl - f.y0 + 3) : (unsigned)(f.xl - f.x0 + 3);
-    const unsigned per = lines * (unsigned)(2 * f.g);
-    const unsigned total = per * nlev;
-    const unsigned plane = (unsigned)f.ny * f.nx;
-    for (unsigned z = (unsigned)blockIdx.x * blockDim.x + threadIdx.x; z < total; z += (unsigned)gridDim.x * blockDim.x) {
-        const int h = (int)(z % (2 * f.g));
-        const int l = (int)((z / (2 * f.g)) % lines);
-        const int k = (int)(z / per) + f.k0;
-        float *lev = f.q + (unsigned)k * plane;
-        if (ew) {
-            const int y = f.y0 - 1 + l;
-            const int x = h < f.g ? f.x0 - f.g + h : f.xl + 1 + (h - f.g);
-            const int src = h < f.g ? f.x0 : f.xl;
-            lev[(unsigned)y * f.nx + x] = lev[(unsigned)y * f.nx + src];
-        } else {
-            const int x = f.x0 - 1 + l;
-            const int y = h < f.g ? f.y0 - f.g + h : f.yl + 1 + (h - f.g);
-            const int src = h < f.g ? f.y0 : f.yl;
-            lev[(unsigned)y * f.nx + x] = lev[(unsigned)src * f.nx + x];
+// The reference fills in two ordered passes: the family's first direction
+// over the rows (columns) y0-1..yl+1, then the second.  One launch leaves the
+// same words: every halo word is a live edge word of its row or column (the
+// diagonal words of the first ring: of the corner cell), except the words
+// beyond the first ring beside a first-ring corner, which the first pass
+// copies from the halo word the second pass then overwrites; the thread that
+// overwrites it copies it first.
+__device__ __forceinline__ void fill_word(const FillGeom &f, unsigned z) {
+    const unsigned w = (unsigned)(f.xl - f.x0 + 1), h = (unsigned)(f.yl - f.y0 + 1), g2 = 2u * f.g;
+    const unsigned na = h * g2, nb = w * g2, per = na + nb + 2 * g2;
+    unsigned r = z % per;
+    float *lev = f.q + ((unsigned)f.k0 + z / per) * (unsigned)f.ny * (unsigned)f.nx;
+    auto word = [&](int y, int x) -> float & { return lev[(unsigned)y * (unsigned)f.nx + (unsigned)x]; };
+    auto halo_x = [&](int q) { return q < f.g ? f.x0 - f.g + q : f.xl + 1 + q - f.g; };
+    auto halo_y = [&](int q) { return q < f.g ? f.y0 - f.g + q : f.yl + 1 + q - f.g; };
+    if (r < na) {  // west and east of the live rows
+        const int q = (int)(r % g2), y = f.y0 + (int)(r / g2), x = halo_x(q);
+        if (!f.ew_first && (x == f.x0 - 1 || x == f.xl + 1) && (y == f.y0 || y == f.yl)) {
+            const float old = word(y, x);
+            for (int t = 2; t <= f.g; ++t) {
+                if (y == f.y0) word(f.y0 - t, x) = old;
+                if (y == f.yl) word(f.yl + t, x) = old;
+            }
+        }
+        word(y, x) = word(y, q < f.g ? f.x0 : f.xl);
+        return;
+    }
+    r -= na;
+    if (r < nb) {  // south and north of the live columns
+        const int q = (int)(r / w), x = f.x0 + (int)(r % w), y = halo_y(q);
+        if (f.ew_first && (y == f.y0 - 1 || y == f.yl + 1) && (x == f.x0 || x == f.xl)) {
+            const float old = word(y, x);
+            for (int t = 2; t <= f.g; ++t) {
+                if (x == f.x0) word(y, f.x0 - t) = old;
+                if (x == f.xl) word(y, f.xl + t) = old;
+            }
+        }
+        word(y, x) = word(q < f.g ? f.y0 : f.yl, x);
+        return;
+    }
+    r -= nb;  // beside the corners: the second direction's halo of the first ring
+    const int q = (int)(r / 2);
+    const bool hi = r % 2 != 0;
+    if (f.ew_first)
+        word(halo_y(q), hi ? f.xl + 1 : f.x0 - 1) = word(q < f.g ? f.y0 : f.yl, hi ? f.xl : f.x0);
+    else
+        word(hi ? f.yl + 1 : f.y0 - 1, halo_x(q)) = word(hi ? f.yl : f.y0, q < f.g ? f.x0 : f.xl);
+}
+
+constexpr int kMostFills = 4;
+struct Fills {
+    FillGeom f[kMostFills];
+    unsigned words[kMostFills];  // fill_word's of each
+    int n;
+};
+
+__global__ void __launch_bounds__(256) open_fill_kernel(const __grid_constant__ Fills a) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (int q = 0; q < a.n; ++q) {
+        const FillGeom &f = a.f[q];
+        for (unsigned z = t; z < a.words[q]; z += step) fill_word(f, z);
+        if (f.zero_w) {
+            const unsigned rows = (unsigned)(f.yl - f.y0 + 3), cols = (unsigned)(f.xl - f.x0 + 3);
+            for (unsigned z = t; z < 2 * rows * cols; z += step) {
+                const int x = f.x0 - 1 + (int)(z % cols);
+                const int y = f.y0 - 1 + (int)((z / cols) % rows);
+                const int k = z / (rows * cols) == 0 ? 1 : f.nk + 1;
+                f.q[((unsigned)k * (unsigned)f.ny + (unsigned)y) * (unsigned)f.nx + (unsigned)x] = 0.0f;
+            }
         }
     }
-    if (zero) {
-        const unsigned rows = (unsigned)(f.yl - f.y0 + 3), cols = (unsigned)(f.xl - f.x0 + 3);
-        for (unsigned z = (unsigned)blockIdx.x * blockDim.x + threadIdx.x; z < 2 * rows * cols;
-             z += (unsigned)gridDim.x * blockDim.x) {
-            const int x = f.x0 - 1 + (int)(z % cols);
-            const int y = f.y0 - 1 + (int)((z / cols) % rows);
-            const int k = z / (rows * cols) == 0 ? 1 : f.nk + 1;
-            f.q[(unsigned)k * plane + (unsigned)y * f.nx + x] = 0.0f;
-        }
-    }
+}
+
+// theta (th0 - 300 + th3d) and the moisture rows into their padded arrays,
+// the halos of levels 1..nk as the open scalar fill leaves them, one launch
+struct PackScalars {
+    const float *th0, *scalar[4];  // th3d, then the moisture rows
+    float *padded[4];
+};
+
+__global__ void __launch_bounds__(256) pack_scalars_kernel(const __grid_constant__ PackScalars a, int ni, int nj) {
+    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y, k = blockIdx.z;
+    const int px = ni + 6, py = nj + 6;
+    if (x >= px || y >= py) return;
+    if ((y < 3 || y > nj + 2) && (x < 2 || x > ni + 3)) return;  // words no fill writes
+    const unsigned c = ((unsigned)k * nj + (unsigned)(min(max(y, 3), nj + 2) - 3)) * (unsigned)ni +
+                       (unsigned)(min(max(x, 3), ni + 2) - 3);
+    const unsigned d = ((unsigned)(k + 1) * py + y) * (unsigned)px + x;
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = __ldg(a.scalar[q] + c);
+    const float base = __ldg(a.th0 + k) - 300.0f;
+    a.padded[0][d] = base + v[0];
+#pragma unroll
+    for (int q = 1; q < 4; ++q) a.padded[q][d] = v[q];
 }
 
 bool fill_geometry(int kind, int ni, int nj, int nk, float *q, FillGeom &f) {
@@ -754,6 +817,39 @@ bool grid_ok(int ni, int nj, int nk, int mi, int mj, int mk, const char *what) {
 }
 }  // namespace
 
+namespace gm1b {
+
+int32_t open_fills(int32_t ni, int32_t nj, int32_t nk, const OpenFill *fills, int n, cudaStream_t st) {
+    Fills a{};
+    size_t work = 0;
+    for (int q = 0; q < n; ++q) {
+        FillGeom &f = a.f[q];
+        if (n > kMostFills || !fill_geometry(fills[q].kind, ni, nj, nk, fills[q].q, f)) return GM1B_ERR_ARGUMENT;
+        const size_t per = ((size_t)(f.xl - f.x0 + 1) + (size_t)(f.yl - f.y0 + 1) + 2) * 2 * f.g;
+        a.words[q] = f.k1 >= f.k0 ? (unsigned)(per * (size_t)(f.k1 - f.k0 + 1)) : 0u;
+        work = std::max(work, (size_t)a.words[q]);
+        if (f.zero_w) work = std::max(work, (size_t)2 * (f.yl - f.y0 + 3) * (f.xl - f.x0 + 3));
+    }
+    a.n = n;
+    ProfScope ps("open_fill_kernel", st);
+    open_fill_kernel<<<grid_for(work), 256, 0, st>>>(a);
+    ps.stop();
+    return launch_ok("open_fill_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
+}
+
+int32_t pack_scalars_open(int32_t ni, int32_t nj, int32_t nk, const float *th0, const float *const scalar[4],
+                          float *const padded[4], cudaStream_t st) {
+    PackScalars a{};
+    a.th0 = th0;
+    for (int q = 0; q < 4; ++q) a.scalar[q] = scalar[q], a.padded[q] = padded[q];
+    ProfScope ps("pack_scalars_kernel", st);
+    pack_scalars_kernel<<<dim3((ni + 6 + 31) / 32, (nj + 6 + 7) / 8, nk), dim3(32, 8), 0, st>>>(a, ni, nj);
+    ps.stop();
+    return launch_ok("pack_scalars_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
+}
+
+}  // namespace gm1b
+
 extern "C" int32_t gm1b_open_fill(int32_t ni, int32_t nj, int32_t nk, int32_t kind, float *q, void *stream) {
     FillGeom f;
     if (q == nullptr || !grid_ok(ni, nj, nk, 2, 2, 2, "gm1b_open_fill") || !fill_geometry(kind, ni, nj, nk, q, f)) {
@@ -761,16 +857,8 @@ extern "C" int32_t gm1b_open_fill(int32_t ni, int32_t nj, int32_t nk, int32_t ki
             gm1b_set_error("gm1b_open_fill: need an array and a GM1B_FILL_* kind");
         return GM1B_ERR_ARGUMENT;
     }
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const size_t work = (size_t)(nk + 2) * (size_t)(std::max(ni, nj) + 8) * 6;
-    for (int pass = 0; pass < 2; ++pass) {
-        const int ew = pass == 0 ? f.ew_first : !f.ew_first;
-        ProfScope ps("open_fill_pass_kernel", st);
-        open_fill_pass_kernel<<<grid_for(work), 256, 0, st>>>(f, ew, pass == 1 && f.zero_w);
-        ps.stop();
-        if (!launch_ok("open_fill_pass_kernel")) return GM1B_ERR_CUDA;
-    }
-    return GM1B_OK;
+    const OpenFill one{kind, q};
+    return open_fills(ni, nj, nk, &one, 1, static_cast<cudaStream_t>(stream));
 }
 
 namespace {

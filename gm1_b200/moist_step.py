@@ -779,8 +779,6 @@ class MoistLargeStep:
         met = {"c1": m["c1"], "c2": m["c2"], "rr0": m["rr0"], "gz": m["gz"]}
         theta_transport_scalar(s["th0"], s["th3d"], s["theta_padded"], **self.k3, stream=st)
         mo.open_fill(s["theta_padded"], "scalar", **self.k3, stream=st)
-        with torch.cuda.stream(st):
-            s["theta_adv"].zero_()
         self._advect(s["theta_padded"], flux, met, s["theta_adv"], theta_weps_f64(), nrk, st)
 
     def _advect(self, padded, flux, met, tendency, weps, nrk: int, st) -> None:
@@ -801,8 +799,6 @@ class MoistLargeStep:
         padded = self.species_scratch[r]["moisture_padded"]
         mo.pack_scalar(self.q_rows[r], padded, **self.k3, stream=st)
         mo.open_fill(padded, "scalar", **self.k3, stream=st)
-        with torch.cuda.stream(st):
-            s["moist_adv"][r].zero_()
         weps = moisture_weps_f64(r)
         if nrk < 3:
             self._advect(padded, {"rru": s["rru"], "rrv": s["rrv"], "rrw": s["rrw"]},
@@ -1132,7 +1128,7 @@ def _native_lib():
 class NativeMoistLargeStep:
     """The composed moist large step through the C ABI's whole-step entry
     point (gm1b_moist_step_create / gm1b_moist_large_step): one library call
-    per step, the same launches in the same order as MoistLargeStep, so the
+    per step, the same operators in the same order as MoistLargeStep, so the
     two leave the same words.  ``state`` and ``metrics`` are the device dicts
     MoistLargeStep takes; the scratch of moisture species 1 and 2 is
     allocated here (zero), everything else is the caller's."""
