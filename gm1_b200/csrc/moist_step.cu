@@ -265,19 +265,16 @@ struct Getdiv {
 
 template <int VM>
 __device__ __forceinline__ float gd_xu(const Getdiv &a, const Lane &L, int k, int j, int f) {
-    if (VM == 2) return a.rru[L.u(k, j + 3, f + 3)];
     return a.rru[L.u(k, j + 3, f + 3)] * a.rgzu[(unsigned)j * (L.ni + 1) + f];
 }
 template <int VM>
 __device__ __forceinline__ float gd_yv(const Getdiv &a, const Lane &L, int k, int f, int i) {
-    if (VM == 2) return a.rrv[L.v(k, f + 3, i + 3)];
     return a.rrv[L.v(k, f + 3, i + 3)] * a.rgzv[(unsigned)f * L.ni + i];
 }
 // transformed w on w levels (getdiv's own grouping: r1 = 0.5 (1 - r2), r2 = 0.5 r2)
 template <int VM>
 __device__ __forceinline__ float gd_wt(const Getdiv &a, const Lane &L, int kf, int j, int i) {
     if (kf == 1 || kf == L.nk + 1) return 0.0f;
-    if (VM == 2) return a.rrw[L.s(kf, j + 3, i + 3)];
     const bool pr = VM == 1;
     const float rds = pr ? a.rds[kf] : 1.0f / a.dz;
     const float sf = pr ? a.sigmaf[kf] : (float)(kf - 1) * a.dz, sm = pr ? a.sigma[kf - 1] : ((float)(kf - 1) - 0.5f) * a.dz;
@@ -301,14 +298,14 @@ __global__ void __launch_bounds__(256) msb_getdiv_kernel(Getdiv a, Lane L) {
         float d = (gd_xu<VM>(a, L, k, j, i + 1) - gd_xu<VM>(a, L, k, j, i)) * a.rdx +
                   (gd_yv<VM>(a, L, k, j + 1, i) - gd_yv<VM>(a, L, k, j, i)) * a.rdy;
         const float dw = gd_wt<VM>(a, L, k + 1, j, i) - gd_wt<VM>(a, L, k, j, i);
-        d = d + (VM == 2 ? (dw * a.rdzm) * a.mh[k] : dw * (VM == 1 ? a.rdsfp[k] : a.rdsf));
-        if (fabsf(d) < (VM == 2 ? 1.0e-30f : 1.0e-20f)) d = 0.0f;
+        d = d + dw * (VM == 1 ? a.rdsfp[k] : a.rdsf);
+        if (fabsf(d) < 1.0e-20f) d = 0.0f;
         a.div[z] = d;
         a.theta_div[z] = d * a.thterm[z];
     }
 }
 
-// vmode 1: base density from the padded rho0p; vmode 2: rho0p(k, 3, 3) alone
+// vmode 1: base density from the padded rho0p
 __global__ void __launch_bounds__(256) msb_getdivx_horizontal_kernel(const float *rho0, const float *rgzu,
                                                                     const float *rgzv, float *rru, float *rrv, Lane L,
                                                                     int vmode, const float *rho0p) {
@@ -318,10 +315,6 @@ __global__ void __launch_bounds__(256) msb_getdivx_horizontal_kernel(const float
         if (z < nu) {
             const int f = (int)(z % (ni + 1)), j = (int)((z / (ni + 1)) % nj), k = (int)(z / ((unsigned)(ni + 1) * nj)) + 1;
             const unsigned p = L.u(k, j + 3, f + 3);
-            if (vmode == 2) {
-                rru[p] = rru[p] * rho0p[L.s(k, 3, 3)];
-                continue;
-            }
             const int l = f == 0 ? 0 : f - 1, r = f == ni ? ni - 1 : f;
             const float den = vmode == 1 ? 0.5f * (rho0p[L.s(k, j + 3, f + 2)] + rho0p[L.s(k, j + 3, f + 3)])
                                          : 0.5f * (rho0[L.m(k - 1, j, l)] + rho0[L.m(k - 1, j, r)]);
@@ -330,10 +323,6 @@ __global__ void __launch_bounds__(256) msb_getdivx_horizontal_kernel(const float
             const unsigned q = z - nu;
             const int i = (int)(q % ni), f = (int)((q / ni) % (nj + 1)), k = (int)(q / ((unsigned)ni * (nj + 1))) + 1;
             const unsigned p = L.v(k, f + 3, i + 3);
-            if (vmode == 2) {
-                rrv[p] = rrv[p] * rho0p[L.s(k, 3, 3)];
-                continue;
-            }
             const int s = f == 0 ? 0 : f - 1, nn = f == nj ? nj - 1 : f;
             const float den = vmode == 1 ? 0.5f * (rho0p[L.s(k, f + 2, i + 3)] + rho0p[L.s(k, f + 3, i + 3)])
                                          : 0.5f * (rho0[L.m(k - 1, s, i)] + rho0[L.m(k - 1, nn, i)]);
@@ -358,10 +347,6 @@ __global__ void __launch_bounds__(256) msb_getdivx_vertical_kernel(const float *
             rrw[p] = 0.0f;
             continue;
         }
-        if (vmode == 2) {  // the flat column: rf0(1,1,k) rrw
-            rrw[p] = rrw[p] * rf0[L.m(kf - 1, 0, 0)];
-            continue;
-        }
         const float sf = pr ? sigmaf[kf] : (float)(kf - 1) * dz, sm = pr ? sigma[kf - 1] : ((float)(kf - 1) - 0.5f) * dz;
         float r2 = (sf - sm) * (pr ? rdsp[kf] : rds);
         const float r1 = 0.5f * (1.0f - r2);
@@ -376,18 +361,63 @@ __global__ void __launch_bounds__(256) msb_getdivx_vertical_kernel(const float *
     }
 }
 
+// The flat column's getdiv and getdivx divergences together, from the
+// averaged velocities before they are scaled to mass fluxes: seven words a
+// cell instead of ten in two passes.
+__global__ void __launch_bounds__(256) msb_flat_divergences_kernel(Getdiv a, const float *rho0p, const float *rf0,
+                                                                   float *divx, Lane L) {
+    // all tiles of a level in one grid dimension, which takes any plane
+    const int tiles = (L.ni + 31) / 32;
+    const int i = blockIdx.x % tiles * 32 + threadIdx.x, j = blockIdx.x / tiles * 8 + threadIdx.y;
+    if (i >= L.ni || j >= L.nj) return;
+    for (int k = blockIdx.y + 1; k <= L.nk; k += gridDim.y) {
+        const unsigned z = L.m(k - 1, j, i), u = L.u(k, j + 3, i + 3), v = L.v(k, j + 3, i + 3), w = L.s(k, j + 3, i + 3);
+        const float u0 = a.rru[u], u1 = a.rru[u + 1], v0 = a.rrv[v], v1 = a.rrv[v + (unsigned)(L.ni + 6)];
+        const float w0 = k == 1 ? 0.0f : a.rrw[w];
+        const float w1 = k == L.nk ? 0.0f : a.rrw[w + (unsigned)(L.nj + 6) * (unsigned)(L.ni + 6)];
+        const float mh = a.mh[k], r = rho0p[L.s(k, 3, 3)];
+        float d = (u1 - u0) * a.rdx + (v1 - v0) * a.rdy;
+        d = d + ((w1 - w0) * a.rdzm) * mh;
+        if (fabsf(d) < 1.0e-30f) d = 0.0f;
+        a.div[z] = d;
+        a.theta_div[z] = d * a.thterm[z];
+        const float m0 = k == 1 ? 0.0f : w0 * rf0[L.m(k - 1, 0, 0)], m1 = k == L.nk ? 0.0f : w1 * rf0[L.m(k, 0, 0)];
+        d = (u1 * r - u0 * r) * a.rdx + (v1 * r - v0 * r) * a.rdy;
+        d = d + ((m1 - m0) * a.rdzm) * mh;
+        divx[z] = fabsf(d) < 1.0e-30f ? 0.0f : d;
+    }
+}
+
+// the flat column's mass fluxes in place: rho0(1,1,k) u, rho0(1,1,k) v,
+// rf0(1,1,k) w with the two end levels of w zero
+__global__ void __launch_bounds__(256) msb_flat_mass_kernel(const float *rho0p, const float *rf0, float *rru, float *rrv,
+                                                            float *rrw, Lane L) {
+    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = ni / 32 + 1;
+    const int x = blockIdx.x % tiles * 32 + threadIdx.x, y = blockIdx.x / tiles * 8 + threadIdx.y;
+    if (x > ni || y > nj) return;
+    for (int k = blockIdx.y + 1; k <= nk + 1; k += gridDim.y) {
+        const unsigned u = L.u(k, y + 3, x + 3), v = L.v(k, y + 3, x + 3), w = L.s(k, y + 3, x + 3);
+        const bool du = k <= nk && y < nj, dv = k <= nk && x < ni, dw = x < ni && y < nj, end = k == 1 || k == nk + 1;
+        const float r = k <= nk ? rho0p[L.s(k, 3, 3)] : 0.0f, rf = end ? 0.0f : rf0[L.m(k - 1, 0, 0)];
+        const float fu = du ? rru[u] : 0.0f, fv = dv ? rrv[v] : 0.0f, fw = dw && !end ? rrw[w] : 0.0f;
+        if (du) rru[u] = fu * r;
+        if (dv) rrv[v] = fv * r;
+        if (dw) rrw[w] = end ? 0.0f : fw * rf;
+    }
+}
+
 __global__ void __launch_bounds__(256) msb_getdivx_divergence_kernel(const float *rru, const float *rrv,
                                                                     const float *rrw, float *divx, float rdx,
                                                                     float rdy, float rdsf, Lane L, int vmode,
-                                                                    const float *rdsfp, const float *mh, float rdzm) {
+                                                                    const float *rdsfp) {
     const unsigned n = (unsigned)L.nk * L.nj * L.ni;
     for (unsigned z = (unsigned)blockIdx.x * blockDim.x + threadIdx.x; z < n; z += (unsigned)gridDim.x * blockDim.x) {
         const int i = (int)(z % L.ni), j = (int)((z / L.ni) % L.nj), k = (int)(z / ((unsigned)L.ni * L.nj)) + 1;
         float d = (rru[L.u(k, j + 3, i + 4)] - rru[L.u(k, j + 3, i + 3)]) * rdx +
                   (rrv[L.v(k, j + 4, i + 3)] - rrv[L.v(k, j + 3, i + 3)]) * rdy;
         const float dw = rrw[L.s(k + 1, j + 3, i + 3)] - rrw[L.s(k, j + 3, i + 3)];
-        d = d + (vmode == 2 ? (dw * rdzm) * mh[k] : dw * (vmode == 1 ? rdsfp[k] : rdsf));
-        divx[z] = fabsf(d) < (vmode == 2 ? 1.0e-30f : 1.0e-20f) ? 0.0f : d;
+        d = d + dw * (vmode == 1 ? rdsfp[k] : rdsf);
+        divx[z] = fabsf(d) < 1.0e-20f ? 0.0f : d;
     }
 }
 
@@ -712,6 +742,270 @@ __global__ void __launch_bounds__(256) pdef_total_kernel(Pdef p, Lane L) {
 }
 
 // ---------------------------------------------------------------------------
+// the same chain for a caller that needs only its advection: two passes and
+// three words of scratch per cell (advx, advy, advz before any repair)
+// instead of ten passes through the face fluxes, the candidates and the
+// corrected rows
+// ---------------------------------------------------------------------------
+constexpr int kPdRows = 8;   // rows of y faces per CTA of the flux pass: 7 rows of cells
+constexpr int kPdOut = 31;   // cells a warp of 32 x faces completes
+constexpr int kRepOut = 28;   // cells a warp completes in the repair pass
+constexpr int kRepRows = 16;  // rows per CTA of the repair pass: 12 rows of cells
+
+// the upwind WENO flux at a face from the six points around it; nothing where
+// no point exceeds the smallness
+__device__ __forceinline__ float pdef_flux(float m, float s0, float s1, float s2, float s3, float s4, float s5,
+                                           double weps, float small) {
+    const bool pos = m >= 0.0f;
+    const float a = pos ? s0 : s5, b = pos ? s1 : s4, c = pos ? s2 : s3, d = pos ? s3 : s2, e = pos ? s4 : s1;
+    return max5abs(a, b, c, d, e) > small ? m * weno5(a, b, c, d, e, weps) : 0.0f;
+}
+
+// vertical flux at face f (2..nk) from levels f-3 .. f+2 (pdef_vertical_flux_kernel)
+__device__ __forceinline__ float pdef_zflux(const Pdef &p, const float win[6], float m, float c1, float c2, int f,
+                                            int nk, float small) {
+    const float ew = (float)p.weps;
+#define Q(l) win[(l) - f + 3]
+    float r;
+    if (f == 2) {
+        r = m >= 0.0f ? c1 * Q(f - 1) + c2 * Q(f) : upstrpd(Q(f + 1), Q(f), Q(f - 1), ew);
+    } else if (f == nk) {
+        r = m > 0.0f ? upstrpd(Q(f - 2), Q(f - 1), Q(f), ew) : c1 * Q(f - 1) + c2 * Q(f);
+    } else if (f == 3 && (p.pdefweno ? m > 0.0f : m >= 0.0f)) {
+        r = upstrpd(Q(f - 2), Q(f - 1), Q(f), ew);
+    } else if (f == nk - 1 && m < 0.0f) {
+        r = f == 3 ? upstrpd(Q(f - 2), Q(f - 1), Q(f), ew) : upstrpd(Q(f + 1), Q(f), Q(f - 1), ew);
+    } else {
+        const bool pos = m >= 0.0f;
+        const float a = pos ? Q(f - 3) : Q(f + 2), b = pos ? Q(f - 2) : Q(f + 1), c = pos ? Q(f - 1) : Q(f);
+        const float d = pos ? Q(f) : Q(f - 1), e = pos ? Q(f + 1) : Q(f - 2);
+        if (p.pdefweno && max5abs(a, b, c, d, e) <= small) return 0.0f;
+        r = weno5(a, b, c, d, e, p.weps);
+    }
+#undef Q
+    return m * r;
+}
+
+// Directional advection: a warp owns the x faces of one row and marches up a
+// chunk of levels as the WENO scalar advection does (x fluxes by shuffle, y
+// fluxes through shared memory, the vertical flux carried); the binary64
+// weights bound it where there is water.
+__global__ void __launch_bounds__(32 * kPdRows, 4) pdef_advection_kernel(const __grid_constant__ Pdef p, Lane L,
+                                                                          int levels_per_chunk, float small) {
+    __shared__ float s_fy[2][kPdRows][32], s_vm[2][kPdRows][32];
+    const int lane = threadIdx.x, ty = threadIdx.y;
+    const int ni = L.ni, nj = L.nj, nk = L.nk;
+    const int sx = ni + 6, sy = nj + 6, sz = sx * sy, uz = (ni + 7) * sy, vz = sx * (nj + 7), cz = ni * nj;
+    const int tiles = ni / kPdOut + 1, i0 = blockIdx.x % tiles * kPdOut + lane;
+    const int row = blockIdx.x / tiles * (kPdRows - 1) + ty;
+    // faces and rows past the domain repeat its last ones and store nothing
+    const int i = min(i0, ni), j = min(row, nj);
+    const bool cell = i0 < ni && row < nj && lane < kPdOut && ty < kPdRows - 1;
+    const int o = (j + 3) * sx + i + 3, ou = (j + 3) * (ni + 7) + i + 3, oc = min(j, nj - 1) * ni + min(i, ni - 1);
+    const bool wo = i0 == 0 && obc_side(p.obc, 0u) == 2u, eo = i0 + 1 == ni && obc_side(p.obc, 1u) == 2u;
+    const bool so = row == 0 && obc_side(p.obc, 2u) == 2u, no = row + 1 == nj && obc_side(p.obc, 3u) == 2u;
+    const int k_lo = 1 + blockIdx.y * levels_per_chunk, k_hi = min(nk, k_lo + levels_per_chunk - 1);
+    float win[6];  // levels k-3 .. k+2; shifted to k-2 .. k+3 for face k+1
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const int l = k_lo - 3 + q;
+        win[q] = l >= 0 && l <= nk + 1 ? __ldg(p.s + l * sz + o) : 0.0f;
+    }
+    auto zflux = [&](int f) {
+        const bool end = f == 2 || f == nk;
+        return pdef_zflux(p, win, __ldg(p.rrw + f * sz + o), end ? __ldg(p.c1 + (f - 1) * cz + oc) : 0.0f,
+                          end ? __ldg(p.c2 + (f - 1) * cz + oc) : 0.0f, f, nk, small);
+    };
+    float zlo = 0.0f;
+    if (k_lo >= 2 && cell) zlo = zflux(k_lo);
+#pragma unroll 1
+    for (int k = k_lo; k <= k_hi; ++k) {
+        const float *pt = p.s + k * sz + o;
+        float px[6], py[6];
+        const float sv = win[3];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            px[q] = q == 3 ? sv : __ldg(pt + (q - 3));
+            py[q] = q == 3 ? sv : __ldg(pt + (q - 3) * sx);
+        }
+        const float next = k + 3 <= nk + 1 ? __ldg(pt + 3 * sz) : 0.0f;
+        const float mw = __ldg(p.rru + k * uz + ou), ms = __ldg(p.rrv + k * vz + o);
+        const float fx = pdef_flux(mw, px[0], px[1], px[2], px[3], px[4], px[5], p.weps, small);
+        const float fy = pdef_flux(ms, py[0], py[1], py[2], py[3], py[4], py[5], p.weps, small);
+        s_fy[k & 1][ty][lane] = fy;
+        s_vm[k & 1][ty][lane] = ms;
+        float fw = fx, fe = __shfl_down_sync(0xffffffffu, fx, 1), fs = fy;
+        const float me = __shfl_down_sync(0xffffffffu, mw, 1);
+        __syncthreads();
+        const int up = min(ty + 1, kPdRows - 1);
+        float fn = s_fy[k & 1][up][lane];
+        const float mn = s_vm[k & 1][up][lane];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) win[q] = win[q + 1];
+        win[5] = next;
+        if (!cell) continue;
+        const float zhi = k < nk ? zflux(k + 1) : 0.0f;
+        const bool iw = wo && mw >= 0.0f, ie = eo && me <= 0.0f, js = so && ms >= 0.0f, jn = no && mn <= 0.0f;
+        if (iw) fw = fe;
+        if (ie) fe = fw;
+        if (js) fs = fn;
+        if (jn) fn = fs;
+        float axv = (fw - fe) * p.rdx, ayv = (fs - fn) * p.rdy;
+        if (iw) axv = axv - (sv * (me - mw)) * p.rdx;
+        if (ie) axv = axv - (sv * (me - mw)) * p.rdx;
+        if (js) ayv = ayv - (sv * (mn - ms)) * p.rdy;
+        if (jn) ayv = ayv - (sv * (mn - ms)) * p.rdy;
+        const unsigned z = (unsigned)(k - 1) * (unsigned)cz + (unsigned)oc;
+        p.ax[z] = axv;
+        p.ay[z] = ayv;
+        p.az[z] = pdef_zterm(p, k == 1 ? -zhi : k == nk ? zlo : zlo - zhi, k);
+        zlo = zhi;
+    }
+}
+
+// a cell's rho0 a, the product both its candidates and its repair start from
+__device__ __forceinline__ float pdef_r0a(const Pdef &p, unsigned level, unsigned q) {
+    return (p.vmode == 2 ? __ldg(p.rho0 + level) : __ldg(p.rho0 + q)) * __ldg(p.a + q);
+}
+
+// the share a negative candidate v between lo and hi takes of each neighbour
+__device__ __forceinline__ float pdef_share(float v, float lo, float hi) {
+    if (v >= 0.0f) return 0.0f;
+    const float sum = fmaxf(0.0f, lo) + fmaxf(0.0f, hi);
+    return sum > 1.0e-30f ? fmaxf(v, -sum) / sum : 0.0f;
+}
+
+// the repair's mass of a cell from the candidates of its line, c-2 .. c+2
+// (pdef_row_mass); false where there is none
+__device__ __forceinline__ bool pdef_mass(float ll, float l, float v, float r, float rr, float &mass) {
+    mass = 0.0f;
+    bool flag = false;
+    if (v < 0.0f) {
+        const float s = pdef_share(v, l, r);
+        if (s != 0.0f) {
+            const float sum = fmaxf(0.0f, l) + fmaxf(0.0f, r);
+            mass = 0.0f - sum * s;
+            flag = true;
+        }
+    } else if (v > 1.0e-30f) {
+        const float sl = pdef_share(l, ll, v), sr = pdef_share(r, v, rr);
+        if (sl != 0.0f) mass = mass + v * sl, flag = true;
+        if (sr != 0.0f) mass = mass + v * sr, flag = true;
+    }
+    return flag;
+}
+
+// Candidates, repair rows and the total in one pass.  Each candidate is
+// formed once: a warp's 32 lanes hold its row's (two of the boundary family's
+// cells, or of the next tiles', on either side of the 28 cells it completes)
+// and pass them by shuffle; the block's 16 rows hand theirs along y through
+// shared memory (two rows on either side of the 12 it completes form only
+// that); the z candidates of levels k-2 .. k+2 are carried up the column.
+__global__ void __launch_bounds__(32 * kRepRows, 2) pdef_repair_kernel(const __grid_constant__ Pdef p,
+                                                                        const __grid_constant__ Lane L,
+                                                                        int levels_per_chunk) {
+    __shared__ float s_y[2][kRepRows][32];
+    const int ni = L.ni, nj = L.nj, nk = L.nk, lane = threadIdx.x, ty = threadIdx.y;
+    const int tiles = (ni + kRepOut - 1) / kRepOut;
+    const int i0 = blockIdx.x % tiles * kRepOut + lane - 2;
+    const int j0 = blockIdx.x / tiles * (kRepRows - 4) + ty - 2;
+    const unsigned so = obc_side(p.obc, 2u), no = obc_side(p.obc, 3u);
+    // beyond the domain the boundary family's cell; further out, any
+    const int i = (int)pdef_cell(min(i0, ni + 1), ni, obc_side(p.obc, 0u), obc_side(p.obc, 1u));
+    const int j = (int)pdef_cell(min(j0, nj + 1), nj, so, no);
+    const bool row = ty >= 2 && ty < kRepRows - 2 && j0 < nj, own = row && lane >= 2 && lane < kRepOut + 2 && i0 < ni;
+    const unsigned cz = (unsigned)ni * nj, sz = (unsigned)(nj + 6) * (ni + 6), uz = (unsigned)(nj + 6) * (ni + 7),
+                   vz = (unsigned)(nj + 7) * (ni + 6);
+    const unsigned oc = (unsigned)j * ni + i, os = (unsigned)(j + 3) * (ni + 6) + (i + 3),
+                   ou = (unsigned)(j + 3) * (ni + 7) + (i + 3);
+    const bool flat = p.vmode == 2;
+    const float gz = flat ? 0.0f : __ldg(p.gz + oc), rgz = flat ? 0.0f : __ldg(p.rgz + oc);
+    const int k_lo = 1 + blockIdx.y * levels_per_chunk, k_hi = min(nk, k_lo + levels_per_chunk - 1);
+    auto step = [&](float r0a, float inc) { return flat ? r0a + inc : r0a + inc * gz; };
+    // z candidates and what the levels k .. k+2 need again
+    float zc[5], r0a[3], s[3], az[3], wlo = 0.0f;
+    auto z_cand = [&](int k, float w0, float w1, float ra, float sv, float dir) {
+        return step(ra, p.dt * (dir + pdef_zterm(p, sv * (w1 - w0), k)));
+    };
+    if (row) {
+        // levels k_lo-2 .. k_lo+1; the loop's first level adds k_lo+2
+        zc[0] = r0a[0] = s[0] = az[0] = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int k = k_lo - 2 + q;
+            float c = 0.0f, ra = 0.0f, sv = 0.0f, dir = 0.0f;
+            if (k >= 1 && k <= nk) {
+                const unsigned z = (unsigned)(k - 1) * cz + oc;
+                ra = pdef_r0a(p, (unsigned)(k - 1) * cz, z);
+                sv = __ldg(p.s + (unsigned)k * sz + os);
+                dir = __ldg(p.az + z);
+                wlo = __ldg(p.rrw + (unsigned)(k + 1) * sz + os);
+                c = z_cand(k, __ldg(p.rrw + (unsigned)k * sz + os), wlo, ra, sv, dir);
+            }
+            zc[q + 1] = c;
+            if (q >= 2) r0a[q - 1] = ra, s[q - 1] = sv, az[q - 1] = dir;
+        }
+    }
+#pragma unroll 1
+    for (int k = k_lo; k <= k_hi; ++k) {
+        const unsigned z = (unsigned)(k - 1) * cz + oc;
+        if (row) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) zc[q] = zc[q + 1];
+            r0a[0] = r0a[1], s[0] = s[1], az[0] = az[1];
+            r0a[1] = r0a[2], s[1] = s[2], az[1] = az[2];
+            zc[4] = 0.0f;
+            if (k + 2 <= nk) {
+                const float whi = __ldg(p.rrw + (unsigned)(k + 3) * sz + os);
+                r0a[2] = pdef_r0a(p, (unsigned)(k + 1) * cz, z + 2 * cz);
+                s[2] = __ldg(p.s + (unsigned)(k + 2) * sz + os);
+                az[2] = __ldg(p.az + z + 2 * cz);
+                zc[4] = z_cand(k + 2, wlo, whi, r0a[2], s[2], az[2]);
+                wlo = whi;
+            }
+        } else {
+            r0a[0] = pdef_r0a(p, (unsigned)(k - 1) * cz, z);
+            s[0] = __ldg(p.s + (unsigned)k * sz + os);
+        }
+        const unsigned v = (unsigned)k * vz + os, u = (unsigned)k * uz + ou;
+        const float v0 = __ldg(p.rrv + v), v1 = __ldg(p.rrv + v + (unsigned)(ni + 6)), ay = __ldg(p.ay + z);
+        const float sdy = (s[0] * (v1 - v0)) * p.rdy;
+        float yc = step(r0a[0], p.dt * (ay + sdy));
+        if ((j == 0 && so == 2u && v0 >= 0.0f) || (j + 1 == nj && no == 2u && v1 <= 0.0f)) yc = r0a[0];
+        s_y[k & 1][ty][lane] = yc;
+        __syncthreads();
+        if (!row) continue;
+        const float u0 = __ldg(p.rru + u), u1 = __ldg(p.rru + u + 1), ax = __ldg(p.ax + z);
+        const float sdx = (s[0] * (u1 - u0)) * p.rdx;
+        float xc = step(r0a[0], p.dt * (ax + sdx));
+        if (inflow_lo(i, p.obc, 0u, u0) || inflow_hi(i, ni, p.obc, 1u, u1)) xc = r0a[0];
+        const float xll = __shfl_up_sync(0xffffffffu, xc, 2), xl = __shfl_up_sync(0xffffffffu, xc, 1);
+        const float xr = __shfl_down_sync(0xffffffffu, xc, 1), xrr = __shfl_down_sync(0xffffffffu, xc, 2);
+        const float (*sy)[32] = s_y[k & 1];
+        const float yl = sy[ty - 1][lane], yr = sy[ty + 1][lane];
+        float dx = ax, dy = ay, dz = az[0], mass;
+        auto repaired = [&](float c, float m, float sd) {
+            float first = ((c + m) - r0a[0]) * p.rdt;
+            if (!flat) first = first * rgz;
+            return first - sd;
+        };
+        if (!(xl >= 0.0f && xc >= 0.0f && xr >= 0.0f) && pdef_mass(xll, xl, xc, xr, xrr, mass))
+            dx = repaired(xc, mass, sdx);
+        if (!(yl >= 0.0f && yc >= 0.0f && yr >= 0.0f) && pdef_mass(sy[ty - 2][lane], yl, yc, yr, sy[ty + 2][lane], mass))
+            dy = repaired(yc, mass, sdy);
+        if (!(zc[1] >= 0.0f && zc[2] >= 0.0f && zc[3] >= 0.0f) && pdef_mass(zc[0], zc[1], zc[2], zc[3], zc[4], mass)) {
+            const unsigned w = (unsigned)k * sz + os;
+            dz = repaired(zc[2], mass, pdef_zterm(p, s[0] * (__ldg(p.rrw + w + sz) - __ldg(p.rrw + w)), k));
+        }
+        if (own) {
+            float t = (dx + dy) + dz;
+            t = t + s[0] * __ldg(p.divx + z);
+            p.adv[z] = flat ? t * __ldg(p.rr0 + (unsigned)(k - 1) * cz) : (t * __ldg(p.rr0 + z)) * gz;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // held tendencies, solve3 density, scalar pack
 // ---------------------------------------------------------------------------
 struct Held {
@@ -937,11 +1231,26 @@ int32_t post_acoustic_launch(int32_t ni, int32_t nj, int32_t nk, const gm1b_post
              a->theta_divergence_term, rdx, rdy, rdsf, dz, zt, 0.0f, vmode,
              c ? c->sigma : nullptr, c ? c->sigmaf : nullptr, c ? c->rds : nullptr, c ? c->rdsf : nullptr,
              c ? c->mh : nullptr, c ? c->rdz : 0.0f};
+    if (vmode == 2) {
+        const dim3 block(32, 8);
+        {
+            ProfScope ps("msb_flat_divergences_kernel", st);
+            msb_flat_divergences_kernel<<<dim3((ni + 31) / 32 * ((nj + 7) / 8), std::min(nk, 65535)), block, 0, st>>>(
+                g, c->rho0_padded, a->rf0, a->divx, L);
+            ps.stop();
+        }
+        if (!launch_ok("msb_flat_divergences_kernel")) return GM1B_ERR_CUDA;
+        {
+            ProfScope ps("msb_flat_mass_kernel", st);
+            msb_flat_mass_kernel<<<dim3((ni / 32 + 1) * (nj / 8 + 1), std::min(nk + 1, 65535)), block, 0, st>>>(
+                c->rho0_padded, a->rf0, a->rru, a->rrv, a->rrw, L);
+            ps.stop();
+        }
+        return launch_ok("msb_flat_mass_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
+    }
     {
         ProfScope ps("msb_getdiv_kernel", st);
-        if (vmode == 2)
-            msb_getdiv_kernel<2><<<grid_for(n), 256, 0, st>>>(g, L);
-        else if (vmode == 1)
+        if (vmode == 1)
             msb_getdiv_kernel<1><<<grid_for(n), 256, 0, st>>>(g, L);
         else
             msb_getdiv_kernel<0><<<grid_for(n), 256, 0, st>>>(g, L);
@@ -966,7 +1275,7 @@ int32_t post_acoustic_launch(int32_t ni, int32_t nj, int32_t nk, const gm1b_post
     {
         ProfScope ps("msb_getdivx_divergence_kernel", st);
         msb_getdivx_divergence_kernel<<<grid_for(n), 256, 0, st>>>(a->rru, a->rrv, a->rrw, a->divx, rdx, rdy, rdsf, L,
-                                                                   vmode, g.rdsfp, g.mh, g.rdzm);
+                                                                   vmode, g.rdsfp);
         ps.stop();
     }
     return launch_ok("msb_getdivx_divergence_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
