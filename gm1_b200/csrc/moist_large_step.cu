@@ -451,13 +451,9 @@ int species_advection(Step &h, int r, int nrk, cudaStream_t st) {
     gm1b_pdef_chain_arrays a{s.qa + (size_t)r * z.mass, sp.padded, m.rho0_3d, m.gz, m.rgz, m.rr0, m.c1, m.c2,
                              s.divx, s.rru, s.rrv, s.rrw, sp.fx, sp.fy, sp.fz, sp.advx, sp.advy, sp.advz,
                              sp.candidate, adv};
-    const float dttmp = c.dt / (float)(4 - nrk);
-    if (c.stretched) {
-        const gm1b_vertical_column col = flat_vertical(h);
-        return gm1b_pdef_moisture_chain_column(c.ni, c.nj, c.nk, &a, dttmp, c.dx, c.dy, weps, h.obc, r == 0 ? 0 : 1,
-                                               &col, st);
-    }
-    return gm1b_pdef_moisture_chain(c.ni, c.nj, c.nk, &a, dttmp, c.dx, c.dy, c.dz, weps, h.obc, r == 0 ? 0 : 1, st);
+    const gm1b_vertical_column col = flat_vertical(h);
+    return gm1b_pdef_moisture_advection(c.ni, c.nj, c.nk, &a, c.dt / (float)(4 - nrk), c.dx, c.dy, c.dz, weps, h.obc,
+                                        r == 0 ? 0 : 1, c.stretched ? &col : nullptr, st);
 }
 
 int record_wait(cudaEvent_t ev, cudaStream_t from, cudaStream_t to) {

@@ -743,14 +743,14 @@ __global__ void __launch_bounds__(256) pdef_total_kernel(Pdef p, Lane L) {
 
 // ---------------------------------------------------------------------------
 // the same chain for a caller that needs only its advection: two passes and
-// three words of scratch per cell (advx, advy, advz before any repair)
-// instead of ten passes through the face fluxes, the candidates and the
-// corrected rows
+// four words of scratch per cell (advx, advy, advz before any repair and the
+// y candidate) instead of ten passes through the face fluxes, the candidates
+// and the corrected rows
 // ---------------------------------------------------------------------------
 constexpr int kPdRows = 8;   // rows of y faces per CTA of the flux pass: 7 rows of cells
 constexpr int kPdOut = 31;   // cells a warp of 32 x faces completes
-constexpr int kRepOut = 28;   // cells a warp completes in the repair pass
-constexpr int kRepRows = 16;  // rows per CTA of the repair pass: 12 rows of cells
+constexpr int kRepOut = 28;  // cells a warp of 32 lanes completes in the repair pass
+constexpr int kRepRows = 8;
 
 // the upwind WENO flux at a face from the six points around it; nothing where
 // no point exceeds the smallness
@@ -784,6 +784,11 @@ __device__ __forceinline__ float pdef_zflux(const Pdef &p, const float win[6], f
     }
 #undef Q
     return m * r;
+}
+
+// a cell's rho0 a, the product both its candidates and its repair start from
+__device__ __forceinline__ float pdef_r0a(const Pdef &p, unsigned level, unsigned q) {
+    return (p.vmode == 2 ? __ldg(p.rho0 + level) : __ldg(p.rho0 + q)) * __ldg(p.a + q);
 }
 
 // Directional advection: a warp owns the x faces of one row and marches up a
@@ -859,13 +864,12 @@ __global__ void __launch_bounds__(32 * kPdRows, 4) pdef_advection_kernel(const _
         p.ax[z] = axv;
         p.ay[z] = ayv;
         p.az[z] = pdef_zterm(p, k == 1 ? -zhi : k == nk ? zlo : zlo - zhi, k);
+        // the y candidate, whose neighbours lie in other rows
+        const float r0a = pdef_r0a(p, (unsigned)(k - 1) * (unsigned)cz, z);
+        const float inc = p.dt * (ayv + (sv * (mn - ms)) * p.rdy);
+        p.dum[z] = js || jn ? r0a : p.vmode == 2 ? r0a + inc : r0a + inc * __ldg(p.gz + oc);
         zlo = zhi;
     }
-}
-
-// a cell's rho0 a, the product both its candidates and its repair start from
-__device__ __forceinline__ float pdef_r0a(const Pdef &p, unsigned level, unsigned q) {
-    return (p.vmode == 2 ? __ldg(p.rho0 + level) : __ldg(p.rho0 + q)) * __ldg(p.a + q);
 }
 
 // the share a negative candidate v between lo and hi takes of each neighbour
@@ -895,31 +899,33 @@ __device__ __forceinline__ bool pdef_mass(float ll, float l, float v, float r, f
     return flag;
 }
 
-// Candidates, repair rows and the total in one pass.  Each candidate is
-// formed once: a warp's 32 lanes hold its row's (two of the boundary family's
-// cells, or of the next tiles', on either side of the 28 cells it completes)
-// and pass them by shuffle; the block's 16 rows hand theirs along y through
-// shared memory (two rows on either side of the 12 it completes form only
-// that); the z candidates of levels k-2 .. k+2 are carried up the column.
-__global__ void __launch_bounds__(32 * kRepRows, 2) pdef_repair_kernel(const __grid_constant__ Pdef p,
+// Candidates, repair rows and the total in one pass: the y candidates come
+// from the first pass, a warp's 32 lanes hold their row's x candidates (two
+// of the boundary family's cells, or of the next tiles', on either side of the
+// 28 cells it completes) and pass them by shuffle, the z candidates of levels
+// k-2 .. k+2 are carried up the column.  No barrier: warps are independent.
+// With the rows handed along y through shared memory instead (two halo rows
+// on either side of 12, a barrier a level) it took 1.07 ms at 640x768x80.
+__global__ void __launch_bounds__(32 * kRepRows, 4) pdef_repair_kernel(const __grid_constant__ Pdef p,
                                                                         const __grid_constant__ Lane L,
                                                                         int levels_per_chunk) {
-    __shared__ float s_y[2][kRepRows][32];
-    const int ni = L.ni, nj = L.nj, nk = L.nk, lane = threadIdx.x, ty = threadIdx.y;
+    const int ni = L.ni, nj = L.nj, nk = L.nk, lane = threadIdx.x;
     const int tiles = (ni + kRepOut - 1) / kRepOut;
-    const int i0 = blockIdx.x % tiles * kRepOut + lane - 2;
-    const int j0 = blockIdx.x / tiles * (kRepRows - 4) + ty - 2;
+    const int i0 = blockIdx.x % tiles * kRepOut + lane - 2, j = blockIdx.x / tiles * kRepRows + threadIdx.y;
+    if (j >= nj) return;  // whole warps
     const unsigned so = obc_side(p.obc, 2u), no = obc_side(p.obc, 3u);
     // beyond the domain the boundary family's cell; further out, any
     const int i = (int)pdef_cell(min(i0, ni + 1), ni, obc_side(p.obc, 0u), obc_side(p.obc, 1u));
-    const int j = (int)pdef_cell(min(j0, nj + 1), nj, so, no);
-    const bool row = ty >= 2 && ty < kRepRows - 2 && j0 < nj, own = row && lane >= 2 && lane < kRepOut + 2 && i0 < ni;
+    const bool own = lane >= 2 && lane < kRepOut + 2 && i0 < ni;
     const unsigned cz = (unsigned)ni * nj, sz = (unsigned)(nj + 6) * (ni + 6), uz = (unsigned)(nj + 6) * (ni + 7),
                    vz = (unsigned)(nj + 7) * (ni + 6);
     const unsigned oc = (unsigned)j * ni + i, os = (unsigned)(j + 3) * (ni + 6) + (i + 3),
                    ou = (unsigned)(j + 3) * (ni + 7) + (i + 3);
+    auto yrow = [&](int c) { return (unsigned)pdef_cell(c, nj, so, no) * (unsigned)ni + (unsigned)i; };
+    const unsigned ys = yrow(j - 1), yn = yrow(j + 1);
     const bool flat = p.vmode == 2;
     const float gz = flat ? 0.0f : __ldg(p.gz + oc), rgz = flat ? 0.0f : __ldg(p.rgz + oc);
+    const bool wo = i == 0 && obc_side(p.obc, 0u) == 2u, eo = i + 1 == ni && obc_side(p.obc, 1u) == 2u;
     const int k_lo = 1 + blockIdx.y * levels_per_chunk, k_hi = min(nk, k_lo + levels_per_chunk - 1);
     auto step = [&](float r0a, float inc) { return flat ? r0a + inc : r0a + inc * gz; };
     // z candidates and what the levels k .. k+2 need again
@@ -927,80 +933,71 @@ __global__ void __launch_bounds__(32 * kRepRows, 2) pdef_repair_kernel(const __g
     auto z_cand = [&](int k, float w0, float w1, float ra, float sv, float dir) {
         return step(ra, p.dt * (dir + pdef_zterm(p, sv * (w1 - w0), k)));
     };
-    if (row) {
-        // levels k_lo-2 .. k_lo+1; the loop's first level adds k_lo+2
-        zc[0] = r0a[0] = s[0] = az[0] = 0.0f;
+    // levels k_lo-2 .. k_lo+1; the loop's first level adds k_lo+2
+    zc[0] = r0a[0] = s[0] = az[0] = 0.0f;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int k = k_lo - 2 + q;
-            float c = 0.0f, ra = 0.0f, sv = 0.0f, dir = 0.0f;
-            if (k >= 1 && k <= nk) {
-                const unsigned z = (unsigned)(k - 1) * cz + oc;
-                ra = pdef_r0a(p, (unsigned)(k - 1) * cz, z);
-                sv = __ldg(p.s + (unsigned)k * sz + os);
-                dir = __ldg(p.az + z);
-                wlo = __ldg(p.rrw + (unsigned)(k + 1) * sz + os);
-                c = z_cand(k, __ldg(p.rrw + (unsigned)k * sz + os), wlo, ra, sv, dir);
-            }
-            zc[q + 1] = c;
-            if (q >= 2) r0a[q - 1] = ra, s[q - 1] = sv, az[q - 1] = dir;
+    for (int q = 0; q < 4; ++q) {
+        const int k = k_lo - 2 + q;
+        float c = 0.0f, ra = 0.0f, sv = 0.0f, dir = 0.0f;
+        if (k >= 1 && k <= nk) {
+            const unsigned z = (unsigned)(k - 1) * cz + oc;
+            ra = pdef_r0a(p, (unsigned)(k - 1) * cz, z);
+            sv = __ldg(p.s + (unsigned)k * sz + os);
+            dir = __ldg(p.az + z);
+            wlo = __ldg(p.rrw + (unsigned)(k + 1) * sz + os);
+            c = z_cand(k, __ldg(p.rrw + (unsigned)k * sz + os), wlo, ra, sv, dir);
         }
+        zc[q + 1] = c;
+        if (q >= 2) r0a[q - 1] = ra, s[q - 1] = sv, az[q - 1] = dir;
     }
 #pragma unroll 1
     for (int k = k_lo; k <= k_hi; ++k) {
-        const unsigned z = (unsigned)(k - 1) * cz + oc;
-        if (row) {
+        const unsigned level = (unsigned)(k - 1) * cz, z = level + oc, u = (unsigned)k * uz + ou;
+        const float yl = __ldg(p.dum + level + ys), yc = __ldg(p.dum + z), yr = __ldg(p.dum + level + yn);
+        const float u0 = __ldg(p.rru + u), u1 = __ldg(p.rru + u + 1);
+        const float ax = __ldg(p.ax + z), ay = __ldg(p.ay + z), div = __ldg(p.divx + z);
+        const float rr0 = __ldg(p.rr0 + (flat ? level : z));
 #pragma unroll
-            for (int q = 0; q < 4; ++q) zc[q] = zc[q + 1];
-            r0a[0] = r0a[1], s[0] = s[1], az[0] = az[1];
-            r0a[1] = r0a[2], s[1] = s[2], az[1] = az[2];
-            zc[4] = 0.0f;
-            if (k + 2 <= nk) {
-                const float whi = __ldg(p.rrw + (unsigned)(k + 3) * sz + os);
-                r0a[2] = pdef_r0a(p, (unsigned)(k + 1) * cz, z + 2 * cz);
-                s[2] = __ldg(p.s + (unsigned)(k + 2) * sz + os);
-                az[2] = __ldg(p.az + z + 2 * cz);
-                zc[4] = z_cand(k + 2, wlo, whi, r0a[2], s[2], az[2]);
-                wlo = whi;
-            }
-        } else {
-            r0a[0] = pdef_r0a(p, (unsigned)(k - 1) * cz, z);
-            s[0] = __ldg(p.s + (unsigned)k * sz + os);
+        for (int q = 0; q < 4; ++q) zc[q] = zc[q + 1];
+        r0a[0] = r0a[1], s[0] = s[1], az[0] = az[1];
+        r0a[1] = r0a[2], s[1] = s[2], az[1] = az[2];
+        zc[4] = 0.0f;
+        if (k + 2 <= nk) {
+            const float whi = __ldg(p.rrw + (unsigned)(k + 3) * sz + os);
+            r0a[2] = pdef_r0a(p, level + 2 * cz, z + 2 * cz);
+            s[2] = __ldg(p.s + (unsigned)(k + 2) * sz + os);
+            az[2] = __ldg(p.az + z + 2 * cz);
+            zc[4] = z_cand(k + 2, wlo, whi, r0a[2], s[2], az[2]);
+            wlo = whi;
         }
-        const unsigned v = (unsigned)k * vz + os, u = (unsigned)k * uz + ou;
-        const float v0 = __ldg(p.rrv + v), v1 = __ldg(p.rrv + v + (unsigned)(ni + 6)), ay = __ldg(p.ay + z);
-        const float sdy = (s[0] * (v1 - v0)) * p.rdy;
-        float yc = step(r0a[0], p.dt * (ay + sdy));
-        if ((j == 0 && so == 2u && v0 >= 0.0f) || (j + 1 == nj && no == 2u && v1 <= 0.0f)) yc = r0a[0];
-        s_y[k & 1][ty][lane] = yc;
-        __syncthreads();
-        if (!row) continue;
-        const float u0 = __ldg(p.rru + u), u1 = __ldg(p.rru + u + 1), ax = __ldg(p.ax + z);
         const float sdx = (s[0] * (u1 - u0)) * p.rdx;
-        float xc = step(r0a[0], p.dt * (ax + sdx));
-        if (inflow_lo(i, p.obc, 0u, u0) || inflow_hi(i, ni, p.obc, 1u, u1)) xc = r0a[0];
-        const float xll = __shfl_up_sync(0xffffffffu, xc, 2), xl = __shfl_up_sync(0xffffffffu, xc, 1);
-        const float xr = __shfl_down_sync(0xffffffffu, xc, 1), xrr = __shfl_down_sync(0xffffffffu, xc, 2);
-        const float (*sy)[32] = s_y[k & 1];
-        const float yl = sy[ty - 1][lane], yr = sy[ty + 1][lane];
+        const float xc = (wo && u0 >= 0.0f) || (eo && u1 <= 0.0f) ? r0a[0] : step(r0a[0], p.dt * (ax + sdx));
+        const float xl = __shfl_up_sync(0xffffffffu, xc, 1), xr = __shfl_down_sync(0xffffffffu, xc, 1);
         float dx = ax, dy = ay, dz = az[0], mass;
         auto repaired = [&](float c, float m, float sd) {
             float first = ((c + m) - r0a[0]) * p.rdt;
             if (!flat) first = first * rgz;
             return first - sd;
         };
-        if (!(xl >= 0.0f && xc >= 0.0f && xr >= 0.0f) && pdef_mass(xll, xl, xc, xr, xrr, mass))
-            dx = repaired(xc, mass, sdx);
-        if (!(yl >= 0.0f && yc >= 0.0f && yr >= 0.0f) && pdef_mass(sy[ty - 2][lane], yl, yc, yr, sy[ty + 2][lane], mass))
-            dy = repaired(yc, mass, sdy);
+        // away from the edge of the water no candidate nearby is negative
+        const bool fx = !(xl >= 0.0f && xc >= 0.0f && xr >= 0.0f);
+        if (__any_sync(0xffffffffu, fx)) {
+            const float xll = __shfl_up_sync(0xffffffffu, xc, 2), xrr = __shfl_down_sync(0xffffffffu, xc, 2);
+            if (fx && pdef_mass(xll, xl, xc, xr, xrr, mass)) dx = repaired(xc, mass, sdx);
+        }
+        if (!(yl >= 0.0f && yc >= 0.0f && yr >= 0.0f) &&
+            pdef_mass(__ldg(p.dum + level + yrow(j - 2)), yl, yc, yr, __ldg(p.dum + level + yrow(j + 2)), mass)) {
+            const unsigned v = (unsigned)k * vz + os;
+            dy = repaired(yc, mass, (s[0] * (__ldg(p.rrv + v + (unsigned)(ni + 6)) - __ldg(p.rrv + v))) * p.rdy);
+        }
         if (!(zc[1] >= 0.0f && zc[2] >= 0.0f && zc[3] >= 0.0f) && pdef_mass(zc[0], zc[1], zc[2], zc[3], zc[4], mass)) {
             const unsigned w = (unsigned)k * sz + os;
             dz = repaired(zc[2], mass, pdef_zterm(p, s[0] * (__ldg(p.rrw + w + sz) - __ldg(p.rrw + w)), k));
         }
         if (own) {
             float t = (dx + dy) + dz;
-            t = t + s[0] * __ldg(p.divx + z);
-            p.adv[z] = flat ? t * __ldg(p.rr0 + (unsigned)(k - 1) * cz) : (t * __ldg(p.rr0 + z)) * gz;
+            t = t + s[0] * div;
+            p.adv[z] = flat ? t * rr0 : (t * rr0) * gz;
         }
     }
 }
@@ -1303,43 +1300,57 @@ extern "C" int32_t gm1b_post_acoustic_flux_column(int32_t ni, int32_t nj, int32_
 }
 
 namespace {
-int32_t pdef_chain_launch(int32_t ni, int32_t nj, int32_t nk, const gm1b_pdef_chain_arrays *a, float dttmp, float dx,
-                          float dy, float dz, double weps, uint32_t lateral_obc, int32_t pdefweno, int vmode,
-                          const float *rdsf, const float *mh, float rdz, void *stream) {
-    if (a == nullptr || !grid_ok(ni, nj, nk, 2, 2, 4, "gm1b_pdef_moisture_chain")) {
-        if (a == nullptr) gm1b_set_error("gm1b_pdef_moisture_chain: NULL arrays");
+// the operator's arguments; `whole` for the chain that leaves every row,
+// false for its advection alone (fx, fy and fz unused)
+int32_t pdef_args(int32_t ni, int32_t nj, int32_t nk, const gm1b_pdef_chain_arrays *a, float dttmp, float dx, float dy,
+                  float dz, double weps, uint32_t lateral_obc, int32_t pdefweno, const gm1b_vertical_column *column,
+                  bool whole, Pdef &p, const char *what) {
+    if (a == nullptr || !grid_ok(ni, nj, nk, 2, 2, 4, what)) {
+        if (a == nullptr) gm1b_set_error("%s: NULL arrays", what);
+        return GM1B_ERR_ARGUMENT;
+    }
+    if (column != nullptr && ((column->flat != 0 && column->flat != 1) ||
+                              (column->flat ? (column->mh == nullptr || !(column->rdz > 0.0f) || !isfinite(column->rdz))
+                                            : column->rdsf == nullptr))) {
+        gm1b_set_error("%s: need a flat column (mh, rdz > 0) or a terrain column (rdsf)", what);
         return GM1B_ERR_ARGUMENT;
     }
     const void *need[] = {a->scalar_a, a->scalar_padded, a->rho0_3d, a->gz, a->rgz, a->rr0, a->c1, a->c2, a->divx,
-                          a->rru, a->rrv, a->rrw, a->fx, a->fy, a->fz, a->advx, a->advy, a->advz, a->candidate,
-                          a->advection};
-    for (const void *q : need)
-        if (q == nullptr) {
-            gm1b_set_error("gm1b_pdef_moisture_chain: NULL array");
-            return GM1B_ERR_ARGUMENT;
-        }
+                          a->rru, a->rrv, a->rrw, a->advx, a->advy, a->advz, a->candidate, a->advection};
+    const void *rows[] = {a->fx, a->fy, a->fz};
+    bool null = false;
+    for (const void *q : need) null = null || q == nullptr;
+    for (const void *q : rows) null = null || (whole && q == nullptr);
+    if (null) {
+        gm1b_set_error("%s: NULL array", what);
+        return GM1B_ERR_ARGUMENT;
+    }
     for (int s = 0; s < 4; ++s) {
         const unsigned v = (lateral_obc >> (4 * s)) & 15u;
         if (v > 4) {
-            gm1b_set_error("gm1b_pdef_moisture_chain: lateral side codes must be 0..4");
+            gm1b_set_error("%s: lateral side codes must be 0..4", what);
             return GM1B_ERR_ARGUMENT;
         }
     }
     if (!(dttmp > 0.0f) || !(dx > 0.0f) || !(dy > 0.0f) || !(dz > 0.0f)) {
-        gm1b_set_error("gm1b_pdef_moisture_chain: dttmp, dx, dy, dz must be > 0");
+        gm1b_set_error("%s: dttmp, dx, dy, dz must be > 0", what);
         return GM1B_ERR_ARGUMENT;
     }
-    Pdef p{};
+    p = Pdef{};
     p.a = a->scalar_a, p.s = a->scalar_padded, p.rho0 = a->rho0_3d, p.gz = a->gz, p.rgz = a->rgz, p.rr0 = a->rr0;
     p.c1 = a->c1, p.c2 = a->c2, p.divx = a->divx, p.rru = a->rru, p.rrv = a->rrv, p.rrw = a->rrw;
     p.fx = a->fx, p.fy = a->fy, p.fz = a->fz, p.ax = a->advx, p.ay = a->advy, p.az = a->advz;
     p.dum = a->candidate, p.adv = a->advection;
+    p.vmode = column == nullptr ? 0 : column->flat ? 2 : 1;
     p.dt = dttmp, p.dx = dx, p.dy = dy, p.dz = dz;
-    p.rdx = 1.0f / dx, p.rdy = 1.0f / dy, p.rdz = vmode == 0 ? 1.0f / dz : rdz, p.rdt = 1.0f / dttmp;
+    p.rdx = 1.0f / dx, p.rdy = 1.0f / dy, p.rdz = column == nullptr ? 1.0f / dz : column->rdz, p.rdt = 1.0f / dttmp;
     p.weps = weps, p.obc = lateral_obc, p.pdefweno = pdefweno ? 1 : 0;
-    p.vmode = vmode, p.rdsf = rdsf, p.mh = mh;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const Lane L{ni, nj, nk};
+    p.rdsf = column ? column->rdsf : nullptr, p.mh = column ? column->mh : nullptr;
+    return GM1B_OK;
+}
+
+int32_t pdef_chain_launch(const Pdef &p, const Lane &L, cudaStream_t st) {
+    const int ni = L.ni, nj = L.nj, nk = L.nk;
     const size_t n = (size_t)ni * nj * nk;
 #define TOS_LAUNCH(name, work, ...)                                    \
     do {                                                               \
@@ -1359,27 +1370,74 @@ int32_t pdef_chain_launch(int32_t ni, int32_t nj, int32_t nk, const gm1b_pdef_ch
 #undef TOS_LAUNCH
     return GM1B_OK;
 }
+
+// levels per chunk of a marching pass: halve until two rounds of `warps` on
+// each of 148 SMs, or four levels, are left
+int march_chunk(long long row_warps, int nk, int warps) {
+    int chunk = nk;
+    while (chunk > 4 && row_warps * ((nk + chunk - 1) / chunk) < 2LL * 148 * warps) chunk = (chunk + 1) / 2;
+    return chunk;
+}
 }  // namespace
 
 extern "C" int32_t gm1b_pdef_moisture_chain(int32_t ni, int32_t nj, int32_t nk, const gm1b_pdef_chain_arrays *a,
                                             float dttmp, float dx, float dy, float dz, double weps,
                                             uint32_t lateral_obc, int32_t pdefweno, void *stream) {
-    return pdef_chain_launch(ni, nj, nk, a, dttmp, dx, dy, dz, weps, lateral_obc, pdefweno, 0, nullptr, nullptr, 0.0f,
-                             stream);
+    Pdef p;
+    const int32_t r = pdef_args(ni, nj, nk, a, dttmp, dx, dy, dz, weps, lateral_obc, pdefweno, nullptr, true, p,
+                                "gm1b_pdef_moisture_chain");
+    return r != GM1B_OK ? r : pdef_chain_launch(p, Lane{ni, nj, nk}, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int32_t gm1b_pdef_moisture_chain_column(int32_t ni, int32_t nj, int32_t nk,
                                                    const gm1b_pdef_chain_arrays *a, float dttmp, float dx, float dy,
                                                    double weps, uint32_t lateral_obc, int32_t pdefweno,
                                                    const gm1b_vertical_column *column, void *stream) {
-    if (column == nullptr || (column->flat != 0 && column->flat != 1) ||
-        (column->flat ? (column->mh == nullptr || !(column->rdz > 0.0f) || !isfinite(column->rdz))
-                      : column->rdsf == nullptr)) {
+    if (column == nullptr) {
         gm1b_set_error("gm1b_pdef_moisture_chain_column: need a flat column (mh, rdz > 0) or a terrain column (rdsf)");
         return GM1B_ERR_ARGUMENT;
     }
-    return pdef_chain_launch(ni, nj, nk, a, dttmp, dx, dy, 1.0f, weps, lateral_obc, pdefweno, column->flat ? 2 : 1,
-                             column->rdsf, column->mh, column->rdz, stream);
+    Pdef p;
+    const int32_t r = pdef_args(ni, nj, nk, a, dttmp, dx, dy, 1.0f, weps, lateral_obc, pdefweno, column, true, p,
+                                "gm1b_pdef_moisture_chain_column");
+    return r != GM1B_OK ? r : pdef_chain_launch(p, Lane{ni, nj, nk}, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int32_t gm1b_pdef_moisture_advection(int32_t ni, int32_t nj, int32_t nk, const gm1b_pdef_chain_arrays *a,
+                                                float dttmp, float dx, float dy, float dz, double weps,
+                                                uint32_t lateral_obc, int32_t pdefweno,
+                                                const gm1b_vertical_column *column, void *stream) {
+    for (int s = 0; s < 4; ++s)
+        if (((lateral_obc >> (4 * s)) & 15u) == 0u) {
+            gm1b_set_error("gm1b_pdef_moisture_advection: lateral code 0x%x: each side is 1..4", lateral_obc);
+            return GM1B_ERR_ARGUMENT;
+        }
+    Pdef p;
+    const int32_t r = pdef_args(ni, nj, nk, a, dttmp, dx, dy, column ? 1.0f : dz, weps, lateral_obc, pdefweno, column,
+                                false, p, "gm1b_pdef_moisture_advection");
+    if (r != GM1B_OK) return r;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const Lane L{ni, nj, nk};
+    // largest float <= weps: x > weps exactly when x > small, for every float x
+    float small = (float)weps;
+    if ((double)small > weps) small = nextafterf(small, -INFINITY);
+    {
+        const int tiles = ni / kPdOut + 1, rows = (nj + kPdRows - 2) / (kPdRows - 1);
+        const int chunk = march_chunk((long long)tiles * nj, nk, 32);
+        ProfScope ps("pdef_advection_kernel", st);
+        pdef_advection_kernel<<<dim3(tiles * rows, (nk + chunk - 1) / chunk), dim3(32, kPdRows), 0, st>>>(p, L, chunk,
+                                                                                                         small);
+        ps.stop();
+    }
+    if (!launch_ok("pdef_advection_kernel")) return GM1B_ERR_CUDA;
+    {
+        const int tiles = (ni + kRepOut - 1) / kRepOut, rows = (nj + kRepRows - 1) / kRepRows;
+        const int chunk = march_chunk((long long)tiles * nj, nk, 32);
+        ProfScope ps("pdef_repair_kernel", st);
+        pdef_repair_kernel<<<dim3(tiles * rows, (nk + chunk - 1) / chunk), dim3(32, kRepRows), 0, st>>>(p, L, chunk);
+        ps.stop();
+    }
+    return launch_ok("pdef_repair_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }
 
 extern "C" int32_t gm1b_held_compose(int32_t ni, int32_t nj, int32_t nk, const gm1b_held_arrays *a, float dt,

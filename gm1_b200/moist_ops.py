@@ -8,6 +8,7 @@ default, and synchronises nothing):
   post_acoustic_flux    launch_cuda_post_acoustic_flux_bridge (:461)
   pdef_moisture_chain   the final-stage moisture chain of launch_cuda_scalar_moist_rk_stage
                         (src/cm1core/cuda_scalar_moist_rk.py:1336-1500)
+  pdef_moisture_advection  its advection alone, in two passes
   held_compose          gm1_child_predict_and_compose_held_base3d_v1
                         (src/cm1core/cuda_gm1_child_step_composer.py:547)
   solve3_density        gm1_solve3_density_v1 (src/cm1core/cuda_gm1_forecast.py:548)
@@ -53,6 +54,9 @@ def _lib():
         lib.gm1b_pdef_moisture_chain_column.argtypes = [i, i, i, c.POINTER(_Chain), f, f, f, c.c_double, c.c_uint32,
                                                         i, c.POINTER(_VerticalColumn), vp]
         lib.gm1b_pdef_moisture_chain_column.restype = i
+        lib.gm1b_pdef_moisture_advection.argtypes = [i, i, i, c.POINTER(_Chain), f, f, f, f, c.c_double, c.c_uint32, i,
+                                                     c.POINTER(_VerticalColumn), vp]
+        lib.gm1b_pdef_moisture_advection.restype = i
         from .momentum import _Column  # noqa: PLC0415
 
         lib.gm1b_post_acoustic_flux_column.argtypes = [i, i, i, c.POINTER(_Post), f, f, c.POINTER(_Column), vp]
@@ -111,6 +115,20 @@ def pdef_moisture_chain(a: Mapping[str, torch.Tensor], *, ni: int, nj: int, nk: 
                                                   pdefweno, _st(stream, a["rru"].device)), "gm1b_pdef_moisture_chain")
 
 
+def _vertical(column: StretchedColumn, nk: int) -> _VerticalColumn:
+    if not isinstance(column, StretchedColumn):
+        raise TypeError("column must be a StretchedColumn")
+    if column.flat:
+        prof = column.mh
+        if not isinstance(prof, torch.Tensor) or tuple(prof.shape) != (nk + 2,):
+            raise ValueError(f"mh must be a ({nk + 2},) tensor")
+        return _VerticalColumn(1, None, _f32(prof, "mh"), float(column.rdz))
+    prof = column.rdsf
+    if not isinstance(prof, torch.Tensor) or tuple(prof.shape) != (nk + 3,):
+        raise ValueError(f"rdsf must be a ({nk + 3},) tensor")
+    return _VerticalColumn(0, _f32(prof, "rdsf"), None, 0.0)
+
+
 def pdef_moisture_chain_column(a: Mapping[str, torch.Tensor], column: StretchedColumn, *, ni: int, nj: int, nk: int,
                                dttmp: float, dx: float, dy: float, weps: float, lateral_obc: int, pdefweno: int,
                                stream: Any | None = None) -> None:
@@ -118,22 +136,26 @@ def pdef_moisture_chain_column(a: Mapping[str, torch.Tensor], column: StretchedC
     (launch_cuda_gm1_child_stretched_pdef_moisture,
     src/cm1core/cuda_gm1_child_stretched_scalar.py:851): the terrain branch's
     rdsf(k), or the flat column's rdz*mh(k) with its own base state."""
-    if not isinstance(column, StretchedColumn):
-        raise TypeError("column must be a StretchedColumn")
-    if column.flat:
-        prof = column.mh
-        if not isinstance(prof, torch.Tensor) or tuple(prof.shape) != (nk + 2,):
-            raise ValueError(f"mh must be a ({nk + 2},) tensor")
-        col = _VerticalColumn(1, None, _f32(prof, "mh"), float(column.rdz))
-    else:
-        prof = column.rdsf
-        if not isinstance(prof, torch.Tensor) or tuple(prof.shape) != (nk + 3,):
-            raise ValueError(f"rdsf must be a ({nk + 3},) tensor")
-        col = _VerticalColumn(0, _f32(prof, "rdsf"), None, 0.0)
+    col = _vertical(column, nk)
     s = _Chain(**{n: _f32(a[n], n) for n in CHAIN_NAMES})
     _native.check(_lib().gm1b_pdef_moisture_chain_column(ni, nj, nk, ctypes.byref(s), dttmp, dx, dy, weps, lateral_obc,
                                                          pdefweno, ctypes.byref(col), _st(stream, a["rru"].device)),
                   "gm1b_pdef_moisture_chain_column")
+
+
+def pdef_moisture_advection(a: Mapping[str, torch.Tensor], column: StretchedColumn | None = None, *, ni: int, nj: int,
+                            nk: int, dttmp: float, dx: float, dy: float, weps: float, lateral_obc: int, pdefweno: int,
+                            dz: float = 0.0, stream: Any | None = None) -> None:
+    """The chain's advection alone, the words pdef_moisture_chain (column
+    None, spacing ``dz``) or pdef_moisture_chain_column leave in
+    ``advection``: fx, fy and fz are not used, advx, advy, advz and candidate
+    are scratch."""
+    col = None if column is None else ctypes.byref(_vertical(column, nk))
+    unused = ("fx", "fy", "fz")
+    s = _Chain(**{n: _f32(a[n], n) for n in CHAIN_NAMES if n not in unused})
+    _native.check(_lib().gm1b_pdef_moisture_advection(ni, nj, nk, ctypes.byref(s), dttmp, dx, dy, dz, weps, lateral_obc,
+                                                      pdefweno, col, _st(stream, a["rru"].device)),
+                  "gm1b_pdef_moisture_advection")
 
 
 def post_acoustic_flux_column(a: Mapping[str, torch.Tensor], column: Any, *, ni: int, nj: int, nk: int, dx: float,

@@ -804,14 +804,10 @@ class MoistLargeStep:
             self._advect(padded, {"rru": s["rru"], "rrv": s["rrv"], "rrw": s["rrw"]},
                          {"c1": m["c1"], "c2": m["c2"], "rr0": m["rr0"], "gz": m["gz"]}, s["moist_adv"][r], weps, nrk,
                          st)
-        elif self.flat:
-            mo.pdef_moisture_chain_column(self.chain_arrays[r], self.scalar_column, **self.k3, dx=cfg.dx, dy=cfg.dy,
-                                          dttmp=scalar_moist_rk_stage_timestep_f32(cfg.dt, nrk), weps=weps,
-                                          lateral_obc=cfg.obc, pdefweno=0 if r == 0 else 1, stream=st)
         else:
-            mo.pdef_moisture_chain(self.chain_arrays[r], **self.grid,
-                                   dttmp=scalar_moist_rk_stage_timestep_f32(cfg.dt, nrk), weps=weps,
-                                   lateral_obc=cfg.obc, pdefweno=0 if r == 0 else 1, stream=st)
+            mo.pdef_moisture_advection(self.chain_arrays[r], self.scalar_column if self.flat else None, **self.grid,
+                                       dttmp=scalar_moist_rk_stage_timestep_f32(cfg.dt, nrk), weps=weps,
+                                       lateral_obc=cfg.obc, pdefweno=0 if r == 0 else 1, stream=st)
 
     def scalar_moist(self, nrk: int) -> None:
         """theta and the moisture species advect (concurrently, each on its own

@@ -690,6 +690,16 @@ GM1B_API int32_t gm1b_pdef_moisture_chain(int32_t ni, int32_t nj, int32_t nk, co
                                           float dttmp, float dx, float dy, float dz, double weps, uint32_t lateral_obc,
                                           int32_t pdefweno, void *stream);
 
+/* The chain's advection alone, the same words as gm1b_pdef_moisture_chain
+ * (column NULL, spacing dz) or gm1b_pdef_moisture_chain_column leave in
+ * `advection`, for a caller that needs none of the rows between: fx, fy and
+ * fz are not used and may be NULL; advx, advy, advz and candidate are scratch.
+ * Every lateral side is 1..4. */
+GM1B_API int32_t gm1b_pdef_moisture_advection(int32_t ni, int32_t nj, int32_t nk, const gm1b_pdef_chain_arrays *arrays,
+                                              float dttmp, float dx, float dy, float dz, double weps,
+                                              uint32_t lateral_obc, int32_t pdefweno,
+                                              const gm1b_vertical_column *column, void *stream);
+
 /* The chain on a stretched column (launch_cuda_gm1_child_stretched_pdef_moisture,
  * src/cm1core/cuda_gm1_child_stretched_scalar.py:851): flat = 0, the
  * terrain branch's rdsf(k) in every vertical derivative; flat = 1, the flat

@@ -149,3 +149,36 @@ def test_flat_tke_diffusion(ni, nj, nk):
     orc.tke_diffusion_flat(a, **kw)
     te.launch_cuda_flat_tke_diffusion(dev, **kw)
     assert _differ(dev, a, ("tketen",)) == []
+
+
+@pytest.mark.parametrize("column", ["uniform", "terrain", "flat"])
+@pytest.mark.parametrize("obc,pdefweno", [(0x2222, 0), (0x2222, 1), (0x1111, 1), (0x3443, 0)])
+@pytest.mark.parametrize("ni,nj,nk", [(29, 7, 4), (30, 8, 5), (31, 9, 6), (61, 14, 9), (5, 15, 33)])
+def test_pdef_advection_is_the_chains(ni, nj, nk, obc, pdefweno, column):
+    """The two-pass moisture advection against the chain's, with negative
+    candidates on every axis and dry air beside the water."""
+    from gm1_b200 import moist_ops as mo
+    from gm1_b200.advection import StretchedColumn
+    from tests.test_oracle_moist_step import chain_arrays
+
+    a = chain_arrays(ni, nj, nk, ni + nk)
+    rng = np.random.default_rng(nk)
+    dry = rng.random(a["scalar_a"].shape) < 0.4
+    a["scalar_a"][dry] = 0.0
+    a["scalar_padded"][1:nk + 1, 3:nj + 3, 3:ni + 3][dry] = 0.0
+    one = _dev(a)
+    two = {k: v.clone() for k, v in one.items()}
+    kw = dict(ni=ni, nj=nj, nk=nk, dttmp=2.0, dx=400.0, dy=300.0, weps=1e-20, lateral_obc=obc, pdefweno=pdefweno)
+    p = _profiles(nk)
+    if column == "uniform":
+        mo.pdef_moisture_chain(one, dz=200.0, **kw)
+        mo.pdef_moisture_advection(two, dz=200.0, **kw)
+    else:
+        col = StretchedColumn(True, mh=_t(p["mh"]), rdz=p["rdz"]) if column == "flat" else \
+            StretchedColumn(False, rdsf=_t(np.abs(p["mf"]) / 100.0))
+        mo.pdef_moisture_chain_column(one, col, **kw)
+        mo.pdef_moisture_advection(two, col, **kw)
+    torch.cuda.synchronize()
+    want = {k: v.cpu().numpy() for k, v in one.items()}
+    assert np.count_nonzero(want["candidate"] < 0.0) > 0
+    assert _differ(two, want, ("advection",)) == []
