@@ -40,7 +40,7 @@ constexpr int kTosWarps = 8;     // k-parallel warps of the column pass
 constexpr int kTosMaxNk = 160;   // column pass keeps 10 words per level per column in shared memory
 constexpr int kTosArrays = 7;
 constexpr int kFlatLevels = 2;   // the same of the flat pressure gradient, which has no vertical coupling
-constexpr int kPgLevels = 4;     // levels whose loads the pressure-gradient march issues together
+constexpr int kPgLevels = 2;     // levels of a thread of the terrain pressure gradient
 constexpr int kA2Levels = 2;     // levels per warp whose column-pass loads are issued together (phase A2)
 constexpr int kColLevels = 2;    // the same for phases A3 and C
 constexpr int kThomasChunk = 8;  // back-substitution levels whose coefficients are read together
@@ -393,10 +393,13 @@ __global__ void __launch_bounds__(128) tos_flat_pgrad_kernel(TosArgs p) {
 // ---------------------------------------------------------------------------
 // terrain pressure gradient on the interior faces (u faces 2..ni of the
 // physical rows, v faces 2..nj of the physical columns).  One thread per
-// pressure point (j, i), j = 0..nj+1, i = 0..ni+1, marching k = 1..nk with
+// pressure point (j, i), j = 0..nj+1, i = 0..ni+1, and kPgLevels levels, with
 // the vertical ppd differences of its own, west and south points carried in
 // registers.  Under diagnostics with the pi' advection ablated, the last
-// small step leaves those differences in hadvp, as the twin does.
+// small step leaves those differences in hadvp, as the twin does.  Two levels
+// a thread against a march of the column four at a time: 53x48x40 23.0 -> 8.6
+// us (too few threads in flight), 256x256x80 65.0 -> 64.1, 640x768x80 422 ->
+// 424; four levels a thread take 8.7, 67.8 and 481.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) tos_pgrad_kernel(TosArgs p) {
     const Ix X{p.ni, p.nj};
@@ -413,15 +416,21 @@ __global__ void __launch_bounds__(128) tos_pgrad_kernel(TosArgs p) {
     if (!du && !dv && !dh && !acc) return;
     const bool sums = acc && p.n > 1;
     const int iw = du ? i - 1 : i, js = dv ? j - 1 : j;   // neighbour points (own point when unused)
-    float pc = __ldg(a.ppd + X.p(1, j, i)), pw = __ldg(a.ppd + X.p(1, j, iw)), ps = __ldg(a.ppd + X.p(1, js, i));
+    const int k0 = 1 + blockIdx.z * kPgLevels;
+    float pc = __ldg(a.ppd + X.p(k0, j, i)), pw = __ldg(a.ppd + X.p(k0, j, iw)), ps = __ldg(a.ppd + X.p(k0, js, i));
     float vc = 0.0f, vw = 0.0f, vs = 0.0f;  // vertical difference at level k (zero at k = 1)
-    float gxu_lo = du ? __ldg(m.gxu + (size_t)(j - 1) * (ni + 1) + (i - 1)) : 0.0f;
-    float gyv_lo = dv ? __ldg(m.gyv + (size_t)(j - 1) * ni + (i - 1)) : 0.0f;
-    // Levels go in chunks of kPgLevels: every load of a chunk is issued before
-    // its first store, so the chunk's loads are in flight together (the
-    // stores to u3d/v3d would otherwise order each level's loads behind the
-    // previous level's stores).
-    for (int k0 = 1; k0 <= nk; k0 += kPgLevels) {
+    if (k0 > 1) {
+        const float r = vrds(p, k0);
+        vc = (pc - __ldg(a.ppd + X.p(k0 - 1, j, i))) * r;
+        vw = (pw - __ldg(a.ppd + X.p(k0 - 1, j, iw))) * r;
+        vs = (ps - __ldg(a.ppd + X.p(k0 - 1, js, i))) * r;
+    }
+    float gxu_lo = du ? __ldg(m.gxu + ((unsigned)(k0 - 1) * (unsigned)nj + (unsigned)(j - 1)) * (unsigned)(ni + 1) + (unsigned)(i - 1)) : 0.0f;
+    float gyv_lo = dv ? __ldg(m.gyv + ((unsigned)(k0 - 1) * (unsigned)(nj + 1) + (unsigned)(j - 1)) * (unsigned)ni + (unsigned)(i - 1)) : 0.0f;
+    // Every load of the chunk is issued before its first store, so they are in
+    // flight together (the stores to u3d/v3d would otherwise order each level's
+    // loads behind the previous level's stores).
+    {
         float lp[kPgLevels], lw[kPgLevels], ls[kPgLevels], lth[kPgLevels], lthw[kPgLevels], lths[kPgLevels];
         float lgx[kPgLevels], lgy[kPgLevels], lut[kPgLevels], luu[kPgLevels], lvt[kPgLevels], lvv[kPgLevels];
         float lru[kPgLevels], lrv[kPgLevels];
@@ -1808,7 +1817,7 @@ int32_t terrain_open_stage(int32_t ni, int32_t nj, int32_t nk, int32_t nrk, floa
         ps.stop();
     }
     if (!launch_ok("tos_prepare_kernel")) return GM1B_ERR_CUDA;
-    const dim3 pg_grid((ni + 2 + 31) / 32, (nj + 2 + 3) / 4), col_grid((ni + 31) / 32, nj);
+    const dim3 pg_grid((ni + 2 + 31) / 32, (nj + 2 + 3) / 4, (nk + kPgLevels - 1) / kPgLevels), col_grid((ni + 31) / 32, nj);
     constexpr uint32_t column_phases = GM1B_TOS_PRESSURE_GRADIENT | GM1B_TOS_TRANSFORMED_DIVERGENCE |
                                        GM1B_TOS_PRESSURE_ADVECTION | GM1B_TOS_IMPLICIT_SOLVE |
                                        GM1B_TOS_BETWEEN_STEP_FILL;
