@@ -9,15 +9,15 @@
 //   cpu_moist_nm_inplace              src/cm1core/cuda_moist_nm.py:292-396
 //
 // Design (B200):
-//  * calcdef is one z-marching tiled kernel.  A 32 x 8 CTA owns a tile of
-//    output columns and walks the face levels upwards; the strain components
-//    at its cells (s11, s22, s33) ride in registers from one level to the
-//    next, the corner shear s12 of the tile's 33 x 9 corners is built in
-//    shared memory (two level buffers), and the face shears s13 (33 x 8) and
-//    s23 (32 x 9) of the current face level are built in shared memory before
-//    the tile's defv and defh are combined.  Every strain word is formed once
-//    and nothing goes through device memory between stages (the reference
-//    stores six scratch volumes and runs three launches).
+//  * calcdef is one z-marching kernel.  A warp owns 32 cells of a row and
+//    walks a chunk of face levels upwards: each lane forms its cell's diagonal
+//    strains, the corner shear s12 of its lower left corner, and the face
+//    shears s13 and s23 of its west and south faces, and takes the other
+//    corners and faces from the next lane (shuffle) and the next row (shared
+//    memory).  The levels' velocities, their face-level sums and the corner
+//    sums ride in registers from one level to the next, so every word is
+//    loaded once a warp and nothing goes through device memory between stages
+//    (the reference stores six scratch volumes and runs three launches).
 //  * calcnm is elementwise per face level: each thread forms the cell
 //    diagnostics of its own level and of the level below and the face value
 //    between them, so columns need no serial walk; the branch counts are
@@ -30,7 +30,8 @@
 namespace gm1b {
 namespace {
 
-constexpr int kDX = 32, kDY = 8;  // calcdef tile
+constexpr int kDefRows = 8;  // rows of corners per calcdef CTA; they complete 7 rows of cells
+constexpr int kDefOut = 31;  // cells a warp of 32 corners completes
 
 struct DefArgs {
     const float *u, *v, *w, *rho, *rf, *c1, *c2, *gz, *rgz, *rgzu, *rgzv, *gx, *gy;
@@ -47,241 +48,169 @@ __device__ __forceinline__ unsigned i3(int k, int j, int i, int ny, int nx) {
     return ((unsigned)k * (unsigned)ny + (unsigned)j) * (unsigned)nx + (unsigned)i;
 }
 
-// face-level value of a u- or v-shaped field (levels nk, rows ny, row nx)
-__device__ __forceinline__ float atw(const float *q, int kf, int j, int i, int nk, int ny, int nx) {
-    if (kf == 0) {
-        float r = 1.875f * q[i3(0, j, i, ny, nx)];
-        r = r + (-1.25f) * q[i3(1, j, i, ny, nx)];
-        return r + 0.375f * q[i3(2, j, i, ny, nx)];
-    }
-    if (kf == nk) {
-        float r = 1.875f * q[i3(nk - 1, j, i, ny, nx)];
-        r = r + (-1.25f) * q[i3(nk - 2, j, i, ny, nx)];
-        return r + 0.375f * q[i3(nk - 3, j, i, ny, nx)];
-    }
-    return 0.5f * (q[i3(kf - 1, j, i, ny, nx)] + q[i3(kf, j, i, ny, nx)]);
-}
-
-// s11, s22, s33 at mass level k, cell (j, i)
-__device__ __forceinline__ void strain_diag(const DefArgs &p, int k, int j, int i, float &s11, float &s22, float &s33) {
-    const int ni = p.ni, nj = p.nj, nk = p.nk, ux = ni + 1, vy = nj + 1;
-    const unsigned c = i3(k, j, i, nj, ni);
-    const float g = p.gz[(unsigned)j * ni + i], r = p.rho[c];
-    float hor = g * (p.u[i3(k, j, i + 1, nj, ux)] * p.rgzu[(unsigned)j * ux + i + 1] -
-                     p.u[i3(k, j, i, nj, ux)] * p.rgzu[(unsigned)j * ux + i]);
-    hor = hor * p.rdx;
-    float up = p.gx[i3(k + 1, j, i, nj, ni)] * (atw(p.u, k + 1, j, i, nk, nj, ux) + atw(p.u, k + 1, j, i + 1, nk, nj, ux));
-    float lo = p.gx[c] * (atw(p.u, k, j, i, nk, nj, ux) + atw(p.u, k, j, i + 1, nk, nj, ux));
-    float vert = ((up - lo) * 0.5f) * p.rds;
-    s11 = (hor + vert) * r;
-    hor = g * (p.v[i3(k, j + 1, i, vy, ni)] * p.rgzv[(unsigned)(j + 1) * ni + i] -
-               p.v[i3(k, j, i, vy, ni)] * p.rgzv[(unsigned)j * ni + i]);
-    hor = hor * p.rdy;
-    up = p.gy[i3(k + 1, j, i, nj, ni)] * (atw(p.v, k + 1, j, i, nk, vy, ni) + atw(p.v, k + 1, j + 1, i, nk, vy, ni));
-    lo = p.gy[c] * (atw(p.v, k, j, i, nk, vy, ni) + atw(p.v, k, j + 1, i, nk, vy, ni));
-    vert = ((up - lo) * 0.5f) * p.rds;
-    s22 = (hor + vert) * r;
-    s33 = (((p.w[i3(k + 1, j, i, nj, ni)] - p.w[c]) * p.rds) * g) * r;
-}
-
-// s12 at mass level k, corner (jc, ic) in [0, nj] x [0, ni]; the open sides
-// use the nearest interior corner (constant extension)
-__device__ __forceinline__ float strain_s12(const DefArgs &p, int k, int jc, int ic) {
-    const int ni = p.ni, nj = p.nj, nk = p.nk, ux = ni + 1, vy = nj + 1;
-    const int jj = jc < 1 ? 1 : (jc > nj - 1 ? nj - 1 : jc);
-    const int ii = ic < 1 ? 1 : (ic > ni - 1 ? ni - 1 : ic);
-    const float sig_lo = (float)k * p.dz, sig_hi = (float)(k + 1) * p.dz;
-    float r1 = p.rho[i3(k, jj - 1, ii - 1, nj, ni)] * p.gz[(unsigned)(jj - 1) * ni + ii - 1] +
-               p.rho[i3(k, jj, ii, nj, ni)] * p.gz[(unsigned)jj * ni + ii];
-    r1 = r1 + (p.rho[i3(k, jj, ii - 1, nj, ni)] * p.gz[(unsigned)jj * ni + ii - 1] +
-               p.rho[i3(k, jj - 1, ii, nj, ni)] * p.gz[(unsigned)(jj - 1) * ni + ii]);
-    r1 = 0.25f * r1;
-    const float rgzu_t = p.rgzu[(unsigned)jj * ux + ii], rgzu_b = p.rgzu[(unsigned)(jj - 1) * ux + ii];
-    const float x1 = (r1 * (p.u[i3(k, jj, ii, nj, ux)] * rgzu_t - p.u[i3(k, jj - 1, ii, nj, ux)] * rgzu_b)) * p.rdy;
-    const float xu = (p.zt - sig_hi) * (atw(p.u, k + 1, jj - 1, ii, nk, nj, ux) + atw(p.u, k + 1, jj, ii, nk, nj, ux));
-    const float xl = (p.zt - sig_lo) * (atw(p.u, k, jj - 1, ii, nk, nj, ux) + atw(p.u, k, jj, ii, nk, nj, ux));
-    const float x2 = ((((0.5f * (xu - xl)) * p.rds) * r1) * (rgzu_t - rgzu_b)) * p.rdy;
-    const float rgzv_r = p.rgzv[(unsigned)jj * ni + ii], rgzv_l = p.rgzv[(unsigned)jj * ni + ii - 1];
-    const float y1 = (r1 * (p.v[i3(k, jj, ii, vy, ni)] * rgzv_r - p.v[i3(k, jj, ii - 1, vy, ni)] * rgzv_l)) * p.rdx;
-    const float yu = (p.zt - sig_hi) * (atw(p.v, k + 1, jj, ii - 1, nk, vy, ni) + atw(p.v, k + 1, jj, ii, nk, vy, ni));
-    const float yl = (p.zt - sig_lo) * (atw(p.v, k, jj, ii - 1, nk, vy, ni) + atw(p.v, k, jj, ii, nk, vy, ni));
-    const float y2 = ((((0.5f * (yu - yl)) * p.rds) * r1) * (rgzv_r - rgzv_l)) * p.rdx;
-    return 0.5f * ((x1 + x2) + (y1 + y2));
-}
-
-// s13 at face level kf (1..nk-1), row j, u-face column ic in [0, ni]
-__device__ __forceinline__ float strain_s13(const DefArgs &p, int kf, int j, int ic) {
-    const int ni = p.ni, nj = p.nj, ux = ni + 1;
-    const int il = ic - 1 < 0 ? 0 : ic - 1, ir = ic < ni - 1 ? ic : ni - 1;
-    const float sig_l = ((float)kf - 0.5f) * p.dz, sig_u = ((float)kf + 0.5f) * p.dz;
-    const float wr = p.w[i3(kf, j, ir, nj, ni)], wl = p.w[i3(kf, j, il, nj, ni)];
-    const float rgr = p.rgz[(unsigned)j * ni + ir], rgl = p.rgz[(unsigned)j * ni + il];
-    const float du = (p.u[i3(kf, j, ic, nj, ux)] - p.u[i3(kf - 1, j, ic, nj, ux)]) * p.rds;
-    const float hw = (wr * rgr - wl * rgl) * p.rdx;
-    const float upper = (p.zt - sig_u) * (0.5f * (wr + p.w[i3(kf + 1, j, ir, nj, ni)]) +
-                                          0.5f * (wl + p.w[i3(kf + 1, j, il, nj, ni)]));
-    const float lower = (p.zt - sig_l) * (0.5f * (p.w[i3(kf - 1, j, ir, nj, ni)] + wr) +
-                                          0.5f * (p.w[i3(kf - 1, j, il, nj, ni)] + wl));
-    const float terrain = (((0.5f * p.rds) * (upper - lower)) * (rgr - rgl)) * p.rdx;
-    const float strain = 0.5f * ((du + hw) + terrain);
-    const float density = 0.5f * (p.gz[(unsigned)j * ni + il] * p.rf[i3(kf, j, il, nj, ni)] +
-                                  p.gz[(unsigned)j * ni + ir] * p.rf[i3(kf, j, ir, nj, ni)]);
-    return strain * density;
-}
-
-// s23 at face level kf (1..nk-1), v-face row jc in [0, nj], column i
-__device__ __forceinline__ float strain_s23(const DefArgs &p, int kf, int jc, int i) {
-    const int ni = p.ni, nj = p.nj, vy = nj + 1;
-    const int jb = jc - 1 < 0 ? 0 : jc - 1, jt = jc < nj - 1 ? jc : nj - 1;
-    const float sig_l = ((float)kf - 0.5f) * p.dz, sig_u = ((float)kf + 0.5f) * p.dz;
-    const float wt = p.w[i3(kf, jt, i, nj, ni)], wb = p.w[i3(kf, jb, i, nj, ni)];
-    const float rgt = p.rgz[(unsigned)jt * ni + i], rgb = p.rgz[(unsigned)jb * ni + i];
-    const float dv = (p.v[i3(kf, jc, i, vy, ni)] - p.v[i3(kf - 1, jc, i, vy, ni)]) * p.rds;
-    const float hw = (wt * rgt - wb * rgb) * p.rdy;
-    const float upper = (p.zt - sig_u) * (0.5f * (wt + p.w[i3(kf + 1, jt, i, nj, ni)]) +
-                                          0.5f * (wb + p.w[i3(kf + 1, jb, i, nj, ni)]));
-    const float lower = (p.zt - sig_l) * (0.5f * (p.w[i3(kf - 1, jt, i, nj, ni)] + wt) +
-                                          0.5f * (p.w[i3(kf - 1, jb, i, nj, ni)] + wb));
-    const float terrain = (((0.5f * p.rds) * (upper - lower)) * (rgt - rgb)) * p.rdy;
-    const float strain = 0.5f * ((dv + hw) + terrain);
-    const float density = 0.5f * (p.gz[(unsigned)jb * ni + i] * p.rf[i3(kf, jb, i, nj, ni)] +
-                                  p.gz[(unsigned)jt * ni + i] * p.rf[i3(kf, jt, i, nj, ni)]);
-    return strain * density;
-}
-
-// ---- flat column (terrain_flag=.false.) strains: rdz*mh(k) / rdz*mf(k)
-// (gm1_flat_calcdef_mass_v1 / _face_v1, src/cm1core/cuda_gm1_flat_stretched_closure.py:76-112;
-// turb.F:4772-4786, :4880-4895)
-
-// s11, s22, s33 at mass level k, cell (j, i)
-__device__ __forceinline__ void strain_diag_flat(const DefArgs &p, int k, int j, int i, float &s11, float &s22,
-                                                 float &s33) {
-    const int ni = p.ni, nj = p.nj, ux = ni + 1, vy = nj + 1;
-    const unsigned c = i3(k, j, i, nj, ni);
-    const float r = p.rho[c];
-    s11 = (r * (p.u[i3(k, j, i + 1, nj, ux)] - p.u[i3(k, j, i, nj, ux)])) * p.rdx;
-    s22 = (r * (p.v[i3(k, j + 1, i, vy, ni)] - p.v[i3(k, j, i, vy, ni)])) * p.rdy;
-    s33 = (r * (p.w[i3(k + 1, j, i, nj, ni)] - p.w[c])) * (p.rdz * p.mhp[k + 1]);
-}
-
-// s12 at mass level k, corner (jc, ic); open sides take the nearest interior corner
-__device__ __forceinline__ float strain_s12_flat(const DefArgs &p, int k, int jc, int ic) {
-    const int ni = p.ni, nj = p.nj, ux = ni + 1, vy = nj + 1;
-    const int jj = jc < 1 ? 1 : (jc > nj - 1 ? nj - 1 : jc);
-    const int ii = ic < 1 ? 1 : (ic > ni - 1 ? ni - 1 : ic);
-    const float x = (p.u[i3(k, jj, ii, nj, ux)] - p.u[i3(k, jj - 1, ii, nj, ux)]) * p.rdy;
-    const float y = (p.v[i3(k, jj, ii, vy, ni)] - p.v[i3(k, jj, ii - 1, vy, ni)]) * p.rdx;
-    const float rs = (p.rho[i3(k, jj - 1, ii - 1, nj, ni)] + p.rho[i3(k, jj, ii, nj, ni)]) +
-                     (p.rho[i3(k, jj, ii - 1, nj, ni)] + p.rho[i3(k, jj - 1, ii, nj, ni)]);
-    return ((0.5f * (x + y)) * 0.25f) * rs;
-}
-
-// s13 at face level kf (1..nk-1), row j, u-face column ic in [0, ni]
-__device__ __forceinline__ float strain_s13_flat(const DefArgs &p, int kf, int j, int ic) {
-    const int ni = p.ni, nj = p.nj, ux = ni + 1;
-    const int il = ic - 1 < 0 ? 0 : ic - 1, ir = ic < ni - 1 ? ic : ni - 1;
-    const float dw = (p.w[i3(kf, j, ir, nj, ni)] - p.w[i3(kf, j, il, nj, ni)]) * p.rdx;
-    const float du = (((p.u[i3(kf, j, ic, nj, ux)] - p.u[i3(kf - 1, j, ic, nj, ux)]) * p.rdz) * 0.5f) *
-                     (p.mf3[i3(kf, j, il, nj, ni)] + p.mf3[i3(kf, j, ir, nj, ni)]);
-    return ((0.5f * (dw + du)) * 0.5f) * (p.rf[i3(kf, j, il, nj, ni)] + p.rf[i3(kf, j, ir, nj, ni)]);
-}
-
-// s23 at face level kf (1..nk-1), v-face row jc in [0, nj], column i
-__device__ __forceinline__ float strain_s23_flat(const DefArgs &p, int kf, int jc, int i) {
-    const int ni = p.ni, nj = p.nj, vy = nj + 1;
-    const int js = jc - 1 < 0 ? 0 : jc - 1, jn = jc < nj - 1 ? jc : nj - 1;
-    const float dw = (p.w[i3(kf, jn, i, nj, ni)] - p.w[i3(kf, js, i, nj, ni)]) * p.rdy;
-    const float dv = (((p.v[i3(kf, jc, i, vy, ni)] - p.v[i3(kf - 1, jc, i, vy, ni)]) * p.rdz) * 0.5f) *
-                     (p.mf3[i3(kf, js, i, nj, ni)] + p.mf3[i3(kf, jn, i, nj, ni)]);
-    return ((0.5f * (dw + dv)) * 0.5f) * (p.rf[i3(kf, js, i, nj, ni)] + p.rf[i3(kf, jn, i, nj, ni)]);
-}
-
-template <bool FLAT>
-__device__ __forceinline__ void strain_diag_t(const DefArgs &p, int k, int j, int i, float &a, float &b, float &c) {
-    if (FLAT) strain_diag_flat(p, k, j, i, a, b, c);
-    else strain_diag(p, k, j, i, a, b, c);
-}
-template <bool FLAT>
-__device__ __forceinline__ float strain_s12_t(const DefArgs &p, int k, int jc, int ic) {
-    return FLAT ? strain_s12_flat(p, k, jc, ic) : strain_s12(p, k, jc, ic);
-}
-template <bool FLAT>
-__device__ __forceinline__ float strain_s13_t(const DefArgs &p, int kf, int j, int ic) {
-    return FLAT ? strain_s13_flat(p, kf, j, ic) : strain_s13(p, kf, j, ic);
-}
-template <bool FLAT>
-__device__ __forceinline__ float strain_s23_t(const DefArgs &p, int kf, int jc, int i) {
-    return FLAT ? strain_s23_flat(p, kf, jc, i) : strain_s23(p, kf, jc, i);
+// face-level value of a column (nk levels, `stride` words apart)
+__device__ __forceinline__ float atw(const float *q, unsigned kf, unsigned nk, unsigned stride) {
+    if (kf != 0 && kf != nk) return 0.5f * (q[(kf - 1) * stride] + q[kf * stride]);
+    const unsigned k0 = kf == 0 ? 0 : nk - 1, k1 = kf == 0 ? 1 : nk - 2, k2 = kf == 0 ? 2 : nk - 3;
+    float r = 1.875f * q[k0 * stride];
+    r = r + (-1.25f) * q[k1 * stride];
+    return r + 0.375f * q[k2 * stride];
 }
 
 __device__ __forceinline__ float sq(float x) { return x * x; }
 
-// One CTA = a 32 x 8 tile of columns, walking face levels 1..nk-1; FLAT
-// selects the flat column's strain texts (the deformation reduction of
-// turb.F:5361-5385 is the same in both branches).
+// Face levels k_lo .. k_hi of a chunk, after the mass level k_lo - 1 below
+// them.  FLAT selects the flat column's strain texts, rdz*mh(k) / rdz*mf(k)
+// (gm1_flat_calcdef_mass_v1 / _face_v1,
+// src/cm1core/cuda_gm1_flat_stretched_closure.py:76-112; turb.F:4772-4786,
+// :4880-4895); the deformation reduction of turb.F:5361-5385 is the same in
+// both branches.  Corners at the open sides are the nearest interior ones
+// (constant extension).  Bound by instruction issue and the loads' latency.
+// One CTA per 32 x 8 columns with every strain in shared memory (33 x 9 corners
+// take its 256 threads two passes, ~125 loads a level) took 473 us at
+// 256x256x80 on terrain and 0.84 ms at 640x768x80 flat; this takes 146 and
+// 0.59 (24 and 32 warps an SM; 16 and 24: 193 and 0.74).
 template <bool FLAT>
-__global__ void __launch_bounds__(kDX *kDY) calcdef_tile_kernel(DefArgs p) {
-    __shared__ float s12[2][kDY + 1][kDX + 1];
-    __shared__ float s13[kDY][kDX + 1];
-    __shared__ float s23[kDY + 1][kDX];
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kDX + tx;
-    const int i0 = blockIdx.x * kDX, j0 = blockIdx.y * kDY;
-    const int i = i0 + tx, j = j0 + ty;
-    const int ni = p.ni, nj = p.nj, nk = p.nk;
-    const bool own = i < ni && j < nj;
-    constexpr int kCorners = (kDY + 1) * (kDX + 1), kXFaces = kDY * (kDX + 1), kYFaces = (kDY + 1) * kDX;
-
-    float p11 = 0.0f, p22 = 0.0f, p33 = 0.0f;  // mass level kf-1 at the own cell
-    if (own) strain_diag_t<FLAT>(p, 0, j, i, p11, p22, p33);
-    for (int e = tid; e < kCorners; e += kDX * kDY) {
-        const int r = e / (kDX + 1), q = e - r * (kDX + 1);
-        if (j0 + r <= nj && i0 + q <= ni) s12[0][r][q] = strain_s12_t<FLAT>(p, 0, j0 + r, i0 + q);
+__global__ void __launch_bounds__(32 * kDefRows, FLAT ? 4 : 3)
+    calcdef_march_kernel(const __grid_constant__ DefArgs p, int levels_per_chunk) {
+    __shared__ float s_12[2][kDefRows][32], s_23[2][kDefRows][32];
+    const int lane = threadIdx.x, ty = threadIdx.y;
+    const int ni = p.ni, nj = p.nj, nk = p.nk, ux = ni + 1, vy = nj + 1;
+    const int tiles = (ni + kDefOut - 1) / kDefOut;
+    const int i0 = blockIdx.x % tiles * kDefOut + lane, row = blockIdx.x / tiles * (kDefRows - 1) + ty;
+    const bool own = i0 < ni && row < nj && lane < kDefOut && ty < kDefRows - 1;
+    const int i = min(i0, ni), j = min(row, nj);  // faces past the domain repeat its last ones
+    const int ic = min(i, ni - 1), jc = min(j, nj - 1), iw = max(i - 1, 0), js = max(j - 1, 0);
+    const int ii = min(max(i, 1), ni - 1), jj = min(max(j, 1), nj - 1);  // the corner
+    const unsigned uz = (unsigned)nj * ux, vz = (unsigned)vy * ni, cz = (unsigned)nj * ni;
+    const unsigned oc = i3(0, jc, ic, nj, ni), ow = i3(0, jc, iw, nj, ni), os = i3(0, js, ic, nj, ni);
+    const unsigned oua = i3(0, jj, ii, nj, ux), oub = oua - ux, ouc = i3(0, jc, i, nj, ux);
+    const unsigned ova = i3(0, jj, ii, vy, ni), ovb = ova - 1, ovc = i3(0, j, ic, vy, ni),
+                   ovd = i3(0, min(j + 1, nj), ic, vy, ni);
+    const unsigned orr = i3(0, jj, ii, nj, ni);  // the corner's north-east cell
+    const int k_lo = 1 + blockIdx.y * levels_per_chunk, k_hi = min(nk - 1, k_lo + levels_per_chunk - 1);
+    const unsigned k0 = k_lo - 1;
+    // a, b: the corner's two faces of each field; c (and d): the cell's
+    float ua = p.u[k0 * uz + oua], ub = p.u[k0 * uz + oub], uc = p.u[k0 * uz + ouc], um = 0.0f;
+    float va = p.v[k0 * vz + ova], vb = p.v[k0 * vz + ovb], vc = p.v[k0 * vz + ovc], vd = p.v[k0 * vz + ovd], vm = 0.0f;
+    float wc = p.w[k0 * cz + oc], ww = p.w[k0 * cz + ow], ws = p.w[k0 * cz + os];
+    // sums at the lower face level of the two faces of each kind, and the
+    // metric there
+    float xl = 0.0f, yl = 0.0f, gl = 0.0f, hl = 0.0f, wlx = 0.0f, wly = 0.0f;
+    if (!FLAT) {
+        xl = atw(p.u + oub, k0, nk, uz) + atw(p.u + oua, k0, nk, uz);
+        yl = atw(p.v + ovb, k0, nk, vz) + atw(p.v + ova, k0, nk, vz);
+        const float fu = atw(p.u + ouc, k0, nk, uz);
+        gl = p.gx[k0 * cz + oc] * (fu + __shfl_down_sync(0xffffffffu, fu, 1));
+        hl = p.gy[k0 * cz + oc] * (atw(p.v + ovc, k0, nk, vz) + atw(p.v + ovd, k0, nk, vz));
     }
-    for (int kf = 1; kf < nk; ++kf) {
-        const int cur = kf & 1;
-        float c11 = 0.0f, c22 = 0.0f, c33 = 0.0f;
-        if (own) strain_diag_t<FLAT>(p, kf, j, i, c11, c22, c33);
-        for (int e = tid; e < kCorners; e += kDX * kDY) {
-            const int r = e / (kDX + 1), q = e - r * (kDX + 1);
-            if (j0 + r <= nj && i0 + q <= ni) s12[cur][r][q] = strain_s12_t<FLAT>(p, kf, j0 + r, i0 + q);
+    float g = 0.0f, gw = 0.0f, gs = 0.0f, rg = 0.0f, rgw = 0.0f, rgs = 0.0f;
+    float ga = 0.0f, gb = 0.0f, gc = 0.0f, gd = 0.0f, rua = 0.0f, rub = 0.0f, ruc = 0.0f, rue = 0.0f, rva = 0.0f,
+          rvb = 0.0f, rvc = 0.0f, rvd = 0.0f;
+    if (!FLAT) {
+        g = p.gz[oc], gw = p.gz[ow], gs = p.gz[os], rg = p.rgz[oc], rgw = p.rgz[ow], rgs = p.rgz[os];
+        ga = p.gz[orr], gb = p.gz[orr - 1], gc = p.gz[orr - ni], gd = p.gz[orr - ni - 1];
+        rua = p.rgzu[oua], rub = p.rgzu[oub], ruc = p.rgzu[ouc];
+        rue = __shfl_down_sync(0xffffffffu, ruc, 1);
+        rva = p.rgzv[ova], rvb = p.rgzv[ovb], rvc = p.rgzv[ovc], rvd = p.rgzv[ovd];
+    }
+    float p11 = 0.0f, p22 = 0.0f, p33 = 0.0f, lo12 = 0.0f;  // the mass level below
+#pragma unroll 1
+    for (int kf = k_lo - 1; kf <= k_hi; ++kf) {
+        const unsigned k = kf, z = k * cz;
+        const bool more = kf + 1 < nk;
+        const unsigned un = (k + 1) * uz, vn = (k + 1) * vz;
+        const float nua = more ? p.u[un + oua] : 0.0f, nub = more ? p.u[un + oub] : 0.0f, nuc = more ? p.u[un + ouc] : 0.0f;
+        const float nva = more ? p.v[vn + ova] : 0.0f, nvb = more ? p.v[vn + ovb] : 0.0f,
+                    nvc = more ? p.v[vn + ovc] : 0.0f, nvd = more ? p.v[vn + ovd] : 0.0f;
+        const float nwc = p.w[z + cz + oc], nww = p.w[z + cz + ow], nws = p.w[z + cz + os];
+        const float rfc = p.rf[z + oc], rfw = p.rf[z + ow], rfs = p.rf[z + os];
+        const float a = p.c1[z + oc], b = p.c2[z + oc];
+        const float r = p.rho[z + oc], ra = p.rho[z + orr], rb = p.rho[z + orr - 1], rc = p.rho[z + orr - ni],
+                    rd = p.rho[z + orr - ni - 1];
+        const float ue = __shfl_down_sync(0xffffffffu, uc, 1);
+        float c11, c22, c33, c12, c13 = 0.0f, c23 = 0.0f;
+        if (FLAT) {
+            c11 = (r * (ue - uc)) * p.rdx;
+            c22 = (r * (vd - vc)) * p.rdy;
+            c33 = (r * (nwc - wc)) * (p.rdz * p.mhp[kf + 1]);
+            const float x = (ua - ub) * p.rdy, y = (va - vb) * p.rdx;
+            c12 = ((0.5f * (x + y)) * 0.25f) * ((rd + ra) + (rb + rc));
+            if (kf >= k_lo) {
+                const float mc = p.mf3[z + oc], mw = p.mf3[z + ow], ms = p.mf3[z + os];
+                const float du = (((uc - um) * p.rdz) * 0.5f) * (mw + mc);
+                c13 = ((0.5f * ((wc - ww) * p.rdx + du)) * 0.5f) * (rfw + rfc);
+                const float dv = (((vc - vm) * p.rdz) * 0.5f) * (ms + mc);
+                c23 = ((0.5f * ((wc - ws) * p.rdy + dv)) * 0.5f) * (rfs + rfc);
+            }
+        } else {
+            // the velocities at the upper face level
+            float xu, yu, fu, fv;
+            if (more) {
+                xu = 0.5f * (ub + nub) + 0.5f * (ua + nua);
+                yu = 0.5f * (vb + nvb) + 0.5f * (va + nva);
+                fu = 0.5f * (uc + nuc);
+                fv = 0.5f * (vc + nvc) + 0.5f * (vd + nvd);
+            } else {
+                xu = atw(p.u + oub, nk, nk, uz) + atw(p.u + oua, nk, nk, uz);
+                yu = atw(p.v + ovb, nk, nk, vz) + atw(p.v + ova, nk, nk, vz);
+                fu = atw(p.u + ouc, nk, nk, uz);
+                fv = atw(p.v + ovc, nk, nk, vz) + atw(p.v + ovd, nk, nk, vz);
+            }
+            const float gu = p.gx[z + cz + oc] * (fu + __shfl_down_sync(0xffffffffu, fu, 1));
+            const float hu = p.gy[z + cz + oc] * fv;
+            float hor = (g * (ue * rue - uc * ruc)) * p.rdx;
+            c11 = (hor + ((gu - gl) * 0.5f) * p.rds) * r;
+            hor = (g * (vd * rvd - vc * rvc)) * p.rdy;
+            c22 = (hor + ((hu - hl) * 0.5f) * p.rds) * r;
+            c33 = (((nwc - wc) * p.rds) * g) * r;
+            const float z_hi = p.zt - (float)(kf + 1) * p.dz, z_lo = p.zt - (float)kf * p.dz;
+            const float r1 = 0.25f * ((rd * gd + ra * ga) + (rb * gb + rc * gc));
+            const float x1 = (r1 * (ua * rua - ub * rub)) * p.rdy;
+            const float x2 = ((((0.5f * (z_hi * xu - z_lo * xl)) * p.rds) * r1) * (rua - rub)) * p.rdy;
+            const float y1 = (r1 * (va * rva - vb * rvb)) * p.rdx;
+            const float y2 = ((((0.5f * (z_hi * yu - z_lo * yl)) * p.rds) * r1) * (rva - rvb)) * p.rdx;
+            c12 = 0.5f * ((x1 + x2) + (y1 + y2));
+            const float zm_u = p.zt - ((float)kf + 0.5f) * p.dz, zm_l = p.zt - ((float)kf - 0.5f) * p.dz;
+            const float hc = 0.5f * (wc + nwc), wux = hc + 0.5f * (ww + nww), wuy = hc + 0.5f * (ws + nws);
+            if (kf >= k_lo) {
+                const float du = (uc - um) * p.rds, hx = (wc * rg - ww * rgw) * p.rdx;
+                const float tx = (((0.5f * p.rds) * (zm_u * wux - zm_l * wlx)) * (rg - rgw)) * p.rdx;
+                c13 = (0.5f * ((du + hx) + tx)) * (0.5f * (gw * rfw + g * rfc));
+                const float dv = (vc - vm) * p.rds, hy = (wc * rg - ws * rgs) * p.rdy;
+                const float ty2 = (((0.5f * p.rds) * (zm_u * wuy - zm_l * wly)) * (rg - rgs)) * p.rdy;
+                c23 = (0.5f * ((dv + hy) + ty2)) * (0.5f * (gs * rfs + g * rfc));
+            }
+            xl = xu, yl = yu, gl = gu, hl = hu, wlx = wux, wly = wuy;
         }
-        for (int e = tid; e < kXFaces; e += kDX * kDY) {
-            const int r = e / (kDX + 1), q = e - r * (kDX + 1);
-            if (j0 + r < nj && i0 + q <= ni) s13[r][q] = strain_s13_t<FLAT>(p, kf, j0 + r, i0 + q);
-        }
-        for (int e = tid; e < kYFaces; e += kDX * kDY) {
-            const int r = e / kDX, q = e - r * kDX;
-            if (j0 + r <= nj && i0 + q < ni) s23[r][q] = strain_s23_t<FLAT>(p, kf, j0 + r, i0 + q);
-        }
+        s_12[kf & 1][ty][lane] = c12;
+        s_23[kf & 1][ty][lane] = c23;
         __syncthreads();
-        if (own) {
-            const unsigned f = i3(kf, j, i, nj, ni);
-            const float a = p.c1[f], b = p.c2[f];
+        const int up = min(ty + 1, kDefRows - 1);
+        const float n12 = s_12[kf & 1][up][lane], ne12 = s_12[kf & 1][up][min(lane + 1, 31)];
+        const float e12 = __shfl_down_sync(0xffffffffu, c12, 1), e13 = __shfl_down_sync(0xffffffffu, c13, 1);
+        const float hi12 = (sq(c12) + sq(ne12)) + (sq(n12) + sq(e12));
+        if (kf >= k_lo && own) {
             const float t11 = a * sq(p11) + b * sq(c11);
             const float t22 = a * sq(p22) + b * sq(c22);
             const float t33 = a * sq(p33) + b * sq(c33);
-            const float(*L)[kDX + 1] = s12[cur ^ 1];
-            const float(*H)[kDX + 1] = s12[cur];
-            const float lo12 = (sq(L[ty][tx]) + sq(L[ty + 1][tx + 1])) + (sq(L[ty + 1][tx]) + sq(L[ty][tx + 1]));
-            const float hi12 = (sq(H[ty][tx]) + sq(H[ty + 1][tx + 1])) + (sq(H[ty + 1][tx]) + sq(H[ty][tx + 1]));
             const float t12 = 0.25f * (a * lo12 + b * hi12);
-            const float t13 = 0.5f * (sq(s13[ty][tx]) + sq(s13[ty][tx + 1]));
-            const float t23 = 0.5f * (sq(s23[ty][tx]) + sq(s23[ty + 1][tx]));
-            const float rfv = p.rf[f];
-            const float rrf = rcp_rn(rfv * rfv);
-            p.defv[f] = (4.0f * (t13 + t23)) * rrf;
-            p.defh[f] = ((2.0f * ((t11 + t22) + t33)) + 4.0f * t12) * rrf;
+            const float t13 = 0.5f * (sq(c13) + sq(e13));
+            const float t23 = 0.5f * (sq(c23) + sq(s_23[kf & 1][up][lane]));
+            const float rrf = rcp_rn(rfc * rfc);
+            p.defv[z + oc] = (4.0f * (t13 + t23)) * rrf;
+            p.defh[z + oc] = ((2.0f * ((t11 + t22) + t33)) + 4.0f * t12) * rrf;
         }
-        p11 = c11;
-        p22 = c22;
-        p33 = c33;
-        __syncthreads();
+        p11 = c11, p22 = c22, p33 = c33, lo12 = hi12;
+        um = uc, uc = nuc, ua = nua, ub = nub;
+        vm = vc, vc = nvc, vd = nvd, va = nva, vb = nvb;
+        wc = nwc, ww = nww, ws = nws;
     }
-    if (own) {
-        p.defv[i3(0, j, i, nj, ni)] = 0.0f;
-        p.defh[i3(0, j, i, nj, ni)] = 0.0f;
-        p.defv[i3(nk, j, i, nj, ni)] = 0.0f;
-        p.defh[i3(nk, j, i, nj, ni)] = 0.0f;
+    if (own && blockIdx.y == 0) {
+        p.defv[oc] = 0.0f;
+        p.defh[oc] = 0.0f;
+        p.defv[(unsigned)nk * cz + oc] = 0.0f;
+        p.defh[(unsigned)nk * cz + oc] = 0.0f;
     }
 }
 
@@ -468,6 +397,21 @@ bool launch_ok(const char *what) {
 
 using namespace gm1b;
 
+namespace {
+// Whole columns leave a small plane too few warps; a chunk of levels forms the
+// strains of the mass level below it again: halve until two rounds of the
+// resident CTAs on 148 SMs, or eight levels, are left
+// (256x256x80 terrain: 246 us with whole columns; 128x100x64 flat: 80 against 27).
+template <bool FLAT>
+void calcdef_launch(const DefArgs &p, cudaStream_t st) {
+    const long long tiles =
+        (long long)((p.ni + kDefOut - 1) / kDefOut) * ((p.nj + kDefRows - 2) / (kDefRows - 1));
+    int chunk = p.nk - 1;
+    while (chunk > 8 && tiles * ((p.nk - 2 + chunk) / chunk) < 3LL * 148 * (FLAT ? 4 : 3)) chunk = (chunk + 1) / 2;
+    calcdef_march_kernel<FLAT><<<dim3((unsigned)tiles, (p.nk - 2 + chunk) / chunk), dim3(32, kDefRows), 0, st>>>(p, chunk);
+}
+}  // namespace
+
 extern "C" int32_t gm1b_terrain_deformation(int32_t ni, int32_t nj, int32_t nk,
                                             const gm1b_deformation_arrays *arrays, float dx, float dy, float dz,
                                             void *stream) {
@@ -516,10 +460,10 @@ extern "C" int32_t gm1b_terrain_deformation(int32_t ni, int32_t nj, int32_t nk,
     p.zt = (float)nk * dz;
     p.dz = dz;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    ProfScope ps("calcdef_tile_kernel", st);
-    calcdef_tile_kernel<false><<<dim3((ni + kDX - 1) / kDX, (nj + kDY - 1) / kDY), dim3(kDX, kDY), 0, st>>>(p);
+    ProfScope ps("calcdef_march_kernel", st);
+    calcdef_launch<false>(p, st);
     ps.stop();
-    return launch_ok("calcdef_tile_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
+    return launch_ok("calcdef_march_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }
 
 extern "C" int32_t gm1b_flat_deformation(int32_t ni, int32_t nj, int32_t nk, const gm1b_flat_deformation_arrays *arrays,
@@ -562,10 +506,10 @@ extern "C" int32_t gm1b_flat_deformation(int32_t ni, int32_t nj, int32_t nk, con
     p.rdy = 1.0f / dy;
     p.rdz = rdz;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    ProfScope ps("calcdef_flat_tile_kernel", st);
-    calcdef_tile_kernel<true><<<dim3((ni + kDX - 1) / kDX, (nj + kDY - 1) / kDY), dim3(kDX, kDY), 0, st>>>(p);
+    ProfScope ps("calcdef_flat_march_kernel", st);
+    calcdef_launch<true>(p, st);
     ps.stop();
-    return launch_ok("calcdef_flat_tile_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
+    return launch_ok("calcdef_flat_march_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }
 
 extern "C" int32_t gm1b_moist_nm(int32_t ni, int32_t nj, int32_t nk, const gm1b_moist_nm_arrays *arrays, float dz,

@@ -151,6 +151,33 @@ def test_flat_tke_diffusion(ni, nj, nk):
     assert _differ(dev, a, ("tketen",)) == []
 
 
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("ni,nj,nk", [(31, 7, 9), (32, 8, 10), (30, 6, 18), (3, 3, 3), (63, 15, 20)])
+def test_deformation(ni, nj, nk, flat):
+    """Runs of levels of the strains' march."""
+    from gm1_b200 import closure
+    from oracle import closure as orc
+    from tests.golden.make_golden import deformation_fixture
+
+    a = deformation_fixture(ni, nj, nk, seed=3 * ni + nk)
+    dx, dy, dz = (float(x) for x in a.pop("_spacing"))
+    g = dict(ni=ni, nj=nj, nk=nk, dx=dx, dy=dy)
+    if flat:
+        p = _profiles(nk)
+        a["mf"] = np.random.default_rng(nk).uniform(0.3, 3.0, (nk + 1, nj, ni)).astype(np.float32)
+        a["mh_profile"] = p["mh"]
+        a = {n: a[n] for n in orc.FLAT_DEFORMATION_INPUTS + ("defv", "defh")}
+        dev = _dev(a)
+        orc.flat_calcdef(a, **g, rdz=p["rdz"])
+        mh = dev.pop("mh_profile")
+        closure.launch_cuda_flat_deformation(dev, mh_profile=mh, **g, rdz=p["rdz"])
+    else:
+        dev = _dev(a)
+        orc.calcdef(a, **g, dz=dz)
+        closure.launch_cuda_terrain_deformation(dev, **g, dz=dz)
+    assert _differ(dev, a, ("defv", "defh")) == []
+
+
 @pytest.mark.parametrize("column", ["uniform", "terrain", "flat"])
 @pytest.mark.parametrize("obc,pdefweno", [(0x2222, 0), (0x2222, 1), (0x1111, 1), (0x3443, 0)])
 @pytest.mark.parametrize("ni,nj,nk", [(29, 7, 4), (30, 8, 5), (31, 9, 6), (61, 14, 9), (5, 15, 33)])
