@@ -410,8 +410,8 @@ constexpr int kStageWRows = 8;  // rows per CTA of the WENO stage: 8 rows of y f
 // level), the last row forming a flux only.  Columns beyond the open sides
 // repeat the edge ones.  Bound by instruction issue (fifth order) and the
 // binary64 weights (WENO); a step's three flat stages at 640x768x80 took 5.04 ms
-// with six fluxes per cell and take 2.87 here (24 warps an SM for WENO: 16
-// warps 1.787 ms a stage, 24 1.624).
+// with six fluxes per cell and take 2.52 here (a fifth-order stage 0.497 ms,
+// 0.624 with every offset clamped; WENO 1.524, and 1.787 with 16 warps an SM).
 // FLAT: the flat column's advw (gm1_flat_tke_advw_rk_v1,
 // src/cm1core/cuda_gm1_flat_stretched_closure.py:401-449; adv.F:3252-3355
 // with terrain_flag=.false.): vertical divergence -(dumz(k)-dumz(k-1))*rdz
@@ -419,7 +419,7 @@ constexpr int kStageWRows = 8;  // rows per CTA of the WENO stage: 8 rows of y f
 // open-side divergence piece (q*d)*rdx evaluated left to right, no gz.
 template <bool W, bool FLAT>
 __global__ void __launch_bounds__(32 * (W ? kStageWRows : kStageRows), W ? 3 : 8)
-    tke_rk_stage_kernel(TkeArgs a, const float *__restrict__ cur, float *__restrict__ nxt, float *__restrict__ nxt2,
+    tke_rk_stage_kernel(const __grid_constant__ TkeArgs a, const float *__restrict__ cur, float *__restrict__ nxt, float *__restrict__ nxt2,
                         int levels_per_chunk, float dttmp, double eps) {
     constexpr int ROWS = W ? kStageWRows : kStageRows;
     __shared__ float s_fy[W ? 2 : 1][W ? ROWS : 1][32], s_my[W ? 2 : 1][W ? ROWS : 1][32];
@@ -435,11 +435,11 @@ __global__ void __launch_bounds__(32 * (W ? kStageWRows : kStageRows), W ? 3 : 8
     const bool own = i0 < ni && row < nj && lane < kStageOut && (!W || ty < ROWS - 1);
     const int jc = min(j, nj - 1), ic = min(i, ni - 1), cc = jc * ni + ic;
     const int ou = (jc + kG) * ux + i + kG, ov = (j + kG) * sx + ic + kG, ow = (jc + kG) * sx + ic + kG;
-    int xo[6], yo[7];  // clamped columns and rows of the two stencils, as offsets in a level
-#pragma unroll
-    for (int q = 0; q < 6; ++q) xo[q] = jc * ni + clampi(i + q - 3, ni);
-#pragma unroll
-    for (int q = 0; q < 7; ++q) yo[q] = clampi(j + q - 3, nj) * ni + ic;
+    // a warp whose stencils stay inside the plane loads them at fixed offsets,
+    // one at its edge at clamped columns and rows
+    const bool inside = __all_sync(0xffffffffu, i >= 3 && i + 2 < ni) && j >= 3 && j + 3 < nj;
+    auto xo = [&](int q) { return jc * ni + clampi(i + q - 3, ni); };
+    auto yo = [&](int q) { return clampi(j + q - 3, nj) * ni + ic; };
     // window of the own column: levels f_lo-4 .. f_lo+1, shifted to f-3 .. f+2
     const int f_lo = blockIdx.y * levels_per_chunk, f_hi = min(nk, f_lo + levels_per_chunk - 1);
     if (f_lo == 0 && own) {
@@ -465,30 +465,50 @@ __global__ void __launch_bounds__(32 * (W ? kStageWRows : kStageRows), W ? 3 : 8
     if (!W) rnl = __ldg(a.rrv + k_lo * vz + ov + sx);
     float dl = __ldg(a.divx + (k_lo - 1) * cz + cc);
     const float gz = FLAT ? 0.0f : __ldg(a.gz + cc);
+    // WENO rows of cells away from the open sides, at levels away from the
+    // column's ends, take a finish without those branches (256x256x80: 249 ->
+    // 234 us; the fifth-order stage gains nothing from it, 86 against 89)
+    const bool edge = !W || __any_sync(0xffffffffu, i == 0 || i == ni - 1) || j == 0 || j == nj - 1;
 #pragma unroll 1
     for (int f = k_lo; f <= k_hi; ++f) {
         const float *lev = cur + f * cz;
         const float q = win[3];
-        float px[6], py[7];
-#pragma unroll
-        for (int e = 0; e < 6; ++e) px[e] = __ldg(lev + xo[e]);
-#pragma unroll
-        for (int e = 0; e < 7; ++e) py[e] = W && e == 6 ? 0.0f : __ldg(lev + yo[e]);
-        const float next = f + 3 <= nk ? __ldg(lev + 3 * cz + cc) : 0.0f;
         const float *c2p = a.c2 + f * cz;
-        const float kw = __ldg(c2p + xo[2]), ke = __ldg(c2p + xo[3]), ks = __ldg(c2p + yo[2]), kn = __ldg(c2p + yo[3]);
+        float px[6], py[7], kw, ks, kn = 0.0f;
+        px[3] = py[3] = q;  // the centre is the own column's
+        py[6] = 0.0f;
+        if (inside) {
+            const float *pt = lev + cc, *pc = c2p + cc;
+            kw = __ldg(pc - 1), ks = __ldg(pc - ni);
+            if (!W) kn = __ldg(pc + ni);
+#pragma unroll
+            for (int e = 0; e < 6; ++e)
+                if (e != 3) px[e] = __ldg(pt + (e - 3));
+#pragma unroll
+            for (int e = 0; e < (W ? 6 : 7); ++e)
+                if (e != 3) py[e] = __ldg(pt + (e - 3) * ni);
+        } else {
+            kw = __ldg(c2p + xo(2)), ks = __ldg(c2p + yo(2));
+            if (!W) kn = __ldg(c2p + yo(4));
+#pragma unroll
+            for (int e = 0; e < 6; ++e)
+                if (e != 3) px[e] = __ldg(lev + xo(e));
+#pragma unroll
+            for (int e = 0; e < (W ? 6 : 7); ++e)
+                if (e != 3) py[e] = __ldg(lev + yo(e));
+        }
+        const float next = f + 3 <= nk ? __ldg(lev + 3 * cz + cc) : 0.0f;
         const float c2 = __ldg(c2p + cc);
         const float ru = __ldg(a.rru + (f + 1) * uz + ou), rs = __ldg(a.rrv + (f + 1) * vz + ov);
         const float rwn = __ldg(a.rrw + (f + 2) * wz + ow), dh = __ldg(a.divx + f * cz + cc);
         const unsigned z = (unsigned)f * (unsigned)cz + (unsigned)cc;
         const float base = a.tkea[z], ten = __ldg(a.tketen + z);
         const float rrf = FLAT ? __ldg(a.rrf0 + f * cz) : __ldg(a.rrf0 + z);
-        const float c2x = 0.5f * (kw + ke), c2y = 0.5f * (ks + kn);
+        const float c2x = 0.5f * (kw + c2), c2y = 0.5f * (ks + c2);
         const float mw = c2x * ru + (1.0f - c2x) * rul, ms = c2y * rs + (1.0f - c2y) * rsl;
         const float fx0 = up6<W>(mw, px[0], px[1], px[2], px[3], px[4], px[5], eps);
         const float fy0 = up6<W>(ms, py[0], py[1], py[2], py[3], py[4], py[5], eps);
-        const float fx1 = __shfl_down_sync(0xffffffffu, fx0, 1), me = __shfl_down_sync(0xffffffffu, mw, 1);
-        const float rue = __shfl_down_sync(0xffffffffu, ru, 1), rule = __shfl_down_sync(0xffffffffu, rul, 1);
+        const float fx1 = __shfl_down_sync(0xffffffffu, fx0, 1);
         float fy1, mn, rn = 0.0f;
         if (W) {
             s_fy[f & 1][ty][lane] = fy0;
@@ -499,32 +519,39 @@ __global__ void __launch_bounds__(32 * (W ? kStageWRows : kStageRows), W ? 3 : 8
             mn = s_my[f & 1][up][lane];
         } else {
             rn = __ldg(a.rrv + (f + 1) * vz + ov + sx);
-            const float c2n = 0.5f * (kn + __ldg(c2p + yo[4]));
+            const float c2n = 0.5f * (c2 + kn);
             mn = c2n * rn + (1.0f - c2n) * rnl;
             fy1 = up6<W>(mn, py[1], py[2], py[3], py[4], py[5], py[6], eps);
-        }
-        // inflow through an open side's face takes the inner neighbour's flux
-        const bool sw = i == 0 && mw >= 0.0f, se = i == ni - 1 && me <= 0.0f;
-        const bool ss = j == 0 && ms >= 0.0f, sn = j == nj - 1 && mn <= 0.0f;
-        float ax = -1.0f * (((se ? fx0 : fx1) - (sw ? fx1 : fx0)) * a.rdx);
-        float ay = -1.0f * (((sn ? fy0 : fy1) - (ss ? fy1 : fy0)) * a.rdy);
-        const float c1 = 1.0f - c2;
-        if (sw || se) {
-            const float du = c1 * (rule - rul) + c2 * (rue - ru);
-            ax = FLAT ? ax - ((q * du) * a.rdx) : ax - q * (du * a.rdx);
-        }
-        if (ss || sn) {
-            if (W) {
-                rn = __ldg(a.rrv + (f + 1) * vz + ov + sx);
-                rnl = __ldg(a.rrv + f * vz + ov + sx);
-            }
-            const float dv = c1 * (rnl - rsl) + c2 * (rn - rs);
-            ay = FLAT ? ay - ((q * dv) * a.rdy) : ay - q * (dv * a.rdy);
         }
 #pragma unroll
         for (int e = 0; e < 5; ++e) win[e] = win[e + 1];
         win[5] = next;
-        const float zhi = vert_flux<W>(win, 0.5f * (rw + rwn), f + 1, nk, eps);
+        const float mz = 0.5f * (rw + rwn), c1 = 1.0f - c2;
+        float ax, ay, zhi;
+        if (!edge && f >= 2 && f < nk - 2) {
+            zhi = up6<W>(mz, win[0], win[1], win[2], win[3], win[4], win[5], eps);
+            ax = -1.0f * ((fx1 - fx0) * a.rdx);
+            ay = -1.0f * ((fy1 - fy0) * a.rdy);
+        } else {
+            const float me = __shfl_down_sync(0xffffffffu, mw, 1), rue = __shfl_down_sync(0xffffffffu, ru, 1);
+            const float rule = __shfl_down_sync(0xffffffffu, rul, 1);
+            // inflow through an open side's face takes the inner neighbour's flux
+            const bool sw = i == 0 && mw >= 0.0f, se = i == ni - 1 && me <= 0.0f;
+            const bool ss = j == 0 && ms >= 0.0f, sn = j == nj - 1 && mn <= 0.0f;
+            zhi = vert_flux<W>(win, mz, f + 1, nk, eps);
+            ax = -1.0f * (((se ? fx0 : fx1) - (sw ? fx1 : fx0)) * a.rdx);
+            ay = -1.0f * (((sn ? fy0 : fy1) - (ss ? fy1 : fy0)) * a.rdy);
+            if (sw || se) {
+                const float du = c1 * (rule - rul) + c2 * (rue - ru);
+                ax = FLAT ? ax - ((q * du) * a.rdx) : ax - q * (du * a.rdx);
+            }
+            if (ss || sn) {
+                const float rnh = W ? __ldg(a.rrv + (f + 1) * vz + ov + sx) : rn;
+                const float rnk = W ? __ldg(a.rrv + f * vz + ov + sx) : rnl;
+                const float dv = c1 * (rnk - rsl) + c2 * (rnh - rs);
+                ay = FLAT ? ay - ((q * dv) * a.rdy) : ay - q * (dv * a.rdy);
+            }
+        }
         const float dvf = zhi - zlo;
         const float az = FLAT ? ((-dvf) * a.rdz) * __ldg(a.mfp + f + 1) : -1.0f * (dvf * a.rdz);
         float total = (ax + ay) + az;
