@@ -117,6 +117,41 @@ int32_t open_fills(int32_t ni, int32_t nj, int32_t nk, const OpenFill *fills, in
 int32_t pack_scalars_open(int32_t ni, int32_t nj, int32_t nk, const float *th0, const float *const scalar[4],
                           float *const padded[4], cudaStream_t st);
 
+constexpr int kSweepChunk = 8;  // back-substitution levels whose words the sweep reads together
+
+// the sweep of a column's tridiagonal rows in shared memory (rows p at stride
+// 32, forward into c and d, the solution left in d), one lane per column; n >= 1
+__device__ __forceinline__ void column_sweep(const float *s_a, const float *s_b, float *s_c, float *s_d, int n) {
+    float cprev = 0.0f, dprev = 0.0f;
+    float cfa = s_a[0], cfb = s_b[0], cfc = s_c[0], cfd = s_d[0];
+    for (int p = 0; p < n - 1; ++p) {
+        const int q = (p + 1) * 32;
+        const float na = s_a[q], nb = s_b[q], nc = s_c[q], nd = s_d[q];
+        const float inv = rcp_rn(p == 0 ? cfb : cfa * cprev + cfb);
+        cprev = -(cfc * inv);
+        dprev = (p == 0 ? cfd : cfd - cfa * dprev) * inv;
+        s_c[p * 32] = cprev;
+        s_d[p * 32] = dprev;
+        cfa = na, cfb = nb, cfc = nc, cfd = nd;
+    }
+    float sol = (cfd - cfa * dprev) * rcp_rn(cfa * cprev + cfb);
+    s_d[(n - 1) * 32] = sol;
+    for (int pb = n - 2; pb >= 0; pb -= kSweepChunk) {
+        float ce[kSweepChunk], de[kSweepChunk];
+#pragma unroll
+        for (int e = 0; e < kSweepChunk; ++e) {
+            const int p = max(pb - e, 0);
+            ce[e] = s_c[p * 32], de[e] = s_d[p * 32];
+        }
+#pragma unroll
+        for (int e = 0; e < kSweepChunk; ++e) {
+            if (pb - e < 0) break;
+            sol = ce[e] * sol + de[e];
+            s_d[(pb - e) * 32] = sol;
+        }
+    }
+}
+
 }  // namespace gm1b
 
 // thread-local error message of the last failed entry point

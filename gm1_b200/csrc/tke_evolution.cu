@@ -10,14 +10,13 @@
 //               (enqueue_flat_turbt :631; CartesianClosure.tke_rk, cuda_cartesian_closure.py:1658-1663)
 //
 // Design (B200):
-//  * turbt is one kernel per 32 x 4 column tile.  Each thread first solves
-//    its column's implicit diffusion (Thomas) with the elimination arrays in
-//    shared memory (the reference's thread-per-column kernel keeps five local
-//    arrays of 74 words, which spill); then the tile walks the face levels
-//    upwards with a three-level ring of the x and y TKE face fluxes (33 x 4
-//    and 32 x 5 per level) in shared memory, so every face flux is formed
-//    once, and each cell adds its horizontal divergence and vertical
-//    diffusion to tketen.  No device scratch.
+//  * turbt is one kernel per 32 columns of a row: eight warps form the
+//    tridiagonal rows of their own runs of levels (the mf/rf divisions and
+//    every load spread over the CTA), one warp sweeps them in shared memory
+//    (the reference's thread-per-column kernel keeps five local arrays of 74
+//    words, which spill), then all warps add the horizontal flux divergence
+//    and the vertical diffusion of their levels to tketen, each face flux of
+//    a column formed once and carried up.  No device scratch.
 //  * an RK stage marches warps of 32 x faces up the face levels: each x and
 //    vertical face flux (fifth order, WENO5 at nrk = 3) is formed once, from
 //    the stage-start field.
@@ -29,8 +28,8 @@
 namespace gm1b {
 namespace {
 
-constexpr int kTTX = 32, kTTY = 4, kTT = kTTX * kTTY;  // turbt tile
-constexpr int kTTChunk = 8;  // levels whose column-solve loads turbt issues together
+constexpr int kTurbtWarps = 8;  // warps of a turbt CTA, which owns 32 columns of a row
+constexpr int kTurbtMostNk = 201;
 constexpr int kG = 3;                                    // padded-lane halo of rru/rrv/rrw
 
 struct TkeArgs {
@@ -45,203 +44,95 @@ struct TkeArgs {
 __device__ __forceinline__ int clampi(int x, int n) { return x < 0 ? 0 : (x >= n ? n - 1 : x); }
 // 32-bit element offsets (the entry points refuse grids whose padded arrays
 // reach 2^31 words)
-__device__ __forceinline__ unsigned f3(const TkeArgs &a, int k, int j, int i) {
-    return ((unsigned)k * (unsigned)a.nj + (unsigned)j) * (unsigned)a.ni + (unsigned)i;
-}
-// value at a clamped column (constant extension beyond the open sides)
-__device__ __forceinline__ float cellc(const TkeArgs &a, const float *p, int k, int j, int i) {
-    return p[f3(a, k, clampi(j, a.nj), clampi(i, a.ni))];
-}
-__device__ __forceinline__ float g2c(const TkeArgs &a, const float *p, int j, int i) {
-    return p[(unsigned)clampi(j, a.nj) * (unsigned)a.ni + (unsigned)clampi(i, a.ni)];
-}
-__device__ __forceinline__ float tsm(const TkeArgs &a, int m, int j, int i) {
-    return 0.5f * (cellc(a, a.t, m, j, i) + cellc(a, a.t, m + 1, j, i));
-}
-
-// x TKE flux at face level f (1..nk-1), row j, u face `face`; 0 elsewhere
-__device__ float tke_tx(const TkeArgs &a, int f, int j, int face) {
+// x TKE flux at face level f (1..nk-1) between the cells l and r (offsets in a
+// level), y likewise with rd = rdy
+__device__ __forceinline__ float tke_flux(const TkeArgs &a, int f, int l, int r, float gl, float gr, float rgl, float rgr,
+                                          float rd) {
     if (f <= 0 || f >= a.nk) return 0.0f;
-    const int l = face - 1, r = face;
-    const float den = g2c(a, a.gz, j, r) * cellc(a, a.rf, f, j, r) + g2c(a, a.gz, j, l) * cellc(a, a.rf, f, j, l);
-    const float kval = cellc(a, a.kmh, f, j, r) + cellc(a, a.kmh, f, j, l);
-    const float gr = g2c(a, a.rgz, j, r), gl = g2c(a, a.rgz, j, l);
-    float term = (cellc(a, a.t, f, j, r) * gr - cellc(a, a.t, f, j, l) * gl) * a.rdx;
-    const float up = (a.zt - ((float)f + 0.5f) * a.dz) * (tsm(a, f, j, l) + tsm(a, f, j, r));
-    const float lo = (a.zt - ((float)f - 0.5f) * a.dz) * (tsm(a, f - 1, j, l) + tsm(a, f - 1, j, r));
-    term = term + 0.5f * ((up - lo) * (a.rdz * ((gr - gl) * a.rdx)));
+    const unsigned cz = (unsigned)a.ni * a.nj, z = (unsigned)f * cz;
+    const float *t = a.t + z, *tu = t + cz, *tl = t - cz;
+    const float cl = t[l], cr = t[r];
+    const float den = gr * a.rf[z + r] + gl * a.rf[z + l];
+    const float kval = a.kmh[z + r] + a.kmh[z + l];
+    float term = (cr * rgr - cl * rgl) * rd;
+    const float up = (a.zt - ((float)f + 0.5f) * a.dz) * (0.5f * (cl + tu[l]) + 0.5f * (cr + tu[r]));
+    const float lo = (a.zt - ((float)f - 0.5f) * a.dz) * (0.5f * (tl[l] + cl) + 0.5f * (tl[r] + cr));
+    term = term + 0.5f * ((up - lo) * (a.rdz * ((rgr - rgl) * rd)));
     return -0.25f * (den * (2.0f * (kval * term)));
 }
 
-// y TKE flux at face level f, v face `face`, column i
-__device__ float tke_ty(const TkeArgs &a, int f, int face, int i) {
-    if (f <= 0 || f >= a.nk) return 0.0f;
-    const int s = face - 1, n = face;
-    const float den = g2c(a, a.gz, n, i) * cellc(a, a.rf, f, n, i) + g2c(a, a.gz, s, i) * cellc(a, a.rf, f, s, i);
-    const float kval = cellc(a, a.kmh, f, n, i) + cellc(a, a.kmh, f, s, i);
-    const float gn = g2c(a, a.rgz, n, i), gs = g2c(a, a.rgz, s, i);
-    float term = (cellc(a, a.t, f, n, i) * gn - cellc(a, a.t, f, s, i) * gs) * a.rdy;
-    const float up = (a.zt - ((float)f + 0.5f) * a.dz) * (tsm(a, f, s, i) + tsm(a, f, n, i));
-    const float lo = (a.zt - ((float)f - 0.5f) * a.dz) * (tsm(a, f - 1, s, i) + tsm(a, f - 1, n, i));
-    term = term + 0.5f * ((up - lo) * (a.rdz * ((gn - gs) * a.rdy)));
-    return -0.25f * (den * (2.0f * (kval * term)));
-}
-
-// dynamic shared memory: cp and dp (the latter becomes the solution), each
-// (nk-1) levels x kTT columns
-__global__ void __launch_bounds__(kTT) tke_turbt_kernel(TkeArgs a, float dt) {
+// dynamic shared memory: the four tridiagonal words of each of the nk-1 rows
+// of 32 columns.  256x256x80: 405 us with a thread per column (its loads a
+// level at a time, most of the chip idle), 223 here.
+__global__ void __launch_bounds__(32 * kTurbtWarps, 3) tke_turbt_kernel(const __grid_constant__ TkeArgs a, float dt) {
     extern __shared__ float s_col[];
-    __shared__ float s_tx[4][kTTY][kTTX + 1];
-    __shared__ float s_ty[4][kTTY + 1][kTTX];
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTTX + tx;
-    const int i0 = blockIdx.x * kTTX, j0 = blockIdx.y * kTTY;
-    const int i = i0 + tx, j = j0 + ty;
-    const int ni = a.ni, nj = a.nj, nk = a.nk, n = nk - 1;
-    const bool own = i < ni && j < nj;
-    float *cp = s_col, *dp = s_col + (size_t)n * kTT;
-#define CP(p) cp[(unsigned)(p) * kTT + tid]
-#define DP(p) dp[(unsigned)(p) * kTT + tid]
-    const float rdt = 1.0f / dt;
-    // ---- vertically implicit diffusion of the own column -------------------
-    if (own) {
-        const float tema = -1.0f * (dt * (a.rdz * a.rdz));
-        int f = 1;
-        unsigned z = f3(a, f, j, i);
-        float rrf = a.mf[z] / a.rf[z];
-        float r2 = (a.kmv[z] + a.kmv[f3(a, f + 1, j, i)]) * (a.mh[f3(a, f, j, i)] * (a.rho[f3(a, f, j, i)] * rrf));
-        float cfc = tema * r2, cfb = 1.0f - cfc, inv = rcp_rn(cfb);
-        float cprev = -1.0f * (cfc * inv), dprev = a.t[z] * inv;
-        CP(0) = cprev;
-        DP(0) = dprev;
-        // kmv(f-1), kmv(f), mh(f-1) and rho(f-1) of the level being
-        // eliminated ride in registers; each chunk of kTTChunk levels issues
-        // all of its loads before its first elimination, so their latency is
-        // paid once per chunk rather than once per level (same operations,
-        // same order)
-        float km1 = a.kmv[z], k0 = a.kmv[f3(a, 2, j, i)], mhm = a.mh[z], rhom = a.rho[z];
-        for (int p0 = 1; p0 < n - 1; p0 += kTTChunk) {
-            float lkn[kTTChunk], lmh[kTTChunk], lrho[kTTChunk], lmf[kTTChunk], lrf[kTTChunk], lt[kTTChunk];
-#pragma unroll
-            for (int q = 0; q < kTTChunk; ++q) {
-                lkn[q] = lmh[q] = lrho[q] = lt[q] = 0.0f;
-                lmf[q] = lrf[q] = 1.0f;
-                if (p0 + q >= n - 1) continue;
-                const unsigned zq = f3(a, p0 + q + 1, j, i);
-                lkn[q] = a.kmv[f3(a, p0 + q + 2, j, i)];
-                lmh[q] = a.mh[zq];
-                lrho[q] = a.rho[zq];
-                lmf[q] = a.mf[zq];
-                lrf[q] = a.rf[zq];
-                lt[q] = a.t[zq];
-            }
-#pragma unroll
-            for (int q = 0; q < kTTChunk; ++q) {
-                const int p = p0 + q;
-                if (p >= n - 1) break;
-                rrf = lmf[q] / lrf[q];
-                const float r1 = (km1 + k0) * (mhm * (rhom * rrf));
-                r2 = (k0 + lkn[q]) * (lmh[q] * (lrho[q] * rrf));
-                const float cfa = tema * r1;
-                cfc = tema * r2;
-                cfb = (1.0f - cfa) - cfc;
-                inv = rcp_rn(cfa * cprev + cfb);
-                cprev = -1.0f * (cfc * inv);
-                dprev = (lt[q] - cfa * dprev) * inv;
-                CP(p) = cprev;
-                DP(p) = dprev;
-                km1 = k0, k0 = lkn[q], mhm = lmh[q], rhom = lrho[q];
-            }
+    const int lane = threadIdx.x, wy = threadIdx.y;
+    const int ni = a.ni, nj = a.nj, nk = a.nk, n = nk - 1, cz = ni * nj, tiles = (ni + 31) / 32;
+    const int i0 = blockIdx.x % tiles * 32 + lane, j = blockIdx.x / tiles;
+    const bool own = i0 < ni;
+    const int i = min(i0, ni - 1), c = j * ni + i;  // lanes past the row's end repeat its last column
+    float *s_a = s_col + lane, *s_b = s_a + n * 32, *s_c = s_b + n * 32, *s_d = s_c + n * 32;  // rows f - 1
+    const float rdt = 1.0f / dt, tema = -1.0f * (dt * (a.rdz * a.rdz));
+    const int run = (n + kTurbtWarps - 1) / kTurbtWarps;
+    const int f_lo = 1 + wy * run, f_hi = min(n, f_lo + run - 1);
+    if (f_lo <= f_hi) {
+        unsigned z = (unsigned)f_lo * (unsigned)cz + (unsigned)c;
+        // level f-1's and f's words ride in registers
+        float km = a.kmv[z - cz], k0 = a.kmv[z], mhm = a.mh[z - cz], rhom = a.rho[z - cz];
+#pragma unroll 4
+        for (int f = f_lo; f <= f_hi; ++f, z += cz) {
+            const float kp = a.kmv[z + cz], mh = a.mh[z], rho = a.rho[z];
+            const float rrf = a.mf[z] / a.rf[z];
+            const float r1 = (km + k0) * (mhm * (rhom * rrf)), r2 = (k0 + kp) * (mh * (rho * rrf));
+            const float cfa = tema * r1, cfc = tema * r2;
+            const int q = (f - 1) * 32;
+            s_a[q] = cfa, s_c[q] = cfc, s_d[q] = a.t[z];
+            s_b[q] = f == 1 ? 1.0f - cfc : f == n ? 1.0f - cfa : (1.0f - cfa) - cfc;
+            km = k0, k0 = kp, mhm = mh, rhom = rho;
         }
-        f = nk - 1;
-        z = f3(a, f, j, i);
-        rrf = a.mf[z] / a.rf[z];
-        const float r1 = (km1 + k0) * (mhm * (rhom * rrf));
-        const float cfa = tema * r1;
-        cfb = 1.0f - cfa;
-        float sol = (a.t[z] - cfa * DP(n - 2)) * rcp_rn(cfa * CP(n - 2) + cfb);
-        DP(n - 1) = sol;
-        for (int p = n - 2; p >= 0; --p) {
-            sol = CP(p) * sol + DP(p);
-            DP(p) = sol;
-        }
-    }
-    // ---- horizontal divergence, walking the face levels --------------------
-    // Four level slots: while level f is formed from slots f-1, f, f+1, this
-    // thread's share of level f+2's face terms is evaluated into registers
-    // (its loads in flight during the level's arithmetic) and stored into the
-    // fourth slot, which no thread reads until after the closing barrier.
-    constexpr int kXF = kTTY * (kTTX + 1), kYF = (kTTY + 1) * kTTX;
-    constexpr int kXE = (kXF + kTT - 1) / kTT, kYE = (kYF + kTT - 1) / kTT;
-    float rx[kXE], ry[kYE];
-    auto eval = [&](int lev) {
-#pragma unroll
-        for (int q2 = 0; q2 < kXE; ++q2) {
-            const int e = tid + q2 * kTT, r = e / (kTTX + 1), q = e - r * (kTTX + 1);
-            rx[q2] = (e < kXF && j0 + r < nj && i0 + q <= ni) ? tke_tx(a, lev, j0 + r, i0 + q) : 0.0f;
-        }
-#pragma unroll
-        for (int q2 = 0; q2 < kYE; ++q2) {
-            const int e = tid + q2 * kTT, r = e / kTTX, q = e - r * kTTX;
-            ry[q2] = (e < kYF && j0 + r <= nj && i0 + q < ni) ? tke_ty(a, lev, j0 + r, i0 + q) : 0.0f;
-        }
-    };
-    auto store = [&](int lev) {
-        const int slot = lev % 4;
-#pragma unroll
-        for (int q2 = 0; q2 < kXE; ++q2) {
-            const int e = tid + q2 * kTT, r = e / (kTTX + 1), q = e - r * (kTTX + 1);
-            if (e < kXF) s_tx[slot][r][q] = rx[q2];
-        }
-#pragma unroll
-        for (int q2 = 0; q2 < kYE; ++q2) {
-            const int e = tid + q2 * kTT, r = e / kTTX, q = e - r * kTTX;
-            if (e < kYF) s_ty[slot][r][q] = ry[q2];
-        }
-    };
-    for (int lev = 0; lev <= 2 && lev <= nk; ++lev) {
-        eval(lev);
-        store(lev);
     }
     __syncthreads();
-    float gzji = 0.0f, ru0 = 0.0f, ru1 = 0.0f, rv0 = 0.0f, rv1 = 0.0f;
-    if (own) {
-        gzji = a.gz[(size_t)j * ni + i];
-        ru0 = a.rgzu[(size_t)j * (ni + 1) + i];
-        ru1 = a.rgzu[(size_t)j * (ni + 1) + i + 1];
-        rv0 = a.rgzv[(size_t)j * ni + i];
-        rv1 = a.rgzv[(size_t)(j + 1) * ni + i];
+    if (wy == 0) column_sweep(s_a, s_b, s_c, s_d, n);
+    __syncthreads();
+    if (f_lo > f_hi || !own) return;
+    // horizontal divergence of the run's levels: the four face fluxes of the
+    // levels f-1, f and f+1, each formed once and carried up
+    const int w = j * ni + max(i - 1, 0), e = j * ni + min(i + 1, ni - 1), s = max(j - 1, 0) * ni + i,
+              t = min(j + 1, nj - 1) * ni + i;
+    const float g = a.gz[c], gw = a.gz[w], ge = a.gz[e], gs = a.gz[s], gt = a.gz[t];
+    const float rg = a.rgz[c], rgw = a.rgz[w], rge = a.rgz[e], rgs = a.rgz[s], rgt = a.rgz[t];
+    const float ru0 = a.rgzu[(unsigned)j * (ni + 1) + i], ru1 = a.rgzu[(unsigned)j * (ni + 1) + i + 1];
+    const float rv0 = a.rgzv[(unsigned)j * ni + i], rv1 = a.rgzv[(unsigned)(j + 1) * ni + i];
+    const bool ex = i == 0 || i == ni - 1, ey = j == 0 || j == nj - 1;
+    auto fluxes = [&](int f, float q[4]) {
+        q[0] = ex ? 0.0f : tke_flux(a, f, w, c, gw, g, rgw, rg, a.rdx);
+        q[1] = ex ? 0.0f : tke_flux(a, f, c, e, g, ge, rg, rge, a.rdx);
+        q[2] = ey ? 0.0f : tke_flux(a, f, s, c, gs, g, rgs, rg, a.rdy);
+        q[3] = ey ? 0.0f : tke_flux(a, f, c, t, g, gt, rg, rgt, a.rdy);
+    };
+    float lo4[4], cur[4], up4[4];
+    fluxes(f_lo - 1, lo4);
+    fluxes(f_lo, cur);
+#pragma unroll 1
+    for (int f = f_lo; f <= f_hi; ++f) {
+        fluxes(f + 1, up4);
+        const unsigned z = (unsigned)f * (unsigned)cz + (unsigned)c;
+        const float hi_z = a.zt - ((float)f + 0.5f) * a.dz, lo_z = a.zt - ((float)f - 0.5f) * a.dz;
+        auto part = [&](int q, float m0, float m1, float rd) {
+            const float x0 = cur[q], x1 = cur[q + 1];
+            float x = -1.0f * ((x1 * m1 - x0 * m0) * (g * rd));
+            const float f0 = 0.5f * (x0 + up4[q]), f1 = 0.5f * (x1 + up4[q + 1]);
+            const float b0 = 0.5f * (lo4[q] + x0), b1 = 0.5f * (lo4[q + 1] + x1);
+            const float up = hi_z * (f0 + f1), lo = lo_z * (b0 + b1);
+            return x - 0.5f * ((up - lo) * (a.rdz * ((m1 - m0) * (g * rd))));
+        };
+        const float hx = ex ? 0.0f : part(0, ru0, ru1, a.rdx), hy = ey ? 0.0f : part(2, rv0, rv1, a.rdy);
+        const float rfz = a.rf[z];
+        const float vz = rfz * ((s_d[(f - 1) * 32] - a.t[z]) * rdt);
+        a.tketen[z] = a.tketen[z] + ((hx + hy) + vz) / rfz;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) lo4[q] = cur[q], cur[q] = up4[q];
     }
-    for (int f = 1; f < nk; ++f) {
-        const bool ahead = f + 2 <= nk;
-        if (ahead) eval(f + 2);
-        if (own) {
-            const int cm = (f - 1) % 4, c0 = f % 4, cpl = (f + 1) % 4;
-            const float x0 = s_tx[c0][ty][tx], x1 = s_tx[c0][ty][tx + 1];
-            float x = -1.0f * ((x1 * ru1 - x0 * ru0) * (gzji * a.rdx));
-            const float sxf0 = 0.5f * (x0 + s_tx[cpl][ty][tx]), sxf1 = 0.5f * (x1 + s_tx[cpl][ty][tx + 1]);
-            const float sxm0 = 0.5f * (s_tx[cm][ty][tx] + x0), sxm1 = 0.5f * (s_tx[cm][ty][tx + 1] + x1);
-            float up = (a.zt - ((float)f + 0.5f) * a.dz) * (sxf0 + sxf1);
-            float lo = (a.zt - ((float)f - 0.5f) * a.dz) * (sxm0 + sxm1);
-            x = x - 0.5f * ((up - lo) * (a.rdz * ((ru1 - ru0) * (gzji * a.rdx))));
-            const float y0 = s_ty[c0][ty][tx], y1 = s_ty[c0][ty + 1][tx];
-            float y = -1.0f * ((y1 * rv1 - y0 * rv0) * (gzji * a.rdy));
-            const float syf0 = 0.5f * (y0 + s_ty[cpl][ty][tx]), syf1 = 0.5f * (y1 + s_ty[cpl][ty + 1][tx]);
-            const float sym0 = 0.5f * (s_ty[cm][ty][tx] + y0), sym1 = 0.5f * (s_ty[cm][ty + 1][tx] + y1);
-            up = (a.zt - ((float)f + 0.5f) * a.dz) * (syf0 + syf1);
-            lo = (a.zt - ((float)f - 0.5f) * a.dz) * (sym0 + sym1);
-            y = y - 0.5f * ((up - lo) * (a.rdz * ((rv1 - rv0) * (gzji * a.rdy))));
-            const float hx = (i == 0 || i == ni - 1) ? 0.0f : x;
-            const float hy = (j == 0 || j == nj - 1) ? 0.0f : y;
-            const unsigned z = f3(a, f, j, i);
-            const float rfz = a.rf[z];
-            const float vz = rfz * ((DP(f - 1) - a.t[z]) * rdt);
-            a.tketen[z] = a.tketen[z] + ((hx + hy) + vz) / rfz;
-        }
-        if (ahead) store(f + 2);
-        __syncthreads();
-    }
-#undef CP
-#undef DP
 }
 
 // ------------------------------------------------- turbt, flat column
@@ -249,22 +140,20 @@ __global__ void __launch_bounds__(kTT) tke_turbt_kernel(TkeArgs a, float dt) {
 // turbtend.F:729-1044 with terrain_flag=.false.): the x/y face fluxes
 // -0.25*(rf(a)+rf(a-1))*2*(kmh(a)+kmh(a-1))*(t(a)-t(a-1))*rdx, no terrain
 // correction, and the implicit diffusion with rdz and the 3-D mh/mf.  One
-// CTA per 32 columns of a row: kFlatTWarps warps form the tridiagonal rows of
+// CTA per 32 columns of a row: kTurbtWarps warps form the tridiagonal rows of
 // their own runs of levels (the mf/rf divisions and every load spread over
 // the CTA), one warp sweeps them in shared memory, then all warps add the
 // horizontal and vertical parts of their levels.  Four shared words per level
 // and column leave five CTAs on an SM at nk = 80.  640x768x80: 3.653 -> 0.603
 // ms against a thread per column (two 128-thread CTAs an SM, its loads one
 // level at a time).
-constexpr int kFlatTWarps = 8;
-
 // the flux through the face between the cells l and r (rd = rdx or rdy)
 __device__ __forceinline__ float tke_flux_flat(float rfr, float rfl, float kr, float kl, float tr, float tl, float rd) {
     const float rs = rfr + rfl, ks = kr + kl, dt = tr - tl;
     return -(((((0.25f * rs) * 2.0f) * ks) * dt) * rd);
 }
 
-__global__ void __launch_bounds__(32 * kFlatTWarps) tke_turbt_flat_kernel(TkeArgs a, float dt) {
+__global__ void __launch_bounds__(32 * kTurbtWarps) tke_turbt_flat_kernel(TkeArgs a, float dt) {
     extern __shared__ float s_col[];
     const int lane = threadIdx.x, wy = threadIdx.y;
     const int ni = a.ni, nj = a.nj, nk = a.nk, n = nk - 1, cz = ni * nj;
@@ -276,7 +165,7 @@ __global__ void __launch_bounds__(32 * kFlatTWarps) tke_turbt_flat_kernel(TkeArg
     const float rdt = 1.0f / dt;
     const float tema = (((-1.0f * dt) * 1.0f) * a.rdz) * a.rdz;
     const float temb = ((dt * 0.0f) * a.rdz) * a.rdz;
-    const int run = (n + kFlatTWarps - 1) / kFlatTWarps;
+    const int run = (n + kTurbtWarps - 1) / kTurbtWarps;
     const int f_lo = 1 + wy * run, f_hi = min(n, f_lo + run - 1);
     if (f_lo <= f_hi) {
         unsigned z = (unsigned)f_lo * (unsigned)cz + (unsigned)c;
@@ -308,36 +197,7 @@ __global__ void __launch_bounds__(32 * kFlatTWarps) tke_turbt_flat_kernel(TkeArg
         }
     }
     __syncthreads();
-    if (wy == 0) {
-        float cprev = 0.0f, dprev = 0.0f;
-        float cfa = s_a[0], cfb = s_b[0], cfc = s_c[0], cfd = s_d[0];
-        for (int p = 0; p < n - 1; ++p) {
-            const int q = (p + 1) * 32;
-            const float na = s_a[q], nb = s_b[q], nc = s_c[q], nd = s_d[q];
-            const float inv = rcp_rn(p == 0 ? cfb : cfa * cprev + cfb);
-            cprev = -(cfc * inv);
-            dprev = (p == 0 ? cfd : cfd - cfa * dprev) * inv;
-            s_c[p * 32] = cprev;
-            s_d[p * 32] = dprev;
-            cfa = na, cfb = nb, cfc = nc, cfd = nd;
-        }
-        float sol = (cfd - cfa * dprev) * rcp_rn(cfa * cprev + cfb);
-        s_d[(n - 1) * 32] = sol;
-        for (int pb = n - 2; pb >= 0; pb -= kTTChunk) {
-            float ce[kTTChunk], de[kTTChunk];
-#pragma unroll
-            for (int e = 0; e < kTTChunk; ++e) {
-                const int p = max(pb - e, 0);
-                ce[e] = s_c[p * 32], de[e] = s_d[p * 32];
-            }
-#pragma unroll
-            for (int e = 0; e < kTTChunk; ++e) {
-                if (pb - e < 0) break;
-                sol = ce[e] * sol + de[e];
-                s_d[(pb - e) * 32] = sol;
-            }
-        }
-    }
+    if (wy == 0) column_sweep(s_a, s_b, s_c, s_d, n);
     __syncthreads();
     if (!own) return;
     const int dw = i > 0 ? -1 : 0, de = i < ni - 1 ? 1 : 0, ds = j > 0 ? -ni : 0, dn = j < nj - 1 ? ni : 0;
@@ -642,11 +502,12 @@ int tke_args(int ni, int nj, int nk, const gm1b_tke_evolution_arrays *s, float d
     return GM1B_OK;
 }
 
-size_t turbt_smem(int nk) { return (size_t)2 * (nk - 1) * kTT * sizeof(float); }
+// four tridiagonal words of each of the nk-1 rows of 32 columns
+size_t turbt_smem(int nk) { return (size_t)4 * (nk - 1) * 32 * sizeof(float); }
 
 int enqueue_diffusion(const TkeArgs &a, float dt, cudaStream_t st) {
     const size_t smem = turbt_smem(a.nk);
-    if (smem > 200 * 1024) {
+    if (a.nk > kTurbtMostNk) {
         gm1b_set_error("gm1b_tke_diffusion: nk=%d exceeds the column solve's shared memory (nk <= 201)", a.nk);
         return GM1B_ERR_ARGUMENT;
     }
@@ -663,7 +524,7 @@ int enqueue_diffusion(const TkeArgs &a, float dt, cudaStream_t st) {
         configured[dev] = 200 * 1024;
     }
     ProfScope ps("tke_turbt_kernel", st);
-    tke_turbt_kernel<<<dim3((a.ni + kTTX - 1) / kTTX, (a.nj + kTTY - 1) / kTTY), dim3(kTTX, kTTY), smem, st>>>(a, dt);
+    tke_turbt_kernel<<<(a.ni + 31) / 32 * a.nj, dim3(32, kTurbtWarps), smem, st>>>(a, dt);
     ps.stop();
     return launch_ok("tke_turbt_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }
@@ -772,7 +633,7 @@ extern "C" int32_t gm1b_tke_diffusion_flat(int32_t ni, int32_t nj, int32_t nk,
     const int r = tke_args_flat(ni, nj, nk, arrays, dx, dy, rdz, dt, a, false, nullptr, "gm1b_tke_diffusion_flat");
     if (r != GM1B_OK) return r;
     const size_t smem = turbt_smem(nk);
-    if (smem > 200 * 1024) {
+    if (nk > kTurbtMostNk) {
         gm1b_set_error("gm1b_tke_diffusion_flat: nk=%d exceeds the column solve's shared memory (nk <= 201)", nk);
         return GM1B_ERR_ARGUMENT;
     }
@@ -790,8 +651,7 @@ extern "C" int32_t gm1b_tke_diffusion_flat(int32_t ni, int32_t nj, int32_t nk,
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     ProfScope ps("tke_turbt_flat_kernel", st);
-    tke_turbt_flat_kernel<<<(ni + 31) / 32 * nj, dim3(32, kFlatTWarps), (size_t)4 * (nk - 1) * 32 * sizeof(float), st>>>(
-        a, dt);
+    tke_turbt_flat_kernel<<<(ni + 31) / 32 * nj, dim3(32, kTurbtWarps), smem, st>>>(a, dt);
     ps.stop();
     return launch_ok("tke_turbt_flat_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }

@@ -151,6 +151,20 @@ def test_flat_tke_diffusion(ni, nj, nk):
     assert _differ(dev, a, ("tketen",)) == []
 
 
+@pytest.mark.parametrize("ni,nj,nk", [(31, 7, 8), (32, 8, 9), (33, 7, 10), (7, 7, 17), (8, 9, 201)])
+def test_terrain_tke_diffusion(ni, nj, nk):
+    from gm1_b200 import tke_evolution as te
+    from oracle import tke_evolution as orc
+    from tests.golden.make_golden import tke_evolution_fixture
+
+    a = tke_evolution_fixture(ni, nj, nk, seed=3 * ni + nk)
+    dev = _dev(a)
+    kw = dict(ni=ni, nj=nj, nk=nk, dx=500.0, dy=450.0, dz=150.0, dt=2.0)
+    orc.tke_diffusion(a, **kw)
+    te.launch_cuda_tke_diffusion(dev, **kw)
+    assert _differ(dev, a, ("tketen",)) == []
+
+
 @pytest.mark.parametrize("flat", [False, True])
 @pytest.mark.parametrize("ni,nj,nk", [(31, 7, 9), (32, 8, 10), (30, 6, 18), (3, 3, 3), (63, 15, 20)])
 def test_deformation(ni, nj, nk, flat):
