@@ -11,9 +11,9 @@
 //
 // Design (B200): the reference runs its column phases one thread per j ROW
 // (serial over i, k and the fallout sub-steps) and its budget finishes on a
-// single thread.  Here every COLUMN is a thread (pdefq x3, fall speed,
-// nfall, the fallout sub-steps marching up k with the flux of the level
-// above carried in a register), every CELL is a thread for the local
+// single thread.  Here a CTA owns 32 columns (pdefq x3, fall speed, nfall and
+// the fallout sub-steps in shared memory, each thread with a run of levels;
+// very tall columns a thread each), every CELL is a thread for the local
 // conversion fused with the saturation adjustment, and the FP64 budgets are
 // reduced in a fixed order: per-column sums in the twin's k order, row sums
 // in its i order, then a short ordered finish.  The budget scratch lives in a
@@ -208,22 +208,204 @@ __global__ void __launch_bounds__(kCX *kCY)
     w.colterm[4 * ncol + col] = bud;
 }
 
-__device__ __forceinline__ double block_sum(double v, double *smem) {
+// ---- the same columns, 32 of a row to a CTA
+constexpr int kTileWarps = 8;
+constexpr int kTileWords = 6;  // shared words per level and column
+constexpr int kTileMostNk = 296;  // taller columns do not fit an SM's shared memory: a thread per column
+
+// A CTA holds 32 columns in shared memory (rho, rmh, the three species and
+// the fall speed).  The level-ordered binary64 sums of a species and column
+// belong to one thread; everything else - the loads, the rescaling, powf, the
+// fallout sub-steps, which read the level above before any level changes - is
+// spread over the CTA's warps, each with a run of levels.  A thread per column
+// (three species one after the other, its loads a level at a time) took 1.373
+// ms at 640x768x80, 261 us at 256x256x80 and 71 us at 53x48x40; this takes
+// 0.790 ms, 120 us and less than 20.
+__global__ void __launch_bounds__(32 * kTileWarps)
+    kessler_tile_kernel(const __grid_constant__ gm1b_kessler_arrays a, KDims d, KWork w, const __grid_constant__ KConst c,
+                        float dt, float rdz) {
+    extern __shared__ float s_tile[];
+    __shared__ double s_t3[3][32];
+    __shared__ float s_cr[kTileWarps][32];
+    __shared__ int s_nfall[32], s_most;
+    const int lane = threadIdx.x, wy = threadIdx.y;
+    const int ni = d.ni, nk = d.nk, tiles = (ni + 31) / 32;
+    const int i0 = blockIdx.x % tiles * 32 + lane, j = blockIdx.x / tiles;
+    const bool own = i0 < ni;
+    const int i = min(i0, ni - 1);  // lanes past the row's end repeat its last column and store nothing
+    const size_t col = (size_t)j * ni + i, ncol = (size_t)ni * d.nj;
+    const int words = nk * 32;
+    float *s_rho = s_tile + lane, *s_rmh = s_rho + words, *s_v = s_rmh + words, *s_q = s_v + words;
+    float *s_qr = s_q + 2 * words;
+    const int run = (nk + kTileWarps - 1) / kTileWarps;
+    const int lo = min(wy * run, nk), hi = min(lo + run, nk);
+#pragma unroll 4
+    for (int k = lo; k < hi; ++k) {
+        const size_t p = (size_t)k * ncol + col;
+        const float rho = a.rho[p], rmh = a.rmh[p], qv = a.qv[p], qc = a.qc[p], qr = a.qr[p];
+        s_rho[k * 32] = rho, s_rmh[k * 32] = rmh;
+        s_q[k * 32] = qv, s_q[words + k * 32] = qc, s_qr[k * 32] = qr;
+    }
+    __syncthreads();
+    const float ruh = a.ruh[i], rvh = a.rvh[j];
+    const float rmax = wy == 0 ? 0.0f : 1.0e-14f;
+    double a1 = 0.0;
+    if (wy < 3) {  // pdefq of species wy: its sums
+        const float *q = s_q + wy * words;
+        double t1 = 0.0, t2 = 0.0;
+#pragma unroll 8
+        for (int k = 0; k < nk; ++k) {
+            const float rho = s_rho[k * 32], qk = q[k * 32];
+            t1 += (double)(rho * qk);
+            a1 += (double)((((rho * qk) * ruh) * rvh) * s_rmh[k * 32]);
+            t2 += (double)(rho * ((qk < rmax) ? 0.0f : qk));
+        }
+        double t3 = (t1 + 1.0e-20) / (t2 + 1.0e-20);
+        if (t3 < 0.0) t3 = 1.0;
+        s_t3[wy][lane] = t3;
+    }
+    __syncthreads();
+    // rescaled species, rain fall speed, largest Courant number of the run
+    const double t3v = s_t3[0][lane], t3c = s_t3[1][lane], t3r = s_t3[2][lane];
+    float crmax = 0.0f;
+#pragma unroll 2
+    for (int k = lo; k < hi; ++k) {
+        const size_t p = (size_t)k * ncol + col;
+        const float rho = s_rho[k * 32], mh = a.mh[p];
+        const float qv = s_q[k * 32], qc = s_q[words + k * 32], qr = s_qr[k * 32];
+        const float nv = (float)(t3v * (double)((qv < 0.0f) ? 0.0f : qv));
+        const float nc = (float)(t3c * (double)((qc < 1.0e-14f) ? 0.0f : qc));
+        const float nr = (float)(t3r * (double)((qr < 1.0e-14f) ? 0.0f : qr));
+        s_q[k * 32] = nv, s_q[words + k * 32] = nc, s_qr[k * 32] = nr;
+        if (own) a.qv[p] = nv, a.qc[p] = nc;
+        float v = 0.0f;
+        if (nr > 1.0e-12f) v = (14.34f * powf(rho * nr, 0.1346f)) * sqrtf(1.15f / rho);
+        s_v[k * 32] = v;
+        crmax = pymax(crmax, ((v * dt) * rdz) * mh);
+    }
+    s_cr[wy][lane] = crmax;
+    __syncthreads();
+    if (wy < 3) {
+        const float *q = s_q + wy * words;
+        double a2 = 0.0;
+#pragma unroll 8
+        for (int k = 0; k < nk; ++k)
+            a2 += (double)((((s_rho[k * 32] * q[k * 32]) * ruh) * rvh) * s_rmh[k * 32]);
+        if (own) w.colterm[wy * ncol + col] = a2 - a1;
+    } else if (wy == 3) {
+        const float temp0 = (a.th0[col] + a.th3d[col]) * (a.pi0[col] + a.pp3d[col]);
+        float term = dt * s_v[0];
+        term = term * a.rr[col];
+        term = term * s_qr[0];
+        term = term * (c.cpl * temp0 - c.lv1);
+        term = term * ruh;
+        term = term * rvh;
+        if (own) w.colterm[3 * ncol + col] = (double)term;
+        // a largest value that skips NaN does not depend on the order
+        crmax = 0.0f;
+        for (int q = 0; q < kTileWarps; ++q) crmax = pymax(crmax, s_cr[q][lane]);
+        int nfall = (int)(crmax + 1.0f);
+        if (nfall < 1) nfall = 1;
+        // A column whose fall Courant number is not finite or above
+        // kMaxFallSubsteps holds no physical state (rain or density already
+        // blew up); int(crmax + 1) would reach 2^31 sub-steps.  It is counted
+        // in status[2] and takes one sub-step, so the launch stays bounded
+        // and the caller refuses the step.
+        if (!(crmax < (float)kMaxFallSubsteps)) {
+            if (own) atomicAdd(&w.status[2], 1);
+            nfall = 1;
+        }
+        if (own && a.nfall != nullptr) a.nfall[col] = nfall;
+        s_nfall[lane] = nfall;
+        const int most = __reduce_max_sync(0xffffffffu, nfall);
+        if (lane == 0) {
+            s_most = most;
+            atomicMax(&w.status[1], most);
+        }
+        // below-threshold rain takes the fall speed of the level above
+        float above = s_v[(nk - 1) * 32];
+#pragma unroll 8
+        for (int k = nk - 2; k >= 0; --k) {
+            const float v = s_v[k * 32];
+            above = s_qr[k * 32] < 1.0e-8f ? above : v;
+            s_v[k * 32] = above;
+        }
+    }
+    __syncthreads();
+    const int nfall = s_nfall[lane], most = s_most;
+    const float dtfall = dt / (float)nfall;
+    const float rr0 = a.rr[col];
+    float rain = wy == 0 ? a.rain[col] : 0.0f, prate = 0.0f;
+    double bud = 0.0;
+    auto flux = [&](int k) { return k < nk ? (s_rho[k * 32] * s_v[k * 32]) * pymax(0.0f, s_qr[k * 32]) : 0.0f; };
+    for (int n = 0; n < most; ++n) {
+        const float rq_hi = flux(hi);  // of the next run, before its levels change
+        __syncthreads();
+        if (n < nfall && lo < hi) {
+            float rq_k = flux(lo);
+            if (wy == 0) prate = rq_k;
+#pragma unroll 2
+            for (int k = lo; k < hi; ++k) {
+                const float rq_up = k + 1 < hi ? flux(k + 1) : rq_hi;
+                const float delta = (((dtfall * (rq_up - rq_k)) * rdz) * a.mh[(size_t)k * ncol + col]) / s_rho[k * 32];
+                s_qr[k * 32] = s_qr[k * 32] + delta;
+                rq_k = rq_up;
+            }
+            if (wy == 0) {
+                rain = rain + (0.1f * dtfall) * prate;
+                float term = dtfall * rr0;
+                term = term * s_v[0];
+                term = term * pymax(0.0f, s_qr[0]);
+                term = term * ruh;
+                term = term * rvh;
+                bud += (double)term;
+            }
+        }
+        __syncthreads();
+    }
+    if (!own) return;
+    if (wy == 0) {
+        a.rain[col] = rain;
+        a.prate[col] = prate;
+        w.colterm[4 * ncol + col] = bud;
+    }
+#pragma unroll 4
+    for (int k = lo; k < hi; ++k) {
+        const size_t p = (size_t)k * ncol + col;
+        a.qr[p] = s_qr[k * 32];
+        a.fall_velocity[p] = s_v[k * 32];
+    }
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
     for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) smem[warp] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += smem[q];
-    __syncthreads();
-    return s;
+    return v;
+}
+
+// acc + term(0) + term(1) + ... in that order, by a warp: its lanes load the
+// terms 32 at a time, the adds alone are a chain
+template <class F>
+__device__ __forceinline__ double ordered_sum(double acc, int n, F term) {
+    const int lane = threadIdx.x & 31;
+    double next = lane < n ? term(lane) : 0.0;
+    for (int base = 0; base < n; base += 32) {
+        const double x = next;
+        next = base + 32 + lane < n ? term(base + 32 + lane) : 0.0;
+        const int m = min(32, n - base);
+        if (m == 32) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) acc += __shfl_sync(0xffffffffu, x, e);
+        } else {
+            for (int e = 0; e < m; ++e) acc += __shfl_sync(0xffffffffu, x, e);
+        }
+    }
+    return acc;
 }
 
 // grid (nbx, nj, nk): one thread per cell; local conversion then satadj
 __global__ void __launch_bounds__(kKX)
     kessler_cell_kernel(gm1b_kessler_arrays a, KDims d, KWork w, KConst c, float dt, int eqtset) {
-    __shared__ double s_red[kKX / 32];
+    __shared__ double s_red[5][kKX / 32];
     const int i = blockIdx.x * kKX + threadIdx.x;
     const int j = blockIdx.y, k = blockIdx.z;
     double terms[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -362,22 +544,30 @@ __global__ void __launch_bounds__(kKX)
     }
     const size_t slot = ((size_t)k * d.nj + j) * w.nbx + blockIdx.x;
     const size_t plane = (size_t)d.nk * d.nj * w.nbx;
+    // the five sums share one barrier
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int t = 0; t < 5; ++t) {
-        const double s = block_sum(terms[t], s_red);
-        if (threadIdx.x == 0) w.partial[t * plane + slot] = s;
+        const double s = warp_sum(terms[t]);
+        if (lane == 0) s_red[t][warp] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x < 5) {
+        double s = 0.0;
+        for (int q = 0; q < kKX / 32; ++q) s += s_red[threadIdx.x][q];
+        w.partial[threadIdx.x * plane + slot] = s;
     }
 }
 
-// one thread per (budget type, row): row sums of the column terms in i order
-__global__ void kessler_rows_kernel(KDims d, KWork w) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= 5 * d.nj) return;
-    const int t = q / d.nj, j = q % d.nj;
-    const size_t ncol = (size_t)d.ni * d.nj;
-    double s = 0.0;
-    for (int i = 0; i < d.ni; ++i) s += w.colterm[t * ncol + (size_t)j * d.ni + i];
-    w.rows[(size_t)t * d.nj + j] = s;
+// one warp per (budget type, row): row sums of the column terms in i order
+constexpr int kRowWarps = 4;
+__global__ void __launch_bounds__(32 * kRowWarps) kessler_rows_kernel(KDims d, KWork w) {
+    const long long q = (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    if (q >= 5LL * d.nj) return;
+    const int t = (int)(q / d.nj), j = (int)(q % d.nj);
+    const double *terms = w.colterm + t * (size_t)d.ni * d.nj + (size_t)j * d.ni;
+    const double s = ordered_sum(0.0, d.ni, [&](int i) { return terms[i]; });
+    if ((threadIdx.x & 31) == 0) w.rows[(size_t)t * d.nj + j] = s;
 }
 
 // grid (nk, 5): block (k, t) sums the nj*nbx cell-kernel partials of budget
@@ -392,40 +582,37 @@ __global__ void __launch_bounds__(kLevelThreads) kessler_levels_kernel(KDims d, 
     double *level = w.partial + (size_t)t * d.nk * n + (size_t)k * n;
     double s = 0.0;
     for (size_t q = threadIdx.x; q < n; q += kLevelThreads) s += level[q];
-    s = block_sum(s, s_red);
-    if (threadIdx.x == 0) level[0] = s;
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = s;
+    __syncthreads();  // every read of the level's first slot is done, too
+    if (threadIdx.x != 0) return;
+    s = 0.0;
+    for (int q = 0; q < kLevelThreads / 32; ++q) s += s_red[q];
+    level[0] = s;
 }
 
-// single thread: ordered finish of every budget (row sums of asq in j order,
+// one CTA, a warp per budget: ordered finish (row sums of asq in j order,
 // level totals of qbudget in k order)
-__global__ void kessler_finish_kernel(gm1b_kessler_arrays a, KDims d, KWork w, double volume, double dxd,
-                                      double dyd, double area) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    // Each budget accumulates in a register in the same order as a running
-    // sum in memory would, and is stored once: the row and level totals are
-    // then independent loads that can all be in flight together.
-    const double *rows = w.rows;
-    for (int s = 0; s < 3; ++s) {
-        double acc = a.asq[s];
-        for (int j = 0; j < d.nj; ++j) acc += rows[(size_t)s * d.nj + j] * volume;
-        a.asq[s] = acc;
+constexpr int kBudgets = 10;
+__global__ void __launch_bounds__(32 * kBudgets) kessler_finish_kernel(gm1b_kessler_arrays a, KDims d, KWork w,
+                                                                       double volume, double dxd, double dyd,
+                                                                       double area) {
+    const int b = threadIdx.x >> 5;
+    const double *rows = w.rows + (size_t)b * d.nj;  // b < 5
+    const size_t n = (size_t)d.nj * w.nbx;
+    double *out = b < 3 ? a.asq + b : a.qbudget + (b == 3 ? 6 : b == 4 ? 5 : b < 8 ? b - 3 : b - 8);
+    double acc = *out;
+    if (b < 3) {
+        acc = ordered_sum(acc, d.nj, [&](int j) { return rows[j] * volume; });
+    } else if (b == 3) {
+        acc = ordered_sum(acc, d.nj, [&](int j) { return rows[j] * dxd * dyd; });
+    } else if (b == 4) {
+        acc = ordered_sum(acc, d.nj, [&](int j) { return rows[j] * area; });
+    } else {
+        const double *levels = w.partial + (size_t)(b - 5) * d.nk * n;
+        acc = ordered_sum(acc, d.nk, [&](int k) { return levels[(size_t)k * n] * volume; });
     }
-    double q6 = a.qbudget[6], q5 = a.qbudget[5];
-    for (int j = 0; j < d.nj; ++j) q6 += rows[(size_t)3 * d.nj + j] * dxd * dyd;
-    for (int j = 0; j < d.nj; ++j) q5 += rows[(size_t)4 * d.nj + j] * area;
-    a.qbudget[6] = q6;
-    a.qbudget[5] = q5;
-    const size_t n = (size_t)d.nj * w.nbx, plane = (size_t)d.nk * n;
-    for (int p = 0; p < 3; ++p) {
-        double acc = a.qbudget[2 + p];
-        for (int k = 0; k < d.nk; ++k) acc = acc + w.partial[p * plane + (size_t)k * n] * volume;
-        a.qbudget[2 + p] = acc;
-    }
-    for (int p = 3; p < 5; ++p) {
-        double acc = a.qbudget[p - 3];
-        for (int k = 0; k < d.nk; ++k) acc += w.partial[p * plane + (size_t)k * n] * volume;
-        a.qbudget[p - 3] = acc;
-    }
+    if ((threadIdx.x & 31) == 0) *out = acc;
 }
 
 bool launched(const char *what) {
@@ -491,13 +678,26 @@ extern "C" int32_t gm1b_kessler_driver(int32_t ni, int32_t nj, int32_t nk, const
         return GM1B_ERR_CUDA;
     }
     const float rdz = 1.0f / dz;
-    {
+    if (nk <= kTileMostNk) {
+        constexpr int kLevelBytes = kTileWords * 32 * (int)sizeof(float);
+        const cudaError_t e = cudaFuncSetAttribute(kessler_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   kLevelBytes * kTileMostNk);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            gm1b_set_error("cudaFuncSetAttribute(kessler_tile_kernel): %s", cudaGetErrorString(e));
+            return GM1B_ERR_CUDA;
+        }
+        ProfScope ps("kessler_tile_kernel", st);
+        const long long tiles = (long long)((ni + 31) / 32) * nj;
+        kessler_tile_kernel<<<(unsigned)tiles, dim3(32, kTileWarps), kLevelBytes * nk, st>>>(a, d, w, c, dt, rdz);
+        ps.stop();
+    } else {
         ProfScope ps("kessler_column_kernel", st);
         kessler_column_kernel<<<dim3((ni + kCX - 1) / kCX, (nj + kCY - 1) / kCY), dim3(kCX, kCY), 0, st>>>(a, d, w, c,
                                                                                                          dt, rdz);
         ps.stop();
     }
-    if (!launched("kessler_column_kernel")) return GM1B_ERR_CUDA;
+    if (!launched("kessler column kernel")) return GM1B_ERR_CUDA;
     {
         ProfScope ps("kessler_cell_kernel", st);
         kessler_cell_kernel<<<dim3(w.nbx, nj, nk), kKX, 0, st>>>(a, d, w, c, dt, equation_set);
@@ -506,7 +706,7 @@ extern "C" int32_t gm1b_kessler_driver(int32_t ni, int32_t nj, int32_t nk, const
     if (!launched("kessler_cell_kernel")) return GM1B_ERR_CUDA;
     {
         ProfScope ps("kessler_rows_kernel", st);
-        kessler_rows_kernel<<<(5 * nj + 127) / 128, 128, 0, st>>>(d, w);
+        kessler_rows_kernel<<<(5 * nj + kRowWarps - 1) / kRowWarps, 32 * kRowWarps, 0, st>>>(d, w);
         ps.stop();
     }
     if (!launched("kessler_rows_kernel")) return GM1B_ERR_CUDA;
@@ -520,7 +720,7 @@ extern "C" int32_t gm1b_kessler_driver(int32_t ni, int32_t nj, int32_t nk, const
     const double area = (double)(dx * dy);
     {
         ProfScope ps("kessler_finish_kernel", st);
-        kessler_finish_kernel<<<1, 1, 0, st>>>(a, d, w, volume, (double)dx, (double)dy, area);
+        kessler_finish_kernel<<<1, 32 * kBudgets, 0, st>>>(a, d, w, volume, (double)dx, (double)dy, area);
         ps.stop();
     }
     if (!launched("kessler_finish_kernel")) return GM1B_ERR_CUDA;

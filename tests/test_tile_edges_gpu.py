@@ -165,6 +165,28 @@ def test_terrain_tke_diffusion(ni, nj, nk):
     assert _differ(dev, a, ("tketen",)) == []
 
 
+@pytest.mark.parametrize("ni,nj,nk", [(31, 3, 1), (32, 2, 7), (33, 5, 8), (65, 2, 9), (5, 3, 296), (5, 3, 297)])
+def test_kessler_columns(ni, nj, nk):
+    """Columns in shared memory (up to 296 levels) and a thread per column:
+    the sub-step counts and the level-ordered sums are the oracle's."""
+    from oracle import kessler as ko
+    from tests.golden.make_golden import kessler_fixture
+    from tests.test_kessler_gpu import run_gpu
+    from tests.kessler_common import assert_budgets_close, assert_fields_close
+
+    dz = 100.0 if nk < 100 else 20.0
+    meta = dict(ni=ni, nj=nj, nk=nk, dx=1000.0, dy=1000.0, dz=dz, dt=0.2 * dz, eqtset=2)
+    inputs = kessler_fixture(ni, nj, nk, dz, ni + nk)
+    want = {k: v.copy() for k, v in inputs.items()}
+    nfall = np.zeros((nj, ni), np.int32)
+    ko.kessler_driver(want, **meta, nfall=nfall)
+    got, _, nf, _ = run_gpu(inputs, meta)
+    assert np.array_equal(nf, nfall)
+    assert_fields_close(want, got)
+    assert np.array_equal(got["asq"].view(np.uint64), want["asq"].view(np.uint64))
+    assert_budgets_close(want["qbudget"], got["qbudget"])
+
+
 @pytest.mark.parametrize("flat", [False, True])
 @pytest.mark.parametrize("ni,nj,nk", [(31, 7, 9), (32, 8, 10), (30, 6, 18), (3, 3, 3), (63, 15, 20)])
 def test_deformation(ni, nj, nk, flat):
