@@ -31,14 +31,15 @@
 //       src/cm1core/cuda_rayleigh_held.py:213-254, :419-488 (solve1.F:412-454)
 //
 // Design: the strain and gettau passes are grid-stride elementwise kernels
-// over the union of their index spaces (one launch each).  The three column
-// solves run one thread per staggered column, 32 x 4 columns per CTA with
-// consecutive threads on consecutive columns of a row (every level's loads
-// coalesce); the forward sweep keeps the face pairs of the level above in
-// registers for the next level and parks the Thomas coefficients in shared
-// memory ([level][thread], conflict-free); the back substitution recomputes
-// the horizontal divergence and the cross term at each level and adds the
-// tendency there, so no column array beyond the two coefficient rows exists.
+// over the union of their index spaces (one launch each).  A column solve's
+// CTA owns 32 columns of a row: eight warps form the tridiagonal rows of their
+// own runs of levels in shared memory ([level][column], conflict-free; every
+// load and division spread over the CTA), one warp sweeps them, then all warps
+// form the horizontal divergence and the cross term of their levels and add
+// the tendency.  Against a thread per column (its loads one level at a time,
+// too few columns in flight), 189x131x64: turbu 207 -> 71 us, turbv 141 ->
+// 54, turbw 90 -> 38; turbs of theta and the three moisture rows, which share
+// the matrix and its reciprocals, 285 -> 99.
 #include "gm1b_common.cuh"
 
 namespace gm1b {
@@ -46,6 +47,8 @@ namespace {
 
 constexpr int kCX = 32, kCY = 4, kCT = kCX * kCY;  // column tile
 constexpr int kEW = 256;                            // elementwise block
+constexpr int kColWarps = 8;                        // warps of a column solve's CTA, which owns 32 columns of a row
+constexpr int kTurbsGroup = 4;                      // scalars the turbs column pass solves together
 
 #define TRY(x)                        \
     do {                              \
@@ -161,187 +164,146 @@ __global__ void __launch_bounds__(kEW) flat_gettau_kernel(StressArgs a) {
 // DIR 0: a u column (j, f), f in [0, ni]; DIR 1: a v column (f, i), f in [0, nj];
 // the cells either side of it are (ja, ia) and (jb, ib).
 template <int DIR>
-__global__ void __launch_bounds__(kCT) flat_turb_uv_kernel(StressArgs a) {
+__global__ void __launch_bounds__(32 * kColWarps) flat_turb_uv_kernel(const __grid_constant__ StressArgs a) {
     extern __shared__ float s_col[];
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kCX + tx;
+    const int lane = threadIdx.x, wy = threadIdx.y;
     const int ni = a.ni, nj = a.nj, K = a.nk, ux = ni + 1, vy = nj + 1;
-    const int cx = blockIdx.x * kCX + tx, cy = blockIdx.y * kCY + ty;
+    const int nx = DIR == 0 ? ux : ni, tiles = (nx + 31) / 32;
+    const int c0 = blockIdx.x % tiles * 32 + lane, cy = blockIdx.x / tiles;
+    const bool own = c0 < nx;
+    const int cx = min(c0, nx - 1);  // lanes past the row's end repeat its last column and store nothing
     // DIR 0: column (j = cy, f = cx); DIR 1: column (f = cy, i = cx)
-    if (DIR == 0 ? (cx > ni || cy >= nj) : (cx >= ni || cy > nj)) return;
-    const int ja = DIR == 0 ? cy : cy - 1, jb = cy, ia = DIR == 0 ? cx - 1 : cx, ib = cx;
+    const int ja = DIR == 0 ? cy : clampi(cy - 1, nj), jb = clampi(cy, nj);
+    const int ia = DIR == 0 ? clampi(cx - 1, ni) : cx, ib = clampi(cx, ni);
+    const unsigned ca = o3(0, ja, ia, nj, ni), cb = o3(0, jb, ib, nj, ni), cz = (unsigned)nj * ni;
     const float *q = DIR == 0 ? a.u : a.v;       // the column's wind
     const float *top = DIR == 0 ? a.t13 : a.t23;  // its t13/t23 (face levels)
     float *ten = DIR == 0 ? a.uten : a.vten;
-    const unsigned col = DIR == 0 ? (unsigned)cy * ux + cx : (unsigned)cy * ni + cx;
-    const unsigned lev = DIR == 0 ? (unsigned)nj * ux : (unsigned)vy * ni;
+    const unsigned col = (unsigned)cy * nx + cx, lev = DIR == 0 ? (unsigned)nj * ux : (unsigned)vy * ni;
     const float rd = DIR == 0 ? a.rdx : a.rdy, rdz = a.rdz, dt = a.dt;
-    float *cp = s_col, *dp = s_col + (size_t)K * kCT;
-#define CP(k) cp[(unsigned)(k) * kCT + tid]
-#define DP(k) dp[(unsigned)(k) * kCT + tid]
-#define PAIR(p, k) (cell(a, p, k, ja, ia) + cell(a, p, k, jb, ib))
-#define QK(k) q[(unsigned)(k) * lev + col]
-#define D7(k) (((((cell(a, a.w, k, jb, ib) - cell(a, a.w, k, ja, ia)) * rd) * 0.25f) * PAIR(a.kmv, k)) * PAIR(a.rf, k))
+    float *s_a = s_col + lane, *s_b = s_a + K * 32, *s_c = s_b + K * 32, *s_d = s_c + K * 32;
+    auto pair = [&](const float *p, int k) { return p[k * cz + ca] + p[k * cz + cb]; };
     const float rdt = 0.5f / dt;
     const float tema = (((-0.0625f * dt) * 1.0f) * rdz) * rdz;
     const float temb = (((0.0625f * dt) * 0.0f) * rdz) * rdz;
     const float temc = (0.5f * dt) * rdz;
-    // k = 0
-    float rr0 = 1.0f / (0.5f * PAIR(a.rho, 0));
-    float mhp = PAIR(a.mh, 0);
-    float tem = mhp * rr0;
-    float kmv_u = PAIR(a.kmv, 1), mf_u = PAIR(a.mf, 1), rf_u = PAIR(a.rf, 1);  // face above
-    float r2 = ((kmv_u * mf_u) * rf_u) * tem;
-    float cfc = tema * r2, cfb = 1.0f - cfc;
-    float qm = QK(0), qk = QK(1);  // q(k-1), q(k) of the next level
-    float cfd = (qm + temb * (r2 * qk - r2 * qm)) - ((temc * top[col]) * mhp) * rr0;
-    float inv = 1.0f / cfb;
-    float cprev = -(cfc * inv), dprev = cfd * inv;
-    CP(0) = cprev;
-    DP(0) = dprev;
-    #pragma unroll 4
-    for (int k = 1; k < K - 1; ++k) {
-        rr0 = 1.0f / (0.5f * PAIR(a.rho, k));
-        tem = PAIR(a.mh, k) * rr0;
-        const float r1 = ((kmv_u * mf_u) * rf_u) * tem;
-        kmv_u = PAIR(a.kmv, k + 1);
-        mf_u = PAIR(a.mf, k + 1);
-        rf_u = PAIR(a.rf, k + 1);
-        r2 = ((kmv_u * mf_u) * rf_u) * tem;
-        const float cfa = tema * r1;
-        cfc = tema * r2;
-        cfb = (1.0f - cfa) - cfc;
-        const float qp = QK(k + 1);
-        cfd = qk + temb * ((r2 * qp - (r1 + r2) * qk) + r1 * qm);
-        inv = 1.0f / (cfa * cprev + cfb);
-        cprev = -(cfc * inv);
-        dprev = (cfd - cfa * dprev) * inv;
-        CP(k) = cprev;
-        DP(k) = dprev;
-        qm = qk;
-        qk = qp;
-    }
-    float sol;
-    {
-        const int k = K - 1;
-        rr0 = 1.0f / (0.5f * PAIR(a.rho, k));
-        mhp = PAIR(a.mh, k);
-        tem = mhp * rr0;
-        const float r1 = ((kmv_u * mf_u) * rf_u) * tem;
-        const float cfa = tema * r1;
-        cfb = 1.0f - cfa;
-        cfd = (qk + temb * (-(r1 * qk) + r1 * qm)) + ((temc * top[(unsigned)K * lev + col]) * mhp) * rr0;
-        inv = 1.0f / (cfa * cprev + cfb);
-        sol = (cfd - cfa * dprev) * inv;
-    }
-    // back substitution, the vertical term and the tendency per level
-    float d7_up = 0.0f;
-    #pragma unroll 4
-    for (int k = K - 1; k >= 0; --k) {
-        if (k < K - 1) sol = CP(k) * sol + DP(k);
-        const float rho_p = PAIR(a.rho, k);
-        float tz = (rho_p * (sol - QK(k))) * rdt;
-        const float d7 = k == 0 ? 0.0f : D7(k);
-        tz = tz + (((d7_up - d7) * rdz) * 0.5f) * PAIR(a.mh, k);
-        d7_up = d7;
-        float hx, hy;
-        if (DIR == 0) {
-            hx = (cell(a, a.t11, k, cy, ib) - cell(a, a.t11, k, cy, ia)) * a.rdx;
-            hy = (a.t12[o3(k, cy + 1, cx, vy, ux)] - a.t12[o3(k, cy, cx, vy, ux)]) * a.rdy;
-            if (cx == 0 || cx == ni) hx = 0.0f;
-            if (cy == 0 || cy == nj - 1) hy = 0.0f;
-        } else {
-            hx = (a.t12[o3(k, cy, cx + 1, vy, ux)] - a.t12[o3(k, cy, cx, vy, ux)]) * a.rdx;
-            hy = (cell(a, a.t22, k, jb, cx) - cell(a, a.t22, k, ja, cx)) * a.rdy;
-            if (cx == 0 || cx == ni - 1) hx = 0.0f;
-            if (cy == 0 || cy == nj) hy = 0.0f;
+    const int run = (K + kColWarps - 1) / kColWarps;
+    const int lo = min(wy * run, K), hi = min(lo + run, K);
+    // the diffusivity product of a face, formed once and carried up
+    auto face = [&](int f) { return f >= 1 && f < K ? (pair(a.kmv, f) * pair(a.mf, f)) * pair(a.rf, f) : 0.0f; };
+    if (lo < hi) {
+        float below = face(lo), qm = lo > 0 ? q[(lo - 1) * lev + col] : 0.0f, qk = q[lo * lev + col];
+#pragma unroll 2
+        for (int k = lo; k < hi; ++k) {
+            const float rr0 = 1.0f / (0.5f * pair(a.rho, k));
+            const float mhp = pair(a.mh, k), tem = mhp * rr0;
+            const float above = face(k + 1), qp = k + 1 < K ? q[(k + 1) * lev + col] : 0.0f;
+            const float r1 = below * tem, r2 = above * tem;
+            const float cfa = tema * r1, cfc = tema * r2;
+            float cfb, cfd;
+            if (k == 0) {
+                cfb = 1.0f - cfc;
+                cfd = (qk + temb * (r2 * qp - r2 * qk)) - ((temc * top[col]) * mhp) * rr0;
+            } else if (k == K - 1) {
+                cfb = 1.0f - cfa;
+                cfd = (qk + temb * (-(r1 * qk) + r1 * qm)) + ((temc * top[(unsigned)K * lev + col]) * mhp) * rr0;
+            } else {
+                cfb = (1.0f - cfa) - cfc;
+                cfd = qk + temb * ((r2 * qp - (r1 + r2) * qk) + r1 * qm);
+            }
+            s_a[k * 32] = cfa, s_b[k * 32] = cfb, s_c[k * 32] = cfc, s_d[k * 32] = cfd;
+            below = above, qm = qk, qk = qp;
         }
-        const float rrk = 1.0f / (0.5f * rho_p);
-        const unsigned p = (unsigned)k * lev + col;
-        ten[p] = ten[p] + ((hx + hy) + tz) * rrk;
     }
-#undef CP
-#undef DP
-#undef PAIR
-#undef QK
-#undef D7
+    __syncthreads();
+    if (wy == 0) column_sweep(s_a, s_b, s_c, s_d, K);
+    __syncthreads();
+    if (lo >= hi || !own) return;
+    // the vertical and horizontal terms and the tendency of each level
+    auto cross = [&](int k) {
+        return k >= 1 && k < K ? ((((a.w[k * cz + cb] - a.w[k * cz + ca]) * rd) * 0.25f) * pair(a.kmv, k)) * pair(a.rf, k)
+                               : 0.0f;
+    };
+    const unsigned corner = (unsigned)vy * ux, oc = o3(0, cy, cx, vy, ux), ou = oc + (DIR == 0 ? ux : 1);
+    const bool ex = DIR == 0 ? cx == 0 || cx == ni : cx == 0 || cx == ni - 1;
+    const bool ey = DIR == 0 ? cy == 0 || cy == nj - 1 : cy == 0 || cy == nj;
+    const float *diag = DIR == 0 ? a.t11 : a.t22;
+    float d7 = cross(lo);
+#pragma unroll 2
+    for (int k = lo; k < hi; ++k) {
+        const unsigned p = (unsigned)k * lev + col;
+        const float rho_p = pair(a.rho, k), old = ten[p];
+        float tz = (rho_p * (s_d[k * 32] - q[p])) * rdt;
+        const float d7_up = cross(k + 1);
+        tz = tz + (((d7_up - d7) * rdz) * 0.5f) * pair(a.mh, k);
+        d7 = d7_up;
+        const float dd = diag[k * cz + cb] - diag[k * cz + ca];
+        const float dc = a.t12[k * corner + ou] - a.t12[k * corner + oc];
+        const float hx = ex ? 0.0f : (DIR == 0 ? dd : dc) * a.rdx;
+        const float hy = ey ? 0.0f : (DIR == 0 ? dc : dd) * a.rdy;
+        const float rrk = 1.0f / (0.5f * rho_p);
+        ten[p] = old + ((hx + hy) + tz) * rrk;
+    }
 }
 
 // ----------------------------------------------------------------- turbw
-__global__ void __launch_bounds__(kCT) flat_turbw_kernel(StressArgs a) {
+__global__ void __launch_bounds__(32 * kColWarps) flat_turbw_kernel(const __grid_constant__ StressArgs a) {
     extern __shared__ float s_col[];
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kCX + tx;
-    const int ni = a.ni, nj = a.nj, K = a.nk, ux = ni + 1, vy = nj + 1;
-    const int i = blockIdx.x * kCX + tx, j = blockIdx.y * kCY + ty;
-    if (i >= ni || j >= nj) return;
+    const int lane = threadIdx.x, wy = threadIdx.y;
+    const int ni = a.ni, nj = a.nj, K = a.nk, n = K - 1, ux = ni + 1, vy = nj + 1, tiles = (ni + 31) / 32;
+    const int i0 = blockIdx.x % tiles * 32 + lane, j = blockIdx.x / tiles;
+    const bool own = i0 < ni;
+    const int i = min(i0, ni - 1);  // lanes past the row's end repeat its last column and store nothing
     const unsigned col = (unsigned)j * ni + i, lev = (unsigned)nj * ni;
     const float rdz = a.rdz, dt = a.dt;
-    float *cp = s_col, *dp = s_col + (size_t)K * kCT;
-#define CP(p) cp[(unsigned)(p) * kCT + tid]
-#define DP(p) dp[(unsigned)(p) * kCT + tid]
-#define PF(p, f) p[(unsigned)(f) * lev + col]
+    float *s_a = s_col + lane, *s_b = s_a + n * 32, *s_c = s_b + n * 32, *s_d = s_c + n * 32;  // rows f - 1
     const float rdt = 1.0f / dt;
     const float tema = (((-1.0f * dt) * 1.0f) * rdz) * rdz;
     const float temb = ((dt * 0.0f) * rdz) * rdz;
     const float temc = dt * rdz;
-    // face 1
-    float rrf = PF(a.mf, 1) / PF(a.rf, 1);
-    float kmh_m = PF(a.kmh, 1), kmh_u = PF(a.kmh, 2);
-    float r2 = (((kmh_m + kmh_u) * PF(a.mh, 1)) * PF(a.rho, 1)) * rrf;
-    float cfc = tema * r2, cfb = 1.0f - cfc;
-    float wm = PF(a.w, 1), wk = PF(a.w, 2);  // w(f-1), w(f) of the next face
-    float cfd = (wm + temb * (r2 * wk - r2 * wm)) - (temc * PF(a.t33, 0)) * rrf;
-    float inv = 1.0f / cfb;
-    float cprev = -(cfc * inv), dprev = cfd * inv;
-    CP(0) = cprev;
-    DP(0) = dprev;
-    #pragma unroll 4
-    for (int f = 2; f < K - 1; ++f) {
-        rrf = PF(a.mf, f) / PF(a.rf, f);
-        const float r1 = (((kmh_m + kmh_u) * PF(a.mh, f - 1)) * PF(a.rho, f - 1)) * rrf;
-        kmh_m = kmh_u;
-        kmh_u = PF(a.kmh, f + 1);
-        r2 = (((kmh_m + kmh_u) * PF(a.mh, f)) * PF(a.rho, f)) * rrf;
-        const float cfa = tema * r1;
-        cfc = tema * r2;
-        cfb = (1.0f - cfa) - cfc;
-        const float wp = PF(a.w, f + 1);
-        cfd = wk + temb * ((r2 * wp - (r1 + r2) * wk) + r1 * wm);
-        inv = 1.0f / (cfa * cprev + cfb);
-        cprev = -(cfc * inv);
-        dprev = (cfd - cfa * dprev) * inv;
-        CP(f - 1) = cprev;
-        DP(f - 1) = dprev;
-        wm = wk;
-        wk = wp;
+    const int run = (n + kColWarps - 1) / kColWarps;
+    const int lo = min(1 + wy * run, K), hi = min(lo + run, K);  // faces lo .. hi-1
+    if (lo < hi) {
+        unsigned z = (unsigned)lo * lev + col;
+        float km = a.kmh[z - lev], k0 = a.kmh[z], mhm = a.mh[z - lev], rhom = a.rho[z - lev], wm = a.w[z - lev],
+              wk = a.w[z];
+#pragma unroll 2
+        for (int f = lo; f < hi; ++f, z += lev) {
+            const float rrf = a.mf[z] / a.rf[z];
+            const float kp = a.kmh[z + lev], mh = a.mh[z], rho = a.rho[z], wp = a.w[z + lev];
+            const float r1 = (((km + k0) * mhm) * rhom) * rrf, r2 = (((k0 + kp) * mh) * rho) * rrf;
+            const float cfa = tema * r1, cfc = tema * r2;
+            float cfb, cfd;
+            if (f == 1) {
+                cfb = 1.0f - cfc;
+                cfd = (wk + temb * (r2 * wp - r2 * wk)) - (temc * a.t33[col]) * rrf;
+            } else if (f == n) {
+                cfb = 1.0f - cfa;
+                cfd = (wk + temb * (-(r1 * wk) + r1 * wm)) + (temc * a.t33[z]) * rrf;
+            } else {
+                cfb = (1.0f - cfa) - cfc;
+                cfd = wk + temb * ((r2 * wp - (r1 + r2) * wk) + r1 * wm);
+            }
+            const int p = (f - 1) * 32;
+            s_a[p] = cfa, s_b[p] = cfb, s_c[p] = cfc, s_d[p] = cfd;
+            km = k0, k0 = kp, mhm = mh, rhom = rho, wm = wk, wk = wp;
+        }
     }
-    float sol;
-    {
-        const int f = K - 1;
-        rrf = PF(a.mf, f) / PF(a.rf, f);
-        const float r1 = (((kmh_m + kmh_u) * PF(a.mh, f - 1)) * PF(a.rho, f - 1)) * rrf;
-        const float cfa = tema * r1;
-        cfb = 1.0f - cfa;
-        cfd = (wk + temb * (-(r1 * wk) + r1 * wm)) + (temc * PF(a.t33, f)) * rrf;
-        inv = 1.0f / (cfa * cprev + cfb);
-        sol = (cfd - cfa * dprev) * inv;
+    __syncthreads();
+    if (wy == 0) column_sweep(s_a, s_b, s_c, s_d, n);
+    __syncthreads();
+    if (!own) return;
+    const bool ex = i == 0 || i == ni - 1, ey = j == 0 || j == nj - 1;
+#pragma unroll 2
+    for (int f = lo; f < hi; ++f) {
+        const unsigned p = (unsigned)f * lev + col, px = o3(f, j, i, nj, ux), py = o3(f, j, i, vy, ni);
+        const float rff = a.rf[p], old = a.wten[p];
+        const float tz = (rff * (s_d[(f - 1) * 32] - a.w[p])) * rdt;
+        const float hx = ex ? 0.0f : (a.t13[px + 1] - a.t13[px]) * a.rdx;
+        const float hy = ey ? 0.0f : (a.t23[py + ni] - a.t23[py]) * a.rdy;
+        a.wten[p] = old + ((hx + hy) + tz) / rff;
     }
-    #pragma unroll 4
-    for (int f = K - 1; f >= 1; --f) {
-        if (f < K - 1) sol = CP(f - 1) * sol + DP(f - 1);
-        const float rff = PF(a.rf, f);
-        const float tz = (rff * (sol - PF(a.w, f))) * rdt;
-        float hx = (a.t13[o3(f, j, i + 1, nj, ux)] - a.t13[o3(f, j, i, nj, ux)]) * a.rdx;
-        float hy = (a.t23[o3(f, j + 1, i, vy, ni)] - a.t23[o3(f, j, i, vy, ni)]) * a.rdy;
-        if (i == 0 || i == ni - 1) hx = 0.0f;
-        if (j == 0 || j == nj - 1) hy = 0.0f;
-        const unsigned p = (unsigned)f * lev + col;
-        a.wten[p] = a.wten[p] + ((hx + hy) + tz) / rff;
-    }
-#undef CP
-#undef DP
-#undef PF
 }
-
 
 // ---------------------------------------------------------- turbs (flat)
 // theta ((th0 - 300) + tha) and numq moisture rows.  The open-halo copies of
@@ -415,77 +377,125 @@ __global__ void __launch_bounds__(kCT) flat_turbs_horizontal_kernel(TurbsArgs a)
     }
 }
 
-__global__ void __launch_bounds__(kCT) flat_turbs_column_kernel(TurbsArgs a) {
+// The matrix and its reciprocals are the same for every scalar: formed and
+// swept once a column, then a warp per scalar of the group sweeps its right
+// side.  Shared words per level and column: the matrix rows (the reciprocal in
+// the diagonal's place) and one of each scalar.
+__global__ void __launch_bounds__(32 * kColWarps) flat_turbs_column_kernel(const __grid_constant__ TurbsArgs a) {
     extern __shared__ float s_col[];
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kCX + tx;
-    const int ni = a.ni, nj = a.nj, nk = a.nk;
-    const int i = blockIdx.x * kCX + tx, j = blockIdx.y * kCY + ty;
-    if (i >= ni || j >= nj) return;
+    const int lane = threadIdx.x, wy = threadIdx.y;
+    const int ni = a.ni, nj = a.nj, nk = a.nk, tiles = (ni + 31) / 32;
+    const int i0 = blockIdx.x % tiles * 32 + lane, j = blockIdx.x / tiles;
+    const bool own = i0 < ni;
+    const int i = min(i0, ni - 1);  // lanes past the row's end repeat its last column and store nothing
     const size_t n = (size_t)ni * nj * nk;
     const unsigned col = (unsigned)j * ni + i, lev = (unsigned)nj * ni;
-    float *cp = s_col, *dp = s_col + (size_t)nk * kCT;
-#define CP(k) cp[(unsigned)(k) * kCT + tid]
-#define DP(k) dp[(unsigned)(k) * kCT + tid]
-#define PF(p, k) p[(unsigned)(k) * lev + col]
-#define COEF(F, K) ((((PF(a.khv, F) * PF(a.mf, F)) * PF(a.rf, F)) * PF(a.mh, K)) * PF(a.rr, K))
+    const int words = nk * 32;
+    float *s_a = s_col + lane, *s_b = s_a + words, *s_c = s_b + words, *s_d = s_c + words;
     const float rz = 1.0f / a.dz, dt = a.dt, rdt = 1.0f / dt;
     const float tema = (((-1.0f * dt) * 1.0f) * rz) * rz;
     const float temb = ((dt * 0.0f) * rz) * rz;
     const float temc = dt * rz;
-    for (int sc = 0; sc < a.nsc; ++sc) {
-        float *target = sc == 0 ? a.thten : a.qten + (size_t)(sc - 1) * n;
-        const float *h = a.work + (size_t)sc * n;
-#define SC(k) sval(a, sc, k, j, i)
-        float sm = SC(0), sk = SC(1);  // scalar at k-1 and k of the next level
-        float r2 = COEF(1, 0);
-        float cfc = tema * r2, cfb = 1.0f - cfc;
-        float ex = (-r2) * sm + r2 * sk;
-        float bc = ((temc * 0.0f) * PF(a.mh, 0)) * PF(a.rr, 0);
-        float cfd = (sm + temb * ex) + bc;
-        float tem = 1.0f / cfb;
-        float cprev = (-cfc) * tem, dprev = cfd * tem;
-        CP(0) = cprev;
-        DP(0) = dprev;
-        for (int k = 1; k + 1 < nk; ++k) {
-            const float r1 = COEF(k, k);
-            r2 = COEF(k + 1, k);
-            const float cfa = tema * r1;
-            cfc = tema * r2;
-            cfb = (1.0f - cfa) - cfc;
-            const float sp1 = SC(k + 1);
-            ex = (r1 * sm - (r1 + r2) * sk) + r2 * sp1;
-            cfd = sk + temb * ex;
-            tem = 1.0f / (cfa * cprev + cfb);
-            cprev = (-cfc) * tem;
-            dprev = (cfd - cfa * dprev) * tem;
-            CP(k) = cprev;
-            DP(k) = dprev;
-            sm = sk;
-            sk = sp1;
+    const int run = (nk + kColWarps - 1) / kColWarps;
+    const int lo = min(wy * run, nk), hi = min(lo + run, nk);
+    auto face = [&](int f) {
+        const unsigned z = (unsigned)f * lev + col;
+        return f >= 1 && f < nk ? (a.khv[z] * a.mf[z]) * a.rf[z] : 0.0f;
+    };
+    for (int first = 0; first < a.nsc; first += kTurbsGroup) {
+        const int group = min(kTurbsGroup, a.nsc - first);
+        const float *src[kTurbsGroup];  // theta is (th0 - 300) + tha
+#pragma unroll
+        for (int g = 0; g < kTurbsGroup; ++g) {
+            const int sc = first + min(g, group - 1);
+            src[g] = (sc == 0 ? a.tha : a.qa + (size_t)(sc - 1) * n) + col;
         }
-        float sol;
-        {
-            const int k = nk - 1;
-            const float r1 = COEF(k, k), cfa = tema * r1;
-            cfb = 1.0f - cfa;
-            ex = r1 * sm - r1 * sk;
-            bc = ((temc * 0.0f) * PF(a.mh, k)) * PF(a.rr, k);
-            cfd = (sk + temb * ex) - bc;
-            tem = 1.0f / (cfa * cprev + cfb);
-            sol = (cfd - cfa * dprev) * tem;
+        auto scalar = [&](int g, int k) {
+            const float x = src[g][(unsigned)k * lev];
+            return first == 0 && g == 0 ? (a.th0[k] - 300.0f) + x : x;
+        };
+        if (lo < hi) {
+            float below = face(lo), sm[kTurbsGroup], sk[kTurbsGroup];
+#pragma unroll
+            for (int g = 0; g < kTurbsGroup; ++g) {
+                sm[g] = lo > 0 ? scalar(g, lo - 1) : 0.0f;
+                sk[g] = scalar(g, lo);
+            }
+            for (int k = lo; k < hi; ++k) {
+                const unsigned z = (unsigned)k * lev + col;
+                const float mh = a.mh[z], rr = a.rr[z], above = face(k + 1);
+                const float r1 = (below * mh) * rr, r2 = (above * mh) * rr;
+                const float cfa = tema * r1, cfc = tema * r2, bc = ((temc * 0.0f) * mh) * rr;
+                if (first == 0) {
+                    s_a[k * 32] = cfa, s_c[k * 32] = cfc;
+                    s_b[k * 32] = k == 0 ? 1.0f - cfc : k == nk - 1 ? 1.0f - cfa : (1.0f - cfa) - cfc;
+                }
+#pragma unroll
+                for (int g = 0; g < kTurbsGroup; ++g) {
+                    if (g >= group) break;
+                    const float sp = k + 1 < nk ? scalar(g, k + 1) : 0.0f;
+                    float cfd;
+                    if (k == 0) {
+                        const float ex = (-r2) * sk[g] + r2 * sp;
+                        cfd = (sk[g] + temb * ex) + bc;
+                    } else if (k == nk - 1) {
+                        const float ex = r1 * sm[g] - r1 * sk[g];
+                        cfd = (sk[g] + temb * ex) - bc;
+                    } else {
+                        const float ex = (r1 * sm[g] - (r1 + r2) * sk[g]) + r2 * sp;
+                        cfd = sk[g] + temb * ex;
+                    }
+                    s_d[g * words + k * 32] = cfd;
+                    sm[g] = sk[g], sk[g] = sp;
+                }
+                below = above;
+            }
         }
-        for (int k = nk - 1; k >= 0; --k) {
-            if (k != nk - 1) sol = CP(k) * sol + DP(k);
-            const float tz = (PF(a.rho, k) * (sol - SC(k))) * rdt;
-            const unsigned p = (unsigned)k * lev + col;
-            target[p] = target[p] + (h[p] + tz) * PF(a.rr, k);
+        __syncthreads();
+        if (first == 0) {
+            if (wy == 0) {
+                float cprev = 0.0f;
+#pragma unroll 4
+                for (int k = 0; k < nk; ++k) {
+                    const float inv = rcp_rn(k == 0 ? s_b[0] : s_a[k * 32] * cprev + s_b[k * 32]);
+                    cprev = (-s_c[k * 32]) * inv;
+                    s_b[k * 32] = inv, s_c[k * 32] = cprev;
+                }
+            }
+            __syncthreads();
         }
-#undef SC
+        if (wy < group) {
+            float *d = s_d + wy * words;
+            float prev = d[0] * s_b[0];
+            d[0] = prev;
+#pragma unroll 8
+            for (int k = 1; k < nk; ++k) {
+                prev = (d[k * 32] - s_a[k * 32] * prev) * s_b[k * 32];
+                d[k * 32] = prev;
+            }
+#pragma unroll 8
+            for (int k = nk - 2; k >= 0; --k) {
+                prev = s_c[k * 32] * prev + d[k * 32];
+                d[k * 32] = prev;
+            }
+        }
+        __syncthreads();
+        if (own) {
+            for (int k = lo; k < hi; ++k) {
+                const unsigned z = (unsigned)k * lev + col;
+                const float rho = a.rho[z], rr = a.rr[z];
+#pragma unroll
+                for (int g = 0; g < kTurbsGroup; ++g) {
+                    if (g >= group) break;
+                    const int sc = first + g;
+                    float *target = sc == 0 ? a.thten : a.qten + (size_t)(sc - 1) * n;
+                    const float tz = (rho * (s_d[g * words + k * 32] - scalar(g, k))) * rdt;
+                    target[z] = target[z] + (a.work[(size_t)sc * n + z] + tz) * rr;
+                }
+            }
+        }
+        __syncthreads();  // the next group's right sides take these words
     }
-#undef CP
-#undef DP
-#undef PF
-#undef COEF
 }
 
 // ------------------------------------------------------ Rayleigh (upper)
@@ -650,28 +660,30 @@ int configure(Kernel kernel, size_t smem, const char *name) {
 }
 
 int enqueue_momentum(const StressArgs &a, cudaStream_t st) {
-    const size_t smem = (size_t)2 * a.nk * kCT * sizeof(float);
-    if (smem > 200 * 1024) {
+    if (a.nk > 200) {
         gm1b_set_error("gm1b_flat_momentum_stress: nk=%d exceeds the column solves' shared memory (nk <= 200)", a.nk);
         return GM1B_ERR_ARGUMENT;
     }
-    TRY(configure(flat_turb_uv_kernel<0>, smem, "flat_turb_uv_kernel<0>"));
-    TRY(configure(flat_turb_uv_kernel<1>, smem, "flat_turb_uv_kernel<1>"));
-    TRY(configure(flat_turbw_kernel, smem, "flat_turbw_kernel"));
+    const size_t words = (size_t)4 * a.nk * 32 * sizeof(float);
+    TRY(configure(flat_turb_uv_kernel<0>, words, "flat_turb_uv_kernel<0>"));
+    TRY(configure(flat_turb_uv_kernel<1>, words, "flat_turb_uv_kernel<1>"));
+    TRY(configure(flat_turbw_kernel, words, "flat_turbw_kernel"));
+    const dim3 cta(32, kColWarps);
+    auto tiles = [](int nx, int ny) { return (unsigned)((nx + 31) / 32) * (unsigned)ny; };
     {
         ProfScope ps("flat_turbu_kernel", st);
-        flat_turb_uv_kernel<0><<<dim3((a.ni + 1 + kCX - 1) / kCX, (a.nj + kCY - 1) / kCY), dim3(kCX, kCY), smem, st>>>(a);
+        flat_turb_uv_kernel<0><<<tiles(a.ni + 1, a.nj), cta, words, st>>>(a);
         ps.stop();
         if (!launch_ok("flat_turbu_kernel")) return GM1B_ERR_CUDA;
     }
     {
         ProfScope ps("flat_turbv_kernel", st);
-        flat_turb_uv_kernel<1><<<dim3((a.ni + kCX - 1) / kCX, (a.nj + 1 + kCY - 1) / kCY), dim3(kCX, kCY), smem, st>>>(a);
+        flat_turb_uv_kernel<1><<<tiles(a.ni, a.nj + 1), cta, words, st>>>(a);
         ps.stop();
         if (!launch_ok("flat_turbv_kernel")) return GM1B_ERR_CUDA;
     }
     ProfScope ps("flat_turbw_kernel", st);
-    flat_turbw_kernel<<<dim3((a.ni + kCX - 1) / kCX, (a.nj + kCY - 1) / kCY), dim3(kCX, kCY), smem, st>>>(a);
+    flat_turbw_kernel<<<tiles(a.ni, a.nj), cta, words, st>>>(a);
     ps.stop();
     return launch_ok("flat_turbw_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }
@@ -750,8 +762,9 @@ extern "C" int32_t gm1b_flat_scalar_turbulence(int32_t ni, int32_t nj, int32_t n
         gm1b_set_error("gm1b_flat_scalar_turbulence: a required array (or the workspace) is NULL");
         return GM1B_ERR_ARGUMENT;
     }
-    const size_t smem = (size_t)2 * nk * kCT * sizeof(float);
-    if (smem > 200 * 1024) {
+    // nk <= 200: 179200 bytes for a full group
+    const size_t smem = (size_t)(3 + (numq + 1 < kTurbsGroup ? numq + 1 : kTurbsGroup)) * nk * 32 * sizeof(float);
+    if (nk > 200) {
         gm1b_set_error("gm1b_flat_scalar_turbulence: nk=%d exceeds the column solve's shared memory (nk <= 200)", nk);
         return GM1B_ERR_ARGUMENT;
     }
@@ -767,7 +780,7 @@ extern "C" int32_t gm1b_flat_scalar_turbulence(int32_t ni, int32_t nj, int32_t n
         if (!launch_ok("flat_turbs_horizontal_kernel")) return GM1B_ERR_CUDA;
     }
     ProfScope ps("flat_turbs_column_kernel", st);
-    flat_turbs_column_kernel<<<cols, tile, smem, st>>>(a);
+    flat_turbs_column_kernel<<<(unsigned)((ni + 31) / 32) * (unsigned)nj, dim3(32, kColWarps), smem, st>>>(a);
     ps.stop();
     return launch_ok("flat_turbs_column_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }

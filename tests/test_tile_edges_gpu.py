@@ -165,6 +165,31 @@ def test_terrain_tke_diffusion(ni, nj, nk):
     assert _differ(dev, a, ("tketen",)) == []
 
 
+@pytest.mark.parametrize("ni,nj,nk,numq", [(31, 3, 7, 2), (32, 4, 8, 3), (33, 3, 9, 4), (64, 3, 17, 5), (3, 5, 200, 6)])
+def test_flat_turbulence_columns(ni, nj, nk, numq):
+    """Runs of levels of the stress and scalar solves, and the scalars'
+    groups of four."""
+    from gm1_b200 import stress
+    from oracle import stress as ost
+    from tests.test_stress_gpu import _inputs, _turbs_inputs
+
+    g = dict(ni=ni, nj=nj, nk=nk, dx=100.0, dy=90.0, dt=0.6)
+    a, rdz = _inputs(ni, nj, nk, ni + nk)
+    rng = np.random.default_rng(nk)
+    for n in ost.TAU_NAMES:
+        a[n][:] = rng.normal(0.0, 1.0, a[n].shape)
+    d = _dev(a)
+    ost.flat_momentum_stress(a, **g, rdz=rdz)
+    stress.launch_cuda_flat_momentum_stress(d, **g, rdz=rdz)
+    assert _differ(d, a, ost.TENDENCY_NAMES) == []
+    a, dz = _turbs_inputs(ni, nj, nk, numq, ni + nk)
+    d = _dev(a)
+    d["workspace"] = stress.scalar_turbulence_workspace(ni, nj, nk, numq, d["tha"].device)
+    ost.flat_scalar_turbulence(a, **g, numq=numq, dz=dz)
+    stress.launch_cuda_flat_scalar_turbulence(d, **g, numq=numq, dz=dz)
+    assert _differ(d, a, ("thten1", "qten")) == []
+
+
 @pytest.mark.parametrize("ni,nj,nk", [(31, 3, 1), (32, 2, 7), (33, 5, 8), (65, 2, 9), (5, 3, 296), (5, 3, 297)])
 def test_kessler_columns(ni, nj, nk):
     """Columns in shared memory (up to 296 levels) and a thread per column:
