@@ -49,14 +49,17 @@ __device__ __forceinline__ float flx3(float s1, float s2, float s3) {
 // (subnormal-adjacent, huge, zero, inf, NaN) it defers to __frcp_rn.
 // gm1b_selftest_reciprocal compares it with __frcp_rn on every one of the
 // 2^32 binary32 words.
-__device__ __forceinline__ float rcp_rn(float b) {
+__device__ __forceinline__ bool rcp_short(float b) {  // the short path holds
     const float ab = fabsf(b);
-    if (!(ab >= 0x1p-125f && ab <= 0x1p125f)) return __frcp_rn(b);
+    return ab >= 0x1p-125f && ab <= 0x1p125f;
+}
+__device__ __forceinline__ float rcp_rn_short(float b) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
     const float e = fmaf(-b, y, 1.0f);
     return fmaf(y, e, y);
 }
+__device__ __forceinline__ float rcp_rn(float b) { return rcp_short(b) ? rcp_rn_short(b) : __frcp_rn(b); }
 
 __device__ __forceinline__ float flx5(float s1, float s2, float s3, float s4, float s5) {
     float r = kF5_1 * s1;
@@ -117,37 +120,75 @@ int32_t open_fills(int32_t ni, int32_t nj, int32_t nk, const OpenFill *fills, in
 int32_t pack_scalars_open(int32_t ni, int32_t nj, int32_t nk, const float *th0, const float *const scalar[4],
                           float *const padded[4], cudaStream_t st);
 
-constexpr int kSweepChunk = 8;  // back-substitution levels whose words the sweep reads together
+// The sweep of a column's tridiagonal rows 0 .. n-1 in shared memory (rows at
+// stride 32, one lane per column, a whole warp; n >= 1): the eliminated
+// coefficients are left in s_c, the solution in s_d.  Bound by the chain of a
+// row's multiply, add, reciprocal and multiply, so the reciprocals' range
+// check, a branch on the chain, is taken once a chunk of rows: the chunk is
+// formed on the short path, and again from its start with rcp_rn if any row's
+// pivot of any lane lay outside it.  Against a row at a time with the branch:
+// turbu at 189x131x64 71 -> 56 us, turbv 54 -> 45, the acoustic column pass at
+// 640x768x80 0.863 -> 0.799 ms.
+constexpr int kSweepChunk = 8;  // rows whose words the back substitution reads together
 
-// the sweep of a column's tridiagonal rows in shared memory (rows p at stride
-// 32, forward into c and d, the solution left in d), one lane per column; n >= 1
+template <int kSweepRows>  // rows of a forward chunk; the next one's words are in flight meanwhile
 __device__ __forceinline__ void column_sweep(const float *s_a, const float *s_b, float *s_c, float *s_d, int n) {
-    float cprev = 0.0f, dprev = 0.0f;
-    float cfa = s_a[0], cfb = s_b[0], cfc = s_c[0], cfd = s_d[0];
-    for (int p = 0; p < n - 1; ++p) {
-        const int q = (p + 1) * 32;
-        const float na = s_a[q], nb = s_b[q], nc = s_c[q], nd = s_d[q];
-        const float inv = rcp_rn(p == 0 ? cfb : cfa * cprev + cfb);
-        cprev = -(cfc * inv);
-        dprev = (p == 0 ? cfd : cfd - cfa * dprev) * inv;
-        s_c[p * 32] = cprev;
-        s_d[p * 32] = dprev;
-        cfa = na, cfb = nb, cfc = nc, cfd = nd;
+    float ec = 0.0f, ed = 0.0f;
+    struct Rows {
+        float a[kSweepRows], b[kSweepRows], c[kSweepRows], d[kSweepRows];
+    };
+    auto load = [&](int p0) {
+        Rows r;
+#pragma unroll
+        for (int q = 0; q < kSweepRows; ++q) {
+            const int z = min(p0 + q, n - 1) * 32;
+            r.a[q] = p0 + q == 0 ? 0.0f : s_a[z], r.b[q] = s_b[z], r.c[q] = s_c[z], r.d[q] = s_d[z];
+        }
+        return r;
+    };
+    Rows next = load(0);
+    for (int p0 = 0; p0 < n; p0 += kSweepRows) {
+        const Rows r = next;
+        next = load(p0 + kSweepRows);  // (rows past the last repeat it)
+        float e[kSweepRows], f[kSweepRows];
+        const float ec0 = ec, ed0 = ed;
+        bool rare = false;
+#pragma unroll
+        for (int q = 0; q < kSweepRows; ++q) {
+            const float piv = r.a[q] * ec + r.b[q];
+            rare |= !rcp_short(piv);
+            const float inv = rcp_rn_short(piv);
+            e[q] = ec = -(r.c[q] * inv);
+            f[q] = ed = (r.d[q] - r.a[q] * ed) * inv;
+        }
+        if (__any_sync(0xffffffffu, rare)) {
+            ec = ec0, ed = ed0;
+#pragma unroll
+            for (int q = 0; q < kSweepRows; ++q) {
+                const float inv = rcp_rn(r.a[q] * ec + r.b[q]);
+                e[q] = ec = -(r.c[q] * inv);
+                f[q] = ed = (r.d[q] - r.a[q] * ed) * inv;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kSweepRows; ++q) {
+            if (p0 + q >= n) break;
+            s_c[(p0 + q) * 32] = e[q], s_d[(p0 + q) * 32] = f[q];
+        }
     }
-    float sol = (cfd - cfa * dprev) * rcp_rn(cfa * cprev + cfb);
-    s_d[(n - 1) * 32] = sol;
+    float sol = s_d[(n - 1) * 32];
     for (int pb = n - 2; pb >= 0; pb -= kSweepChunk) {
         float ce[kSweepChunk], de[kSweepChunk];
 #pragma unroll
-        for (int e = 0; e < kSweepChunk; ++e) {
-            const int p = max(pb - e, 0);
-            ce[e] = s_c[p * 32], de[e] = s_d[p * 32];
+        for (int q = 0; q < kSweepChunk; ++q) {
+            const int p = max(pb - q, 0);
+            ce[q] = s_c[p * 32], de[q] = s_d[p * 32];
         }
 #pragma unroll
-        for (int e = 0; e < kSweepChunk; ++e) {
-            if (pb - e < 0) break;
-            sol = ce[e] * sol + de[e];
-            s_d[(pb - e) * 32] = sol;
+        for (int q = 0; q < kSweepChunk; ++q) {
+            if (pb - q < 0) break;
+            sol = ce[q] * sol + de[q];
+            s_d[(pb - q) * 32] = sol;
         }
     }
 }

@@ -37,8 +37,8 @@
 // load and division spread over the CTA), one warp sweeps them, then all warps
 // form the horizontal divergence and the cross term of their levels and add
 // the tendency.  Against a thread per column (its loads one level at a time,
-// too few columns in flight), 189x131x64: turbu 207 -> 71 us, turbv 141 ->
-// 54, turbw 90 -> 38; turbs of theta and the three moisture rows, which share
+// too few columns in flight), 189x131x64: turbu 207 -> 56 us, turbv 141 ->
+// 45, turbw 90 -> 39; turbs of theta and the three moisture rows, which share
 // the matrix and its reciprocals, 285 -> 99.
 #include "gm1b_common.cuh"
 
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(32 * kColWarps) flat_turb_uv_kernel(const __gr
         }
     }
     __syncthreads();
-    if (wy == 0) column_sweep(s_a, s_b, s_c, s_d, K);
+    if (wy == 0) column_sweep<4>(s_a, s_b, s_c, s_d, K);
     __syncthreads();
     if (lo >= hi || !own) return;
     // the vertical and horizontal terms and the tendency of each level
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(32 * kColWarps) flat_turbw_kernel(const __grid
         }
     }
     __syncthreads();
-    if (wy == 0) column_sweep(s_a, s_b, s_c, s_d, n);
+    if (wy == 0) column_sweep<4>(s_a, s_b, s_c, s_d, n);
     __syncthreads();
     if (!own) return;
     const bool ex = i == 0 || i == ni - 1, ey = j == 0 || j == nj - 1;

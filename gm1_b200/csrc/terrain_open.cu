@@ -993,15 +993,17 @@ __global__ void __launch_bounds__(32 * kTosWarps, 3) tos_column_kernel(TosArgs p
 // pressure-gradient pass, which holds u and v.
 // Bound by load latency and the barriers around the sweep (24 warps an SM:
 // the five shared words and 80 registers allow three CTAs).  Measured on one
-// B200, per launch: flat column 640x768x80 1.583 -> 0.878 ms, uniform column
-// 256x256x80 271 -> 177 us against the phase-by-phase pass and its separate
-// open-edge launch of 11 us; 16 warps 1.007 ms, 10 warps 1.048, 4 warps 1.228,
+// B200, per launch: flat column 640x768x80 1.583 -> 0.799 ms, uniform column
+// 256x256x80 271 -> 170 us against the phase-by-phase pass and its separate
+// open-edge launch of 11 us.  With the sweep a row at a time (0.863-0.878): 16 warps 1.007 ms, 10 warps 1.048, 4 warps 1.228,
 // two CTAs an SM 1.175, four (64 registers) 1.144, four without the next
 // level's prefetch 1.179; the last phase's loads two levels at a time 0.900,
-// one 0.962.
+// one 0.962.  Prefetching the rows of the next levels into L2 made it slower
+// (1.03 ms, whatever the distance).
 // ---------------------------------------------------------------------------
 constexpr int kMarchWarps = 8;
 constexpr int kMarchArrays = 5;
+constexpr int kMarchSweep = 3;   // rows of the sweep's chunk (640x768x80 flat: 2 0.916 ms, 3 0.799, 4 0.872)
 constexpr int kMarchLevels = 4;  // levels of the last phase whose loads are issued together
 
 // the transformed face velocities of one level, and (terrain column) their
@@ -1137,6 +1139,7 @@ __device__ __forceinline__ float edge_velocity(const TosArgs &p, const Ix &X, in
 template <int VM>
 __global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(const __grid_constant__ TosArgs p) {
     extern __shared__ float sh[];
+    __shared__ float s_mm[kMarchWarps][32];  // mm of the runs' first rows
     const Ix X{p.ni, p.nj};
     const int ni = p.ni, nk = p.nk, L = nk + 2;
     const int lane = threadIdx.x, wy = threadIdx.y;
@@ -1152,7 +1155,6 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(c
     const int run = (nk + kMarchWarps - 1) / kMarchWarps;
     const int k_lo = 1 + wy * run, k_hi = min(nk, k_lo + run - 1);
     const bool busy = k_lo <= nk;
-    float f_base = 0.0f, f_mm = 0.0f, f_sum = 0.0f;  // the run's first row, completed after the barrier
     if (busy) {
         float gz = 0.0f, dzdx = 0.0f, dzdy = 0.0f, rgw = 0.0f, rge = 0.0f, rgs = 0.0f, rgn = 0.0f;
         if (VM != 2) {
@@ -1239,8 +1241,8 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(c
                 const float pd = ld.pp - ppm;
                 const float fwk = p.dts * ld.wt + p.beta * ((-mmk) * pd);
                 const float base = wk + fwk;
-                if (k == k_lo)
-                    f_base = base, f_mm = mmk, f_sum = sum;
+                if (k == k_lo)  // completed after the barrier
+                    s_dd[k * 32] = base, s_mm[wy][lane] = mmk;
                 else
                     s_dd[k * 32] = base + p.alph * ((-mmk) * (sum - summ));
             }
@@ -1266,49 +1268,15 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(c
     };
     if (busy) c_loads(k_lo);
     __syncthreads();
-    if (busy && k_lo >= 2) s_dd[k_lo * 32] = f_base + p.alph * ((-f_mm) * (f_sum - s_sum[(k_lo - 1) * 32]));
-    __syncthreads();
-    // Thomas sweep, one lane per column, as in tos_column_kernel
     if (wy == 0) {
-        float ec = 0.0f, ed = 0.0f, wn = 0.0f;
-        float aa = s_aa[2 * 32], bb = s_bb[2 * 32], cc = s_cc[2 * 32], dd = s_dd[2 * 32];
-        for (int k = 2; k <= nk; ++k) {
-            float naa = 0.0f, nbb = 0.0f, ncc = 0.0f, ndd = 0.0f;
-            if (k < nk) {
-                naa = s_aa[(k + 1) * 32];
-                nbb = s_bb[(k + 1) * 32];
-                ncc = s_cc[(k + 1) * 32];
-                ndd = s_dd[(k + 1) * 32];
-            }
-            const float piv = k == 2 ? bb : aa * ec + bb;
-            const float inv = rcp_rn(piv);
-            if (k < nk) {
-                ec = (-cc) * inv;
-                ed = (k == 2 ? dd : dd - aa * ed) * inv;
-                s_cc[k * 32] = ec;
-                s_dd[k * 32] = ed;
-            } else {
-                wn = (dd - aa * ed) * inv;
-                s_dd[k * 32] = wn;
-            }
-            aa = naa, bb = nbb, cc = ncc, dd = ndd;
-        }
-        for (int kb = nk - 1; kb >= 2; kb -= kThomasChunk) {
-            float ce[kThomasChunk], ee[kThomasChunk];
+        // the runs' first rows, which need the run below: base is in dd
 #pragma unroll
-            for (int q = 0; q < kThomasChunk; ++q) {
-                const int k = kb - q;
-                ce[q] = k >= 2 ? s_cc[k * 32] : 0.0f;
-                ee[q] = k >= 2 ? s_dd[k * 32] : 0.0f;
-            }
-#pragma unroll
-            for (int q = 0; q < kThomasChunk; ++q) {
-                const int k = kb - q;
-                if (k < 2) break;
-                wn = ce[q] * wn + ee[q];
-                s_dd[k * 32] = wn;
-            }
+        for (int r = 1; r < kMarchWarps; ++r) {
+            const int k = min(1 + r * run, nk);
+            const float sum = s_sum[k * 32], below = s_sum[(k - 1) * 32];
+            if (1 + r * run <= nk) s_dd[k * 32] = s_dd[k * 32] + p.alph * ((-s_mm[r][lane]) * (sum - below));
         }
+        column_sweep<kMarchSweep>(s_aa + 2 * 32, s_bb + 2 * 32, s_cc + 2 * 32, s_dd + 2 * 32, nk - 1);
     }
     __syncthreads();
     // pressure update, filter, halo copy, rrw average

@@ -63,7 +63,7 @@ __device__ __forceinline__ float tke_flux(const TkeArgs &a, int f, int l, int r,
 
 // dynamic shared memory: the four tridiagonal words of each of the nk-1 rows
 // of 32 columns.  256x256x80: 405 us with a thread per column (its loads a
-// level at a time, most of the chip idle), 223 here.
+// level at a time, most of the chip idle), 220 here.
 __global__ void __launch_bounds__(32 * kTurbtWarps, 3) tke_turbt_kernel(const __grid_constant__ TkeArgs a, float dt) {
     extern __shared__ float s_col[];
     const int lane = threadIdx.x, wy = threadIdx.y;
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(32 * kTurbtWarps, 3) tke_turbt_kernel(const __
         }
     }
     __syncthreads();
-    if (wy == 0) column_sweep(s_a, s_b, s_c, s_d, n);
+    if (wy == 0) column_sweep<4>(s_a, s_b, s_c, s_d, n);
     __syncthreads();
     if (f_lo > f_hi || !own) return;
     // horizontal divergence of the run's levels: the four face fluxes of the
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(32 * kTurbtWarps) tke_turbt_flat_kernel(TkeArg
         }
     }
     __syncthreads();
-    if (wy == 0) column_sweep(s_a, s_b, s_c, s_d, n);
+    if (wy == 0) column_sweep<4>(s_a, s_b, s_c, s_d, n);
     __syncthreads();
     if (!own) return;
     const int dw = i > 0 ? -1 : 0, de = i < ni - 1 ? 1 : 0, ds = j > 0 ? -ni : 0, dn = j < nj - 1 ? ni : 0;
