@@ -98,7 +98,8 @@ def test_scalar_advection(ni, nj, nk, chunk, nrk):
 
 
 @pytest.mark.parametrize("sides", [(2, 2, 2, 2), (1, 1, 1, 1)])
-@pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (32, 9, 10), (62, 11, 13), (63, 12, 33)])
+@pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (32, 9, 10), (62, 11, 13), (63, 12, 33),
+                                      (33, 800, 9), (32, 1200, 17)])
 def test_momentum_advection(ni, nj, nk, sides):
     from gm1_b200 import momentum as mom
     from oracle import momentum as orc
