@@ -115,6 +115,30 @@ def test_momentum_advection(ni, nj, nk, sides):
     assert _differ({**dev, "divx": out.divx}, ref, OUTS) == []
 
 
+@pytest.mark.parametrize("ni,nj,nk", [(31, 8, 2), (33, 9, 3), (33, 800, 9), (32, 1200, 17)])
+def test_column_marches(ni, nj, nk):
+    """Buoyancy and the post-acoustic divergences, which march two, four or
+    eight levels a thread."""
+    from gm1_b200 import moist_ops as mo
+    from oracle import moist_step as om
+    from tests.golden.make_golden import moist_piece_fixture
+
+    g = dict(ni=ni, nj=nj, nk=nk)
+    a = moist_piece_fixture(ni, nj, nk, 3 * ni + nk)
+    for n in ("divergence", "theta_divergence_term"):
+        a[n] = np.zeros((nk, nj, ni), np.float32)
+    d = _dev(a)
+    names = ("dum8", "c1", "c2", "gxu", "gyv", "uten", "vten", "wten")
+    om.moist_buoyancy(*(a[n] for n in names), **g)
+    mo.moist_buoyancy(*(d[n] for n in names), **g)
+    assert _differ(d, a, ("uten", "vten", "wten")) == []
+    om.moist_buoyancy_flat(a["dum8"], a["c1"], a["c2"], a["wten"], **g)
+    mo.moist_buoyancy_flat(d["dum8"], d["c1"], d["c2"], d["wten"], **g)
+    om.post_acoustic_flux(a, **g, dx=400.0, dy=350.0, dz=180.0)
+    mo.post_acoustic_flux(d, **g, dx=400.0, dy=350.0, dz=180.0)
+    assert _differ(d, a, ("wten", "rru", "rrv", "rrw", "divergence", "theta_divergence_term", "divx")) == []
+
+
 @pytest.mark.parametrize("flat", [False, True])
 @pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (32, 14, 11), (62, 15, 12), (7, 9, 40)])
 def test_tke_stages(ni, nj, nk, flat):
