@@ -295,3 +295,26 @@ def test_pdef_advection_is_the_chains(ni, nj, nk, obc, pdefweno, column):
     want = {k: v.cpu().numpy() for k, v in one.items()}
     assert np.count_nonzero(want["candidate"] < 0.0) > 0
     assert _differ(two, want, ("advection",)) == []
+
+
+@pytest.mark.parametrize("nrk", [1, 3])
+@pytest.mark.parametrize("ni,nj,nk", [(8, 8, 8), (9, 33, 9), (34, 9, 12), (65, 10, 17)])
+def test_advection_adjoint_in_one_pass(ni, nj, nk, nrk):
+    """An output that overlaps the tendency adjoint takes the two passes over
+    the face scratch: the fifth-order words are those of the one pass; and the
+    edge cells sum the carrier adjoint's words."""
+    from gm1_b200 import adjoint as adj
+    from tests.test_adjoint_gpu import _flow, warm_rain_case
+
+    state, fr, g = warm_rain_case(ni=ni, nj=nj, nk=nk, seed=ni + nk)
+    flow = _flow(fr, g)
+    s, rng = _t(state["qv"]), np.random.default_rng(nj)
+    lam = _t(rng.standard_normal((nk, nj, ni)))
+    got = adj.advection_tendency_adjoint(flow, s, lam, nrk)
+    in_place = lam.clone()
+    assert torch.equal(adj.advection_tendency_adjoint(flow, s, in_place, nrk, out=in_place), got)
+    padded = adj.advection_carrier_adjoint(flow, adj._carrier(flow, s), lam, nrk)
+    assert torch.equal(padded[1:-1, 4:-4, 4:-4], got[:, 1:-1, 1:-1])
+    west = padded[1:-1, 4:-4, :4].double().sum(-1)
+    # four float32 words of at most the largest one's size
+    assert torch.allclose(west, got[:, 1:-1, 0].double(), rtol=0.0, atol=float(padded.abs().max()) * 2.0 ** -21)
