@@ -7,7 +7,10 @@ every operator raises.  Build it with ``python -m gm1_b200.csrc.build``.
 from __future__ import annotations
 
 import ctypes
+from contextlib import nullcontext
 from pathlib import Path
+
+import torch
 
 from .arrays import ALL_ARRAY_NAMES
 
@@ -47,6 +50,17 @@ _lib: ctypes.CDLL | None = None
 
 class Gm1bError(RuntimeError):
     """A libgm1b.so entry point returned a non-zero status."""
+
+
+def device_guard(device: torch.device):
+    """torch.cuda.device(device), or nothing where it is the current device
+    already (the guard's own calls cost more than a small launch's)."""
+    return nullcontext() if device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
+
+
+def raw_stream(device: torch.device) -> ctypes.c_void_p:
+    """The current stream of a CUDA tensor's device."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(device.index))
 
 
 def lib() -> ctypes.CDLL:

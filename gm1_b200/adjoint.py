@@ -45,7 +45,7 @@ import torch
 import torch.utils.checkpoint
 
 from . import _native
-from .advection import launch_cuda_scalar_advection5, padded_shapes
+from .advection import enqueue_scalar_advection5, padded_shapes
 from .autotune import Autotuner
 from .periodic import rk_stage_dt_f32
 
@@ -96,8 +96,7 @@ def _ptr(t: torch.Tensor, name: str) -> int:
     return t.data_ptr()
 
 
-def _stream(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+_stream = _native.raw_stream
 
 
 @dataclass(frozen=True)
@@ -137,7 +136,7 @@ OBC_OPEN = 0x2222
 def _tendency(flow: FrozenFlow, padded: torch.Tensor, nrk: int, weps: float, chunk: int | None = None) -> torch.Tensor:
     f = flow.fields
     ten = torch.empty((flow.nk, flow.nj, flow.ni), dtype=torch.float32, device=padded.device)
-    launch_cuda_scalar_advection5(
+    enqueue_scalar_advection5(
         padded, {n: f[n] for n in FLUX_NAMES}, {n: f[n] for n in ("c1", "c2", "rr0", "gz")}, f["divx"], ten, None,
         ni=flow.ni, nj=flow.nj, nk=flow.nk, nrk=nrk, dx=flow.dx, dy=flow.dy, dz=flow.dz, weps=weps,
         lateral_sides=LATERAL_OPEN, write_fluxes=False, levels_per_chunk=chunk)

@@ -142,7 +142,7 @@ def _validated_spacing(name: str, value: float) -> float:
 def _require(value: Any, name: str, shape: tuple[int, ...]) -> torch.Tensor:
     if not isinstance(value, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
-    if not value.is_cuda or value.dtype != torch.float32 or tuple(value.shape) != shape or not value.is_contiguous():
+    if not value.is_cuda or value.dtype != torch.float32 or value.shape != shape or not value.is_contiguous():
         raise ValueError(f"{name} must be a contiguous float32 CUDA tensor of shape {shape}")
     return value
 
@@ -230,19 +230,15 @@ def launch_cuda_terrain_mass_flux5(
     return CudaLaunch(ev, {"operation": "terrain-mass-flux-and-divergence", "domain": {"ni": ni, "nj": nj, "nk": nk}})
 
 
-def launch_cuda_scalar_advection5(
+def enqueue_scalar_advection5(
     scalar: Any, arrays: Mapping[str, Any], metrics: Mapping[str, Any], divx: Any, tendency: Any,
     fluxes: Mapping[str, Any] | None, *, ni: int, nj: int, nk: int, nrk: int, dx: float, dy: float, dz: float,
     weps: float, wflag: bool = True, selection: Advection5Selection = DEFAULT_ADVECTION5_SELECTION,
     stream: Any | None = None, lateral_sides: tuple[int, int, int, int] | None = None,
     write_fluxes: bool = True, levels_per_chunk: int | None = None,
-) -> CudaLaunch:
-    """Enqueue one scalar's fifth-order/WENO5 tendency for RK stage ``nrk``.
-
-    ``lateral_sides`` is CM1's (wbc, ebc, sbc, nbc) of a whole-domain launch;
-    None is a tile-local launch whose outer three cells are not written.
-    ``write_fluxes`` also stores the face fluxes into ``fluxes`` x/y/z as the
-    reference does; False skips those HBM writes (``fluxes`` may be None)."""
+) -> tuple[bool, int]:
+    """The checks and the launch of launch_cuda_scalar_advection5 without its
+    event; (weno, packed sides)."""
     use_weno = scalar_advection_uses_weno(nrk, wflag=wflag, selection=selection)
     _validated_grid(ni, nj, nk)
     dx, dy, dz = (_validated_spacing(n, v) for n, v in (("dx", dx), ("dy", dy), ("dz", dz)))
@@ -270,13 +266,35 @@ def launch_cuda_scalar_advection5(
     _no_alias(list(a.values()), "scalar advection inputs, flux scratch, and tendency")
     s = _ScalarAdvArrays(**{n: t.data_ptr() for n, t in a.items()})
     device = a["scalar"].device
-    st = torch.cuda.current_stream(device) if stream is None else stream
-    with torch.cuda.device(device):
+    st = _native.raw_stream(device) if stream is None else ctypes.c_void_p(stream.cuda_stream)
+    with _native.device_guard(device):
         _native.check(_bind().gm1b_scalar_advection5(ni, nj, nk, ctypes.byref(s), nrk, 1 if wflag else 0, dx, dy, dz,
-                                                     weps, obc, int(levels_per_chunk or 0),
-                                                     ctypes.c_void_p(st.cuda_stream)), "gm1b_scalar_advection5")
+                                                     weps, obc, int(levels_per_chunk or 0), st),
+                      "gm1b_scalar_advection5")
+    return use_weno, obc
+
+
+def launch_cuda_scalar_advection5(
+    scalar: Any, arrays: Mapping[str, Any], metrics: Mapping[str, Any], divx: Any, tendency: Any,
+    fluxes: Mapping[str, Any] | None, *, ni: int, nj: int, nk: int, nrk: int, dx: float, dy: float, dz: float,
+    weps: float, wflag: bool = True, selection: Advection5Selection = DEFAULT_ADVECTION5_SELECTION,
+    stream: Any | None = None, lateral_sides: tuple[int, int, int, int] | None = None,
+    write_fluxes: bool = True, levels_per_chunk: int | None = None,
+) -> CudaLaunch:
+    """Enqueue one scalar's fifth-order/WENO5 tendency for RK stage ``nrk``.
+
+    ``lateral_sides`` is CM1's (wbc, ebc, sbc, nbc) of a whole-domain launch;
+    None is a tile-local launch whose outer three cells are not written.
+    ``write_fluxes`` also stores the face fluxes into ``fluxes`` x/y/z as the
+    reference does; False skips those HBM writes (``fluxes`` may be None)."""
+    use_weno, obc = enqueue_scalar_advection5(
+        scalar, arrays, metrics, divx, tendency, fluxes, ni=ni, nj=nj, nk=nk, nrk=nrk, dx=dx, dy=dy, dz=dz, weps=weps,
+        wflag=wflag, selection=selection, stream=stream, lateral_sides=lateral_sides, write_fluxes=write_fluxes,
+        levels_per_chunk=levels_per_chunk)
+    device = scalar.device
+    with _native.device_guard(device):
         ev = torch.cuda.Event()
-        ev.record(st)
+        ev.record(torch.cuda.current_stream(device) if stream is None else stream)
     return CudaLaunch(ev, {"operation": "scalar-advection5", "nrk": nrk, "weno": use_weno, "lateral_obc": obc})
 
 
