@@ -17,18 +17,18 @@
 // (--fmad=false); open sides are index clamps (the twins' edge padding).
 //
 // Design as csrc/stress.cu: elementwise grid-stride passes for the strain
-// and gettau, one thread per staggered column (32 x 4 columns per CTA, the
-// Thomas coefficients in shared memory [level][thread]) for the implicit
-// solves, the horizontal terms and the cross term formed in the back
-// substitution; turbs forms its x/y fluxes of every scalar in one pass into
-// the workspace (their w-level interpolation is read back there), then solves
-// each column.
+// and gettau, a CTA of eight warps per 32 columns for the implicit solves
+// (rows formed by all warps, swept in shared memory by one), the horizontal
+// terms and the cross term formed with the tendency; turbs forms its x/y
+// fluxes of every scalar in one pass into the workspace (their w-level
+// interpolation is read back there), then solves each column.
 #include "gm1b_common.cuh"
 
 namespace gm1b {
 namespace {
 
-constexpr int kCX = 32, kCY = 4, kCT = kCX * kCY;
+constexpr int kColWarps = 8;    // warps of a column solve's CTA, which owns 32 columns of a row
+constexpr int kTurbsGroup = 4;  // scalars the turbs column pass solves together
 constexpr int kEW = 256;
 
 #define TRY(x)                        \
@@ -204,66 +204,74 @@ __global__ void __launch_bounds__(kEW) terrain_gettau_kernel(TArgs a) {
 }
 
 // ------------------------------------------------------- turbu and turbv
+// A CTA owns 32 columns of a row: its warps form the tridiagonal rows of their
+// own runs of levels in shared memory, one warp sweeps them, then all warps
+// add the tendencies of their levels.  256x256x80 against a thread per column,
+// its loads a level at a time: turbu 615 -> 246 us, turbv 596 -> 243, turbw 386
+// -> 107 (24 warps an SM 339, 285 and 125).
 template <int DIR>
-__global__ void __launch_bounds__(kCT) terrain_turb_uv_kernel(TArgs a) {
+__global__ void __launch_bounds__(32 * kColWarps, 4) terrain_turb_uv_kernel(const __grid_constant__ TArgs a) {
     extern __shared__ float s_col[];
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kCX + tx;
+    const int lane = threadIdx.x, wy = threadIdx.y;
     const int ni = a.ni, nj = a.nj, nk = a.nk, ux = ni + 1, vy = nj + 1;
-    const int cx = blockIdx.x * kCX + tx, cy = blockIdx.y * kCY + ty;
-    if (DIR == 0 ? (cx > ni || cy >= nj) : (cx >= ni || cy > nj)) return;
+    const int nx = DIR == 0 ? ux : ni, tiles = (nx + 31) / 32;
+    const int c0 = blockIdx.x % tiles * 32 + lane, cy = blockIdx.x / tiles;
+    const bool own = c0 < nx;
+    const int cx = min(c0, nx - 1);  // lanes past the row's end repeat its last column and store nothing
     // DIR 0: u column (j = cy, iface = cx), cells (j, cx-1), (j, cx); DIR 1: v column (jface = cy, i = cx)
     const int ja = DIR == 0 ? cy : cy - 1, jb = cy, ia = DIR == 0 ? cx - 1 : cx, ib = cx;
     const float *q = DIR == 0 ? a.u : a.v, *top = DIR == 0 ? a.t13 : a.t23;
     float *ten = DIR == 0 ? a.uten : a.vten;
-    const unsigned col = DIR == 0 ? (unsigned)cy * ux + cx : (unsigned)cy * ni + cx;
+    const unsigned col = (unsigned)cy * nx + cx;
     const unsigned lev = DIR == 0 ? (unsigned)nj * ux : (unsigned)vy * ni;
     const float rdx = 1.0f / a.dx, rdy = 1.0f / a.dy, dz = a.dz, dt = a.dt, rdz = 1.0f / dz, zt = (float)nk * dz;
     const float rd = DIR == 0 ? rdx : rdy;
     const float tema = -0.0625f * (dt * (rdz * rdz)), temc = 0.5f * (dt * rdz), rdt = 0.5f / dt;
-    float *cp = s_col, *dp = s_col + (size_t)nk * kCT;
-#define CP(k) cp[(unsigned)(k) * kCT + tid]
-#define DP(k) dp[(unsigned)(k) * kCT + tid]
+    float *s_a = s_col + lane, *s_b = s_a + nk * 32, *s_c = s_b + nk * 32, *s_d = s_c + nk * 32;
 #define PAIR(p, k) (c3(a, p, k, ja, ia) + c3(a, p, k, jb, ib))
 #define QK(k) q[(unsigned)(k) * lev + col]
 #define WA(k) a.w[o3(k, cl(ja, nj), cl(ia, ni), nj, ni)]
 #define WB(k) a.w[o3(k, cl(jb, nj), cl(ib, ni), nj, ni)]
     const float rg_a = c2(a, a.rgz, ja, ia), rg_b = c2(a, a.rgz, jb, ib);
     const float gza = c2(a, a.gz, ja, ia), gzb = c2(a, a.gz, jb, ib);
-    // forward elimination
-    float kmv_u = PAIR(a.kmv, 1), mf_u = PAIR(a.mf, 1), rf_u = PAIR(a.rf, 1);
-    {
-        const float rr0 = 1.0f / (0.5f * PAIR(a.rho, 0)), mhp = PAIR(a.mh, 0);
-        const float r2v = kmv_u * (mf_u * (rf_u * (mhp * rr0)));
-        const float cfc = tema * r2v, cfb = 1.0f - cfc, cfd = QK(0) - temc * (top[col] * (mhp * rr0));
-        const float inv = 1.0f / cfb;
-        CP(0) = -1.0f * (cfc * inv);
-        DP(0) = cfd * inv;
+    const int run = (nk + kColWarps - 1) / kColWarps;
+    const int lo = min(wy * run, nk), hi = min(lo + run, nk);
+    if (lo < hi) {
+        float kmv_l = lo > 0 ? PAIR(a.kmv, lo) : 0.0f, mf_l = lo > 0 ? PAIR(a.mf, lo) : 0.0f;
+        float rf_l = lo > 0 ? PAIR(a.rf, lo) : 0.0f;
+#pragma unroll 2
+        for (int k = lo; k < hi; ++k) {
+            const bool more = k + 1 < nk;
+            const float kmv_u = more ? PAIR(a.kmv, k + 1) : 0.0f, mf_u = more ? PAIR(a.mf, k + 1) : 0.0f;
+            const float rf_u = more ? PAIR(a.rf, k + 1) : 0.0f;
+            const float rr0 = 1.0f / (0.5f * PAIR(a.rho, k)), common = PAIR(a.mh, k) * rr0;
+            const float r1v = kmv_l * (mf_l * (rf_l * common)), r2v = kmv_u * (mf_u * (rf_u * common));
+            const float cfa = tema * r1v, cfc = tema * r2v;
+            float cfb = (1.0f - cfa) - cfc, cfd = QK(k);
+            if (k == 0) {
+                cfb = 1.0f - cfc;
+                cfd = cfd - temc * (top[col] * common);
+            } else if (k == nk - 1) {
+                cfb = 1.0f - cfa;
+                cfd = cfd + temc * (top[(unsigned)nk * lev + col] * common);
+            }
+            s_a[k * 32] = cfa, s_b[k * 32] = cfb, s_c[k * 32] = cfc, s_d[k * 32] = cfd;
+            kmv_l = kmv_u, mf_l = mf_u, rf_l = rf_u;
+        }
     }
-    float cprev = CP(0), dprev = DP(0);
-    #pragma unroll 4
-    for (int k = 1; k < nk - 1; ++k) {
-        const float rr0 = 1.0f / (0.5f * PAIR(a.rho, k)), common = PAIR(a.mh, k) * rr0;
-        const float r1v = kmv_u * (mf_u * (rf_u * common));
-        kmv_u = PAIR(a.kmv, k + 1);
-        mf_u = PAIR(a.mf, k + 1);
-        rf_u = PAIR(a.rf, k + 1);
-        const float r2v = kmv_u * (mf_u * (rf_u * common));
-        const float cfa = tema * r1v, cfc = tema * r2v, cfb = (1.0f - cfa) - cfc;
-        const float inv = 1.0f / (cfa * cprev + cfb);
-        cprev = -1.0f * (cfc * inv);
-        dprev = (QK(k) - cfa * dprev) * inv;
-        CP(k) = cprev;
-        DP(k) = dprev;
-    }
-    float sol;
-    {
-        const int k = nk - 1;
-        const float rr0 = 1.0f / (0.5f * PAIR(a.rho, k)), mhp = PAIR(a.mh, k);
-        const float r1v = kmv_u * (mf_u * (rf_u * (mhp * rr0)));
-        const float cfa = tema * r1v, cfb = 1.0f - cfa;
-        const float cfd = QK(k) + temc * (top[(unsigned)nk * lev + col] * (mhp * rr0));
-        sol = (cfd - cfa * dprev) * (1.0f / (cfa * cprev + cfb));
-    }
+    __syncthreads();
+    if (wy == 0) column_sweep<4>(s_a, s_b, s_c, s_d, nk);
+    __syncthreads();
+    if (lo >= hi || !own) return;
+    auto cross_at = [&](int k) {
+        if (k < 1 || k >= nk) return 0.0f;
+        const float wm = 0.5f * (WB(k) + WB(k + 1)), wl = 0.5f * (WA(k) + WA(k + 1));
+        const float grad = (WB(k) * rg_b - WA(k) * rg_a) * rd;
+        const float below = 0.5f * (WB(k - 1) + WB(k)) + 0.5f * (WA(k - 1) + WA(k));
+        const float terrain = 0.5f * (((zt - ((float)k + 0.5f) * dz) * (wm + wl) - (zt - ((float)k - 0.5f) * dz) * below) *
+                                      (rdz * ((rg_b - rg_a) * rd)));
+        return (grad + terrain) * (0.25f * (PAIR(a.kmv, k) * (gza * c3(a, a.rf, k, ja, ia) + gzb * c3(a, a.rf, k, jb, ib))));
+    };
     // back substitution, the cross term and the tendency per level
     float r1 = 0.0f, r2 = 0.0f;
     if (DIR == 0) {
@@ -274,19 +282,9 @@ __global__ void __launch_bounds__(kCT) terrain_turb_uv_kernel(TArgs a) {
         r2 = 0.25f * ((c2(a, a.rgz, ja, cx + 1) + c2(a, a.rgz, jb, cx)) + (c2(a, a.rgz, jb, cx + 1) + c2(a, a.rgz, ja, cx)));
     }
     const float g = DIR == 0 ? a.gzu[(unsigned)cy * ux + cx] : a.gzv[(unsigned)cy * ni + cx];
-    float cross_up = 0.0f;  // cross(k+1); zero above the top level
-    #pragma unroll 4
-    for (int k = nk - 1; k >= 0; --k) {
-        if (k < nk - 1) sol = CP(k) * sol + DP(k);
-        float cross = 0.0f;
-        if (k >= 1) {
-            const float wm = 0.5f * (WB(k) + WB(k + 1)), wl = 0.5f * (WA(k) + WA(k + 1));
-            const float grad = (WB(k) * rg_b - WA(k) * rg_a) * rd;
-            const float below = 0.5f * (WB(k - 1) + WB(k)) + 0.5f * (WA(k - 1) + WA(k));
-            const float terrain = 0.5f * (((zt - ((float)k + 0.5f) * dz) * (wm + wl) - (zt - ((float)k - 0.5f) * dz) * below) *
-                                          (rdz * ((rg_b - rg_a) * rd)));
-            cross = (grad + terrain) * (0.25f * (PAIR(a.kmv, k) * (gza * c3(a, a.rf, k, ja, ia) + gzb * c3(a, a.rf, k, jb, ib))));
-        }
+    float cross = cross_at(lo);
+    for (int k = lo; k < hi; ++k) {
+        const float cross_up = cross_at(k + 1);  // zero above the top level
         float hx, hy;
         if (DIR == 0) {
             const float x = g * ((c3(a, a.t11, k, cy, ib) * rg_b - c3(a, a.t11, k, cy, ia) * rg_a) * rdx);
@@ -312,14 +310,12 @@ __global__ void __launch_bounds__(kCT) terrain_turb_uv_kernel(TArgs a) {
             if (cy == 0 || cy == nj) hy = 0.0f;
         }
         const float rho_p = PAIR(a.rho, k), mhp = PAIR(a.mh, k);
-        float vert = rho_p * ((sol - QK(k)) * rdt);
+        float vert = rho_p * ((s_d[k * 32] - QK(k)) * rdt);
         vert = vert + (cross_up - cross) * (rdz * (0.5f * mhp));
-        cross_up = cross;
+        cross = cross_up;
         const unsigned p = (unsigned)k * lev + col;
         ten[p] = ten[p] + ((hx + hy) + vert) / (0.5f * rho_p);
     }
-#undef CP
-#undef DP
 #undef PAIR
 #undef QK
 #undef WA
@@ -327,55 +323,49 @@ __global__ void __launch_bounds__(kCT) terrain_turb_uv_kernel(TArgs a) {
 }
 
 // ----------------------------------------------------------------- turbw
-__global__ void __launch_bounds__(kCT) terrain_turbw_kernel(TArgs a) {
+__global__ void __launch_bounds__(32 * kColWarps, 4) terrain_turbw_kernel(const __grid_constant__ TArgs a) {
     extern __shared__ float s_col[];
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kCX + tx;
-    const int ni = a.ni, nj = a.nj, nk = a.nk, ux = ni + 1, vy = nj + 1;
-    const int i = blockIdx.x * kCX + tx, j = blockIdx.y * kCY + ty;
-    if (i >= ni || j >= nj) return;
+    const int lane = threadIdx.x, wy = threadIdx.y;
+    const int ni = a.ni, nj = a.nj, nk = a.nk, n = nk - 1, ux = ni + 1, vy = nj + 1, tiles = (ni + 31) / 32;
+    const int i0 = blockIdx.x % tiles * 32 + lane, j = blockIdx.x / tiles;
+    const bool own = i0 < ni;
+    const int i = min(i0, ni - 1);  // lanes past the row's end repeat its last column and store nothing
     const unsigned col = (unsigned)j * ni + i, lev = (unsigned)nj * ni;
     const float rdx = 1.0f / a.dx, rdy = 1.0f / a.dy, dz = a.dz, dt = a.dt, rdz = 1.0f / dz, zt = (float)nk * dz;
     const float tema = -1.0f * (dt * (rdz * rdz)), temc = dt * rdz, rdt = 1.0f / dt;
-    float *cp = s_col, *dp = s_col + (size_t)nk * kCT;
-#define CP(p) cp[(unsigned)(p) * kCT + tid]
-#define DP(p) dp[(unsigned)(p) * kCT + tid]
+    float *s_a = s_col + lane, *s_b = s_a + n * 32, *s_c = s_b + n * 32, *s_d = s_c + n * 32;  // rows f - 1
 #define PF(p, f) p[(unsigned)(f) * lev + col]
 #define T13(f, ii) a.t13[o3(f, j, ii, nj, ux)]
 #define T23(f, jj) a.t23[o3(f, jj, i, vy, ni)]
-    {
-        const int f = 1;
-        const float rrf = PF(a.mf, f) / PF(a.rf, f);
-        const float r2v = (PF(a.kmh, f) + PF(a.kmh, f + 1)) * (PF(a.mh, f) * (PF(a.rho, f) * rrf));
-        const float cfc = tema * r2v, cfb = 1.0f - cfc, cfd = PF(a.w, f) - temc * (PF(a.t33, 0) * rrf);
-        const float inv = 1.0f / cfb;
-        CP(0) = -1.0f * (cfc * inv);
-        DP(0) = cfd * inv;
+    const int run = (n + kColWarps - 1) / kColWarps;
+    const int lo = min(1 + wy * run, nk), hi = min(lo + run, nk);  // faces lo .. hi-1
+    if (lo < hi) {
+        float km = PF(a.kmh, lo - 1), k0 = PF(a.kmh, lo), mhm = PF(a.mh, lo - 1), rhom = PF(a.rho, lo - 1);
+#pragma unroll 2
+        for (int f = lo; f < hi; ++f) {
+            const float rrf = PF(a.mf, f) / PF(a.rf, f);
+            const float kp = PF(a.kmh, f + 1), mh = PF(a.mh, f), rho = PF(a.rho, f);
+            const float r1v = (km + k0) * (mhm * (rhom * rrf)), r2v = (k0 + kp) * (mh * (rho * rrf));
+            const float cfa = tema * r1v, cfc = tema * r2v;
+            float cfb = (1.0f - cfa) - cfc, cfd = PF(a.w, f);
+            if (f == 1) {
+                cfb = 1.0f - cfc;
+                cfd = cfd - temc * (PF(a.t33, 0) * rrf);
+            } else if (f == n) {
+                cfb = 1.0f - cfa;
+                cfd = cfd + temc * (PF(a.t33, nk - 1) * rrf);
+            }
+            const int p = (f - 1) * 32;
+            s_a[p] = cfa, s_b[p] = cfb, s_c[p] = cfc, s_d[p] = cfd;
+            km = k0, k0 = kp, mhm = mh, rhom = rho;
+        }
     }
-    float cprev = CP(0), dprev = DP(0);
-    #pragma unroll 4
-    for (int f = 2; f < nk - 1; ++f) {
-        const float rrf = PF(a.mf, f) / PF(a.rf, f);
-        const float r1v = (PF(a.kmh, f - 1) + PF(a.kmh, f)) * (PF(a.mh, f - 1) * (PF(a.rho, f - 1) * rrf));
-        const float r2v = (PF(a.kmh, f) + PF(a.kmh, f + 1)) * (PF(a.mh, f) * (PF(a.rho, f) * rrf));
-        const float cfa = tema * r1v, cfc = tema * r2v, cfb = (1.0f - cfa) - cfc;
-        const float inv = 1.0f / (cfa * cprev + cfb);
-        cprev = -1.0f * (cfc * inv);
-        dprev = (PF(a.w, f) - cfa * dprev) * inv;
-        CP(f - 1) = cprev;
-        DP(f - 1) = dprev;
-    }
-    float sol;
-    {
-        const int f = nk - 1;
-        const float rrf = PF(a.mf, f) / PF(a.rf, f);
-        const float r1v = (PF(a.kmh, f - 1) + PF(a.kmh, f)) * (PF(a.mh, f - 1) * (PF(a.rho, f - 1) * rrf));
-        const float cfa = tema * r1v, cfb = 1.0f - cfa, cfd = PF(a.w, f) + temc * (PF(a.t33, nk - 1) * rrf);
-        sol = (cfd - cfa * dprev) * (1.0f / (cfa * cprev + cfb));
-    }
+    __syncthreads();
+    if (wy == 0) column_sweep<4>(s_a, s_b, s_c, s_d, n);
+    __syncthreads();
+    if (!own) return;
     const float g = a.gz[col];
-    #pragma unroll 4
-    for (int f = nk - 1; f >= 1; --f) {
-        if (f < nk - 1) sol = CP(f - 1) * sol + DP(f - 1);
+    for (int f = lo; f < hi; ++f) {
         const float d1 = 0.25f * ((T13(f + 1, i) + T13(f + 1, i + 1)) + (T13(f, i) + T13(f, i + 1)));
         const float d0 = 0.25f * ((T13(f, i) + T13(f, i + 1)) + (T13(f - 1, i) + T13(f - 1, i + 1)));
         float x = g * ((T13(f, i + 1) * a.rgzu[j * ux + i + 1] - T13(f, i) * a.rgzu[j * ux + i]) * rdx);
@@ -388,12 +378,10 @@ __global__ void __launch_bounds__(kCT) terrain_turbw_kernel(TArgs a) {
                     (g * ((a.rgzv[(j + 1) * ni + i] - a.rgzv[j * ni + i]) * (rdy * rdz)));
         const float h = (i == 0 || i == ni - 1 ? 0.0f : x) + (j == 0 || j == nj - 1 ? 0.0f : y);
         const float rff = PF(a.rf, f);
-        const float vert = rff * ((sol - PF(a.w, f)) * rdt);
+        const float vert = rff * ((s_d[(f - 1) * 32] - PF(a.w, f)) * rdt);
         const unsigned p = (unsigned)f * lev + col;
         a.wten[p] = a.wten[p] + (h + vert) / rff;
     }
-#undef CP
-#undef DP
 #undef PF
 #undef T13
 #undef T23
@@ -433,41 +421,48 @@ __device__ __forceinline__ float *fx_of(const SArgs &a, int sc) {
 }
 __device__ __forceinline__ float *fy_of(const SArgs &a, int sc) { return fx_of(a, sc) + (size_t)a.nk * a.nj * (a.ni + 1); }
 
-__global__ void __launch_bounds__(kEW) terrain_turbs_flux_kernel(SArgs a) {
-    const int ni = a.ni, nj = a.nj, nk = a.nk, ux = ni + 1, vy = nj + 1;
+// A thread owns the west x face and south y face (face, row) of a cell and
+// marches a chunk of levels for one scalar at a time, the two cells' face
+// values (sw) of the level below carried up; the faces beyond the last cells
+// belong to one more column and row of threads.  256x256x80, four scalars:
+// 1139 -> 385 us against a thread per face from a divided linear index.
+__global__ void __launch_bounds__(256, 4) terrain_turbs_flux_kernel(const __grid_constant__ SArgs a, int chunk) {
+    const int ni = a.ni, nj = a.nj, nk = a.nk, ux = ni + 1, vy = nj + 1, tiles = (ux + 31) / 32;
+    const int x = blockIdx.x % tiles * 32 + threadIdx.x, y = blockIdx.x / tiles * 8 + threadIdx.y;
+    if (x > ni || y > nj) return;
     const float rdx = 1.0f / a.dx, rdy = 1.0f / a.dy, rdz = 1.0f / a.dz;
-    const size_t nxf = (size_t)nk * nj * ux, nyf = (size_t)nk * vy * ni, total = nxf + nyf;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
-        if (q < nxf) {
-            const int face = (int)(q % ux), j = (int)((q / ux) % nj), k = (int)(q / ((size_t)ux * nj));
-            const int il = face - 1, ir = face;
-            const float den = sc2(a, a.gz, j, ir) * sc3(a, a.rho, k, j, ir) + sc2(a, a.gz, j, il) * sc3(a, a.rho, k, j, il);
-            const float dif = (sc3(a, a.khh, k, j, ir) + sc3(a, a.khh, k, j, il)) + (sc3(a, a.khh, k + 1, j, ir) + sc3(a, a.khh, k + 1, j, il));
-            const float fac = (-0.125f * den) * dif;
-            const float rr_ = sc2(a, a.rgz, j, ir), rl_ = sc2(a, a.rgz, j, il);
-            const float gu = a.gxu[o3(k + 1, j, face, nj, ux)], gl = a.gxu[o3(k, j, face, nj, ux)], rzu = a.rgzu[j * ux + face];
-            for (int sc = 0; sc < a.nsc; ++sc) {
-                const float hor = (sv(a, sc, k, j, ir) * rr_ - sv(a, sc, k, j, il) * rl_) * rdx;
-                const float up = gu * (sw(a, sc, k + 1, j, ir) + sw(a, sc, k + 1, j, il));
-                const float lo = gl * (sw(a, sc, k, j, ir) + sw(a, sc, k, j, il));
-                const float ter = ((0.5f * (up - lo)) * rdz) * rzu;
-                fx_of(a, sc)[q] = fac * (hor + ter);
-            }
-        } else {
-            const size_t z = q - nxf;
-            const int i = (int)(z % ni), face = (int)((z / ni) % vy), k = (int)(z / ((size_t)ni * vy));
-            const int js = face - 1, jn = face;
-            const float den = sc2(a, a.gz, jn, i) * sc3(a, a.rho, k, jn, i) + sc2(a, a.gz, js, i) * sc3(a, a.rho, k, js, i);
-            const float dif = (sc3(a, a.khh, k, jn, i) + sc3(a, a.khh, k, js, i)) + (sc3(a, a.khh, k + 1, jn, i) + sc3(a, a.khh, k + 1, js, i));
-            const float fac = (-0.125f * den) * dif;
-            const float rn_ = sc2(a, a.rgz, jn, i), rs_ = sc2(a, a.rgz, js, i);
-            const float gu = a.gyv[o3(k + 1, face, i, vy, ni)], gl = a.gyv[o3(k, face, i, vy, ni)], rzv = a.rgzv[face * ni + i];
-            for (int sc = 0; sc < a.nsc; ++sc) {
-                const float hor = (sv(a, sc, k, jn, i) * rn_ - sv(a, sc, k, js, i) * rs_) * rdy;
-                const float up = gu * (sw(a, sc, k + 1, jn, i) + sw(a, sc, k + 1, js, i));
-                const float lo = gl * (sw(a, sc, k, jn, i) + sw(a, sc, k, js, i));
-                const float ter = ((0.5f * (up - lo)) * rdz) * rzv;
-                fy_of(a, sc)[z] = fac * (hor + ter);
+    const int k_lo = blockIdx.y * chunk, k_hi = min(nk, k_lo + chunk);
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir) {
+        if (dir == 0 ? y >= nj : x >= ni) continue;
+        // the cells r and l either side of the face
+        const int jr = y, ir = x, jl = dir == 0 ? y : y - 1, il = dir == 0 ? x - 1 : x;
+        const float gr = sc2(a, a.gz, jr, ir), gl = sc2(a, a.gz, jl, il), rgr = sc2(a, a.rgz, jr, ir), rgl = sc2(a, a.rgz, jl, il);
+        const float *slope = dir == 0 ? a.gxu : a.gyv;
+        const int ny = dir == 0 ? nj : vy, nx = dir == 0 ? ux : ni;
+        const float rz = dir == 0 ? a.rgzu[y * ux + x] : a.rgzv[y * ni + x], rd = dir == 0 ? rdx : rdy;
+        for (int sc = 0; sc < a.nsc; ++sc) {
+            float *out = dir == 0 ? fx_of(a, sc) : fy_of(a, sc);
+            float khr = sc3(a, a.khh, k_lo, jr, ir), khl = sc3(a, a.khh, k_lo, jl, il);
+            float lower = slope[o3(k_lo, y, x, ny, nx)] * (sw(a, sc, k_lo, jr, ir) + sw(a, sc, k_lo, jl, il));
+            float sr = sv(a, sc, k_lo, jr, ir), sl = sv(a, sc, k_lo, jl, il);
+#pragma unroll 2
+            for (int k = k_lo; k < k_hi; ++k) {
+                const float nkr = sc3(a, a.khh, k + 1, jr, ir), nkl = sc3(a, a.khh, k + 1, jl, il);
+                const float den = gr * sc3(a, a.rho, k, jr, ir) + gl * sc3(a, a.rho, k, jl, il);
+                const float fac = (-0.125f * den) * ((khr + khl) + (nkr + nkl));
+                const float hor = (sr * rgr - sl * rgl) * rd;
+                float nr = 0.0f, nl = 0.0f, at_r, at_l;  // the face values above
+                if (k + 1 < nk) {
+                    nr = sv(a, sc, k + 1, jr, ir), nl = sv(a, sc, k + 1, jl, il);
+                    at_r = 0.5f * sr + 0.5f * nr, at_l = 0.5f * sl + 0.5f * nl;
+                } else {
+                    at_r = sw(a, sc, nk, jr, ir), at_l = sw(a, sc, nk, jl, il);
+                }
+                const float upper = slope[o3(k + 1, y, x, ny, nx)] * (at_r + at_l);
+                const float ter = ((0.5f * (upper - lower)) * rdz) * rz;
+                out[o3(k, y, x, ny, nx)] = fac * (hor + ter);
+                khr = nkr, khl = nkl, lower = upper, sr = nr, sl = nl;
             }
         }
     }
@@ -480,92 +475,138 @@ __device__ __forceinline__ float fw(const float *col, size_t stride, int f, int 
     return 0.5f * col[(f - 1) * stride] + 0.5f * col[f * stride];
 }
 
-__global__ void __launch_bounds__(kCT) terrain_turbs_column_kernel(SArgs a) {
+// The matrix and its reciprocals are the same for every scalar: formed and
+// swept once a column, then a warp per scalar of the group sweeps its right
+// side (the flat column's solve, with the terrain's flux divergence).
+// 256x256x80, four scalars: 1572 -> 693 us against a thread per column solving
+// each scalar's own matrix.
+__global__ void __launch_bounds__(32 * kColWarps, 3) terrain_turbs_column_kernel(const __grid_constant__ SArgs a) {
     extern __shared__ float s_col[];
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kCX + tx;
-    const int ni = a.ni, nj = a.nj, nk = a.nk, ux = ni + 1, vy = nj + 1;
-    const int i = blockIdx.x * kCX + tx, j = blockIdx.y * kCY + ty;
-    if (i >= ni || j >= nj) return;
+    const int lane = threadIdx.x, wy = threadIdx.y;
+    const int ni = a.ni, nj = a.nj, nk = a.nk, ux = ni + 1, vy = nj + 1, tiles = (ni + 31) / 32;
+    const int i0 = blockIdx.x % tiles * 32 + lane, j = blockIdx.x / tiles;
+    const bool own = i0 < ni;
+    const int i = min(i0, ni - 1);  // lanes past the row's end repeat its last column and store nothing
     const size_t n = (size_t)ni * nj * nk, zu = (size_t)nj * ux, zv = (size_t)vy * ni;
     const unsigned col = (unsigned)j * ni + i, lev = (unsigned)nj * ni;
-    float *cp = s_col, *dp = s_col + (size_t)nk * kCT;
-#define CP(k) cp[(unsigned)(k) * kCT + tid]
-#define DP(k) dp[(unsigned)(k) * kCT + tid]
-#define PF(p, k) p[(unsigned)(k) * lev + col]
-#define COEF(F, K) ((((PF(a.khv, F) * PF(a.mf, F)) * PF(a.rf, F)) * PF(a.mh, K)) * PF(a.rr, K))
+    const int words = nk * 32;
+    float *s_a = s_col + lane, *s_b = s_a + words, *s_c = s_b + words, *s_d = s_c + words;
     const float rdx = 1.0f / a.dx, rdy = 1.0f / a.dy, rdz = 1.0f / a.dz, dt = a.dt, rdt = 1.0f / dt;
     const float tema = (((-1.0f * dt) * 1.0f) * rdz) * rdz;
     const float temb = ((dt * 0.0f) * rdz) * rdz;
     const float temc = dt * rdz;
     const float g = a.gz[col];
-    for (int sc = 0; sc < a.nsc; ++sc) {
-        float *target = sc == 0 ? a.thten : a.qten + (size_t)(sc - 1) * n;
-        const float *fxc = fx_of(a, sc) + (size_t)j * ux + i, *fyc = fy_of(a, sc) + (size_t)j * ni + i;
-#define SC(k) sv(a, sc, k, j, i)
-        float sm = SC(0), sk = SC(1);
-        float r2 = COEF(1, 0);
-        float cfc = tema * r2, cfb = 1.0f - cfc;
-        float ex = (-r2) * sm + r2 * sk;
-        float bc = ((temc * 0.0f) * PF(a.mh, 0)) * PF(a.rr, 0);
-        float cfd = (sm + temb * ex) + bc;
-        float tem = 1.0f / cfb;
-        float cprev = (-cfc) * tem, dprev = cfd * tem;
-        CP(0) = cprev;
-        DP(0) = dprev;
-        #pragma unroll 4
-        for (int k = 1; k + 1 < nk; ++k) {
-            const float r1 = COEF(k, k);
-            r2 = COEF(k + 1, k);
-            const float cfa = tema * r1;
-            cfc = tema * r2;
-            cfb = (1.0f - cfa) - cfc;
-            const float sp1 = SC(k + 1);
-            ex = (r1 * sm - (r1 + r2) * sk) + r2 * sp1;
-            cfd = sk + temb * ex;
-            tem = 1.0f / (cfa * cprev + cfb);
-            cprev = (-cfc) * tem;
-            dprev = (cfd - cfa * dprev) * tem;
-            CP(k) = cprev;
-            DP(k) = dprev;
-            sm = sk;
-            sk = sp1;
+    const float ruw = a.rgzu[j * ux + i], rue = a.rgzu[j * ux + i + 1], rvs = a.rgzv[j * ni + i], rvn = a.rgzv[(j + 1) * ni + i];
+    const bool ex = i == 0 || i == ni - 1, ey = j == 0 || j == nj - 1;
+    const int run = (nk + kColWarps - 1) / kColWarps;
+    const int lo = min(wy * run, nk), hi = min(lo + run, nk);
+    auto face = [&](int f) {
+        const unsigned z = (unsigned)f * lev + col;
+        return f >= 1 && f < nk ? (a.khv[z] * a.mf[z]) * a.rf[z] : 0.0f;
+    };
+    for (int first = 0; first < a.nsc; first += kTurbsGroup) {
+        const int group = min(kTurbsGroup, a.nsc - first);
+        const float *src[kTurbsGroup];  // theta is (th0 - 300) + tha
+#pragma unroll
+        for (int q = 0; q < kTurbsGroup; ++q) {
+            const int sc = first + min(q, group - 1);
+            src[q] = (sc == 0 ? a.tha : a.qa + (size_t)(sc - 1) * n) + col;
         }
-        float sol;
-        {
-            const int k = nk - 1;
-            const float r1 = COEF(k, k), cfa = tema * r1;
-            cfb = 1.0f - cfa;
-            ex = r1 * sm - r1 * sk;
-            bc = ((temc * 0.0f) * PF(a.mh, k)) * PF(a.rr, k);
-            cfd = (sk + temb * ex) - bc;
-            tem = 1.0f / (cfa * cprev + cfb);
-            sol = (cfd - cfa * dprev) * tem;
+        auto scalar = [&](int q, int k) {
+            const float x = src[q][(unsigned)k * lev];
+            return first == 0 && q == 0 ? (a.th0[k] - 300.0f) + x : x;
+        };
+        if (lo < hi) {
+            float below = face(lo), sm[kTurbsGroup], sk[kTurbsGroup];
+#pragma unroll
+            for (int q = 0; q < kTurbsGroup; ++q) {
+                sm[q] = lo > 0 ? scalar(q, lo - 1) : 0.0f;
+                sk[q] = scalar(q, lo);
+            }
+            for (int k = lo; k < hi; ++k) {
+                const unsigned z = (unsigned)k * lev + col;
+                const float mh = a.mh[z], rr = a.rr[z], above = face(k + 1);
+                const float r1 = (below * mh) * rr, r2 = (above * mh) * rr;
+                const float cfa = tema * r1, cfc = tema * r2, bc = ((temc * 0.0f) * mh) * rr;
+                if (first == 0) {
+                    s_a[k * 32] = cfa, s_c[k * 32] = cfc;
+                    s_b[k * 32] = k == 0 ? 1.0f - cfc : k == nk - 1 ? 1.0f - cfa : (1.0f - cfa) - cfc;
+                }
+#pragma unroll
+                for (int q = 0; q < kTurbsGroup; ++q) {
+                    if (q >= group) break;
+                    const float sp = k + 1 < nk ? scalar(q, k + 1) : 0.0f;
+                    float cfd;
+                    if (k == 0) {
+                        const float e = (-r2) * sk[q] + r2 * sp;
+                        cfd = (sk[q] + temb * e) + bc;
+                    } else if (k == nk - 1) {
+                        const float e = r1 * sm[q] - r1 * sk[q];
+                        cfd = (sk[q] + temb * e) - bc;
+                    } else {
+                        const float e = (r1 * sm[q] - (r1 + r2) * sk[q]) + r2 * sp;
+                        cfd = sk[q] + temb * e;
+                    }
+                    s_d[q * words + k * 32] = cfd;
+                    sm[q] = sk[q], sk[q] = sp;
+                }
+                below = above;
+            }
         }
-        #pragma unroll 4
-        for (int k = nk - 1; k >= 0; --k) {
-            if (k != nk - 1) sol = CP(k) * sol + DP(k);
-            const float turbz = (PF(a.rho, k) * (sol - SC(k))) * rdt;
-            const float right = fxc[(size_t)k * zu + 1] * a.rgzu[j * ux + i + 1], left = fxc[(size_t)k * zu] * a.rgzu[j * ux + i];
-            const float tx0 = ((-g) * (right - left)) * rdx;
-            const float upx = a.gx[o3(k + 1, j, i, nj, ni)] * (fw(fxc, zu, k + 1, nk) + fw(fxc + 1, zu, k + 1, nk));
-            const float lox = a.gx[o3(k, j, i, nj, ni)] * (fw(fxc, zu, k, nk) + fw(fxc + 1, zu, k, nk));
-            float txv = tx0 + ((-(upx - lox)) * 0.5f) * rdz;
-            if (i == 0 || i == ni - 1) txv = 0.0f;
-            const float north = fyc[(size_t)k * zv + ni] * a.rgzv[(j + 1) * ni + i], south = fyc[(size_t)k * zv] * a.rgzv[j * ni + i];
-            const float ty0 = ((-g) * (north - south)) * rdy;
-            const float upy = a.gy[o3(k + 1, j, i, nj, ni)] * (fw(fyc, zv, k + 1, nk) + fw(fyc + ni, zv, k + 1, nk));
-            const float loy = a.gy[o3(k, j, i, nj, ni)] * (fw(fyc, zv, k, nk) + fw(fyc + ni, zv, k, nk));
-            float tyv = ty0 + ((-(upy - loy)) * 0.5f) * rdz;
-            if (j == 0 || j == nj - 1) tyv = 0.0f;
-            const unsigned p = (unsigned)k * lev + col;
-            target[p] = target[p] + ((txv + tyv) + turbz) * PF(a.rr, k);
+        __syncthreads();
+        if (first == 0) {
+            if (wy == 0) {
+                float cprev = 0.0f;
+#pragma unroll 4
+                for (int k = 0; k < nk; ++k) {
+                    const float inv = rcp_rn(k == 0 ? s_b[0] : s_a[k * 32] * cprev + s_b[k * 32]);
+                    cprev = (-s_c[k * 32]) * inv;
+                    s_b[k * 32] = inv, s_c[k * 32] = cprev;
+                }
+            }
+            __syncthreads();
         }
-#undef SC
+        if (wy < group) {
+            float *d = s_d + wy * words;
+            float prev = d[0] * s_b[0];
+            d[0] = prev;
+#pragma unroll 8
+            for (int k = 1; k < nk; ++k) {
+                prev = (d[k * 32] - s_a[k * 32] * prev) * s_b[k * 32];
+                d[k * 32] = prev;
+            }
+#pragma unroll 8
+            for (int k = nk - 2; k >= 0; --k) {
+                prev = s_c[k * 32] * prev + d[k * 32];
+                d[k * 32] = prev;
+            }
+        }
+        __syncthreads();
+        for (int q = 0; own && q < group; ++q) {
+            if (lo >= hi) break;
+            const int sc = first + q;
+            float *target = sc == 0 ? a.thten : a.qten + (size_t)(sc - 1) * n;
+            const float *fxc = fx_of(a, sc) + (size_t)j * ux + i, *fyc = fy_of(a, sc) + (size_t)j * ni + i;
+            // the slope terms at the lower face of the run's first level, then carried up
+            float lox = a.gx[o3(lo, j, i, nj, ni)] * (fw(fxc, zu, lo, nk) + fw(fxc + 1, zu, lo, nk));
+            float loy = a.gy[o3(lo, j, i, nj, ni)] * (fw(fyc, zv, lo, nk) + fw(fyc + ni, zv, lo, nk));
+            for (int k = lo; k < hi; ++k) {
+                const unsigned z = (unsigned)k * lev + col;
+                const float turbz = (a.rho[z] * (s_d[q * words + k * 32] - sv(a, sc, k, j, i))) * rdt;
+                const float right = fxc[(size_t)k * zu + 1] * rue, left = fxc[(size_t)k * zu] * ruw;
+                const float tx0 = ((-g) * (right - left)) * rdx;
+                const float upx = a.gx[o3(k + 1, j, i, nj, ni)] * (fw(fxc, zu, k + 1, nk) + fw(fxc + 1, zu, k + 1, nk));
+                const float txv = ex ? 0.0f : tx0 + ((-(upx - lox)) * 0.5f) * rdz;
+                const float north = fyc[(size_t)k * zv + ni] * rvn, south = fyc[(size_t)k * zv] * rvs;
+                const float ty0 = ((-g) * (north - south)) * rdy;
+                const float upy = a.gy[o3(k + 1, j, i, nj, ni)] * (fw(fyc, zv, k + 1, nk) + fw(fyc + ni, zv, k + 1, nk));
+                const float tyv = ey ? 0.0f : ty0 + ((-(upy - loy)) * 0.5f) * rdz;
+                target[z] = target[z] + ((txv + tyv) + turbz) * a.rr[z];
+                lox = upx, loy = upy;
+            }
+        }
+        __syncthreads();  // the next group's right sides take these words
     }
-#undef CP
-#undef DP
-#undef PF
-#undef COEF
 }
 
 bool all_set(std::initializer_list<const void *> ps) {
@@ -661,24 +702,26 @@ extern "C" int32_t gm1b_terrain_stress(int32_t ni, int32_t nj, int32_t nk, const
         ps.stop();
         if (!launch_ok("terrain_gettau_kernel")) return GM1B_ERR_CUDA;
     }
-    const size_t smem = (size_t)2 * nk * kCT * sizeof(float);
+    const size_t smem = (size_t)4 * nk * 32 * sizeof(float);  // 102400 bytes at nk = 200
+    const dim3 cta(32, kColWarps);
+    auto tiles = [](int nx, int ny) { return (unsigned)((nx + 31) / 32) * (unsigned)ny; };
     TRY(configure(terrain_turb_uv_kernel<0>, smem, "terrain_turb_uv_kernel<0>"));
     TRY(configure(terrain_turb_uv_kernel<1>, smem, "terrain_turb_uv_kernel<1>"));
     TRY(configure(terrain_turbw_kernel, smem, "terrain_turbw_kernel"));
     {
         ProfScope ps("terrain_turbu_kernel", st);
-        terrain_turb_uv_kernel<0><<<dim3((ni + 1 + kCX - 1) / kCX, (nj + kCY - 1) / kCY), dim3(kCX, kCY), smem, st>>>(a);
+        terrain_turb_uv_kernel<0><<<tiles(ni + 1, nj), cta, smem, st>>>(a);
         ps.stop();
         if (!launch_ok("terrain_turbu_kernel")) return GM1B_ERR_CUDA;
     }
     {
         ProfScope ps("terrain_turbv_kernel", st);
-        terrain_turb_uv_kernel<1><<<dim3((ni + kCX - 1) / kCX, (nj + 1 + kCY - 1) / kCY), dim3(kCX, kCY), smem, st>>>(a);
+        terrain_turb_uv_kernel<1><<<tiles(ni, nj + 1), cta, smem, st>>>(a);
         ps.stop();
         if (!launch_ok("terrain_turbv_kernel")) return GM1B_ERR_CUDA;
     }
     ProfScope ps("terrain_turbw_kernel", st);
-    terrain_turbw_kernel<<<dim3((ni + kCX - 1) / kCX, (nj + kCY - 1) / kCY), dim3(kCX, kCY), smem, st>>>(a);
+    terrain_turbw_kernel<<<tiles(ni, nj), cta, smem, st>>>(a);
     ps.stop();
     return launch_ok("terrain_turbw_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }
@@ -715,14 +758,17 @@ extern "C" int32_t gm1b_terrain_scalar_turbulence(int32_t ni, int32_t nj, int32_
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     {
         ProfScope ps("terrain_turbs_flux_kernel", st);
-        terrain_turbs_flux_kernel<<<ew_blocks((size_t)nk * nj * (ni + 1) + (size_t)nk * (nj + 1) * ni), kEW, 0, st>>>(a);
+        const unsigned tiles = (unsigned)((ni + 1 + 31) / 32) * (unsigned)((nj + 1 + 7) / 8);
+        const int chunk = level_chunk(tiles, nk);
+        terrain_turbs_flux_kernel<<<dim3(tiles, (nk + chunk - 1) / chunk), dim3(32, 8), 0, st>>>(a, chunk);
         ps.stop();
         if (!launch_ok("terrain_turbs_flux_kernel")) return GM1B_ERR_CUDA;
     }
-    const size_t smem = (size_t)2 * nk * kCT * sizeof(float);
+    // 179200 bytes for a full group at nk = 200
+    const size_t smem = (size_t)(3 + (numq + 1 < kTurbsGroup ? numq + 1 : kTurbsGroup)) * nk * 32 * sizeof(float);
     TRY(configure(terrain_turbs_column_kernel, smem, "terrain_turbs_column_kernel"));
     ProfScope ps("terrain_turbs_column_kernel", st);
-    terrain_turbs_column_kernel<<<dim3((ni + kCX - 1) / kCX, (nj + kCY - 1) / kCY), dim3(kCX, kCY), smem, st>>>(a);
+    terrain_turbs_column_kernel<<<(unsigned)((ni + 31) / 32) * (unsigned)nj, dim3(32, kColWarps), smem, st>>>(a);
     ps.stop();
     return launch_ok("terrain_turbs_column_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }

@@ -215,6 +215,30 @@ def test_flat_turbulence_columns(ni, nj, nk, numq):
     assert _differ(d, a, ("thten1", "qten")) == []
 
 
+@pytest.mark.parametrize("ni,nj,nk,numq", [(31, 3, 7, 2), (32, 8, 8, 3), (33, 7, 9, 4), (64, 3, 17, 5), (3, 5, 200, 6)])
+def test_terrain_turbulence_columns(ni, nj, nk, numq):
+    from gm1_b200 import stress
+    from oracle import stress as ost
+    from tests.test_stress_terrain_gpu import _stress_inputs, _turbs_inputs
+
+    g = dict(ni=ni, nj=nj, nk=nk, dx=1000.0, dy=900.0, dz=250.0)
+    a = _stress_inputs(ni, nj, nk, ni + nk)
+    rng = np.random.default_rng(nk)
+    for n in ost.STRAIN_NAMES:
+        a[n][:] = rng.normal(0.0, 1.0, a[n].shape)
+    d = _dev(a)
+    ost.terrain_gettau(a, ni=ni, nj=nj, nk=nk)
+    ost.terrain_momentum_stress(a, **g, dt=5.0)
+    stress.launch_cuda_terrain_stress(d, **g, dt=5.0)
+    assert _differ(d, a, ("uten", "vten", "wten")) == []
+    a = _turbs_inputs(ni, nj, nk, ni + nk)
+    d = _dev(a)
+    d["workspace"] = stress.terrain_scalar_turbulence_workspace(ni, nj, nk, numq, d["tha"].device)
+    ost.terrain_scalar_turbulence(a, **g, numq=numq, dt=5.0)
+    stress.launch_cuda_terrain_scalar_turbulence(d, **g, numq=numq, dt=5.0)
+    assert _differ(d, a, ("thten1", "qten")) == []
+
+
 @pytest.mark.parametrize("ni,nj,nk", [(31, 3, 1), (32, 2, 7), (33, 5, 8), (65, 2, 9), (5, 3, 296), (5, 3, 297)])
 def test_kessler_columns(ni, nj, nk):
     """Columns in shared memory (up to 296 levels) and a thread per column:
