@@ -216,7 +216,9 @@ __global__ void __launch_bounds__(32 * kColWarps) flat_turb_uv_kernel(const __gr
         }
     }
     __syncthreads();
-    if (wy == 0) column_sweep<4>(s_a, s_b, s_c, s_d, K);
+    // (chunks of four rows cost registers and CTAs an SM: 640x768x80 turbu 1115
+    // us against 1005, turbw 828 against 541)
+    if (wy == 0) column_sweep<2>(s_a, s_b, s_c, s_d, K);
     __syncthreads();
     if (lo >= hi || !own) return;
     // the vertical and horizontal terms and the tendency of each level
@@ -290,7 +292,7 @@ __global__ void __launch_bounds__(32 * kColWarps) flat_turbw_kernel(const __grid
         }
     }
     __syncthreads();
-    if (wy == 0) column_sweep<4>(s_a, s_b, s_c, s_d, n);
+    if (wy == 0) column_sweep<2>(s_a, s_b, s_c, s_d, n);
     __syncthreads();
     if (!own) return;
     const bool ex = i == 0 || i == ni - 1, ey = j == 0 || j == nj - 1;
