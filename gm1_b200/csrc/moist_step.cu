@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(256) open_fill_kernel(const __grid_constant__ 
 }
 
 // theta (th0 - 300 + th3d) and the moisture rows into their padded arrays,
-// the halos of levels 1..nk as the open scalar fill leaves them, one launch
+// the halos of levels 1..nk as the open scalar fill leaves them (fill_word's,
+// the words beyond the first ring beside its corners among them), one launch
 struct PackScalars {
     const float *th0, *scalar[4];  // th3d, then the moisture rows
     float *padded[4];
@@ -136,13 +137,22 @@ __global__ void __launch_bounds__(256) pack_scalars_kernel(const __grid_constant
     const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y, k = blockIdx.z;
     const int px = ni + 6, py = nj + 6;
     if (x >= px || y >= py) return;
-    if ((y < 3 || y > nj + 2) && (x < 2 || x > ni + 3)) return;  // words no fill writes
+    if ((y < 3 || y > nj + 2) && (x < 2 || x > ni + 3)) return;  // left alone, or a first-ring thread's below
     const unsigned c = ((unsigned)k * nj + (unsigned)(min(max(y, 3), nj + 2) - 3)) * (unsigned)ni +
                        (unsigned)(min(max(x, 3), ni + 2) - 3);
     const unsigned d = ((unsigned)(k + 1) * py + y) * (unsigned)px + x;
     float v[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) v[q] = __ldg(a.scalar[q] + c);
+    if ((y == 2 || y == nj + 3) && (x == 3 || x == ni + 2)) {
+        // the west/east pass copied this word outward before the other overwrote it
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float old = a.padded[q][d];
+            if (x == 3) a.padded[q][d - 2] = a.padded[q][d - 3] = old;
+            if (x == ni + 2) a.padded[q][d + 2] = a.padded[q][d + 3] = old;
+        }
+    }
     const float base = __ldg(a.th0 + k) - 300.0f;
     a.padded[0][d] = base + v[0];
 #pragma unroll

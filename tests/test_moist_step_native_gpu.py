@@ -92,3 +92,21 @@ def test_native_step_refuses_a_courant_stop():
     with pytest.raises(CourantStop):
         nat.check()
     nat.close()
+
+
+@pytest.mark.parametrize("stretched", [False, True])
+def test_native_step_leaves_the_python_composition_carriers(stretched):
+    """The padded carriers whole: the halos of the second and later stages
+    hold words of the stage before beyond the first ring at the corners."""
+    cfg, host, metrics = _case(stretched)
+    py = MoistLargeStep(cfg, upload(host), upload(metrics), concurrent=False)
+    nat = NativeMoistLargeStep(cfg, upload(host), upload(metrics))
+    for _ in range(2):
+        py.step()
+        nat.step()
+    torch.cuda.synchronize()
+    names = ("theta_padded", "moisture_padded", "moisture_padded_1", "moisture_padded_2")
+    want = {"theta_padded": py.s["theta_padded"],
+            **{n: py.species_scratch[r]["moisture_padded"] for r, n in enumerate(names[1:])}}
+    assert _same(want, {**nat.s, **nat.scratch}, names) == []
+    nat.close()
