@@ -77,6 +77,7 @@ struct gm1b_moist_step {
     float *ones_i = nullptr, *ones_j = nullptr, *mh_col = nullptr;
     float rdz = 0.0f;
     uint32_t obc = 0;
+    bool pack_together = false;  // carriers_apart
 };
 
 namespace {
@@ -422,7 +423,12 @@ int advect(Step &h, float *padded, float *tendency, double weps, int nrk, cudaSt
 }
 
 int theta_advection(Step &h, int nrk, cudaStream_t st) {
+    const gm1b_moist_step_config &c = h.c;
     const gm1b_moist_state &s = h.s;
+    if (!h.pack_together) {
+        TRY(gm1b_theta_transport_pack(c.ni, c.nj, c.nk, s.th0, s.th3d, s.theta_padded, st));
+        TRY(gm1b_open_fill(c.ni, c.nj, c.nk, GM1B_FILL_SCALAR, s.theta_padded, st));
+    }
     return advect(h, s.theta_padded, s.theta_adv, weps_of(10.0f), nrk, st);
 }
 
@@ -439,6 +445,32 @@ Species species(const Step &h, int r) {
     return {s.moisture_padded, s.fx, s.fy, s.fz, s.advx, s.advy, s.advz, s.candidate};
 }
 
+// Whether the carriers of every lane can be packed before the first lane runs:
+// none shares words with another's carrier or scratch.  (Lanes that run one
+// after another may be given one scratch.)
+bool carriers_apart(const Step &h) {
+    const Sizes z(h.c);
+    struct Span {
+        const float *p;
+        size_t n;
+    };
+    auto apart = [](Span a, Span b) { return a.p + a.n <= b.p || b.p + b.n <= a.p; };
+    const Span theta{h.s.theta_padded, z.scalar};
+    for (int r = 0; r < kNumq; ++r) {
+        const Span mine{species(h, r).padded, z.scalar};
+        if (!apart(theta, mine)) return false;
+        for (int q = 0; q < kNumq; ++q) {
+            if (q == r) continue;
+            const Species o = species(h, q);
+            const Span theirs[] = {{o.padded, z.scalar}, {o.advx, z.mass}, {o.advy, z.mass}, {o.advz, z.mass},
+                                   {o.candidate, z.mass}};
+            for (const Span &t : theirs)
+                if (!apart(mine, t)) return false;
+        }
+    }
+    return true;
+}
+
 int species_advection(Step &h, int r, int nrk, cudaStream_t st) {
     const gm1b_moist_step_config &c = h.c;
     const gm1b_moist_state &s = h.s;
@@ -447,6 +479,10 @@ int species_advection(Step &h, int r, int nrk, cudaStream_t st) {
     const Species sp = species(h, r);
     float *adv = s.moist_adv + (size_t)r * z.mass;
     const double weps = weps_of(1.0e-2f);
+    if (!h.pack_together) {
+        TRY(gm1b_pack_scalar(c.ni, c.nj, c.nk, s.q3d + (size_t)r * z.mass, sp.padded, st));
+        TRY(gm1b_open_fill(c.ni, c.nj, c.nk, GM1B_FILL_SCALAR, sp.padded, st));
+    }
     if (nrk < 3) return advect(h, sp.padded, adv, weps, nrk, st);
     gm1b_pdef_chain_arrays a{s.qa + (size_t)r * z.mass, sp.padded, m.rho0_3d, m.gz, m.rgz, m.rr0, m.c1, m.c2,
                              s.divx, s.rru, s.rrv, s.rrw, sp.fx, sp.fy, sp.fz, sp.advx, sp.advy, sp.advz,
@@ -464,9 +500,9 @@ int record_wait(cudaEvent_t ev, cudaStream_t from, cudaStream_t to) {
 int scalar_moist(Step &h, int nrk, cudaStream_t st) {
     const gm1b_moist_step_config &c = h.c;
     const gm1b_moist_state &s = h.s;
-    {
-        // every scalar's carrier in one launch; the advections write whole
-        // tendencies on these whole-domain sides, so nothing is zeroed
+    // the advections write whole tendencies on these whole-domain sides, so
+    // nothing is zeroed
+    if (h.pack_together) {  // every scalar's carrier in one launch
         const size_t mass = Sizes(c).mass;
         const float *scalar[4] = {s.th3d, s.q3d, s.q3d + mass, s.q3d + 2 * mass};
         float *padded[4] = {s.theta_padded, species(h, 0).padded, species(h, 1).padded, species(h, 2).padded};
@@ -660,6 +696,7 @@ extern "C" int32_t gm1b_moist_step_create(const gm1b_moist_step_config *config, 
     h->obc = (uint32_t)c.lateral_sides[0] | ((uint32_t)c.lateral_sides[1] << 4) |
              ((uint32_t)c.lateral_sides[2] << 8) | ((uint32_t)c.lateral_sides[3] << 12);
     h->rdz = 1.0f / c.dz;
+    h->pack_together = carriers_apart(*h);
     bool good = ok(cudaGetDevice(&h->device), "cudaGetDevice");
     for (auto &q : h->side)
         if (good) good = ok(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "cudaStreamCreateWithFlags");

@@ -1345,8 +1345,8 @@ GM1B_API int32_t gm1b_warm_rain_cell_adjoint(size_t cells, const float *th0, con
  * (ni), rvh (nj); saturation_mask (uint8, mass); asq (3) and qbudget (10)
  * FP64; and the scratch of moisture species 1 and 2 (each padded scalar,
  * fx, fy, fz, advx, advy, advz, candidate), which lets the three species
- * advect concurrently (species 0 uses the state's own).  The caller owns
- * every array.
+ * advect concurrently (species 0 uses the state's own); with concurrent = 0
+ * they may be the state's own again.  The caller owns every array.
  * ---------------------------------------------------------------------- */
 typedef struct gm1b_moist_state {
     float *ua, *u3d, *uten, *rru, *va, *v3d, *vten, *rrv, *wa, *w3d, *wten, *rrw, *fz, *fx, *fy;

@@ -7,12 +7,15 @@ graph; and the folded failure words read back through the ABI."""
 
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
-from gm1_b200.moist_step import (CourantStop, MoistLargeStep, MoistStepConfig, NativeMoistLargeStep,
-                                 StretchedColumnSpec, upload, weisman_klemp_initial_state)
+from gm1_b200._native import check
+from gm1_b200.moist_step import (SPECIES_SCRATCH, CourantStop, MoistLargeStep, MoistStepConfig, NativeMoistLargeStep,
+                                 StretchedColumnSpec, _native_lib, upload, weisman_klemp_initial_state)
 
 pytestmark = pytest.mark.gpu
 
@@ -109,4 +112,30 @@ def test_native_step_leaves_the_python_composition_carriers(stretched):
     want = {"theta_padded": py.s["theta_padded"],
             **{n: py.species_scratch[r]["moisture_padded"] for r, n in enumerate(names[1:])}}
     assert _same(want, {**nat.s, **nat.scratch}, names) == []
+    nat.close()
+
+
+@pytest.mark.parametrize("stretched,shared", [(True, "scratch"), (False, "scratch"), (False, "carrier")])
+def test_native_step_runs_its_lanes_in_one_scratch(stretched, shared):
+    """concurrent = 0: the species may be given the state's own scratch, and
+    their carrier may be theta's."""
+    cfg, host, metrics = _case(stretched)
+    py = MoistLargeStep(cfg, upload(host), upload(metrics), concurrent=False)
+    nat = NativeMoistLargeStep(cfg, upload(host), upload(metrics), concurrent=False)
+    nat.close()
+    for n in SPECIES_SCRATCH:
+        for r in (1, 2):
+            setattr(nat._state, f"{n}_{r}", nat.s[n].data_ptr())
+    if shared == "carrier":
+        nat._state.moisture_padded = nat.s["theta_padded"].data_ptr()
+    handle = ctypes.c_void_p()
+    check(_native_lib().gm1b_moist_step_create(ctypes.byref(nat._config), ctypes.byref(nat._state),
+                                               ctypes.byref(nat._metrics), ctypes.byref(handle)),
+          "gm1b_moist_step_create")
+    nat._handle = handle
+    for _ in range(2):
+        py.step()
+        nat.step()
+    torch.cuda.synchronize()
+    assert _same(py.s, nat.s) == []
     nat.close()
