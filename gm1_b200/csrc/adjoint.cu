@@ -958,7 +958,8 @@ int32_t advection_adjoint_launch(const char *who, int32_t ni, int32_t nj, int32_
     const struct {
         const float *p;
         size_t words;
-    } shared[] = {{a.lam, cells}, {a.rr0, cells}, {a.gz, (size_t)ni * nj}, {a.rru, (size_t)(nk + 2) * (nj + 6) * (ni + 7)},
+    } shared[] = {{a.lam, cells}, {a.rr0, cells}, {a.c1, cells + (size_t)ni * nj}, {a.c2, cells + (size_t)ni * nj},
+                  {a.gz, (size_t)ni * nj}, {a.rru, (size_t)(nk + 2) * (nj + 6) * (ni + 7)},
                   {a.rrv, (size_t)(nk + 2) * (nj + 7) * (ni + 6)}, {a.rrw, (size_t)(nk + 3) * (nj + 6) * (ni + 6)}};
     for (const auto &s : shared)
         one_pass = one_pass && apart(s.p, s.words, a.out, out_words) && apart(s.p, s.words, a.sum_out, cells);

@@ -342,3 +342,27 @@ def test_advection_adjoint_in_one_pass(ni, nj, nk, nrk):
     west = padded[1:-1, 4:-4, :4].double().sum(-1)
     # four float32 words of at most the largest one's size
     assert torch.allclose(west, got[:, 1:-1, 0].double(), rtol=0.0, atol=float(padded.abs().max()) * 2.0 ** -21)
+
+
+@pytest.mark.parametrize("name", ["c1", "c2"])
+@pytest.mark.parametrize("running", [False, True])
+def test_advection_adjoint_over_its_face_weights(name, running):
+    """An output over c1 or c2, which the cells beside the column's ends read
+    at their neighbours' levels, takes the two passes."""
+    import dataclasses
+
+    from gm1_b200 import adjoint as adj
+    from tests.test_adjoint_gpu import _flow, warm_rain_case
+
+    ni, nj, nk = 34, 9, 12
+    state, fr, g = warm_rain_case(ni=ni, nj=nj, nk=nk, seed=3)
+    flow = _flow(fr, g)
+    s, lam = _t(state["qv"]), _t(np.random.default_rng(4).standard_normal((nk, nj, ni)))
+    got = adj.advection_tendency_adjoint(flow, s, lam, 1)
+    over = flow.fields[name].clone()
+    flow = dataclasses.replace(flow, fields={**flow.fields, name: over})
+    if running:
+        adj.advection_tendency_adjoint(flow, s, lam, 1, accumulate=torch.zeros_like(lam), running_sum=over[:nk])
+    else:
+        adj.advection_tendency_adjoint(flow, s, lam, 1, out=over[:nk])
+    assert torch.equal(over[:nk], got)
