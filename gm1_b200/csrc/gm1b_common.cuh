@@ -196,10 +196,12 @@ __device__ __forceinline__ void column_sweep(const float *s_a, const float *s_b,
 // Levels a thread of a memory-bound column march takes: eight, or fewer (two at
 // the least) until four CTAs of its 256 threads lie on each of 148 SMs (mass
 // fluxes of 128x100x64: eight levels 15.1 us, two 12.8; of 256x256x80: 76 and 93).
+// The chunks of a column lie in a grid dimension of at most 65535.
 inline int level_chunk(size_t tiles, int nk) {
     int chunk = 8;
     while (chunk > 2 && tiles * (size_t)((nk + chunk - 1) / chunk) < 4 * 148) chunk /= 2;
-    return chunk;
+    const int least = (int)(((size_t)nk + 65534) / 65535);
+    return chunk < least ? least : chunk;
 }
 
 }  // namespace gm1b

@@ -139,6 +139,25 @@ def test_column_marches(ni, nj, nk):
     assert _differ(d, a, ("wten", "rru", "rrv", "rrw", "divergence", "theta_divergence_term", "divx")) == []
 
 
+def test_column_marches_of_more_chunks_than_a_grid_takes():
+    """2x2 columns whose chunks of eight levels exceed a grid dimension's
+    65535: the whole column against the same columns cut in two."""
+    from gm1_b200 import moist_ops as mo
+
+    ni, nj, nk, cut = 2, 2, 524300, 262144
+    g = torch.Generator(device="cuda").manual_seed(1)
+    r = lambda *s: torch.rand(*s, generator=g, device="cuda")  # noqa: E731
+    a = {"dum8": r(nk + 2, 8, 8), "c1": r(nk + 1, 2, 2), "c2": r(nk + 1, 2, 2), "wten": r(nk + 3, 8, 8)}
+    parts = []
+    for lo, hi in ((1, cut + 1), (cut, nk)):  # two levels in common: the faces at either end are not formed
+        p = {n: a[n][lo - 1:hi + k].contiguous() for n, k in (("dum8", 2), ("c1", 1), ("c2", 1), ("wten", 3))}
+        mo.moist_buoyancy_flat(*p.values(), ni=ni, nj=nj, nk=hi - lo + 1)
+        parts.append(p["wten"])
+    mo.moist_buoyancy_flat(*a.values(), ni=ni, nj=nj, nk=nk)
+    want = torch.cat((parts[0][:cut + 1], parts[1][2:]))
+    assert torch.equal(a["wten"], want)
+
+
 @pytest.mark.parametrize("flat", [False, True])
 @pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (32, 14, 11), (62, 15, 12), (7, 9, 40)])
 def test_tke_stages(ni, nj, nk, flat):
