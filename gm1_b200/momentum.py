@@ -266,7 +266,7 @@ def launch_cuda_terrain_open_momentum_advection5(
                       "lateral_boundaries": list(lateral_sides), "nrk": nrk},
         "boundary_faces": momentum_boundary_faces(lateral_sides),
         "domain": {"ni": ni, "nj": nj, "nk": nk},
-        "launches": 3,
+        "launches": 2,
     }
     if rrw_receipt is not None:
         receipt["rrw_open_boundary"] = dict(rrw_receipt)
@@ -347,7 +347,7 @@ def launch_cuda_gm1_child_stretched_momentum5(
         ev.record(st)
     receipt: dict[str, Any] = {"terrain": not vertical.flat, "stretch_z": 1, "nrk": nrk,
                                "lateral_boundaries": list(lateral_sides), "domain": {"ni": ni, "nj": nj, "nk": nk},
-                               "launches": 3}
+                               "launches": 2}
     if rrw_receipt is not None:
         receipt["rrw_open_boundary"] = dict(rrw_receipt)
     return CudaMomentumAdvection5Launch(divx, ev, receipt)

@@ -140,3 +140,30 @@ def test_stretched_column_matches_oracle(flat, tag):
     for n in ("uten", "vten", "wten", "rru", "rrv", "rrw", "divx"):
         got = d[n].cpu().numpy()
         assert np.array_equal(got.view(np.uint32), want[n].view(np.uint32)), n
+
+
+@pytest.mark.parametrize("column", ["uniform", "terrain", "flat"])
+def test_receipt_counts_the_launches(column):
+    from gm1_b200 import _native
+    from gm1_b200.vertical import uniform_vertical_levels
+    from tests.test_oracle_momentum import _padded_rho0
+
+    ni, nj, nk = 9, 8, 9
+    a, m, _ = momentum_fixture(ni, nj, nk, 3)
+    dev = _dev({**a, **m})
+    kw = dict(ni=ni, nj=nj, nk=nk, nrk=1, dx=500.0, dy=450.0)
+    rho0p = torch.from_numpy(_padded_rho0(m["rho0_3d"], ni, nj, nk)).cuda()
+    lv = uniform_vertical_levels(nk, 150.0)
+    _native.profiler_enable(True)
+    if column == "uniform":
+        out = mom.launch_cuda_terrain_open_momentum_advection5(dev, dev, dz=150.0, **kw)
+    else:
+        col = mom.StretchedMomentumColumn(False, rho0p, ztop=lv.ztop_m, **{
+            n: torch.from_numpy(np.array(getattr(lv, n), np.float32)).cuda() for n in ("sigma", "sigmaf", "rds", "rdsf")}) \
+            if column == "terrain" else mom.StretchedMomentumColumn(
+                True, rho0p, mh=torch.ones(nk + 2, device="cuda"), mf=torch.ones(nk + 3, device="cuda"),
+                rr0=torch.ones((nk, nj, ni), device="cuda"), rdz=1.0 / 150.0)
+        out = mom.launch_cuda_gm1_child_stretched_momentum5(dev, dev, col, **kw)
+    torch.cuda.synchronize()
+    _native.profiler_enable(False)
+    assert out.receipt["launches"] == sum(k["launches"] for k in _native.profiler_collect())
