@@ -129,6 +129,20 @@ def _ablation_mask(ablations: TerrainOpenSoundAblations) -> int:
     return sum(bit for name, bit in _ABLATION_BITS.items() if getattr(ablations, name))
 
 
+def _launches_per_stage(ablations: TerrainOpenSoundAblations) -> str:
+    """Kernels of one stage, "a + b*nloop + c": the stage start; each small
+    step's pressure gradient and column pass; radiation and the two fill
+    passes.  The open sides take a launch a small step, or one a stage where
+    whole small steps let the column pass leave the next one's."""
+    opened = int(ablations.open_consumption)
+    whole = (ablations.terrain_pressure_gradient and ablations.transformed_divergence and ablations.pressure_advection
+             and ablations.implicit_vertical_solve and ablations.between_step_pressure_fill)
+    start = 1 + (opened if whole else 0)
+    step = 1 + int(ablations.terrain_pressure_gradient) + (0 if whole else opened)
+    end = int(ablations.radiation_history_production) + 2 * int(ablations.stage_family_fills)
+    return f"{start} + {step}*nloop + {end}"
+
+
 def terrain_static_shapes(*, ni: int, nj: int, nk: int) -> dict[str, tuple[int, ...]]:
     for name, value, minimum in (("ni", ni, 3), ("nj", nj, 3), ("nk", nk, 3)):
         if isinstance(value, bool) or not isinstance(value, int) or value < minimum:
@@ -344,7 +358,7 @@ def launch_cuda_psolver3_terrain_open_three_stage(
         "comparison_contract": {"mode": "raw-bit", "max_ulp": 0, "null_or_missing_is_pass": False},
         "lateral_boundaries": {"selection": {"wbc": 2, "ebc": 2, "sbc": 2, "nbc": 2, "irbc": 4, "roflux": 0,
                                              "nudgeobc": 0}},
-        "launches_per_stage": "1 + 3*nloop + 3",
+        "launches_per_stage": _launches_per_stage(ablations),
     }
     if not retain:
         receipt["column_diagnostics"] = {"retained": False, "omitted_arrays": list(COLUMN_DIAGNOSTIC_NAMES) + [

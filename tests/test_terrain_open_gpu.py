@@ -250,3 +250,25 @@ def test_flat_stretched_stage_replays_from_a_cuda_graph():
     g.replay()
     torch.cuda.synchronize()
     assert _bad(graphed, {k: v.cpu().numpy() for k, v in eager.items()}, tos.ALL_ARRAY_NAMES) == []
+
+
+@pytest.mark.parametrize("retain", [True, False])
+@pytest.mark.parametrize("off", [None, *orc.ABLATION_BITS])
+def test_receipt_counts_the_launches(off, retain):
+    from gm1_b200 import _native
+
+    ni, nj, nk = 9, 7, 8
+    a, m = terrain_open_fixture(ni, nj, nk, 4)
+    dev, mdev = _dev(a), _dev(m)
+    if not retain:
+        for n in tos.COLUMN_DIAGNOSTIC_NAMES:
+            dev[n] = torch.zeros(1, device="cuda")
+    _native.profiler_enable(True)
+    r = tos.launch_cuda_psolver3_terrain_open_stage(
+        dev, mdev, nrk=3, ni=ni, nj=nj, nk=nk, dt=2.0, nsound=6, dx=450.0, dy=520.0, dz=210.0,
+        compiled=tos.compile_cuda_psolver3_terrain_open(retain_column_diagnostics=retain),
+        ablations=tos.TerrainOpenSoundAblations(**({} if off is None else {off: False})))
+    torch.cuda.synchronize()
+    _native.profiler_enable(False)
+    start, step, end = (int(x.split("*")[0]) for x in r.receipt["launches_per_stage"].split(" + "))
+    assert start + step * r.cadence[0]["nloop"] + end == sum(k["launches"] for k in _native.profiler_collect())
