@@ -735,7 +735,7 @@ def run_ensemble(args) -> None:
                    "mode": "ensemble", "cells": total_cells, "members": args.members,
                    "batched": "one CUDA graph per ensemble step, members over 8 streams",
                    "autotune": {"shapes": len(tuner.table) // 2, "set_up_s": round(t_tune, 2),
-                                "chunks": {k: v["best"] for k, v in list(tuner.table.items())[:8]}},
+                                "chunks": {k: v["chosen"] for k, v in list(tuner.table.items())[:8]}},
                    "plain_cell_updates_per_s": plain_value, "plain_ms_per_step": p_ms / args.steps,
                    "batched_over_plain": value / plain_value,
                    "l2": "flushed before every timed step (256 MiB write, outside the event pair)",
