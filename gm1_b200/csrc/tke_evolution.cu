@@ -10,7 +10,7 @@
 //               (enqueue_flat_turbt :631; CartesianClosure.tke_rk, cuda_cartesian_closure.py:1658-1663)
 //
 // Design (B200):
-//  * turbt is one kernel per 32 columns of a row: eight warps form the
+//  * turbt is one kernel per 32 columns of a row: eight warps (or three) form the
 //    tridiagonal rows of their own runs of levels (the mf/rf divisions and
 //    every load spread over the CTA), one warp sweeps them in shared memory
 //    (the reference's thread-per-column kernel keeps five local arrays of 74
@@ -28,7 +28,7 @@
 namespace gm1b {
 namespace {
 
-constexpr int kTurbtWarps = 8;  // warps of a turbt CTA, which owns 32 columns of a row
+constexpr int kTurbtWarps = 8;  // warps of a flat turbt CTA, which owns 32 columns of a row
 constexpr int kTurbtMostNk = 201;
 constexpr int kG = 3;                                    // padded-lane halo of rru/rrv/rrw
 
@@ -63,8 +63,12 @@ __device__ __forceinline__ float tke_flux(const TkeArgs &a, int f, int l, int r,
 
 // dynamic shared memory: the four tridiagonal words of each of the nk-1 rows
 // of 32 columns.  256x256x80: 405 us with a thread per column (its loads a
-// level at a time, most of the chip idle), 220 here.
-__global__ void __launch_bounds__(32 * kTurbtWarps, 3) tke_turbt_kernel(const __grid_constant__ TkeArgs a, float dt) {
+// level at a time, most of the chip idle), 220 here with eight warps.  Three
+// warps where short columns of a large plane make enough CTAs of them: a run
+// of levels forms the face fluxes of one level more at either end, and one
+// warp sweeps while the others wait (turbt_warps).
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 24 / WARPS) tke_turbt_kernel(const __grid_constant__ TkeArgs a, float dt) {
     extern __shared__ float s_col[];
     const int lane = threadIdx.x, wy = threadIdx.y;
     const int ni = a.ni, nj = a.nj, nk = a.nk, n = nk - 1, cz = ni * nj, tiles = (ni + 31) / 32;
@@ -73,7 +77,7 @@ __global__ void __launch_bounds__(32 * kTurbtWarps, 3) tke_turbt_kernel(const __
     const int i = min(i0, ni - 1), c = j * ni + i;  // lanes past the row's end repeat its last column
     float *s_a = s_col + lane, *s_b = s_a + n * 32, *s_c = s_b + n * 32, *s_d = s_c + n * 32;  // rows f - 1
     const float rdt = 1.0f / dt, tema = -1.0f * (dt * (a.rdz * a.rdz));
-    const int run = (n + kTurbtWarps - 1) / kTurbtWarps;
+    const int run = (n + WARPS - 1) / WARPS;
     const int f_lo = 1 + wy * run, f_hi = min(n, f_lo + run - 1);
     if (f_lo <= f_hi) {
         unsigned z = (unsigned)f_lo * (unsigned)cz + (unsigned)c;
@@ -507,6 +511,14 @@ int tke_args(int ni, int nj, int nk, const gm1b_tke_evolution_arrays *s, float d
 // four tridiagonal words of each of the nk-1 rows of 32 columns
 size_t turbt_smem(int nk) { return (size_t)4 * (nk - 1) * 32 * sizeof(float); }
 
+// Three warps a CTA for columns of up to 64 levels on a plane that gives the
+// eight-warp CTAs (three an SM) three rounds of 148 SMs, else eight.  Eight and
+// three warps, us: 256x256 of 24 levels 61 and 47, 40 levels 104 and 86, 64
+// levels 159 and 148, 80 levels 196 and 249; 512x400x30 264 and 209; 179x261x32
+// 58 and 51; 128x100x24 15 and 19.  (A thread per column: 47, 88, 312, 401;
+// 233; 61; 39.)
+int turbt_warps(unsigned tiles, int nk) { return nk <= 64 && tiles >= 3 * 3 * 148 ? 3 : 8; }
+
 int enqueue_diffusion(const TkeArgs &a, float dt, cudaStream_t st) {
     const size_t smem = turbt_smem(a.nk);
     if (a.nk > kTurbtMostNk) {
@@ -516,8 +528,10 @@ int enqueue_diffusion(const TkeArgs &a, float dt, cudaStream_t st) {
     static size_t configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && configured[dev] < smem) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(tke_turbt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaError_t e =
+            cudaFuncSetAttribute(tke_turbt_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(tke_turbt_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) {
             cudaGetLastError();
             gm1b_set_error("cudaFuncSetAttribute(tke_turbt_kernel): %s", cudaGetErrorString(e));
@@ -525,8 +539,12 @@ int enqueue_diffusion(const TkeArgs &a, float dt, cudaStream_t st) {
         }
         configured[dev] = 200 * 1024;
     }
+    const unsigned tiles = (unsigned)((a.ni + 31) / 32) * (unsigned)a.nj;
     ProfScope ps("tke_turbt_kernel", st);
-    tke_turbt_kernel<<<(a.ni + 31) / 32 * a.nj, dim3(32, kTurbtWarps), smem, st>>>(a, dt);
+    if (turbt_warps(tiles, a.nk) == 3)
+        tke_turbt_kernel<3><<<tiles, dim3(32, 3), smem, st>>>(a, dt);
+    else
+        tke_turbt_kernel<8><<<tiles, dim3(32, 8), smem, st>>>(a, dt);
     ps.stop();
     return launch_ok("tke_turbt_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }

@@ -195,8 +195,11 @@ def test_flat_tke_diffusion(ni, nj, nk):
     assert _differ(dev, a, ("tketen",)) == []
 
 
-@pytest.mark.parametrize("ni,nj,nk", [(31, 7, 8), (32, 8, 9), (33, 7, 10), (7, 7, 17), (8, 9, 201)])
+@pytest.mark.parametrize("ni,nj,nk", [(31, 7, 8), (32, 8, 9), (33, 7, 10), (7, 7, 17), (8, 9, 201),
+                                      (7, 1332, 8), (33, 666, 9), (31, 1340, 10), (7, 1331, 9), (7, 1332, 64),
+                                      (7, 1332, 65)])
 def test_terrain_tke_diffusion(ni, nj, nk):
+    """Columns to a CTA, the eight warps' and the three warps' runs of levels."""
     from gm1_b200 import tke_evolution as te
     from oracle import tke_evolution as orc
     from tests.golden.make_golden import tke_evolution_fixture
