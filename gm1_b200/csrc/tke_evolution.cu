@@ -551,12 +551,16 @@ int enqueue_diffusion(const TkeArgs &a, float dt, cudaStream_t st) {
 
 // Levels per chunk: long chunks re-load and re-form less (each starts with
 // six window loads and its lower flux), short ones give a small plane warps
-// enough: halve until two rounds of `warps` on each of 148 SMs, or four
-// levels, are left.
+// enough: halve until two rounds of `warps` on each of 148 SMs, or at most
+// four levels, are left, and to two where eight warps an SM are not (a WENO
+// stage: 37x24x24 12.9 -> 8.5 us, 28x44x49 13.0 -> 10.2, a thread per cell 10.7
+// and 11.7; 64x64x64 gains nothing, 128x100x64 loses 5%).
 int stage_chunk(const TkeArgs &a, int warps) {
     const long long rows = (long long)(a.ni / kStageOut + 1) * a.nj;
     int chunk = a.nk + 1;
-    while (chunk > 4 && rows * ((a.nk + chunk) / chunk) < 2LL * 148 * warps) chunk = (chunk + 1) / 2;
+    auto row_warps = [&] { return rows * ((a.nk + chunk) / chunk); };
+    while (chunk > 4 && row_warps() < 2LL * 148 * warps) chunk = (chunk + 1) / 2;
+    if (chunk > 2 && row_warps() < 148 * 8) chunk = 2;
     return chunk;
 }
 

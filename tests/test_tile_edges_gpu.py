@@ -159,7 +159,8 @@ def test_column_marches_of_more_chunks_than_a_grid_takes():
 
 
 @pytest.mark.parametrize("flat", [False, True])
-@pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (32, 14, 11), (62, 15, 12), (7, 9, 40)])
+@pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (32, 14, 11), (62, 15, 12), (7, 9, 40),
+                                      (30, 147, 23), (30, 148, 23)])
 def test_tke_stages(ni, nj, nk, flat):
     from gm1_b200 import tke_evolution as te
     from oracle import tke_evolution as orc
