@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(32 * (WENO ? kWenoRows : kFifthRows), WENO ? 4
     const int ni = d.ni, nj = d.nj, nk = d.nk;
     const int sx = ni + 2 * NG, sy = nj + 2 * NG, ux = ni + 1 + 2 * NG, vy = nj + 1 + 2 * NG;
     const int splane = sx * sy, uplane = ux * sy, vplane = sx * vy, cplane = ni * nj;
-    const int xtiles = ni / kFaceOut + 1;  // tiles in one grid dimension, which takes any plane
+    const int xtiles = (ni + kFaceOut - 1) / kFaceOut;  // tiles in one grid dimension, which takes any plane
     const int i = blockIdx.x % xtiles * kFaceOut + lane;
     const int row = blockIdx.x / xtiles * (WENO ? ROWS - 1 : ROWS) + ty;
     if (!WENO && row >= nj) return;  // whole warps: the fifth-order pass has no barrier
@@ -457,7 +457,7 @@ int32_t scalar_advection5_launch(int32_t ni, int32_t nj, int32_t nk, const gm1b_
     }
     const bool weno = wflag != 0 && nrk == 3;
     const PaddedDims d{ni, nj, nk};
-    const int xtiles = ni / kFaceOut + 1;  // faces 0..ni
+    const int xtiles = (ni + kFaceOut - 1) / kFaceOut;  // a warp's 32 faces complete 31 cells
     const int rows = weno ? kWenoRows - 1 : kFifthRows, ytiles = (nj + rows - 1) / rows;
     const int chunk = levels_per_chunk > 0 ? std::min(levels_per_chunk, nk) : default_chunk(xtiles * nj, nk, weno);
     const dim3 grid(xtiles * ytiles, (nk + chunk - 1) / chunk);

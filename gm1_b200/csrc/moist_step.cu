@@ -873,7 +873,7 @@ __global__ void __launch_bounds__(32 * kPdRows, 4) pdef_advection_kernel(const _
     const int lane = threadIdx.x, ty = threadIdx.y;
     const int ni = L.ni, nj = L.nj, nk = L.nk;
     const int sx = ni + 6, sy = nj + 6, sz = sx * sy, uz = (ni + 7) * sy, vz = sx * (nj + 7), cz = ni * nj;
-    const int tiles = ni / kPdOut + 1, i0 = blockIdx.x % tiles * kPdOut + lane;
+    const int tiles = (ni + kPdOut - 1) / kPdOut, i0 = blockIdx.x % tiles * kPdOut + lane;
     const int row = blockIdx.x / tiles * (kPdRows - 1) + ty;
     // faces and rows past the domain repeat its last ones and store nothing
     const int i = min(i0, ni), j = min(row, nj);
@@ -1500,7 +1500,7 @@ extern "C" int32_t gm1b_pdef_moisture_advection(int32_t ni, int32_t nj, int32_t 
     float small = (float)weps;
     if ((double)small > weps) small = nextafterf(small, -INFINITY);
     {
-        const int tiles = ni / kPdOut + 1, rows = (nj + kPdRows - 2) / (kPdRows - 1);
+        const int tiles = (ni + kPdOut - 1) / kPdOut, rows = (nj + kPdRows - 2) / (kPdRows - 1);
         const int chunk = march_chunk((long long)tiles * nj, nk, 32);
         ProfScope ps("pdef_advection_kernel", st);
         pdef_advection_kernel<<<dim3(tiles * rows, (nk + chunk - 1) / chunk), dim3(32, kPdRows), 0, st>>>(p, L, chunk,

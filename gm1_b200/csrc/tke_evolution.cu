@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(32 * (W ? kStageWRows : kStageRows), W ? 3 : 8
     const int ni = a.ni, nj = a.nj, nk = a.nk;
     const int ux = ni + 1 + 2 * kG, sx = ni + 2 * kG, uz = (nj + 2 * kG) * ux, vz = (nj + 1 + 2 * kG) * sx,
               wz = (nj + 2 * kG) * sx, cz = ni * nj;
-    const int tiles = ni / kStageOut + 1;  // all tiles in one grid dimension, which takes any plane
+    const int tiles = (ni + kStageOut - 1) / kStageOut;  // all tiles in one grid dimension, which takes any plane
     const int i0 = blockIdx.x % tiles * kStageOut + lane, row = blockIdx.x / tiles * (W ? ROWS - 1 : ROWS) + ty;
     if (!W && row >= nj) return;  // whole warps: the fifth-order stage has no barrier
     // faces and rows past the domain repeat its last ones and store nothing
@@ -556,7 +556,7 @@ int enqueue_diffusion(const TkeArgs &a, float dt, cudaStream_t st) {
 // stage: 37x24x24 12.9 -> 8.5 us, 28x44x49 13.0 -> 10.2, a thread per cell 10.7
 // and 11.7; 64x64x64 gains nothing, 128x100x64 loses 5%).
 int stage_chunk(const TkeArgs &a, int warps) {
-    const long long rows = (long long)(a.ni / kStageOut + 1) * a.nj;
+    const long long rows = (long long)((a.ni + kStageOut - 1) / kStageOut) * a.nj;
     int chunk = a.nk + 1;
     auto row_warps = [&] { return rows * ((a.nk + chunk) / chunk); };
     while (chunk > 4 && row_warps() < 2LL * 148 * warps) chunk = (chunk + 1) / 2;
@@ -570,7 +570,7 @@ int enqueue_stage(const TkeArgs &a, const float *cur, float *nxt, float *nxt2, i
     const double eps = (double)(100.0f * 1e-18f);
     const bool weno = nrk == 3;
     const int rows = weno ? kStageWRows - 1 : kStageRows, chunk = stage_chunk(a, weno ? 16 : 24);
-    const dim3 grid((a.ni / kStageOut + 1) * ((a.nj + rows - 1) / rows), (a.nk + chunk) / chunk);
+    const dim3 grid((a.ni + kStageOut - 1) / kStageOut * ((a.nj + rows - 1) / rows), (a.nk + chunk) / chunk);
     const char *name = FLAT ? "tke_rk_stage_flat_kernel" : "tke_rk_stage_kernel";
     ProfScope ps(name, st);
     if (weno)

@@ -72,7 +72,7 @@ def test_compact_acoustic_stage(column, ni, nj, nk):
 
 @pytest.mark.parametrize("nrk", [1, 3])
 @pytest.mark.parametrize("ni,nj,nk,chunk", [(30, 8, 8, None), (31, 13, 9, 4), (32, 14, 11, 5), (61, 15, 8, 1),
-                                            (62, 9, 21, None), (8, 8, 40, 7)])
+                                            (62, 9, 21, None), (8, 8, 40, 7), (124, 8, 8, None), (248, 9, 9, 5)])
 def test_scalar_advection(ni, nj, nk, chunk, nrk):
     """Open sides with the face fluxes written, each word of the tendency and
     the fluxes (the warps' shared faces among them)."""
@@ -160,7 +160,7 @@ def test_column_marches_of_more_chunks_than_a_grid_takes():
 
 @pytest.mark.parametrize("flat", [False, True])
 @pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (32, 14, 11), (62, 15, 12), (7, 9, 40),
-                                      (30, 147, 23), (30, 148, 23)])
+                                      (124, 7, 8), (248, 8, 9), (30, 147, 23), (30, 148, 23)])
 def test_tke_stages(ni, nj, nk, flat):
     from gm1_b200 import tke_evolution as te
     from oracle import tke_evolution as orc
@@ -313,7 +313,8 @@ def test_deformation(ni, nj, nk, flat):
 
 @pytest.mark.parametrize("column", ["uniform", "terrain", "flat"])
 @pytest.mark.parametrize("obc,pdefweno", [(0x2222, 0), (0x2222, 1), (0x1111, 1), (0x3443, 0)])
-@pytest.mark.parametrize("ni,nj,nk", [(29, 7, 4), (30, 8, 5), (31, 9, 6), (61, 14, 9), (5, 15, 33)])
+@pytest.mark.parametrize("ni,nj,nk", [(29, 7, 4), (30, 8, 5), (31, 9, 6), (61, 14, 9), (5, 15, 33), (62, 7, 5),
+                                      (124, 8, 4)])
 def test_pdef_advection_is_the_chains(ni, nj, nk, obc, pdefweno, column):
     """The two-pass moisture advection against the chain's, with negative
     candidates on every axis and dry air beside the water."""
