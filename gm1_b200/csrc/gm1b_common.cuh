@@ -196,10 +196,14 @@ __device__ __forceinline__ void column_sweep(const float *s_a, const float *s_b,
 // Levels a thread of a memory-bound column march takes: eight, or fewer (two at
 // the least) until four CTAs of its 256 threads lie on each of 148 SMs (mass
 // fluxes of 128x100x64: eight levels 15.1 us, two 12.8; of 256x256x80: 76 and 93).
+// `light`: a march that carries little up takes single levels where two leave
+// fewer than 2.5 CTAs an SM (buoyancy of 37x24x24: two levels 4.2 us, one 3.1;
+// 53x48x40: 4.8 and 4.3; 26x115x55, with 2.8 CTAs an SM: 5.4 and 5.6).
 // The chunks of a column lie in a grid dimension of at most 65535.
-inline int level_chunk(size_t tiles, int nk) {
+inline int level_chunk(size_t tiles, int nk, bool light = false) {
     int chunk = 8;
     while (chunk > 2 && tiles * (size_t)((nk + chunk - 1) / chunk) < 4 * 148) chunk /= 2;
+    if (light && 2 * tiles * (size_t)((nk + chunk - 1) / chunk) < 5 * 148) chunk = 1;
     const int least = (int)(((size_t)nk + 65534) / 65535);
     return chunk < least ? least : chunk;
 }

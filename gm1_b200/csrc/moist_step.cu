@@ -17,6 +17,7 @@
 // the second), the halo corners among them.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "gm1b_common.cuh"
 #include "weno.cuh"
@@ -219,15 +220,15 @@ struct Lane {
 // Inputs and the three tendencies are distinct arrays (the entry point
 // refuses a call that passes one array twice), so every load may be issued
 // ahead of the stores.
-template <bool W_ONLY>
+template <bool W_ONLY, int W>
 __global__ void __launch_bounds__(256) msb_buoyancy_kernel(const float *__restrict__ dum8,
                                                           const float *__restrict__ c1, const float *__restrict__ c2,
                                                           const float *__restrict__ gxu,
                                                           const float *__restrict__ gyv, float *__restrict__ uten,
                                                           float *__restrict__ vten, float *__restrict__ wten, Lane L,
                                                           int chunk) {
-    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = (ni + 31) / 32;
-    const int i = blockIdx.x % tiles * 32 + threadIdx.x, j = blockIdx.x / tiles * 8 + threadIdx.y;
+    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = (ni + W - 1) / W;
+    const int i = blockIdx.x % tiles * W + threadIdx.x, j = blockIdx.x / tiles * (256 / W) + threadIdx.y;
     if (i >= ni || j >= nj) return;
     const bool du = !W_ONLY && i > 0, dv = !W_ONLY && j > 0;
     const int iw = du ? i - 1 : i, js = dv ? j - 1 : j;  // neighbour cells (the own one when unused)
@@ -310,10 +311,10 @@ __device__ __forceinline__ SlopeWeights slope_weights(bool pr, int kf, float dz,
 // column's levels with the face terms and the transformed w of the level below
 // carried up.  Bound by memory; 256x256x80: a thread per cell 86 us, 45 here
 // (two levels a thread 58).
-template <int VM>
+template <int VM, int W>
 __global__ void __launch_bounds__(256) msb_getdiv_kernel(const __grid_constant__ Getdiv a, Lane L, int chunk) {
-    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = (ni + 31) / 32;
-    const int i = blockIdx.x % tiles * 32 + threadIdx.x, j = blockIdx.x / tiles * 8 + threadIdx.y;
+    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = (ni + W - 1) / W;
+    const int i = blockIdx.x % tiles * W + threadIdx.x, j = blockIdx.x / tiles * (256 / W) + threadIdx.y;
     if (i >= ni || j >= nj) return;
     const unsigned c2d = (unsigned)j * ni + i, u2d = (unsigned)j * (ni + 1) + i;
     const float gu0 = a.rgzu[u2d], gu1 = a.rgzu[u2d + 1], gv0 = a.rgzv[c2d], gv1 = a.rgzv[c2d + ni];
@@ -354,14 +355,15 @@ __global__ void __launch_bounds__(256) msb_getdiv_kernel(const __grid_constant__
 
 // the terrain column's horizontal mass fluxes in place (vmode 1: base density
 // from the padded rho0p)
+template <int W>
 __global__ void __launch_bounds__(256) msb_getdivx_horizontal_kernel(const float *__restrict__ rho0,
                                                                     const float *__restrict__ rgzu,
                                                                     const float *__restrict__ rgzv,
                                                                     float *__restrict__ rru, float *__restrict__ rrv,
                                                                     Lane L, int vmode,
                                                                     const float *__restrict__ rho0p, int chunk) {
-    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = ni / 32 + 1;
-    const int x = blockIdx.x % tiles * 32 + threadIdx.x, y = blockIdx.x / tiles * 8 + threadIdx.y;
+    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = ni / W + 1;
+    const int x = blockIdx.x % tiles * W + threadIdx.x, y = blockIdx.x / tiles * (256 / W) + threadIdx.y;
     if (x > ni || y > nj) return;
     const bool du = y < nj, dv = x < ni;
     const int xl = max(x - 1, 0), xr = min(x, ni - 1), yl = max(y - 1, 0), yr = min(y, nj - 1);
@@ -385,6 +387,7 @@ __global__ void __launch_bounds__(256) msb_getdivx_horizontal_kernel(const float
 
 // the terrain column's vertical mass flux in place, from the horizontal ones;
 // a thread marches a chunk of levels with the sums of the level below carried up
+template <int W>
 __global__ void __launch_bounds__(256) msb_getdivx_vertical_kernel(const float *__restrict__ rf0, const float *dzdx,
                                                                   const float *dzdy, const float *gz,
                                                                   const float *__restrict__ rru,
@@ -394,8 +397,8 @@ __global__ void __launch_bounds__(256) msb_getdivx_vertical_kernel(const float *
                                                                   const float *__restrict__ sigmaf,
                                                                   const float *__restrict__ rdsp, float ztop,
                                                                   int chunk) {
-    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = (ni + 31) / 32;
-    const int i = blockIdx.x % tiles * 32 + threadIdx.x, j = blockIdx.x / tiles * 8 + threadIdx.y;
+    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = (ni + W - 1) / W;
+    const int i = blockIdx.x % tiles * W + threadIdx.x, j = blockIdx.x / tiles * (256 / W) + threadIdx.y;
     if (i >= ni || j >= nj) return;
     const bool pr = vmode == 1;
     const float rds = 1.0f / dz, zt = pr ? ztop : (float)nk * dz, rzt = 1.0f / zt;
@@ -470,14 +473,15 @@ __global__ void __launch_bounds__(256) msb_flat_mass_kernel(const float *rho0p, 
     }
 }
 
+template <int W>
 __global__ void __launch_bounds__(256) msb_getdivx_divergence_kernel(const float *__restrict__ rru,
                                                                     const float *__restrict__ rrv,
                                                                     const float *__restrict__ rrw,
                                                                     float *__restrict__ divx, float rdx, float rdy,
                                                                     float rdsf, Lane L, int vmode,
                                                                     const float *__restrict__ rdsfp, int chunk) {
-    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = (ni + 31) / 32;
-    const int i = blockIdx.x % tiles * 32 + threadIdx.x, j = blockIdx.x / tiles * 8 + threadIdx.y;
+    const int ni = L.ni, nj = L.nj, nk = L.nk, tiles = (ni + W - 1) / W;
+    const int i = blockIdx.x % tiles * W + threadIdx.x, j = blockIdx.x / tiles * (256 / W) + threadIdx.y;
     if (i >= ni || j >= nj) return;
     const int k_lo = 1 + blockIdx.y * chunk, k_hi = min(nk, k_lo + chunk - 1);
     float lo = rrw[L.s(k_lo, j + 3, i + 3)];
@@ -1225,6 +1229,24 @@ extern "C" int32_t gm1b_open_fill(int32_t ni, int32_t nj, int32_t nk, int32_t ki
 }
 
 namespace {
+// CTAs of W x (256/W) columns, all in one grid dimension, which takes any plane
+template <int W>
+unsigned march_tiles(int nx, int ny) {
+    return (unsigned)((nx + W - 1) / W) * (unsigned)((ny + 256 / W - 1) / (256 / W));
+}
+
+// Runs f with the width of a march's CTAs: 32 columns, or 16 where that leaves
+// a third fewer CTAs, on planes up to 16 cells wide (9x200x150: buoyancy 11.7
+// -> 7.8 us, the post-acoustic divergences 24.0 -> 18.1, a thread per point 8.2
+// and 18.1; 12x300x60: 8.5 -> 5.9 and 18.9 -> 13.0, 7.1 and 15.3).
+template <class F>
+void with_tile_width(int ni, int nj, F f) {
+    if (3ull * march_tiles<16>(ni, nj) <= 2ull * march_tiles<32>(ni, nj))
+        f(std::integral_constant<int, 16>());
+    else
+        f(std::integral_constant<int, 32>());
+}
+
 int32_t buoyancy_launch(int32_t ni, int32_t nj, int32_t nk, const float *dum8, const float *c1, const float *c2,
                         const float *gxu, const float *gyv, float *uten, float *vten, float *wten, int w_only,
                         void *stream) {
@@ -1243,14 +1265,17 @@ int32_t buoyancy_launch(int32_t ni, int32_t nj, int32_t nk, const float *dum8, c
             }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const Lane L{ni, nj, nk};
-    const unsigned tiles = (unsigned)((ni + 31) / 32) * (unsigned)((nj + 7) / 8);
-    const int chunk = level_chunk(tiles, nk);
-    const dim3 grid(tiles, (nk + chunk - 1) / chunk), block(32, 8);
     ProfScope ps("msb_buoyancy_kernel", st);
-    if (w_only)
-        msb_buoyancy_kernel<true><<<grid, block, 0, st>>>(dum8, c1, c2, gxu, gyv, uten, vten, wten, L, chunk);
-    else
-        msb_buoyancy_kernel<false><<<grid, block, 0, st>>>(dum8, c1, c2, gxu, gyv, uten, vten, wten, L, chunk);
+    with_tile_width(ni, nj, [&](auto width) {
+        constexpr int W = decltype(width)::value;
+        const unsigned tiles = march_tiles<W>(ni, nj);
+        const int chunk = level_chunk(tiles, nk, true);
+        const dim3 grid(tiles, (nk + chunk - 1) / chunk), block(W, 256 / W);
+        if (w_only)
+            msb_buoyancy_kernel<true, W><<<grid, block, 0, st>>>(dum8, c1, c2, gxu, gyv, uten, vten, wten, L, chunk);
+        else
+            msb_buoyancy_kernel<false, W><<<grid, block, 0, st>>>(dum8, c1, c2, gxu, gyv, uten, vten, wten, L, chunk);
+    });
     ps.stop();
     return launch_ok("msb_buoyancy_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
 }
@@ -1321,39 +1346,45 @@ int32_t post_acoustic_launch(int32_t ni, int32_t nj, int32_t nk, const gm1b_post
         }
         return launch_ok("msb_flat_mass_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
     }
-    const unsigned tiles = (unsigned)((ni + 31) / 32) * (unsigned)((nj + 7) / 8);
-    const int chunk = level_chunk(tiles, nk);
-    const dim3 grid(tiles, (nk + chunk - 1) / chunk), block(32, 8);
-    {
-        ProfScope ps("msb_getdiv_kernel", st);
-        if (vmode == 1)
-            msb_getdiv_kernel<1><<<grid, block, 0, st>>>(g, L, chunk);
-        else
-            msb_getdiv_kernel<0><<<grid, block, 0, st>>>(g, L, chunk);
-        ps.stop();
-    }
-    if (!launch_ok("msb_getdiv_kernel")) return GM1B_ERR_CUDA;
-    {
-        ProfScope ps("msb_getdivx_horizontal_kernel", st);
-        msb_getdivx_horizontal_kernel<<<dim3((unsigned)(ni / 32 + 1) * (unsigned)(nj / 8 + 1), grid.y), block, 0, st>>>(
-            a->rho0_3d, a->rgzu, a->rgzv, a->rru, a->rrv, L, vmode, c ? c->rho0_padded : nullptr, chunk);
-        ps.stop();
-    }
-    if (!launch_ok("msb_getdivx_horizontal_kernel")) return GM1B_ERR_CUDA;
-    {
-        ProfScope ps("msb_getdivx_vertical_kernel", st);
-        msb_getdivx_vertical_kernel<<<grid, block, 0, st>>>(a->rf0, a->dzdx, a->dzdy, a->gz, a->rru, a->rrv, a->rrw, dz,
-                                                           L, vmode, g.sigma, g.sigmaf, g.rds, zt, chunk);
-        ps.stop();
-    }
-    if (!launch_ok("msb_getdivx_vertical_kernel")) return GM1B_ERR_CUDA;
-    {
-        ProfScope ps("msb_getdivx_divergence_kernel", st);
-        msb_getdivx_divergence_kernel<<<grid, block, 0, st>>>(a->rru, a->rrv, a->rrw, a->divx, rdx, rdy, rdsf, L, vmode,
-                                                             g.rdsfp, chunk);
-        ps.stop();
-    }
-    return launch_ok("msb_getdivx_divergence_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
+    int32_t result = GM1B_ERR_CUDA;
+    with_tile_width(ni, nj, [&](auto width) {
+        constexpr int W = decltype(width)::value;
+        const unsigned tiles = march_tiles<W>(ni, nj), faces = march_tiles<W>(ni + 1, nj + 1);
+        const int chunk = level_chunk(tiles, nk, true);
+        const dim3 grid(tiles, (nk + chunk - 1) / chunk), block(W, 256 / W);
+        {
+            ProfScope ps("msb_getdiv_kernel", st);
+            if (vmode == 1)
+                msb_getdiv_kernel<1, W><<<grid, block, 0, st>>>(g, L, chunk);
+            else
+                msb_getdiv_kernel<0, W><<<grid, block, 0, st>>>(g, L, chunk);
+            ps.stop();
+        }
+        if (!launch_ok("msb_getdiv_kernel")) return;
+        {
+            ProfScope ps("msb_getdivx_horizontal_kernel", st);
+            msb_getdivx_horizontal_kernel<W><<<dim3(faces, grid.y), block, 0, st>>>(
+                a->rho0_3d, a->rgzu, a->rgzv, a->rru, a->rrv, L, vmode, c ? c->rho0_padded : nullptr, chunk);
+            ps.stop();
+        }
+        if (!launch_ok("msb_getdivx_horizontal_kernel")) return;
+        {
+            ProfScope ps("msb_getdivx_vertical_kernel", st);
+            msb_getdivx_vertical_kernel<W><<<grid, block, 0, st>>>(a->rf0, a->dzdx, a->dzdy, a->gz, a->rru, a->rrv,
+                                                                  a->rrw, dz, L, vmode, g.sigma, g.sigmaf, g.rds, zt,
+                                                                  chunk);
+            ps.stop();
+        }
+        if (!launch_ok("msb_getdivx_vertical_kernel")) return;
+        {
+            ProfScope ps("msb_getdivx_divergence_kernel", st);
+            msb_getdivx_divergence_kernel<W><<<grid, block, 0, st>>>(a->rru, a->rrv, a->rrw, a->divx, rdx, rdy, rdsf, L,
+                                                                    vmode, g.rdsfp, chunk);
+            ps.stop();
+        }
+        if (launch_ok("msb_getdivx_divergence_kernel")) result = GM1B_OK;
+    });
+    return result;
 }
 }  // namespace
 

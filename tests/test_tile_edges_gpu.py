@@ -115,10 +115,11 @@ def test_momentum_advection(ni, nj, nk, sides):
     assert _differ({**dev, "divx": out.divx}, ref, OUTS) == []
 
 
-@pytest.mark.parametrize("ni,nj,nk", [(31, 8, 2), (33, 9, 3), (33, 800, 9), (32, 1200, 17)])
+@pytest.mark.parametrize("ni,nj,nk", [(31, 8, 2), (33, 9, 3), (33, 800, 9), (32, 1200, 17), (2, 17, 2), (15, 33, 5),
+                                      (16, 32, 24), (17, 32, 24), (48, 16, 9), (33, 64, 40), (9, 500, 33), (16, 4000, 9)])
 def test_column_marches(ni, nj, nk):
-    """Buoyancy and the post-acoustic divergences, which march two, four or
-    eight levels a thread."""
+    """Buoyancy and the post-acoustic divergences, which march one, two, four
+    or eight levels a thread, in CTAs of 32 and of 16 columns."""
     from gm1_b200 import moist_ops as mo
     from oracle import moist_step as om
     from tests.golden.make_golden import moist_piece_fixture
