@@ -301,8 +301,12 @@ __device__ void zface_coefficients(const AdvAdjArgs &a, int K, int j, int i, flo
 // pass 1: grid (ceil((ni+1)/32), ceil((nj+1)/8), nk+1); one thread per
 // face site (column i = 0..ni, row j = 0..nj, level L = 0..nk) writes the
 // slots of its x face, y face and z face (K = L + 1)
-// (32 warps an SM: WENO 200x180x40 228 -> 190 us, 96x96x48 73 -> 68)
-__global__ void __launch_bounds__(256, 4) advection_adjoint_faces_kernel(const __grid_constant__ AdvAdjArgs a) {
+// CTAS an SM: four at 64 registers, which spill 436 bytes (WENO 200x180x40 228
+// -> 190 us, 96x96x48 73 -> 68), or two without a spill where the plane gives
+// no more than three an SM anyway (with the gather pass, 28x44x49 19.8 -> 17.4
+// us, 30x40x50 19.5 -> 17.3; 26x97x42, with 3.8 an SM, takes 26.1 and 28.2).
+template <int CTAS>
+__global__ void __launch_bounds__(256, CTAS) advection_adjoint_faces_kernel(const __grid_constant__ AdvAdjArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, L = blockIdx.z;
     if (i > a.ni || j > a.nj) return;
     {
@@ -965,7 +969,11 @@ int32_t advection_adjoint_launch(const char *who, int32_t ni, int32_t nj, int32_
         one_pass = one_pass && apart(s.p, s.words, a.out, out_words) && apart(s.p, s.words, a.sum_out, cells);
     if (!one_pass) {
         ProfScope ps(a.weno ? "advection_adjoint_faces_weno_kernel" : "advection_adjoint_faces_kernel", st);
-        advection_adjoint_faces_kernel<<<dim3((ni + 1 + 31) / 32, (nj + 1 + 7) / 8, nk + 1), dim3(32, 8), 0, st>>>(a);
+        const dim3 grid((ni + 1 + 31) / 32, (nj + 1 + 7) / 8, nk + 1), block(32, 8);
+        if ((size_t)grid.x * grid.y * grid.z <= 3 * 148)
+            advection_adjoint_faces_kernel<2><<<grid, block, 0, st>>>(a);
+        else
+            advection_adjoint_faces_kernel<4><<<grid, block, 0, st>>>(a);
         ps.stop();
         if (!launch_ok("advection_adjoint_faces_kernel")) return GM1B_ERR_CUDA;
     }
