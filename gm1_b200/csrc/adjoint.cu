@@ -989,7 +989,13 @@ int32_t advection_adjoint_launch(const char *who, int32_t ni, int32_t nj, int32_
         ps.stop();
         return launch_ok("advection_adjoint_gather_compact_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
     }
-    const dim3 grid((ni + 6 + 31) / 32, (nj + 6 + 7) / 8, nk + 2), block(32, 8);
+    // 32 x 8 words a CTA, or 16 x 16 where that leaves a tenth fewer CTAs (fifth
+    // order: 28x44x49 12.5 -> 10.4 us, 30x40x50 11.4 -> 9.9, a face pass and a
+    // gather 10.9 and 10.4; 64x64x40, with 7% fewer, 16.0 and 17.0)
+    const unsigned nx = ni + 6, ny = nj + 6;
+    const bool wide = 9ull * ((nx + 31) / 32) * ((ny + 7) / 8) < 10ull * ((nx + 15) / 16) * ((ny + 15) / 16);
+    const dim3 block(wide ? 32 : 16, wide ? 8 : 16);
+    const dim3 grid((nx + block.x - 1) / block.x, (ny + block.y - 1) / block.y, nk + 2);
     ProfScope ps(one_pass ? "advection_adjoint5_kernel" : "advection_adjoint_gather_kernel", st);
     if (one_pass)
         advection_adjoint_gather_kernel<true><<<grid, block, 0, st>>>(a);

@@ -347,7 +347,8 @@ def test_pdef_advection_is_the_chains(ni, nj, nk, obc, pdefweno, column):
 
 
 @pytest.mark.parametrize("nrk", [1, 3])
-@pytest.mark.parametrize("ni,nj,nk", [(8, 8, 8), (9, 33, 9), (34, 9, 12), (65, 10, 17)])
+@pytest.mark.parametrize("ni,nj,nk", [(8, 8, 8), (9, 33, 9), (34, 9, 12), (65, 10, 17), (28, 44, 9), (42, 42, 9),
+                                      (43, 43, 9)])
 def test_advection_adjoint_in_one_pass(ni, nj, nk, nrk):
     """An output that overlaps the tendency adjoint takes the two passes over
     the face scratch: the fifth-order words are those of the one pass; and the
