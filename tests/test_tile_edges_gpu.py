@@ -392,3 +392,86 @@ def test_advection_adjoint_over_its_face_weights(name, running):
     else:
         adj.advection_tendency_adjoint(flow, s, lam, 1, out=over[:nk])
     assert torch.equal(over[:nk], got)
+
+
+def _columns(nk, rho0p):
+    """The terrain and the flat stretched column: the profiles for the oracle
+    and their device form."""
+    from gm1_b200.momentum import StretchedMomentumColumn
+    from gm1_b200.vertical import uniform_vertical_levels
+
+    lv, p = uniform_vertical_levels(nk, 150.0), _profiles(nk)
+    names = ("sigma", "sigmaf", "rds", "rdsf")
+    shape = (nk, rho0p.shape[1] - 6, rho0p.shape[2] - 6)
+    rr0 = np.random.default_rng(nk).uniform(0.8, 1.4, shape).astype(np.float32)
+    terrain = {"flat": False, "rho0p": rho0p, **{n: getattr(lv, n) for n in names}, "ztop": lv.ztop_m, "mh": lv.mh,
+               "mf": lv.mf, "rr0": rr0, "rdz": p["rdz"]}
+    flat = {"flat": True, "rho0p": rho0p, **dict.fromkeys(names), "ztop": 0.0, "mh": p["mh"], "mf": p["mf"], "rr0": rr0,
+            "rdz": p["rdz"]}
+    return {"terrain": (terrain, StretchedMomentumColumn(False, _t(rho0p), ztop=lv.ztop_m,
+                                                         **{n: _t(terrain[n]) for n in names})),
+            "flat": (flat, StretchedMomentumColumn(True, _t(rho0p), mh=_t(p["mh"]), mf=_t(p["mf"]), rr0=_t(rr0),
+                                                   rdz=p["rdz"]))}
+
+
+@pytest.mark.parametrize("column", ["terrain", "flat"])
+@pytest.mark.parametrize("sides", [(2, 2, 2, 2), (1, 1, 3, 2)])
+@pytest.mark.parametrize("ni,nj,nk", [(30, 7, 8), (31, 8, 9), (33, 9, 21), (62, 13, 10), (32, 1200, 9)])
+def test_momentum_advection_on_a_column(ni, nj, nk, sides, column):
+    from gm1_b200 import momentum as mom
+    from oracle import momentum as orc
+    from tests.golden.make_golden import momentum_fixture
+    from tests.test_oracle_momentum import OUTS, _padded_rho0
+
+    a, m, _ = momentum_fixture(ni, nj, nk, 7 * ni + nk)
+    ref = {**a, **m, "divx": np.zeros((nk, nj, ni), np.float32)}
+    host, vertical = _columns(nk, _padded_rho0(m["rho0_3d"], ni, nj, nk))[column]
+    d = _dev(ref)
+    kw = dict(ni=ni, nj=nj, nk=nk, dx=500.0, dy=450.0, lateral_sides=sides)
+    orc.momentum_advection5_column(ref, host, **kw)
+    mom.launch_cuda_gm1_child_stretched_momentum5(d, d, vertical, nrk=1, divx=d["divx"], **kw)
+    assert _differ(d, ref, OUTS) == []
+
+
+@pytest.mark.parametrize("column", ["terrain", "flat"])
+@pytest.mark.parametrize("ni,nj,nk", [(31, 8, 4), (33, 9, 5), (2, 17, 4), (16, 32, 24), (33, 800, 9), (9, 500, 33)])
+def test_post_acoustic_marches_on_a_column(ni, nj, nk, column):
+    from gm1_b200 import moist_ops as mo
+    from oracle import moist_step as om
+    from tests.golden.make_golden import moist_piece_fixture
+    from tests.test_oracle_momentum import _padded_rho0
+
+    a = moist_piece_fixture(ni, nj, nk, 3 * ni + nk)
+    for n in ("divergence", "theta_divergence_term"):
+        a[n] = np.zeros((nk, nj, ni), np.float32)
+    host, vertical = _columns(nk, _padded_rho0(a["rho0_3d"], ni, nj, nk))[column]
+    d = _dev(a)
+    om.post_acoustic_flux_column(a, host, ni=ni, nj=nj, nk=nk, dx=400.0, dy=350.0)
+    mo.post_acoustic_flux_column(d, vertical, ni=ni, nj=nj, nk=nk, dx=400.0, dy=350.0)
+    assert _differ(d, a, ("rru", "rrv", "rrw", "divergence", "theta_divergence_term", "divx")) == []
+
+
+@pytest.mark.parametrize("column", ["terrain", "flat"])
+@pytest.mark.parametrize("nrk", [1, 3])
+@pytest.mark.parametrize("ni,nj,nk,chunk", [(30, 8, 8, None), (31, 13, 9, 4), (32, 14, 11, 5), (62, 9, 21, None)])
+def test_scalar_advection_on_a_column(ni, nj, nk, chunk, nrk, column):
+    from gm1_b200.advection import (StretchedColumn, launch_cuda_gm1_child_stretched_scalar_advection5, padded_shapes)
+    from oracle import advection as adv
+
+    rng = np.random.default_rng(ni + nk)
+    sh, p = padded_shapes(ni, nj, nk), _profiles(nk)
+    f = lambda s, lo, hi: rng.uniform(lo, hi, s).astype(np.float32)  # noqa: E731
+    h = {"scalar": f(sh["scalar"], -1, 1), "rru": f(sh["u"], -9, 9), "rrv": f(sh["v"], -9, 9), "rrw": f(sh["w"], -2, 2),
+         "c1": f(sh["face"], 0.3, 0.7), "c2": f(sh["face"], 0.3, 0.7), "rr0": f(sh["cell"], 0.8, 3.0),
+         "gz": f((nj, ni), 0.8, 1.2), "divx": f(sh["cell"], -1e-3, 1e-3), "tendency": np.zeros(sh["cell"], np.float32),
+         **{"flux_" + q: np.zeros(sh[s], np.float32) for q, s in zip("xyz", "uvw")}}
+    d = _dev(h)
+    kw = dict(ni=ni, nj=nj, nk=nk, nrk=nrk, dx=400.0, dy=350.0, weps=1.0e-20)
+    flat = column == "flat"
+    profile = p["mh"] if flat else p["mf"] / np.float32(100.0)
+    adv.scalar_advection5_column(h, flat=flat, profile=profile, rdz=p["rdz"], lateral_obc=0x2222, **kw)
+    launch_cuda_gm1_child_stretched_scalar_advection5(
+        d["scalar"], d, d, d["divx"], d["tendency"], None if chunk else {q: d["flux_" + q] for q in "xyz"},
+        StretchedColumn(True, mh=_t(profile), rdz=p["rdz"]) if flat else StretchedColumn(False, rdsf=_t(profile)),
+        lateral_sides=(2, 2, 2, 2), levels_per_chunk=chunk, write_fluxes=chunk is None, **kw)
+    assert _differ(d, h, ("tendency",) if chunk else ("tendency", "flux_x", "flux_y", "flux_z")) == []
