@@ -193,7 +193,8 @@ constexpr int kWenoRows = 8;    // rows per CTA of the WENO pass: 8 rows of y fa
 
 // levels per chunk when the caller leaves it open: long chunks re-read and
 // re-form less (each chunk starts with six window loads and its lower face
-// flux), short ones give a small plane warps enough for 148 SMs
+// flux), short ones give a small plane warps enough: halve until two rounds of
+// 48 (WENO 32) row warps on each of 148 SMs, or at most four levels, are left
 inline int default_chunk(int row_warps, int nk, bool weno) {
     const int want = 148 * (weno ? 32 : 48);  // warps in flight worth of work
     int chunk = nk;
@@ -213,11 +214,12 @@ inline int default_chunk(int row_warps, int nk, bool weno) {
 // Measured on one B200, per launch at 640x768x80: fifth order 1.105 -> 0.430
 // ms, WENO 2.572 -> 1.290 against CTAs that stage each level's plane in shared
 // memory (WENO with 24 warps an SM 1.336, with 16 rows 1.836; fifth order with
-// 24 warps 0.402 but 72 us for 68 at 256x256x80, with 40 warps 0.602).
+// 24 warps 0.402 but 72 us for 68 at 256x256x80, with 40 warps 0.602; up to 44
+// bytes spill at 32).
 // Warps away from open sides, at levels away from the column's ends and with
 // no flux outputs take a finish without those branches.
 template <bool WENO, bool FLAT>
-__global__ void __launch_bounds__(32 * (WENO ? kWenoRows : kFifthRows), WENO ? 4 : 4)
+__global__ void __launch_bounds__(32 * (WENO ? kWenoRows : kFifthRows), 4)
     scalar_advection5_march_kernel(const __grid_constant__ gm1b_scalar_advection5_arrays a,
                                    const __grid_constant__ PaddedDims d, int levels_per_chunk, float rdx, float rdy,
                                    float rdsf, double eps, float wepsf, unsigned obc,

@@ -69,7 +69,10 @@ __device__ __forceinline__ float sq(float x) { return x * x; }
 // One CTA per 32 x 8 columns with every strain in shared memory (33 x 9 corners
 // take its 256 threads two passes, ~125 loads a level) took 473 us at
 // 256x256x80 on terrain and 0.84 ms at 640x768x80 flat; this takes 146 and
-// 0.59 (24 and 32 warps an SM; 16 and 24: 193 and 0.74).
+// 0.59 (24 and 32 warps an SM; 16 and 24: 193 and 0.74).  At 24 warps the
+// terrain strains spill 132 bytes; with 16 and no spill 256x256x80 takes 161 us
+// for 140, 300x301x30 85 for 77, and the smallest planes less (53x48x40 7.4 for
+// 9.1).
 template <bool FLAT>
 __global__ void __launch_bounds__(32 * kDefRows, FLAT ? 4 : 3)
     calcdef_march_kernel(const __grid_constant__ DefArgs p, int levels_per_chunk) {
@@ -399,8 +402,8 @@ using namespace gm1b;
 
 namespace {
 // Whole columns leave a small plane too few warps; a chunk of levels forms the
-// strains of the mass level below it again: halve until two rounds of the
-// resident CTAs on 148 SMs, or eight levels, are left
+// strains of the mass level below it again: halve until three rounds of the
+// resident CTAs on 148 SMs, or at most eight levels, are left
 // (256x256x80 terrain: 246 us with whole columns; 128x100x64 flat: 80 against 27).
 template <bool FLAT>
 void calcdef_launch(const DefArgs &p, cudaStream_t st) {

@@ -220,7 +220,9 @@ constexpr int kTileMostNk = 296;  // taller columns do not fit an SM's shared me
 // spread over the CTA's warps, each with a run of levels.  A thread per column
 // (three species one after the other, its loads a level at a time) took 1.373
 // ms at 640x768x80, 261 us at 256x256x80 and 71 us at 53x48x40; this takes
-// 0.790 ms, 120 us and less than 20.
+// 0.790 ms, 120 us and less than 20.  Tall columns leave an SM one CTA (from
+// about 150 levels) and it is still the faster: 256x256 of 150 levels 940 ->
+// 509 us, of 296 levels 2289 -> 1161; 96x96 of 296 levels 1070 -> 164.
 __global__ void __launch_bounds__(32 * kTileWarps)
     kessler_tile_kernel(const __grid_constant__ gm1b_kessler_arrays a, KDims d, KWork w, const __grid_constant__ KConst c,
                         float dt, float rdz) {

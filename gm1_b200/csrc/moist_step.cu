@@ -1481,7 +1481,7 @@ int32_t pdef_chain_launch(const Pdef &p, const Lane &L, cudaStream_t st) {
 }
 
 // levels per chunk of a marching pass: halve until two rounds of `warps` on
-// each of 148 SMs, or four levels, are left
+// each of 148 SMs, or at most four levels, are left
 int march_chunk(long long row_warps, int nk, int warps) {
     int chunk = nk;
     while (chunk > 4 && row_warps * ((nk + chunk - 1) / chunk) < 2LL * 148 * warps) chunk = (chunk + 1) / 2;

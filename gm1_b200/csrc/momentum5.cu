@@ -9,10 +9,9 @@
 //   lateral families (periodic wrap, open-side inflow substitution and
 //   edits)  :103-208
 //
-// Design (B200): three launches instead of the reference's six.  (1) every
-// u and v face's mass flux; (2) rrw and divx together (each cell forms the
-// two rrw words its divergence needs, writing its own); (3) one momentum
-// pass whose warps march rows of u, v or w faces up the column (below).
+// Design (B200): two launches instead of the reference's six.  (1) every mass
+// flux and divx, in a march of the cells' columns; (2) one momentum pass whose
+// warps march rows of u, v or w faces up the column.
 // Upwind face fluxes read the six points that hold both upwind stencils
 // before the mass-flux sign is known, so no load waits on it.
 // Binary32 one operation at a time in the reference's order: word-identical.
@@ -191,7 +190,7 @@ __global__ void __launch_bounds__(32 * kFluxRows) mom5_flux_kernel(const __grid_
 }
 
 // ---------------------------------------------------------------------------
-// (3) advu / advv / advw.  A warp owns 32 x faces of one row of one component
+// (2) advu / advv / advw.  A warp owns 32 x faces of one row of one component
 // and marches up a chunk of levels: each lane forms the x flux of one face
 // and takes the next face's from the lane above (31 points per 32 lanes, no
 // divergent edge), the upper vertical flux is carried down as the next
@@ -201,8 +200,8 @@ __global__ void __launch_bounds__(32 * kFluxRows) mom5_flux_kernel(const __grid_
 // L2.  Bound by instruction issue (the upwind selects on the half-rate ALU).
 // Measured on one B200, per launch at 640x768x80: 3.085 ms with a thread per
 // point forming all its fluxes, 1.596 with one finish for every line, 1.127
-// here (32 warps an SM; 24 warps 1.169, 40 warps 1.267, two levels a trip
-// 1.353).
+// here (32 warps an SM, the terrain instantiation spilling 16 bytes; 24 warps
+// 1.169, 40 warps 1.267, two levels a trip 1.353).
 // ---------------------------------------------------------------------------
 constexpr int kMomOut = 31;   // points a warp of 32 faces completes
 constexpr int kMomRows = 4;   // rows (independent warps) per CTA
@@ -634,7 +633,8 @@ int enqueue_transport(const MomArgs &a, cudaStream_t st) {
     const int tiles = a.ni / kMomOut + 1, ytiles = (a.nj + 1 + kMomRows - 1) / kMomRows;
     // long chunks re-load and re-form less (each starts with six window loads
     // and its lower flux), short ones give a small plane warps enough: halve
-    // until two rounds of 24 warps on each of 148 SMs, or four levels, are left
+    // until two rounds of 24 warps on each of 148 SMs, or at most four levels,
+    // are left
     int chunk = a.nk;
     while (chunk > 4 && 3LL * tiles * (a.nj + 1) * ((a.nk + chunk - 1) / chunk) < 2LL * 148 * 24) chunk = (chunk + 1) / 2;
     ProfScope ps("mom5_adv_kernel", st);

@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(32 * kColWarps) flat_turb_uv_kernel(const __gr
     }
     __syncthreads();
     // (chunks of four rows cost registers and CTAs an SM: 640x768x80 turbu 1115
-    // us against 1005, turbw 828 against 541)
+    // us against 1005, turbw 828 against 541; with two the u columns spill 8 bytes)
     if (wy == 0) column_sweep<2>(s_a, s_b, s_c, s_d, K);
     __syncthreads();
     if (lo >= hi || !own) return;

@@ -208,7 +208,8 @@ __global__ void __launch_bounds__(kEW) terrain_gettau_kernel(TArgs a) {
 // own runs of levels in shared memory, one warp sweeps them, then all warps
 // add the tendencies of their levels.  256x256x80 against a thread per column,
 // its loads a level at a time: turbu 615 -> 246 us, turbv 596 -> 243, turbw 386
-// -> 107 (24 warps an SM 339, 285 and 125).
+// -> 107 at 32 warps an SM, which spill 44 to 60 bytes (24 warps 339, 285 and
+// 125; the sweep in chunks of two rows instead of four 250, 269 and 115).
 template <int DIR>
 __global__ void __launch_bounds__(32 * kColWarps, 4) terrain_turb_uv_kernel(const __grid_constant__ TArgs a) {
     extern __shared__ float s_col[];
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(32 * kColWarps, 4) terrain_turb_uv_kernel(cons
                                       (rdz * ((rg_b - rg_a) * rd)));
         return (grad + terrain) * (0.25f * (PAIR(a.kmv, k) * (gza * c3(a, a.rf, k, ja, ia) + gzb * c3(a, a.rf, k, jb, ib))));
     };
-    // back substitution, the cross term and the tendency per level
+    // the horizontal, vertical and cross terms and the tendency per level
     float r1 = 0.0f, r2 = 0.0f;
     if (DIR == 0) {
         r1 = 0.25f * ((c2(a, a.rgz, cy - 1, ia) + c2(a, a.rgz, cy, ib)) + (c2(a, a.rgz, cy, ia) + c2(a, a.rgz, cy - 1, ib)));
@@ -425,7 +426,9 @@ __device__ __forceinline__ float *fy_of(const SArgs &a, int sc) { return fx_of(a
 // marches a chunk of levels for one scalar at a time, the two cells' face
 // values (sw) of the level below carried up; the faces beyond the last cells
 // belong to one more column and row of threads.  256x256x80, four scalars:
-// 1139 -> 385 us against a thread per face from a divided linear index.
+// 1139 -> 385 us against a thread per face from a divided linear index (32 warps
+// an SM, which spill 160 bytes; 24 warps with fewer 450, and 250 for 212 at
+// 300x301x30).
 __global__ void __launch_bounds__(256, 4) terrain_turbs_flux_kernel(const __grid_constant__ SArgs a, int chunk) {
     const int ni = a.ni, nj = a.nj, nk = a.nk, ux = ni + 1, vy = nj + 1, tiles = (ux + 31) / 32;
     const int x = blockIdx.x % tiles * 32 + threadIdx.x, y = blockIdx.x / tiles * 8 + threadIdx.y;

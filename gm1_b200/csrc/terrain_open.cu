@@ -13,33 +13,35 @@
 //   cpu_bc{p,s,u,v,w}_open_inplace            src/cm1core/cuda_sound3_open_boundary.py:249-335
 //   cpu_radiation4_inplace                    src/cm1core/cuda_lateral_closure.py:390-472
 //
-// Design (B200).  Per stage: one prepare pass.  Per small step: three
-// launches - (1) the four open edges (a CTA per boundary line snapshots both
-// w-level interpolations of its two face columns in shared memory, then
-// advances every level at once), (2) the terrain pressure gradient on the
-// interior faces (a 32x4 tile marching up the column, each vertical ppd
-// difference formed once), (3) one column pass per 32 columns of a row that
-// keeps the whole column in shared memory: transformed divergence, surface
-// w, pi' advection and fpk, the tridiagonal coefficients, the Thomas sweep,
-// the pi' update with the kdiv filter, the ppd halo copy between small steps
-// and the rru/rrv/rrw averages (the reference takes eight launches and
-// global elimination scratch for the same small step).  After the last small
-// step: the radiation histories (one warp per boundary line, the column sum
-// in level order) and the stage fills in two ordered passes (the first
-// direction of every fill, then the second).  Scratch arrays are written only
-// at the last small step, and only under GM1B_TOS_DIAGNOSTICS: their final
-// words are the CPU twin's.  The vertical coordinate is formed in-kernel with
-// the twin's own float32 operations.  Binary32 one operation at a time in the
-// reference's order: word-identical.
+// Design (B200).  Per stage: one prepare pass and the four open edges of the
+// first small step (a CTA per boundary line snapshots both w-level
+// interpolations of its two face columns in shared memory, then advances every
+// level at once).  Per small step: two launches - (1) the pressure gradient on
+// the interior faces, two levels a thread, with the rru/rrv sums, (2) one
+// column pass per 32 columns of a row that keeps the tridiagonal rows in shared
+// memory: transformed divergence, surface w, pi' advection and fpk, the
+// coefficients, the sweep, the pi' update with the kdiv filter, the ppd halo
+// copy between small steps, the rrw average and the next small step's open
+// edges (the reference takes eight launches and global elimination scratch for
+// the same small step).  An ablated small step, and the last one under
+// GM1B_TOS_DIAGNOSTICS, take a column pass phase by phase instead, which forms
+// every average and leaves the edges to their own launch; it alone writes the
+// scratch arrays, at the last small step under that flag: their final words are
+// the CPU twin's.  After the last small step: the radiation histories (one warp
+// per boundary line, the column sum in level order) and the stage fills in two
+// ordered passes (the first direction of every fill, then the second).  The
+// vertical coordinate is formed in-kernel with the twin's own float32
+// operations.  Binary32 one operation at a time in the reference's order:
+// word-identical.
 #include "gm1b_common.cuh"
 
 namespace gm1b {
 namespace {
 
-constexpr int kTosWarps = 8;     // k-parallel warps of the column pass
-constexpr int kTosMaxNk = 160;   // column pass keeps 10 words per level per column in shared memory
-constexpr int kTosArrays = 7;
-constexpr int kFlatLevels = 2;   // the same of the flat pressure gradient, which has no vertical coupling
+constexpr int kTosWarps = 8;     // k-parallel warps of the phase-by-phase column pass
+constexpr int kTosArrays = 7;    // its shared words per level and column (three more on the stretched terrain column)
+constexpr int kTosMaxNk = 160;   // most levels: 207 KB of those ten
+constexpr int kFlatLevels = 2;   // levels of a thread of the flat pressure gradient
 constexpr int kPgLevels = 2;     // levels of a thread of the terrain pressure gradient
 constexpr int kA2Levels = 2;     // levels per warp whose column-pass loads are issued together (phase A2)
 constexpr int kColLevels = 2;    // the same for phases A3 and C
@@ -979,7 +981,7 @@ __global__ void __launch_bounds__(32 * kTosWarps, 3) tos_column_kernel(TosArgs p
 
 // ---------------------------------------------------------------------------
 // column pass of one small step with every phase on and no diagnostics (the
-// composed steps and the compact stage; tos_column_kernel below keeps the
+// composed steps and the compact stage; tos_column_kernel above keeps the
 // diagnostic words and the ablations).  CTA = 32 consecutive columns of row
 // j, kMarchWarps warps each marching up its own run of consecutive levels.
 // One pass forms fpk and the tridiagonal row of each level: what levels k-1
@@ -995,8 +997,8 @@ __global__ void __launch_bounds__(32 * kTosWarps, 3) tos_column_kernel(TosArgs p
 // the five shared words and 80 registers allow three CTAs).  Measured on one
 // B200, per launch: flat column 640x768x80 1.583 -> 0.799 ms, uniform column
 // 256x256x80 271 -> 170 us against the phase-by-phase pass and its separate
-// open-edge launch of 11 us.  With the sweep a row at a time (0.863-0.878): 16 warps 1.007 ms, 10 warps 1.048, 4 warps 1.228,
-// two CTAs an SM 1.175, four (64 registers) 1.144, four without the next
+// open-edge launch of 11 us.  With the sweep a row at a time (0.863-0.878): 16
+// warps 1.007 ms, 10 warps 1.048, 4 warps 1.228, two CTAs an SM 1.175, four (64 registers) 1.144, four without the next
 // level's prefetch 1.179; the last phase's loads two levels at a time 0.900,
 // one 0.962.  Prefetching the rows of the next levels into L2 made it slower
 // (1.03 ms, whatever the distance).
