@@ -1001,7 +1001,10 @@ __global__ void __launch_bounds__(32 * kTosWarps, 3) tos_column_kernel(TosArgs p
 // warps 1.007 ms, 10 warps 1.048, 4 warps 1.228, two CTAs an SM 1.175, four (64 registers) 1.144, four without the next
 // level's prefetch 1.179; the last phase's loads two levels at a time 0.900,
 // one 0.962.  Prefetching the rows of the next levels into L2 made it slower
-// (1.03 ms, whatever the distance).
+// (1.03 ms, whatever the distance).  The stretched terrain
+// column carries four more words a face and spills 112 bytes at three CTAs an
+// SM, so it takes two: 256x256x80 280 -> 199 us, 512x400x40 400 -> 305,
+// 128x100x64 unchanged at 50.
 // ---------------------------------------------------------------------------
 constexpr int kMarchWarps = 8;
 constexpr int kMarchArrays = 5;
@@ -1139,7 +1142,7 @@ __device__ __forceinline__ float edge_velocity(const TosArgs &p, const Ix &X, in
 }
 
 template <int VM>
-__global__ void __launch_bounds__(32 * kMarchWarps, 3) tos_column_march_kernel(const __grid_constant__ TosArgs p) {
+__global__ void __launch_bounds__(32 * kMarchWarps, VM == 1 ? 2 : 3) tos_column_march_kernel(const __grid_constant__ TosArgs p) {
     extern __shared__ float sh[];
     __shared__ float s_mm[kMarchWarps][32];  // mm of the runs' first rows
     const Ix X{p.ni, p.nj};
