@@ -32,11 +32,11 @@
 //
 // Design: the strain and gettau passes are grid-stride elementwise kernels
 // over the union of their index spaces (one launch each).  A column solve's
-// CTA owns 32 columns of a row: eight warps form the tridiagonal rows of their
-// own runs of levels in shared memory ([level][column], conflict-free; every
-// load and division spread over the CTA), one warp sweeps them, then all warps
-// form the horizontal divergence and the cross term of their levels and add
-// the tendency.  Against a thread per column (its loads one level at a time,
+// CTA owns 32 columns of a row: eight warps (or four) form the tridiagonal rows
+// of their own runs of levels in shared memory ([level][column], conflict-free;
+// every load and division spread over the CTA), one warp sweeps them, then all
+// warps form the horizontal divergence and the cross term of their levels and
+// add the tendency.  Against a thread per column (its loads one level at a time,
 // too few columns in flight), 189x131x64: turbu 207 -> 56 us, turbv 141 ->
 // 45, turbw 90 -> 39; turbs of theta and the three moisture rows, which share
 // the matrix and its reciprocals, 285 -> 99.
@@ -47,7 +47,7 @@ namespace {
 
 constexpr int kCX = 32, kCY = 4, kCT = kCX * kCY;  // column tile
 constexpr int kEW = 256;                            // elementwise block
-constexpr int kColWarps = 8;                        // warps of a column solve's CTA, which owns 32 columns of a row
+constexpr int kColWarps = 8;                        // warps of the scalar solve's CTA, which owns 32 columns of a row
 constexpr int kTurbsGroup = 4;                      // scalars the turbs column pass solves together
 
 #define TRY(x)                        \
@@ -163,8 +163,8 @@ __global__ void __launch_bounds__(kEW) flat_gettau_kernel(StressArgs a) {
 // ------------------------------------------------------- turbu and turbv
 // DIR 0: a u column (j, f), f in [0, ni]; DIR 1: a v column (f, i), f in [0, nj];
 // the cells either side of it are (ja, ia) and (jb, ib).
-template <int DIR>
-__global__ void __launch_bounds__(32 * kColWarps) flat_turb_uv_kernel(const __grid_constant__ StressArgs a) {
+template <int DIR, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) flat_turb_uv_kernel(const __grid_constant__ StressArgs a) {
     extern __shared__ float s_col[];
     const int lane = threadIdx.x, wy = threadIdx.y;
     const int ni = a.ni, nj = a.nj, K = a.nk, ux = ni + 1, vy = nj + 1;
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(32 * kColWarps) flat_turb_uv_kernel(const __gr
     const float tema = (((-0.0625f * dt) * 1.0f) * rdz) * rdz;
     const float temb = (((0.0625f * dt) * 0.0f) * rdz) * rdz;
     const float temc = (0.5f * dt) * rdz;
-    const int run = (K + kColWarps - 1) / kColWarps;
+    const int run = (K + WARPS - 1) / WARPS;
     const int lo = min(wy * run, K), hi = min(lo + run, K);
     // the diffusivity product of a face, formed once and carried up
     auto face = [&](int f) { return f >= 1 && f < K ? (pair(a.kmv, f) * pair(a.mf, f)) * pair(a.rf, f) : 0.0f; };
@@ -249,7 +249,8 @@ __global__ void __launch_bounds__(32 * kColWarps) flat_turb_uv_kernel(const __gr
 }
 
 // ----------------------------------------------------------------- turbw
-__global__ void __launch_bounds__(32 * kColWarps) flat_turbw_kernel(const __grid_constant__ StressArgs a) {
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) flat_turbw_kernel(const __grid_constant__ StressArgs a) {
     extern __shared__ float s_col[];
     const int lane = threadIdx.x, wy = threadIdx.y;
     const int ni = a.ni, nj = a.nj, K = a.nk, n = K - 1, ux = ni + 1, vy = nj + 1, tiles = (ni + 31) / 32;
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(32 * kColWarps) flat_turbw_kernel(const __grid
     const float tema = (((-1.0f * dt) * 1.0f) * rdz) * rdz;
     const float temb = ((dt * 0.0f) * rdz) * rdz;
     const float temc = dt * rdz;
-    const int run = (n + kColWarps - 1) / kColWarps;
+    const int run = (n + WARPS - 1) / WARPS;
     const int lo = min(1 + wy * run, K), hi = min(lo + run, K);  // faces lo .. hi-1
     if (lo < hi) {
         unsigned z = (unsigned)lo * lev + col;
@@ -661,33 +662,44 @@ int configure(Kernel kernel, size_t smem, const char *name) {
     return GM1B_OK;
 }
 
-int enqueue_momentum(const StressArgs &a, cudaStream_t st) {
-    if (a.nk > 200) {
-        gm1b_set_error("gm1b_flat_momentum_stress: nk=%d exceeds the column solves' shared memory (nk <= 200)", a.nk);
-        return GM1B_ERR_ARGUMENT;
-    }
+template <int WARPS>
+int momentum_solves(const StressArgs &a, cudaStream_t st) {
     const size_t words = (size_t)4 * a.nk * 32 * sizeof(float);
-    TRY(configure(flat_turb_uv_kernel<0>, words, "flat_turb_uv_kernel<0>"));
-    TRY(configure(flat_turb_uv_kernel<1>, words, "flat_turb_uv_kernel<1>"));
-    TRY(configure(flat_turbw_kernel, words, "flat_turbw_kernel"));
-    const dim3 cta(32, kColWarps);
+    TRY(configure(flat_turb_uv_kernel<0, WARPS>, words, "flat_turb_uv_kernel<0>"));
+    TRY(configure(flat_turb_uv_kernel<1, WARPS>, words, "flat_turb_uv_kernel<1>"));
+    TRY(configure(flat_turbw_kernel<WARPS>, words, "flat_turbw_kernel"));
+    const dim3 cta(32, WARPS);
     auto tiles = [](int nx, int ny) { return (unsigned)((nx + 31) / 32) * (unsigned)ny; };
     {
         ProfScope ps("flat_turbu_kernel", st);
-        flat_turb_uv_kernel<0><<<tiles(a.ni + 1, a.nj), cta, words, st>>>(a);
+        flat_turb_uv_kernel<0, WARPS><<<tiles(a.ni + 1, a.nj), cta, words, st>>>(a);
         ps.stop();
         if (!launch_ok("flat_turbu_kernel")) return GM1B_ERR_CUDA;
     }
     {
         ProfScope ps("flat_turbv_kernel", st);
-        flat_turb_uv_kernel<1><<<tiles(a.ni, a.nj + 1), cta, words, st>>>(a);
+        flat_turb_uv_kernel<1, WARPS><<<tiles(a.ni, a.nj + 1), cta, words, st>>>(a);
         ps.stop();
         if (!launch_ok("flat_turbv_kernel")) return GM1B_ERR_CUDA;
     }
     ProfScope ps("flat_turbw_kernel", st);
-    flat_turbw_kernel<<<tiles(a.ni, a.nj), cta, words, st>>>(a);
+    flat_turbw_kernel<WARPS><<<tiles(a.ni, a.nj), cta, words, st>>>(a);
     ps.stop();
     return launch_ok("flat_turbw_kernel") ? GM1B_OK : GM1B_ERR_CUDA;
+}
+
+int enqueue_momentum(const StressArgs &a, cudaStream_t st) {
+    if (a.nk > 200) {
+        gm1b_set_error("gm1b_flat_momentum_stress: nk=%d exceeds the column solves' shared memory (nk <= 200)", a.nk);
+        return GM1B_ERR_ARGUMENT;
+    }
+    // Four warps a CTA for columns of up to 40 levels on a plane that gives nine
+    // CTAs an SM, else eight: short runs of levels form their end faces twice, and
+    // the other warps wait for the sweep.  The three solves of 640x500x24 with
+    // eight and four warps 524 and 477 us (a thread per column 508), 256x256x40
+    // 198 and 196, 640x500x56 1119 and 1362, 128x100x24 38 and 47.
+    const size_t tiles = (size_t)((a.ni + 31) / 32) * a.nj;
+    return a.nk <= 40 && tiles >= 9 * 148 ? momentum_solves<4>(a, st) : momentum_solves<8>(a, st);
 }
 
 }  // namespace

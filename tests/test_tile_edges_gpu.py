@@ -214,7 +214,9 @@ def test_terrain_tke_diffusion(ni, nj, nk):
     assert _differ(dev, a, ("tketen",)) == []
 
 
-@pytest.mark.parametrize("ni,nj,nk,numq", [(31, 3, 7, 2), (32, 4, 8, 3), (33, 3, 9, 4), (64, 3, 17, 5), (3, 5, 200, 6)])
+@pytest.mark.parametrize("ni,nj,nk,numq", [(31, 3, 7, 2), (32, 4, 8, 3), (33, 3, 9, 4), (64, 3, 17, 5), (3, 5, 200, 6),
+                                           (3, 1332, 4, 1), (31, 1331, 5, 1), (33, 666, 7, 1), (4, 1332, 40, 1),
+                                           (4, 1332, 41, 1)])
 def test_flat_turbulence_columns(ni, nj, nk, numq):
     """Runs of levels of the stress and scalar solves, and the scalars'
     groups of four."""
