@@ -44,6 +44,7 @@ of the same workload and the same metric.
 from __future__ import annotations
 
 import argparse
+import dataclasses
 import json
 import os
 import subprocess
@@ -458,8 +459,6 @@ def run_moist(args) -> None:
     # columns only) --------------------------------------------------------
     stress_step = None
     if cfg.stretched:
-        import dataclasses
-
         scfg = dataclasses.replace(cfg, sgs_diffusion=True, rayleigh=True, dissipative_heating=True)
         with torch.cuda.stream(stream):
             smodel = NativeMoistLargeStep(scfg, dev_state, dev_metrics, stream=stream)
@@ -1138,7 +1137,9 @@ def main() -> None:
     barrier()
     clocks = sampler.stop()
     if use_graph:
-        captured.check()  # raises if a persistent stage's grid barrier gave up
+        # raises if a persistent stage's grid barrier gave up (the launch's own
+        # event was recorded into the graph and cannot be waited for)
+        dataclasses.replace(captured, ready_event=ends[-1]).check()
     local_ms = sum(s.elapsed_time(e) for s, e in zip(starts, ends))
     total_ms = max_over_ranks(local_ms)
     ms_per_step = total_ms / args.steps
