@@ -1,6 +1,6 @@
 """The whole moist step through the C ABI (gm1b_moist_large_step, driven by
 ctypes alone through NativeMoistLargeStep) against the Python composition
-MoistLargeStep: the same launches in the same order, so every word of every
+MoistLargeStep: the same operators in the same order, so every word of every
 state array the step writes must be identical, on the uniform and on the
 stretched column, sequential and concurrent, eager and captured in a CUDA
 graph; and the folded failure words read back through the ABI."""
